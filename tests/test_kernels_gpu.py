@@ -106,6 +106,32 @@ def test_gemm_ref_float32_rows_do_not_depend_on_the_batch(k):
         assert torch.equal(part, full[13:13 + rows])
 
 
+@pytest.mark.parametrize("m,n,kk", [(1, 31, 4), (4, 32, 64), (5, 1033, 1023), (8, 4100, 128), (17, 9000, 36), (33, 4096, 260),
+                                    (100, 6144, 68), (301, 6144, 100), (129, 19000, 33), (700, 4000, 16)])
+def test_gemm_ref_float32_gives_the_same_bits_on_every_tile(k, m, n, kk):
+    """Sizes that reach each tile, with remainders in every direction; rows that start at 16-byte boundaries and rows that
+    do not.  A row alone runs on the smallest tile: its bits must be those of the row among the others."""
+    torch.manual_seed(m + n)
+    wide = torch.randn(m, kk + 5, device="cuda")
+    w = torch.randn(n, kk, device="cuda")
+    bias, scale = torch.randn(n, device="cuda"), torch.randn(n, device="cuda")
+    for x in (wide[:, 1:1 + kk], wide[:, :kk].contiguous()):
+        ref = x.double() @ w.double().T
+        out = torch.empty(m, n, device="cuda")
+        k.gemm_ref(x, w, out)
+        # a sum of kk products rounded kk times
+        bound = kk * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T) + 1e-30
+        assert ((out.double() - ref).abs() <= bound).all()
+        for row in {0, m // 2, m - 1}:
+            alone = torch.empty(1, n, device="cuda")
+            k.gemm_ref(x[row:row + 1], w, alone)
+            assert torch.equal(alone[0], out[row])
+        acc = torch.full((m, n), 2.0, device="cuda")
+        k.gemm_ref(x, w, acc, bias, accumulate=True, act="gelu", col_scale=scale)
+        want = 2.0 + torch.nn.functional.gelu(ref + bias.double()) * scale.double()
+        assert ((acc.double() - want).abs() <= 1.2 * bound * scale.double().abs() + 2.0 ** -21 * (want.abs() + 4.0 + ref.abs())).all()
+
+
 def test_gemm_refuses_what_it_cannot_take(k):
     x = torch.randn(4, 100, device="cuda").bfloat16()
     w = torch.randn(8, 100, device="cuda").bfloat16()
