@@ -1,75 +1,213 @@
 // Plain causal grouped-query attention over the paged cache, for prompts and for decoding alike.
 //
-// One block per (token, query head).  The query at position p of head h uses kv head
-// h / (nh / nkv) and the keys lo..p, lo = max(0, p + 1 - window) with a window, else 0
+// One block per (TOKENS tokens, up to HEADS query heads of one kv head).  The query at position p of head h
+// uses kv head h / (nh / nkv) and the keys lo..p, lo = max(0, p + 1 - window) with a window, else 0
 // (src/model.rs:1187-1226).  Softmax is m = max, e = exp(s - m), e / sum (src/kernels.rs:1550-1561),
 // computed online over chunks of 128 keys that start at lo.  The arithmetic for one
 // (token, head) is a function of its position and of the cache contents alone, so whole
 // prompts, single tokens and any batch give the same bits.  Everything is float32 arithmetic;
 // it is the attention of the float32 engine and the plain reference of the faster kernels.
+//
+// A chunk's keys come into shared memory with neighbouring threads on neighbouring dims, a thread then
+// walks the dims of its own key for all of the block's queries; its values take the same place with
+// neighbouring threads on neighbouring positions, a thread then walks the positions of its own dim.  What
+// bounds it: the shared-memory reads of those walks.  (Read from memory by the walking threads themselves,
+// 32 lines a load, a query a block, the kernel was bound by its requests: 301 tokens of three prompts, 16
+// heads of 128 over 8 kv heads, took 336 us a layer; in this form 55, the same sums in the same order.)
 #include "common.cuh"
 
 constexpr int CHUNK = 128;
 
-template <typename T>
+// Rows of the chunk in shared memory: a key's dims, or a dim's positions, a multiple of 4 and 4 more.
+static __host__ __device__ inline int quads(int n) { return (n + 3) & ~3; }
+static __host__ __device__ inline size_t tile_floats(int hd) {
+  const size_t keys = (size_t)CHUNK * (quads(hd) + 4), values = (size_t)hd * (CHUNK + 4);
+  return keys > values ? keys : values;
+}
+
+__device__ __forceinline__ float dot4(float d, float4 a, float4 b) {      // one sum, in order
+  d = fmaf(a.x, b.x, d);
+  d = fmaf(a.y, b.y, d);
+  d = fmaf(a.z, b.z, d);
+  return fmaf(a.w, b.w, d);
+}
+
+// One or four neighbouring elements into shared memory as float32: copies in flight for float32 (waited for by
+// copies_done), loads and conversions for bfloat16.
+__device__ __forceinline__ void bring1(float* dst, const float* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void bring4(float* dst, const float* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void bring1(float* dst, const bf16* src) { *dst = to_f32(*src); }
+__device__ __forceinline__ void bring4(float* dst, const bf16* src) {
+#pragma unroll
+  for (int e = 0; e < 4; ++e) dst[e] = to_f32(src[e]);
+}
+__device__ __forceinline__ void copies_done() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+template <typename T, int TOKENS, int HEADS>
 __global__ void __launch_bounds__(CHUNK) attention_ref_kernel(
     const T* __restrict__ q, long long q_stride, T* __restrict__ out, long long out_stride,
     const T* __restrict__ kcache, const T* __restrict__ vcache, PagedKV kv, const int* __restrict__ tok_pos,
-    const int* __restrict__ tok_seq, const int* __restrict__ seq_slot, int nh, int window) {
-  extern __shared__ float smem[];
+    const int* __restrict__ tok_seq, const int* __restrict__ seq_slot, int ntok, int nh, int window, int wide) {
+  constexpr int NQ = TOKENS * HEADS, WARPS = CHUNK / 32;
+  extern __shared__ __align__(16) float smem[];
   pdl_release_next();
   pdl_wait_prior();
-  const int hd = kv.head_dim;
-  float* qs = smem;                    // [hd]
-  float* p = qs + hd;                  // [CHUNK]
-  float* scratch = p + CHUNK;          // [33]
-  // [CHUNK]; 8-byte aligned whatever the head size (the launcher adds the 8 bytes this may skip)
-  size_t* rows = (size_t*)(((uintptr_t)(scratch + 34) + 7) & ~(uintptr_t)7);
-  const int t = blockIdx.x, h = blockIdx.y, tid = threadIdx.x;
-  const int g = h / (nh / kv.num_kv_heads);
-  const int pos = tok_pos[t];
-  const int slot = seq_slot[tok_seq[t]];
-  const int hi = pos + 1;
-  const int lo = window > 0 ? max(0, hi - window) : 0;
-  const T* qrow = q + (size_t)t * q_stride + (size_t)h * hd;
-  for (int i = tid; i < hd; i += CHUNK) qs[i] = to_f32(qrow[i]);
-  __syncthreads();
-  float m = -INFINITY, l = 0.f, acc[2] = {0.f, 0.f};
-  for (int c0 = lo; c0 < hi; c0 += CHUNK) {
-    const int j = c0 + tid;
-    float s = -INFINITY;
-    if (j < hi) {
-      const T* kr = kcache + kv.row(slot, j, g);
-      rows[tid] = kv.vcol(slot, j, g);
-      float d = 0.f;
-      for (int i = 0; i < hd; ++i) d = fmaf(qs[i], to_f32(kr[i]), d);
-      s = d;
-    }
-    const float m_new = fmaxf(m, block_max(s, scratch));
-    const float pj = j < hi ? expf(s - m_new) : 0.f;
-    p[tid] = pj;
-    const float csum = block_sum(pj, scratch);  // also orders the writes of p and rows
-    const float alpha = expf(m - m_new);
-    l = l * alpha + csum;
-    const int n = min(CHUNK, hi - c0);
+  const int hd = kv.head_dim, hq = quads(hd), ld = hq + 4;
+  float* qs = smem;                          // [NQ][hq], zeros beyond hd
+  float* p = qs + NQ * hq;                   // [NQ][CHUNK]
+  float* sums = p + NQ * CHUNK;              // [2][NQ][WARPS] the warps' maxima and sums
+  float* tile = sums + 2 * NQ * WARPS;       // keys [CHUNK][ld], then values [hd][CHUNK + 4]
+  size_t* rows = (size_t*)(tile + tile_floats(hd));   // [2][CHUNK] where a position's key and value lie
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int rep = nh / kv.num_kv_heads, parts = (rep + HEADS - 1) / HEADS;
+  const int g = blockIdx.y / parts, h0 = g * rep + blockIdx.y % parts * HEADS;
+  const int live = min(HEADS, (g + 1) * rep - h0);
+  const int last = min(ntok, (int)(blockIdx.x + 1) * TOKENS);
+  // the block's tokens that read the same keys from the same first one on are worked together
+  for (int t = blockIdx.x * TOKENS, together; t < last; t += together) {
+    const int seq = tok_seq[t], slot = seq_slot[seq];
+    const int lo = window > 0 ? max(0, tok_pos[t] + 1 - window) : 0;
+    int hi[TOKENS], most = 0, fewest = 0x7fffffff;
+    together = 0;
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      const int d = tid + u * CHUNK;
-      if (d < hd) {
-        float a = acc[u] * alpha;
-        for (int jj = 0; jj < n; ++jj) a = fmaf(p[jj], to_f32(vcache[rows[jj] + (size_t)d * kv.page_size]), a);
-        acc[u] = a;
+    for (int i = 0; i < TOKENS; ++i) {
+      const bool in = together == i && t + i < last && tok_seq[t + i] == seq &&
+                      (window > 0 ? max(0, tok_pos[t + i] + 1 - window) : 0) == lo;
+      hi[i] = in ? tok_pos[t + i] + 1 : lo;
+      most = max(most, hi[i]);
+      if (in) fewest = min(fewest, hi[i]);
+      together += in;
+    }
+    __syncthreads();                         // the tokens before have been worked
+    for (int e = tid; e < NQ * hq; e += CHUNK) {
+      const int c = e / hq, i = e % hq, tok = c / HEADS, h = c % HEADS;
+      qs[e] = tok < together && h < live && i < hd ? to_f32(q[(size_t)(t + tok) * q_stride + (size_t)(h0 + h) * hd + i]) : 0.f;
+    }
+    float m[NQ], l[NQ], acc[NQ][2];
+#pragma unroll
+    for (int c = 0; c < NQ; ++c) m[c] = -INFINITY, l[c] = 0.f, acc[c][0] = acc[c][1] = 0.f;
+    for (int c0 = lo; c0 < most; c0 += CHUNK) {
+      const int n = min(CHUNK, most - c0);
+      __syncthreads();                       // the chunk before has been read
+      if (tid < n) {
+        rows[tid] = kv.row(slot, c0 + tid, g);
+        rows[CHUNK + tid] = kv.vcol(slot, c0 + tid, g);
+      }
+      __syncthreads();
+      if (wide) {                            // hd is a multiple of 4 and rows start at 16-byte boundaries
+        for (int e = tid; e < n * (hd / 4); e += CHUNK) {
+          const int j = e / (hd / 4), i = e % (hd / 4) * 4;
+          bring4(tile + j * ld + i, kcache + rows[j] + i);
+        }
+      } else {
+        for (int j = warp; j < n; j += WARPS)
+          for (int i = lane; i < hq; i += 32)
+            if (i < hd) bring1(tile + j * ld + i, kcache + rows[j] + i);
+            else tile[j * ld + i] = 0.f;
+      }
+      copies_done();
+      __syncthreads();
+      float s[NQ];
+#pragma unroll
+      for (int c = 0; c < NQ; ++c) s[c] = 0.f;
+      if (tid < n) {
+        const float4* kr = (const float4*)(tile + tid * ld);
+#pragma unroll 2
+        for (int i = 0; i < hq / 4; ++i) {
+          const float4 kd = kr[i];
+#pragma unroll
+          for (int c = 0; c < NQ; ++c) s[c] = dot4(s[c], ((const float4*)(qs + c * hq))[i], kd);
+        }
+      }
+      // maxima and sums of all queries meet over the four warps at once, in the order of block_max and block_sum
+#pragma unroll
+      for (int c = 0; c < NQ; ++c) {
+        s[c] = c0 + tid < hi[c / HEADS] ? s[c] : -INFINITY;
+        const float v = warp_max(s[c]);
+        if (lane == 0) sums[c * WARPS + warp] = v;
+      }
+      __syncthreads();                       // also: every thread is past its own key
+      const bool whole = wide && kv.page_size % 4 == 0 && c0 % 4 == 0;     // four positions side by side in one page
+      if (whole) {
+        for (int e = tid; e < (n / 4) * hd; e += CHUNK) {
+          const int d = e / (n / 4), j = e % (n / 4) * 4;
+          bring4(tile + d * (CHUNK + 4) + j, vcache + rows[CHUNK + j] + (size_t)d * kv.page_size);
+        }
+      }
+      for (int j0 = whole ? n / 4 * 4 : 0; j0 < n; j0 += 32)
+        for (int d = warp; d < hd; d += WARPS)
+          if (j0 + lane < n) bring1(tile + d * (CHUNK + 4) + j0 + lane, vcache + rows[CHUNK + j0 + lane] + (size_t)d * kv.page_size);
+      float alpha[NQ];
+#pragma unroll
+      for (int c = 0; c < NQ; ++c) {
+        const float* w = sums + c * WARPS;
+        const float m_new = fmaxf(m[c], fmaxf(fmaxf(w[0], w[2]), fmaxf(w[1], w[3])));
+        // a token none of whose keys lie in this chunk keeps what it has
+        const bool any = c0 < hi[c / HEADS];
+        const float pj = c0 + tid < hi[c / HEADS] ? expf(s[c] - m_new) : 0.f;
+        p[c * CHUNK + tid] = pj;
+        const float v = warp_sum(pj);
+        if (lane == 0) sums[(NQ + c) * WARPS + warp] = v;
+        alpha[c] = any ? expf(m[c] - m_new) : 1.f;
+        if (any) m[c] = m_new;
+      }
+      copies_done();
+      __syncthreads();
+#pragma unroll
+      for (int c = 0; c < NQ; ++c) {
+        const float* w = sums + (NQ + c) * WARPS;
+        if (c0 < hi[c / HEADS]) l[c] = l[c] * alpha[c] + ((w[0] + w[2]) + (w[1] + w[3]));
+      }
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int d = tid + u * CHUNK;
+        if (d >= hd) continue;
+        const float4* vr = (const float4*)(tile + d * (CHUNK + 4));
+#pragma unroll
+        for (int c = 0; c < NQ; ++c) acc[c][u] *= alpha[c];
+        // positions that every query of the group sees, four at a time, then each query's own last ones
+        const int least = min(CHUNK, max(0, fewest - c0)) / 4 * 4;
+#pragma unroll 2
+        for (int j = 0; j < least / 4; ++j) {
+          const float4 vd = vr[j];
+#pragma unroll
+          for (int c = 0; c < NQ; ++c) acc[c][u] = dot4(acc[c][u], ((const float4*)(p + c * CHUNK))[j], vd);
+        }
+        for (int j = least; j < n; ++j) {
+          const float vd = tile[d * (CHUNK + 4) + j];
+#pragma unroll
+          for (int c = 0; c < NQ; ++c)
+            if (c0 + j < hi[c / HEADS]) acc[c][u] = fmaf(p[c * CHUNK + j], vd, acc[c][u]);
+        }
       }
     }
-    m = m_new;
-    __syncthreads();
-  }
-  T* orow = out + (size_t)t * out_stride + (size_t)h * hd;
 #pragma unroll
-  for (int u = 0; u < 2; ++u) {
-    const int d = tid + u * CHUNK;
-    if (d < hd) orow[d] = from_f32<T>(acc[u] / l);
+    for (int c = 0; c < NQ; ++c) {
+      if (c / HEADS >= together || c % HEADS >= live) continue;
+      T* orow = out + (size_t)(t + c / HEADS) * out_stride + (size_t)(h0 + c % HEADS) * hd;
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int d = tid + u * CHUNK;
+        if (d < hd) orow[d] = from_f32<T>(acc[c][u] / l[c]);
+      }
+    }
   }
+}
+
+template <typename T, int TOKENS, int HEADS, typename... Args>
+static int launch_ref(int ntok, int rep, const PagedKV& kv, cudaStream_t stream, Args... args) {
+  constexpr int NQ = TOKENS * HEADS;
+  const size_t smem = (NQ * (size_t)(quads(kv.head_dim) + CHUNK + 2 * CHUNK / 32) + tile_floats(kv.head_dim)) * sizeof(float) +
+                      2 * CHUNK * sizeof(size_t);
+  auto kernel = attention_ref_kernel<T, TOKENS, HEADS>;
+  if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const dim3 grid((ntok + TOKENS - 1) / TOKENS, kv.num_kv_heads * ((rep + HEADS - 1) / HEADS));
+  gb_launch(kernel, grid, CHUNK, smem, stream, args...);
+  return gb_launch_status();
 }
 
 // q: [ntok, nh, hd] rows q_stride apart (already normed, rotated, scaled); out likewise.
@@ -80,17 +218,18 @@ GB_EXPORT int gb_attention_ref(const void* q, long long q_stride, void* out, lon
   if (ntok <= 0) return 0;
   if (hd <= 0 || hd > 2 * CHUNK || nkv <= 0 || nh % nkv) return GB_ERR_SIZE;
   PagedKV kv{page_table, table_width, page_size, nkv, hd};
-  const size_t smem = (size_t)(hd + CHUNK + 34) * sizeof(float) + CHUNK * sizeof(size_t) + 8;
-  dim3 grid(ntok, nh);
-  if (dtype == GB_F32)
-    gb_launch(attention_ref_kernel<float>, grid, CHUNK, smem, stream, (const float*)q, q_stride, (float*)out, out_stride,
-                                                              (const float*)kcache, (const float*)vcache, kv,
-                                                              tok_pos, tok_seq, seq_slot, nh, window);
-  else if (dtype == GB_BF16)
-    gb_launch(attention_ref_kernel<bf16>, grid, CHUNK, smem, stream, (const bf16*)q, q_stride, (bf16*)out, out_stride,
-                                                             (const bf16*)kcache, (const bf16*)vcache, kv, tok_pos,
-                                                             tok_seq, seq_slot, nh, window);
-  else
-    return GB_ERR_DTYPE;
-  return gb_launch_status();
+  const int rep = nh / nkv, heads = rep >= 3 ? 4 : rep;
+  // Positions of a prompt share their keys: four tokens a block, once that leaves two blocks an SM
+  const bool four = (long long)ntok * nkv * ((rep + heads - 1) / heads) >= 4 * 2 * 148;
+  const int wide = hd % 4 == 0 && (((uintptr_t)kcache | (uintptr_t)vcache) & 15) == 0;
+#define REF(T, TOKENS, HEADS)                                                                                              \
+  launch_ref<T, TOKENS, HEADS>(ntok, rep, kv, stream, (const T*)q, q_stride, (T*)out, out_stride, (const T*)kcache, (const T*)vcache, \
+                               kv, tok_pos, tok_seq, seq_slot, ntok, nh, window, wide)
+#define REF_HEADS(T) (heads == 1 ? (four ? REF(T, 4, 1) : REF(T, 1, 1)) : heads == 2 ? (four ? REF(T, 4, 2) : REF(T, 1, 2)) \
+                                                                                   : (four ? REF(T, 4, 4) : REF(T, 1, 4)))
+  if (dtype == GB_F32) return REF_HEADS(float);
+  if (dtype == GB_BF16) return REF_HEADS(bf16);
+#undef REF_HEADS
+#undef REF
+  return GB_ERR_DTYPE;
 }

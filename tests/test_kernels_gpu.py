@@ -272,6 +272,32 @@ def test_attention_kernels_against_plain(k, hd, nh, nkv, window):
                 assert err <= tol * max(1.0, ref.abs().max().item()), f"shares={shares}: {err}"
 
 
+@pytest.mark.parametrize("hd,nh,nkv,window", [(128, 16, 8, None), (128, 8, 8, 70), (30, 12, 2, None), (256, 5, 1, None), (64, 36, 4, 130)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_attention_ref_of_prompts_gives_the_bits_of_single_tokens(k, hd, nh, nkv, window, dtype):
+    """Prompts of unequal lengths (blocks of four tokens across the border of two sequences, chunks of 128 keys begun by
+    some of a block's tokens only) against plain sums, and against the same tokens one at a time."""
+    torch.manual_seed(hd + nh)
+    lengths = [190, 1, 61, 126, 131, 67]
+    kc, vc, table, dense = _paged(len(lengths), lengths, nkv, hd, dtype, seed=hd)
+    tok_seq = torch.tensor([i for i, n in enumerate(lengths) for _ in range(n)], dtype=torch.int32, device="cuda")
+    tok_pos = torch.tensor([j for n in lengths for j in range(n)], dtype=torch.int32, device="cuda")
+    slots = torch.arange(len(lengths), dtype=torch.int32, device="cuda")
+    t = len(tok_pos)
+    q = (torch.randn(t, nh * hd, device="cuda") * 2 * hd ** -0.5).to(dtype)
+    out = torch.zeros(t, nh * hd, device="cuda", dtype=dtype)
+    k.attention_ref(q, out, nh, kc, vc, table, 64, tok_pos, tok_seq, slots, window)
+    tol = 2e-5 if dtype == torch.float32 else 2 ** -7
+    for i in (0, 125, 189, 190, 191, 255, 300, t - 1):
+        s = int(tok_seq[i])
+        ref = _attn_ref(q[i].float().view(nh, hd), *dense[s], int(tok_pos[i]), nh, window).view(-1)
+        assert (out[i].float() - ref).abs().max().item() <= tol * max(1.0, ref.abs().max().item())
+    alone = torch.zeros_like(out)
+    for i in range(0, t, 7):
+        k.attention_ref(q[i:i + 1], alone[i:i + 1], nh, kc, vc, table, 64, tok_pos[i:i + 1], tok_seq[i:i + 1], slots, window)
+        assert torch.equal(alone[i], out[i])
+
+
 @pytest.mark.parametrize("hd,nh,nkv,window,ring", [(64, 4, 2, None, None), (128, 8, 2, 100, None), (64, 12, 1, None, None),
                                                     (128, 32, 8, None, None), (128, 6, 3, 128, 3), (64, 16, 1, 70, None)])
 def test_attention_decode_stream_against_plain(k, hd, nh, nkv, window, ring):
