@@ -1,0 +1,550 @@
+// Prompts through the recurrent mixers in chunks of 16 tokens: the delta rule (a decay per head or per key
+// channel), the selective state space, and linear attention with a decay per key channel (read before or
+// after the write).  recurrent.cu walks a sequence token by token; there a prompt of one sequence is bound by
+// the chain from one token's state to the next (0.6 us a token at heads of 128 x 128).  Here the chain is from
+// chunk to chunk, and what a chunk does to the state is three small matrix products on the tensor cores.
+//
+// With S the state before a chunk, and for its tokens i the decay products G_i (up to and with token i, a number
+// per key channel, or one for all), K~ and Q~ rows that carry them, all four recurrences are
+//     U  = T V - W S                  (what the tokens write; the state space and linear attention: U = V)
+//     Y  = Q~ S + P U                 P[i, j], j <= i: what token i reads of token j's write
+//     S <- G_16 S + Kd^T U            Kd[j]: k of token j, decayed to the chunk's end
+// where for the delta rule A[i, j] = beta_i k_i . (G_i / G_j) k_j (j < i), T = (1 + A)^-1 diag(beta) and
+// W = (1 + A)^-1 diag(beta) (G K).  Ratios of decays are products over the tokens between, never quotients, so a
+// decay of zero is no exception.
+//
+// chunk_prepare_kernel makes Q~, Kd, W, P, T and G of every (chunk, head): all chunks side by side, nothing of it
+// depends on the state.  chunk_scan_kernel walks the chunks: a warp holds 16 columns of the state, transposed,
+// as accumulators of mma.sync m16n8k8, which are at the same time the next product's left operand (the inner
+// index may be taken in any order, and lane t's two neighbouring columns of an accumulator stand for inner
+// indexes t and t + 4).
+//
+// Numbers: everything is float32.  A product's operands are split into two tf32 halves, hi + lo (hi rounded to
+// nearest, so lo is at most 2^-12 of the number), and hi hi + hi lo + lo hi is summed in float32: what is left out
+// is 2^-22 of a product, as much as float32 rounding itself.  The state's own sum, S <- G S + (chunk's part), is a
+// float32 fused multiply-add outside the tensor cores.  A value that is not finite reaches the outputs of its whole
+// chunk (zero times infinity), not only of the tokens from its own on.
+#include "common.cuh"
+
+namespace {
+
+constexpr int CT = 16;      // tokens of a chunk
+enum { DELTA = 0, CHANNEL_DELTA = 1, STATE_SPACE = 2, READ_BEFORE = 3, READ_AFTER = 4 };
+__host__ __device__ constexpr bool is_delta(int mode) { return mode == DELTA || mode == CHANNEL_DELTA; }
+__host__ __device__ constexpr bool per_channel(int mode) { return mode == CHANNEL_DELTA || mode == READ_BEFORE || mode == READ_AFTER; }
+
+// A (chunk, head)'s block in memory, in floats: Q~, Kd (, W), P (, T) as the scan's lanes read them, G.
+template <int DP, bool HAS_W>
+struct Block {
+  static constexpr int Q = 0, K = DP * CT, W = 2 * DP * CT, P = (HAS_W ? 3 : 2) * DP * CT, T = P + CT * CT,
+                       G = T + (HAS_W ? CT * CT : 0), FLOATS = G + DP;
+};
+
+__device__ __forceinline__ float sigmoid_f(float z) { return 1.0f / (1.0f + expf(-z)); }
+__device__ __forceinline__ float softplus_f(float z) { return z > 20.0f ? z : log1pf(expf(z)); }
+
+__device__ __forceinline__ void split(float v, uint32_t& hi, uint32_t& lo) {
+  hi = (__float_as_uint(v) + 0x1000u) & 0xffffe000u;
+  lo = __float_as_uint(v - __uint_as_float(hi));
+}
+__device__ __forceinline__ void mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// d += a b in three parts: hi hi into d, the two cross parts into x.
+__device__ __forceinline__ void mma3(float (&d)[4], float (&x)[4], const uint32_t (&ahi)[4], const uint32_t (&alo)[4], float b0, float b1) {
+  uint32_t h0, l0, h1, l1;
+  split(b0, h0, l0);
+  split(b1, h1, l1);
+  mma(d, ahi, h0, h1);
+  mma(x, ahi, l0, l1);
+  mma(x, alo, h0, h1);
+}
+
+// Chunks are numbered over the whole step: sequence b's are cu[b] / 16 + b and those after it, which leaves room
+// for every sequence's last, partly filled one.
+__host__ __device__ inline int chunk_slots(int ntok, int nseq) { return ntok / CT + nseq; }
+
+struct Prepare {
+  const float *q, *k;                   // rows of ldqk floats, head group g at g * D
+  long long ldqk;
+  const float *first, *second;          // delta: logits of beta (and of the decay); state space: dt
+  long long ldg;
+  const float* decay;                   // per channel: rows of ldd floats, head h at h * D
+  long long ldd;
+  const float *A_log, *dt_bias, *skip, *bonus;
+  const int* cu;
+  int nseq, H, G, D, head0;
+  float qscale;
+  float* blocks;
+  int slots;
+};
+
+template <int DP, int MODE>
+__global__ void __launch_bounds__(128) chunk_prepare_kernel(const Prepare a) {
+  constexpr bool HAS_W = is_delta(MODE), CH = per_channel(MODE);
+  using B = Block<DP, HAS_W>;
+  constexpr int LD = DP + 4;
+  __shared__ float ks[CT][LD], qs[CT][LD], extra[HAS_W || CH ? CT : 1][LD];    // extra: the decays, then W
+  __shared__ float kk[CT][CT + 1], qk[CT][CT + 1], tb[HAS_W ? CT : 1][CT + 1];
+  __shared__ float gate[CT], beta[CT];
+  pdl_release_next();
+  pdl_wait_prior();
+  const int slot = blockIdx.x, head = a.head0 + blockIdx.y, g = head / (a.H / a.G), tid = threadIdx.x, D = a.D;
+  int b = 0;
+  for (int step = 1 << 30; step > 0; step >>= 1)     // the last sequence whose chunks start at or before this one
+    if (b + step < a.nseq && a.cu[b + step] / CT + b + step <= slot) b += step;
+  const int first = a.cu[b] + (slot - (a.cu[b] / CT + b)) * CT, n = min(CT, a.cu[b + 1] - first);
+  if (n <= 0) return;
+  for (int e = tid; e < CT * DP; e += 128) {
+    const int i = e / DP, d = e % DP;
+    const bool in = i < n && d < D;
+    ks[i][d] = in ? a.k[(size_t)(first + i) * a.ldqk + (size_t)g * D + d] : 0.f;
+    qs[i][d] = in ? a.q[(size_t)(first + i) * a.ldqk + (size_t)g * D + d] : 0.f;
+    if (CH) extra[i][d] = in ? a.decay[(size_t)(first + i) * a.ldd + (size_t)head * D + d] : 1.f;
+  }
+  if (tid < CT) {          // tokens beyond the end write nothing and keep everything
+    float bt = 0.f, gt = 1.f;
+    if (tid < n) {
+      const size_t row = (size_t)(first + tid) * a.ldg + head;
+      if (HAS_W) bt = sigmoid_f(a.first[row]);
+      if (MODE == DELTA) gt = expf(-expf(a.A_log[head]) * softplus_f(a.second[row] + a.dt_bias[head]));
+      if (MODE == STATE_SPACE) {
+        bt = softplus_f(a.first[row] + a.dt_bias[head]);
+        gt = expf(-expf(a.A_log[head]) * bt);
+      }
+    }
+    beta[tid] = bt;
+    gate[tid] = gt;
+  }
+  __syncthreads();
+  const int warp = tid >> 5, lane = tid & 31;
+  if (HAS_W) {             // unit vectors
+    for (int i = warp; i < CT; i += 4) {
+      float k2 = 0.f, q2 = 0.f;
+#pragma unroll
+      for (int d = lane; d < DP; d += 32) k2 = fmaf(ks[i][d], ks[i][d], k2), q2 = fmaf(qs[i][d], qs[i][d], q2);
+      const float ik = 1.0f / sqrtf(warp_sum(k2) + 1e-6f), iq = a.qscale / sqrtf(warp_sum(q2) + 1e-6f);
+#pragma unroll
+      for (int d = lane; d < DP; d += 32) ks[i][d] *= ik, qs[i][d] *= iq;
+    }
+    __syncthreads();
+  }
+  if (!CH) {
+    // k_i . k_j and q_i . k_j on the tensor cores, a warp 16 x 8 of either; the decays between come after
+    const int gr = lane >> 2, t = lane & 3, nt = warp & 1, which = warp >> 1;
+    if (which == 0 || HAS_W) {
+      const float(*rows)[LD] = which ? ks : qs;
+      float d[4] = {}, x[4] = {};
+#pragma unroll
+      for (int s = 0; s < DP / 8; ++s) {
+        uint32_t hi[4], lo[4];
+        split(rows[gr][8 * s + t], hi[0], lo[0]);
+        split(rows[gr + 8][8 * s + t], hi[1], lo[1]);
+        split(rows[gr][8 * s + t + 4], hi[2], lo[2]);
+        split(rows[gr + 8][8 * s + t + 4], hi[3], lo[3]);
+        mma3(d, x, hi, lo, ks[8 * nt + gr][8 * s + t], ks[8 * nt + gr][8 * s + t + 4]);
+      }
+      float(*out)[CT + 1] = which ? kk : qk;
+      out[gr][8 * nt + 2 * t] = d[0] + x[0];
+      out[gr][8 * nt + 2 * t + 1] = d[1] + x[1];
+      out[gr + 8][8 * nt + 2 * t] = d[2] + x[2];
+      out[gr + 8][8 * nt + 2 * t + 1] = d[3] + x[3];
+    }
+    __syncthreads();
+    const int j = tid >> 3, i0 = (tid & 7) * 2;       // two neighbouring rows of a column
+    float r = 1.f;
+#pragma unroll
+    for (int l = 1; l < CT; ++l)
+      if (l > j && l <= i0) r *= gate[l];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int i = i0 + u;
+      if (u && i > j) r *= gate[i];
+      float p = i >= j ? qk[i][j] * r : 0.f;
+      if (MODE == STATE_SPACE) p = p * beta[j] + (i == j ? a.skip[head] : 0.f);
+      qk[i][j] = p;
+      if (HAS_W) kk[i][j] = i > j ? beta[i] * (kk[i][j] * r) : 0.f;
+    }
+  } else {
+    // a decay per channel stands inside the sums: 16 lanes take a column's sums, DP / 16 channels each, and carry
+    // k_j times the decays since j from row to row; columns j and 15 - j together have 17 rows
+    const int pair = tid >> 4, part = tid & 15;
+    const unsigned mine = 0xffffu << (lane & 16);       // the halves of a warp walk columns of unequal length
+#pragma unroll 1
+    for (int half = 0; half < 2; ++half) {
+      const int j = half ? CT - 1 - pair : pair;
+      float kr[DP / 16];
+#pragma unroll
+      for (int e = 0; e < DP / 16; ++e) kr[e] = ks[j][part + 16 * e];
+      for (int i = j; i < CT; ++i) {
+        float sq = 0.f, sk = 0.f;
+#pragma unroll
+        for (int e = 0; e < DP / 16; ++e) {
+          const int d = part + 16 * e;
+          if (MODE == READ_BEFORE) {                  // token i reads before its own decay and write
+            sq = fmaf(qs[i][d], i == j ? (d < D ? a.bonus[(size_t)head * D + d] : 0.f) * kr[e] : kr[e], sq);
+            if (i > j) kr[e] *= extra[i][d];
+          } else {
+            if (i > j) kr[e] *= extra[i][d];
+            sq = fmaf(qs[i][d], kr[e], sq);
+            if (HAS_W) sk = fmaf(ks[i][d], kr[e], sk);
+          }
+        }
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) {
+          sq += __shfl_xor_sync(mine, sq, o, 16);
+          if (HAS_W) sk += __shfl_xor_sync(mine, sk, o, 16);
+        }
+        if (part == 0) {
+          qk[i][j] = sq;
+          if (HAS_W) kk[i][j] = i > j ? beta[i] * sk : 0.f;
+        }
+      }
+      if (part < j) qk[part][j] = 0.f;
+    }
+  }
+  __syncthreads();
+  // a thread a channel: Q~, Kd and G, and W by forward substitution; then T's columns in the same way
+  if (tid < DP) {
+    float c = 1.f, w[HAS_W ? CT : 1];
+#pragma unroll
+    for (int i = 0; i < CT; ++i) {
+      const float gi = CH ? extra[i][tid] : gate[i];
+      if (MODE == READ_BEFORE) {
+        qs[i][tid] *= c;
+        c *= gi;
+      } else {
+        c *= gi;
+        qs[i][tid] *= c;
+      }
+      if (HAS_W) {
+        float v = beta[i] * (c * ks[i][tid]);
+#pragma unroll
+        for (int j = 0; j < i; ++j) v = fmaf(-kk[i][j], w[j], v);
+        w[HAS_W ? i : 0] = v;
+      }
+    }
+    a.blocks[((size_t)blockIdx.y * a.slots + slot) * B::FLOATS + B::G + tid] = c;
+    float r = 1.f;
+#pragma unroll
+    for (int i = CT - 1; i >= 0; --i) {
+      const float gi = CH ? extra[i][tid] : gate[i];
+      ks[i][tid] *= MODE == STATE_SPACE ? r * beta[i] : r;
+      r *= gi;
+    }
+    if (HAS_W) {
+#pragma unroll
+      for (int i = 0; i < CT; ++i) extra[i][tid] = w[HAS_W ? i : 0];
+    }
+  }
+  if (HAS_W && tid >= 128 - CT) {
+    const int c = tid - (128 - CT);
+    float t[CT];
+#pragma unroll
+    for (int i = 0; i < CT; ++i) {
+      float v = i == c ? beta[i] : 0.f;
+#pragma unroll
+      for (int j = 0; j < i; ++j) v = fmaf(-kk[i][j], t[j], v);
+      tb[HAS_W ? i : 0][c] = t[i] = v;
+    }
+  }
+  __syncthreads();
+  float4* out = (float4*)(a.blocks + ((size_t)blockIdx.y * a.slots + slot) * B::FLOATS);
+  for (int e = tid; e < DP * CT / 4; e += 128) {
+    const int l = e & 31, gr = l >> 2, t = l & 3;
+    const int row = 8 * ((e >> 5) & 1) + gr, col = 16 * (e >> 6) + 2 * t;
+    out[B::Q / 4 + e] = make_float4(qs[row][col], qs[row][col + 1], qs[row][col + 8], qs[row][col + 9]);
+    if (HAS_W) out[B::W / 4 + e] = make_float4(extra[row][col], extra[row][col + 1], extra[row][col + 8], extra[row][col + 9]);
+    const int dim = 8 * (e >> 5) + gr;
+    out[B::K / 4 + e] = make_float4(ks[2 * t][dim], ks[2 * t + 1][dim], ks[8 + 2 * t][dim], ks[9 + 2 * t][dim]);
+  }
+  if (tid < CT * CT / 4) {
+    const int l = tid & 31, gr = l >> 2, t = l & 3, row = 8 * (tid >> 5) + gr;
+    out[B::P / 4 + tid] = make_float4(qk[row][2 * t], qk[row][2 * t + 1], qk[row][8 + 2 * t], qk[row][9 + 2 * t]);
+    if (HAS_W) out[B::T / 4 + tid] = make_float4(tb[row][2 * t], tb[row][2 * t + 1], tb[row][8 + 2 * t], tb[row][9 + 2 * t]);
+  }
+}
+
+struct Scan {
+  const float* blocks;
+  int slots;
+  const float* v;                       // rows of ldv floats, head h at h * V
+  long long ldv;
+  float* state;                         // [slots, H, 8 V lanes 4]: the order of recurrent.cu
+  const int *cu, *seq_slot;
+  float* y;                             // [ntok, H * V]
+  int H, head0, V, lanes;               // lanes: 32 channels of a column each, as the state lies in memory
+  float yscale;
+};
+
+// NV groups of 16 columns a CTA; a group's channels are shared by DS warps (their parts of U and Y meet in shared
+// memory, added in one order).  Blocks of coming chunks arrive by asynchronous copies, STAGES - 1 ahead.
+template <int DP, int DS, int NV, bool HAS_W, int STAGES>
+__global__ void __launch_bounds__(32 * DS * NV) chunk_scan_kernel(const Scan a) {
+  using B = Block<DP, HAS_W>;
+  constexpr int NT = 32 * DS * NV, DW = DP / DS, NJ = DW / 8;
+  extern __shared__ __align__(16) float smem[];
+  float* exch = smem + STAGES * B::FLOATS;             // [2][warps][12][32], with DS 2
+  pdl_wait_prior();
+  const int b = blockIdx.x, head = a.head0 + blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int gr = lane >> 2, t = lane & 3, part = warp % DS, V = a.V;
+  const int col0 = (blockIdx.z * NV + warp / DS) * 16, d0 = part * DW;
+  const int t0 = a.cu[b], t1 = a.cu[b + 1], chunks = (t1 - t0 + CT - 1) / CT;
+  const float* blocks = a.blocks + ((size_t)blockIdx.y * a.slots + t0 / CT + b) * B::FLOATS;
+  auto bring = [&](int c) {
+    if (c < chunks) {
+      const float* src = blocks + (size_t)c * B::FLOATS;
+      const uint32_t dst = (uint32_t)__cvta_generic_to_shared(smem + (c % STAGES) * B::FLOATS);
+      for (int e = tid; e < B::FLOATS / 4; e += NT)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16 * e), "l"(src + 4 * e) : "memory");
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+#pragma unroll
+  for (int c = 0; c < STAGES - 1; ++c) bring(c);
+  const bool in0 = col0 + gr < V, in1 = col0 + gr + 8 < V;
+  const float* vcol = a.v + (size_t)head * V + col0 + gr;
+  float vn[2][4];
+  auto fetch_v = [&](int c) {          // V transposed as a left operand: columns gr, gr + 8; tokens 2 t, 2 t + 1 of each half
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int tok = t0 + c * CT + 8 * h + 2 * t + (e >> 1);
+        vn[h][e] = tok < t1 && ((e & 1) ? in1 : in0) ? vcol[(size_t)tok * a.ldv + 8 * (e & 1)] : 0.f;
+      }
+  };
+  if (chunks > 0) fetch_v(0);
+  float* st = a.state + ((size_t)a.seq_slot[b] * a.H + head) * 32 * V * a.lanes;
+  auto place = [&](int j, int col) {   // of channels d0 + 8 j + 2 t and the next
+    const int d = d0 + 8 * j + 2 * t;
+    return ((size_t)((d & 31) >> 2) * V + col) * a.lanes * 4 + (d >> 5) * 4 + (d & 3);
+  };
+  float S[NJ][4];
+#pragma unroll
+  for (int j = 0; j < NJ; ++j) {
+    const bool in = d0 + 8 * j < 32 * a.lanes;
+    const float2 x = in && in0 ? *(const float2*)(st + place(j, col0 + gr)) : make_float2(0.f, 0.f);
+    const float2 z = in && in1 ? *(const float2*)(st + place(j, col0 + gr + 8)) : make_float2(0.f, 0.f);
+    S[j][0] = x.x; S[j][1] = x.y; S[j][2] = z.x; S[j][3] = z.y;
+  }
+  asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
+  __syncthreads();
+#pragma unroll 1
+  for (int c = 0; c < chunks; ++c) {
+    const float4* blk = (const float4*)(smem + (c % STAGES) * B::FLOATS);
+    uint32_t vhi[2][4], vlo[2][4];
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) split(vn[h][e], vhi[h][e], vlo[h][e]);
+    if (c + 1 < chunks) fetch_v(c + 1);
+    // W S and Q~ S over this warp's channels, transposed: 16 columns by 16 tokens
+    float y[2][4] = {}, yx[2][4] = {}, u[2][4] = {}, ux[2][4] = {};
+#pragma unroll
+    for (int jp = 0; jp < NJ / 2; ++jp) {
+      const int at = (d0 / 16 + jp) * 64 + lane;
+      float4 qf[2], wf[2];
+#pragma unroll
+      for (int nt = 0; nt < 2; ++nt) {
+        qf[nt] = blk[B::Q / 4 + at + 32 * nt];
+        if (HAS_W) wf[nt] = blk[B::W / 4 + at + 32 * nt];
+      }
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const float(&s)[4] = S[2 * jp + h];
+        uint32_t hi[4], lo[4];
+        split(s[0], hi[0], lo[0]);
+        split(s[2], hi[1], lo[1]);
+        split(s[1], hi[2], lo[2]);
+        split(s[3], hi[3], lo[3]);
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt) {
+          if (HAS_W) mma3(u[nt], ux[nt], hi, lo, h ? wf[nt].z : wf[nt].x, h ? wf[nt].w : wf[nt].y);
+          mma3(y[nt], yx[nt], hi, lo, h ? qf[nt].z : qf[nt].x, h ? qf[nt].w : qf[nt].y);
+        }
+      }
+    }
+#pragma unroll
+    for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        y[nt][e] += yx[nt][e];
+        if (HAS_W) u[nt][e] = -(u[nt][e] + ux[nt][e]);
+      }
+    if (HAS_W && part == 0) {           // + T V
+#pragma unroll
+      for (int nt = 0; nt < 2; ++nt) {
+        const float4 tf = blk[B::T / 4 + 32 * nt + lane];
+        float d[4] = {}, x[4] = {};
+        mma3(d, x, vhi[0], vlo[0], tf.x, tf.y);
+        mma3(d, x, vhi[1], vlo[1], tf.z, tf.w);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) u[nt][e] += d[e] + x[e];
+      }
+    }
+    if (DS == 2) {
+      float* mine = exch + ((c & 1) * DS * NV + warp) * 384 + lane;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        if (HAS_W) mine[32 * e] = u[0][e], mine[32 * (4 + e)] = u[1][e];
+        mine[32 * (8 + e)] = part ? y[0][e] : y[1][e];         // the half of the tokens that the other warp finishes
+      }
+    }
+    asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2 > 0 ? STAGES - 3 : 0) : "memory");
+    __syncthreads();                    // block c + 1 is there; all have left block c - 1
+    bring(c + STAGES - 1);
+    if (DS == 2) {
+      const float* other = exch + ((c & 1) * DS * NV + (warp ^ 1)) * 384 + lane;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        if (HAS_W) u[0][e] += other[32 * e], u[1][e] += other[32 * (4 + e)];
+        y[0][e] = (part ? y[1][e] : y[0][e]) + other[32 * (8 + e)];
+      }
+    }
+    uint32_t uhi[2][4], ulo[2][4];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      if (HAS_W) {
+        split(u[h][0], uhi[h][0], ulo[h][0]);
+        split(u[h][2], uhi[h][1], ulo[h][1]);
+        split(u[h][1], uhi[h][2], ulo[h][2]);
+        split(u[h][3], uhi[h][3], ulo[h][3]);
+      } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) uhi[h][e] = vhi[h][e], ulo[h][e] = vlo[h][e];
+      }
+    }
+    // S <- G S + Kd^T U
+    const float* gs = (const float*)blk + B::G + d0;
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) {
+      const float4 kf = blk[B::K / 4 + (d0 / 8 + j) * 32 + lane];
+      const float2 gf = *(const float2*)(gs + 8 * j + 2 * t);
+      float d[4] = {}, x[4] = {};
+      mma3(d, x, uhi[0], ulo[0], kf.x, kf.y);
+      mma3(d, x, uhi[1], ulo[1], kf.z, kf.w);
+      S[j][0] = fmaf(gf.x, S[j][0], d[0] + x[0]);
+      S[j][1] = fmaf(gf.y, S[j][1], d[1] + x[1]);
+      S[j][2] = fmaf(gf.x, S[j][2], d[2] + x[2]);
+      S[j][3] = fmaf(gf.y, S[j][3], d[3] + x[3]);
+    }
+    // Y = Q~ S + P U, of the tokens that this warp finishes
+#pragma unroll
+    for (int i = 0; i < 2 / DS; ++i) {
+      const int nt = DS == 2 ? part : i;
+      const float4 pf = blk[B::P / 4 + 32 * nt + lane];
+      float d[4] = {}, x[4] = {};
+      mma3(d, x, uhi[0], ulo[0], pf.x, pf.y);
+      mma3(d, x, uhi[1], ulo[1], pf.z, pf.w);
+      const int tok = t0 + c * CT + 8 * nt + 2 * t;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int to = tok + (e & 1);
+        if (to < t1 && (e < 2 ? in0 : in1))
+          a.y[(size_t)to * a.H * V + (size_t)head * V + col0 + gr + 8 * (e >> 1)] = (y[i][e] + (d[e] + x[e])) * a.yscale;
+      }
+    }
+  }
+  pdl_release_next();
+#pragma unroll
+  for (int j = 0; j < NJ; ++j) {
+    if (d0 + 8 * j >= 32 * a.lanes) continue;
+    if (in0) *(float2*)(st + place(j, col0 + gr)) = make_float2(S[j][0], S[j][1]);
+    if (in1) *(float2*)(st + place(j, col0 + gr + 8)) = make_float2(S[j][2], S[j][3]);
+  }
+}
+
+template <int DP, int DS, int NV, bool HAS_W>
+static void launch_scan(const Scan& s, int nseq, int heads, cudaStream_t stream) {
+  constexpr int STAGES = 3;
+  constexpr size_t smem = (STAGES * Block<DP, HAS_W>::FLOATS + (DS == 2 ? 2 * DS * NV * 384 : 0)) * sizeof(float);
+  auto kernel = chunk_scan_kernel<DP, DS, NV, HAS_W, STAGES>;
+  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const dim3 grid(nseq, heads, (s.V + 16 * NV - 1) / (16 * NV));
+  // without the attribute that lets it start under the kernel before it, so that its few, long blocks spread one to
+  // an SM (see launch_scan in recurrent.cu)
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = 32 * DS * NV;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchKernelEx(&cfg, kernel, s);
+}
+
+template <int DP, int MODE>
+static int run(Prepare p, Scan s, int ntok, int heads_at_once, cudaStream_t stream) {
+  constexpr bool HAS_W = is_delta(MODE);
+  p.slots = s.slots = chunk_slots(ntok, p.nseq);
+  for (int h = 0; h < p.H; h += heads_at_once) {
+    const int heads = p.H - h < heads_at_once ? p.H - h : heads_at_once;
+    p.head0 = s.head0 = h;
+    gb_launch(chunk_prepare_kernel<DP, MODE>, dim3(p.slots, heads), 128, 0, stream, p);
+    const long long groups = (long long)p.nseq * heads * ((s.V + 15) / 16);
+    if (groups <= 2 * 148) {
+      if constexpr (DP == 128)
+        launch_scan<DP, 2, 2, HAS_W>(s, p.nseq, heads, stream);
+      else
+        launch_scan<DP, 1, 2, HAS_W>(s, p.nseq, heads, stream);
+    } else {
+      launch_scan<DP, 1, 4, HAS_W>(s, p.nseq, heads, stream);
+    }
+  }
+  return gb_launch_status();
+}
+
+template <int MODE>
+static int run_any(const Prepare& p, const Scan& s, int ntok, long long scratch_floats, cudaStream_t stream) {
+  constexpr bool HAS_W = is_delta(MODE);
+  if (p.nseq <= 0 || ntok <= 0) return 0;
+  if (p.D <= 0 || p.D > 128 || s.V <= 0 || p.H <= 0 || p.G <= 0 || p.H % p.G || ((uintptr_t)s.state & 15) ||
+      ((uintptr_t)p.blocks & 15))
+    return GB_ERR_SIZE;
+  const long long head = (long long)chunk_slots(ntok, p.nseq) * (p.D <= 64 ? Block<64, HAS_W>::FLOATS : Block<128, HAS_W>::FLOATS);
+  const long long most = scratch_floats / head;
+  if (most < 1) return GB_ERR_SIZE;
+  const int heads = most < p.H ? (int)most : p.H;
+  return p.D <= 64 ? run<64, MODE>(p, s, ntok, heads, stream) : run<128, MODE>(p, s, ntok, heads, stream);
+}
+
+static int lanes_for(int dims) { return dims <= 32 ? 1 : (dims <= 64 ? 2 : 4); }
+
+}  // namespace
+
+// Floats of scratch that one head of a step needs (delta: the two forms of the delta rule); the entry points below
+// take as many heads at once as their scratch holds.
+GB_EXPORT long long gb_chunk_floats(int ntok, int nseq, int dims, int delta) {
+  const int per = dims <= 64 ? (delta ? Block<64, true>::FLOATS : Block<64, false>::FLOATS)
+                             : (delta ? Block<128, true>::FLOATS : Block<128, false>::FLOATS);
+  return (long long)chunk_slots(ntok, nseq) * per;
+}
+
+// The arguments are those of the entry points of recurrent.cu, with the step's tokens and the scratch; D up to 128.
+// decay null: the delta rule with a decay per head (a_logit, A_log, dt_bias); else with a decay per channel.
+GB_EXPORT int gb_chunk_delta_rule(const float* q, const float* k, const float* v, long long ld, const float* beta_logit,
+                                  const float* a_logit, long long ldg, const float* A_log, const float* dt_bias, const float* decay,
+                                  long long ldd, float* state, const int* cu, const int* seq_slot, float* y, int ntok, int nseq, int H,
+                                  int G, int D, int V, float qscale, float* scratch, long long scratch_floats, cudaStream_t stream) {
+  Prepare p = {q, k, ld, beta_logit, a_logit, ldg, decay, ldd, A_log, dt_bias, nullptr, nullptr, cu, nseq, H, G, D, 0, qscale, scratch, 0};
+  Scan s = {scratch, 0, v, ld, state, cu, seq_slot, y, H, 0, V, lanes_for(D), 1.0f};
+  return decay ? run_any<CHANNEL_DELTA>(p, s, ntok, scratch_floats, stream) : run_any<DELTA>(p, s, ntok, scratch_floats, stream);
+}
+
+GB_EXPORT int gb_chunk_ssd_scan(const float* x, const float* Bm, const float* Cm, long long ld, const float* dt_raw, long long ldd,
+                                const float* A_log, const float* dt_bias, const float* skip, float* state, const int* cu,
+                                const int* seq_slot, float* y, int ntok, int nseq, int H, int G, int N, int V, float* scratch,
+                                long long scratch_floats, cudaStream_t stream) {
+  Prepare p = {Cm, Bm, ld, dt_raw, nullptr, ldd, nullptr, 0, A_log, dt_bias, skip, nullptr, cu, nseq, H, G, N, 0, 1.0f, scratch, 0};
+  Scan s = {scratch, 0, x, ld, state, cu, seq_slot, y, H, 0, V, lanes_for(N), 1.0f};
+  return run_any<STATE_SPACE>(p, s, ntok, scratch_floats, stream);
+}
+
+GB_EXPORT int gb_chunk_wkv_scan(const float* r, const float* k, const float* w, long long ld, long long ldw, const float* v, long long ldv,
+                                const float* bonus, float* state, const int* cu, const int* seq_slot, float* y, int ntok, int nseq,
+                                int H, int D, int V, float yscale, float* scratch, long long scratch_floats, cudaStream_t stream) {
+  Prepare p = {r, k, ld, nullptr, nullptr, 0, w, ldw, nullptr, nullptr, nullptr, bonus, cu, nseq, H, H, D, 0, 1.0f, scratch, 0};
+  Scan s = {scratch, 0, v, ldv, state, cu, seq_slot, y, H, 0, V, lanes_for(D), yscale};
+  return bonus ? run_any<READ_BEFORE>(p, s, ntok, scratch_floats, stream) : run_any<READ_AFTER>(p, s, ntok, scratch_floats, stream);
+}

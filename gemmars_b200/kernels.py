@@ -1665,13 +1665,53 @@ def recurrent_state_matrix(head_state: torch.Tensor, dims: int, vdim: int) -> to
     return head_state.reshape(8, vdim, lanes, 4).permute(2, 0, 3, 1).reshape(32 * lanes, vdim)[:dims]
 
 
+# A prompt step takes the recurrences in chunks of 16 tokens (recurrent_chunk.cu) where a sequence brings at least
+# this many, in the bfloat16 engine only: the float32 engine's results must not depend on how a prompt is cut into
+# steps, bit for bit, and a chunk's sums are grouped by where the step begins.
+CHUNK_SCAN_MIN_TOKENS = 32
+CHUNK_SCAN_MAX_DIM = 128
+#: bytes of scratch a step's chunks may take (a block a chunk and head); the kernels take the heads in turns beyond it
+CHUNK_SCAN_SCRATCH = 128 << 20
+
+
+def chunk_scan_usable(compute: str, max_new: int, dim: int) -> bool:
+    """Whether a step whose longest sequence brings ``max_new`` tokens walks its recurrences chunk by chunk."""
+    return compute != "float32" and max_new >= CHUNK_SCAN_MIN_TOKENS and dim <= CHUNK_SCAN_MAX_DIM
+
+
+def recurrent_units(compute: str, dim: int):
+    """The units a recurrent mixer with keys of ``dim`` launches."""
+    return [("recurrent", ())] + ([("recurrent_chunk", ())] if chunk_scan_usable(compute, CHUNK_SCAN_MIN_TOKENS, dim) else [])
+
+
+def _chunk_scratch(ntok: int, nseq: int, heads: int, dim: int, delta: bool, device) -> torch.Tensor:
+    f = _fn("recurrent_chunk", "gb_chunk_floats", [c_int, c_int, c_int, c_int])
+    f.restype = c_longlong
+    per = f(ntok, nseq, dim, int(delta))
+    at_once = max(1, min(heads, CHUNK_SCAN_SCRATCH // (4 * per)))
+    turns = -(-heads // at_once)
+    return torch.empty(per * -(-heads // turns), dtype=torch.float32, device=device)
+
+
+def _chunk_delta(q, k, v, ld, beta_logit, a_logit, ldg, a_log, dt_bias, decay, ldd, state, cu_seqlens, seq_slot, y, heads, groups, dim,
+                 vdim, q_scale):
+    scratch = _chunk_scratch(y.shape[0], seq_slot.numel(), heads, dim, True, y.device)
+    f = _fn("recurrent_chunk", "gb_chunk_delta_rule",
+            [c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_longlong,
+             c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p, c_longlong, c_void_p])
+    return f(q, k, v, ld, beta_logit, a_logit, ldg, _ptr(a_log), _ptr(dt_bias), decay, ldd, state.data_ptr(), cu_seqlens.data_ptr(),
+             seq_slot.data_ptr(), y.data_ptr(), y.shape[0], seq_slot.numel(), heads, groups, dim, vdim, q_scale, scratch.data_ptr(),
+             scratch.numel(), _stream())
+
+
 def delta_rule(q, k, v, beta_logit, a_logit, a_log, dt_bias, state, cu_seqlens, seq_slot, y, heads, groups, dim, vdim,
-               q_scale):
+               q_scale, chunked: bool = False):
     """The gated delta rule over each sequence of the packed step (float32 throughout):
     S <- g S; u = beta (v - S^T k^); S <- S + k^ u^T; y = S^T q^, with k^, q^ the unit vectors of k
     and q (q^ times ``q_scale``), beta = sigmoid(beta_logit), g = exp(-exp(a_log) softplus(a_logit +
     dt_bias)).  q, k, v: slices of columns of one [T, *] tensor; ``state`` [slots + 1, heads,
-    recurrent_state_floats(dim, vdim)] (see recurrent_state_matrix); dim up to 256."""
+    recurrent_state_floats(dim, vdim)] (see recurrent_state_matrix); dim up to 256.  ``chunked``: in chunks of 16
+    tokens instead of token by token (dim up to 128)."""
     _cuda(q, k, v, beta_logit, a_logit, a_log, dt_bias, state, cu_seqlens, seq_slot, y)
     for t in (q, k, v, beta_logit, a_logit, y, state):
         assert t.dtype == torch.float32
@@ -1682,6 +1722,11 @@ def delta_rule(q, k, v, beta_logit, a_logit, a_log, dt_bias, state, cu_seqlens, 
     ap, lda = _cols(a_logit)
     assert ld == ldk == ldv and ldg == lda and y.is_contiguous() and y.shape[1] == heads * vdim
     assert state.is_contiguous() and tuple(state.shape[1:]) == (heads, recurrent_state_floats(dim, vdim))
+    if chunked:
+        _check(_chunk_delta(qp, kp, vp, ld, bp, ap, ldg, a_log, dt_bias, None, 0, state, cu_seqlens, seq_slot, y, heads, groups, dim,
+                            vdim, q_scale), "chunk_delta_rule", "attention",
+               _nbytes(y) * 2 + 2 * seq_slot.numel() * heads * dim * vdim * 4)
+        return
     f = _fn("recurrent", "gb_delta_rule",
             [c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_void_p,
              c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p])
@@ -1690,11 +1735,13 @@ def delta_rule(q, k, v, beta_logit, a_logit, a_log, dt_bias, state, cu_seqlens, 
            "delta_rule", "attention", _nbytes(y) * 2 + 2 * seq_slot.numel() * heads * dim * vdim * 4)
 
 
-def ssd_scan(x, b, c, dt_raw, a_log, dt_bias, skip, state, cu_seqlens, seq_slot, y, heads, groups, n_state, vdim):
+def ssd_scan(x, b, c, dt_raw, a_log, dt_bias, skip, state, cu_seqlens, seq_slot, y, heads, groups, n_state, vdim,
+             chunked: bool = False):
     """The state-space recurrence with one decay per head over each sequence of the packed step
     (float32): dt = softplus(dt_raw + dt_bias); S <- exp(-exp(a_log) dt) S + dt B x^T; y = S^T C +
     skip x.  x, b, c: slices of columns of one tensor; ``state`` [slots + 1, heads,
-    recurrent_state_floats(n_state, vdim)]; n_state up to 256."""
+    recurrent_state_floats(n_state, vdim)]; n_state up to 256.  ``chunked``: in chunks of 16 tokens instead of token
+    by token (n_state up to 128)."""
     _cuda(x, b, c, dt_raw, a_log, dt_bias, skip, state, cu_seqlens, seq_slot, y)
     for t in (x, b, c, dt_raw, y, state):
         assert t.dtype == torch.float32
@@ -1704,6 +1751,16 @@ def ssd_scan(x, b, c, dt_raw, a_log, dt_bias, skip, state, cu_seqlens, seq_slot,
     dp, ldd = _cols(dt_raw)
     assert ld == ldb == ldc and y.is_contiguous() and y.shape[1] == heads * vdim
     assert state.is_contiguous() and tuple(state.shape[1:]) == (heads, recurrent_state_floats(n_state, vdim))
+    if chunked:
+        scratch = _chunk_scratch(y.shape[0], seq_slot.numel(), heads, n_state, False, y.device)
+        f = _fn("recurrent_chunk", "gb_chunk_ssd_scan",
+                [c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
+                 c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_longlong, c_void_p])
+        _check(f(xp, bp, cp, ld, dp, ldd, a_log.data_ptr(), dt_bias.data_ptr(), skip.data_ptr(), state.data_ptr(),
+                 cu_seqlens.data_ptr(), seq_slot.data_ptr(), y.data_ptr(), y.shape[0], seq_slot.numel(), heads, groups, n_state, vdim,
+                 scratch.data_ptr(), scratch.numel(), _stream()), "chunk_ssd_scan", "attention",
+               _nbytes(y) * 2 + 2 * seq_slot.numel() * heads * n_state * vdim * 4)
+        return
     f = _fn("recurrent", "gb_ssd_scan",
             [c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
              c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p])
@@ -1792,12 +1849,13 @@ def lowrank_map(z, w2, base, mode: str, rate=None, rate_group: int = 1, tau: flo
     return out
 
 
-def channel_delta_rule(q, k, v, beta_logit, decay, state, cu_seqlens, seq_slot, y, heads, groups, dim, vdim, q_scale):
+def channel_delta_rule(q, k, v, beta_logit, decay, state, cu_seqlens, seq_slot, y, heads, groups, dim, vdim, q_scale,
+                       chunked: bool = False):
     """The delta rule with a decay per head and key channel over each sequence of the packed step
     (float32 throughout): S <- diag(g) S; u = beta (v - S^T k^); S <- S + k^ u^T; y = S^T q^, with k^,
     q^ the unit vectors of k and q (q^ times ``q_scale``), beta = sigmoid(beta_logit), g = ``decay``
     [T, heads * dim] as given.  q, k, v: slices of columns of one [T, *] tensor, q/k head
-    i // (heads / groups) for head i; ``state`` as for delta_rule; dim up to 256."""
+    i // (heads / groups) for head i; ``state`` as for delta_rule; dim up to 256; ``chunked`` as there."""
     _cuda(q, k, v, beta_logit, decay, state, cu_seqlens, seq_slot, y)
     for t in (q, k, v, beta_logit, decay, y, state):
         assert t.dtype == torch.float32
@@ -1808,6 +1866,11 @@ def channel_delta_rule(q, k, v, beta_logit, decay, state, cu_seqlens, seq_slot, 
     dp, ldd = _cols(decay)
     assert ld == ldk == ldv and y.is_contiguous() and y.shape[1] == heads * vdim and decay.shape[1] == heads * dim
     assert state.is_contiguous() and tuple(state.shape[1:]) == (heads, recurrent_state_floats(dim, vdim))
+    if chunked:
+        _check(_chunk_delta(qp, kp, vp, ld, bp, None, ldb, None, None, dp, ldd, state, cu_seqlens, seq_slot, y, heads, groups, dim,
+                            vdim, q_scale), "chunk_channel_delta_rule", "attention",
+               _nbytes(y) * 2 + _nbytes(decay) + 2 * seq_slot.numel() * heads * dim * vdim * 4)
+        return
     f = _fn("recurrent", "gb_channel_delta_rule",
             [c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p,
              c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p])
@@ -1816,13 +1879,14 @@ def channel_delta_rule(q, k, v, beta_logit, decay, state, cu_seqlens, seq_slot, 
            "channel_delta_rule", "attention", _nbytes(y) * 2 + _nbytes(decay) + 2 * seq_slot.numel() * heads * dim * vdim * 4)
 
 
-def wkv_scan(r, k, w, v, bonus, state, cu_seqlens, seq_slot, y, heads, dim, vdim, out_scale: float = 1.0):
+def wkv_scan(r, k, w, v, bonus, state, cu_seqlens, seq_slot, y, heads, dim, vdim, out_scale: float = 1.0, chunked: bool = False):
     """Linear attention with a decay per key channel over each sequence of the packed step (float32):
     y = S^T r + (sum_d r_d bonus_d k_d) v, then S <- diag(w) S + k v^T, per head.  r, k: [T, heads *
     dim] with equal row strides; w: [T, heads * dim]; v: [T, heads * vdim]; ``bonus`` [heads, dim]; ``state`` [slots + 1,
     heads, recurrent_state_floats(dim, vdim)] (see recurrent_state_matrix); dim up to 256.
     ``bonus`` None: the read-out follows the write, S <- diag(w) S + k v^T; y = S^T r (gated linear
-    attention).  ``out_scale`` multiplies y (a factor on r, which y is linear in)."""
+    attention).  ``out_scale`` multiplies y (a factor on r, which y is linear in).  ``chunked``: in chunks of 16
+    tokens instead of token by token (dim up to 128)."""
     _cuda(r, k, w, v, bonus, state, cu_seqlens, seq_slot, y)
     for t in (r, k, w, v, bonus, state, y):
         assert t is None or t.dtype == torch.float32
@@ -1833,6 +1897,15 @@ def wkv_scan(r, k, w, v, bonus, state, cu_seqlens, seq_slot, y, heads, dim, vdim
     assert ld == ldk and y.is_contiguous() and y.shape[1] == heads * vdim
     assert bonus is None or (bonus.is_contiguous() and bonus.numel() == heads * dim)
     assert state.is_contiguous() and tuple(state.shape[1:]) == (heads, recurrent_state_floats(dim, vdim))
+    if chunked:
+        scratch = _chunk_scratch(y.shape[0], seq_slot.numel(), heads, dim, False, y.device)
+        f = _fn("recurrent_chunk", "gb_chunk_wkv_scan",
+                [c_void_p, c_void_p, c_void_p, c_longlong, c_longlong, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_void_p,
+                 c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p, c_longlong, c_void_p])
+        _check(f(rp, kp, wp, ld, ldw, vp, ldv, _ptr(bonus), state.data_ptr(), cu_seqlens.data_ptr(), seq_slot.data_ptr(),
+                 y.data_ptr(), y.shape[0], seq_slot.numel(), heads, dim, vdim, float(out_scale), scratch.data_ptr(), scratch.numel(),
+                 _stream()), "chunk_wkv_scan", "attention", _nbytes(y) * 5 + 2 * seq_slot.numel() * heads * dim * vdim * 4)
+        return
     f = _fn("recurrent", "gb_wkv_scan_scaled", [c_void_p, c_void_p, c_void_p, c_longlong, c_longlong, c_void_p, c_longlong, c_void_p,
                                                 c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_float,
                                                 c_void_p])

@@ -70,7 +70,7 @@ class ChannelDeltaRule(Part):
         self.a_log, self.dt_bias, self.norm = t["A_log"].contiguous(), t["dt_bias"].contiguous(), t["norm"].contiguous()
 
     def kernel_units(self):
-        return kernels.gemm_units(self.compute) + [("recurrent", ())]
+        return kernels.gemm_units(self.compute) + kernels.recurrent_units(self.compute, self.dim)
 
     def cache_needs(self):
         return [StateNeed((self.taps - 1, self.channels)), StateNeed((self.heads, kernels.recurrent_state_floats(self.dim, self.vdim)))]
@@ -95,7 +95,8 @@ class ChannelDeltaRule(Part):
         gate = kernels.lowrank_map(p[:, g_at:g_at + self.gate_rank], self.g2, None, "plain")
         y = torch.empty((t, hv), dtype=torch.float32, device=p.device)
         kernels.channel_delta_rule(f[:, :qk], f[:, qk:2 * qk], f[:, 2 * qk:], p[:, c:c + nh], decay, state, ctx.cu_seqlens,
-                                   ctx.seq_slot, y, nh, self.kv_heads, self.dim, self.vdim, float(self.dim) ** -0.5)
+                                   ctx.seq_slot, y, nh, self.kv_heads, self.dim, self.vdim, float(self.dim) ** -0.5,
+                                   chunked=kernels.chunk_scan_usable(self.compute, ctx.max_new, self.dim))
         out = torch.empty((t, hv), dtype=self.act_dtype, device=p.device)
         kernels.gated_group_norm(y, gate, self.norm, out, self.vdim, self.eps, False, self.out_scale, gate_act="sigmoid")
         self.o.add_into(out, residual)

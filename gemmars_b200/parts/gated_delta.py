@@ -62,7 +62,7 @@ class GatedDeltaRule(Part):
         self.a_log, self.dt_bias, self.norm = t["A_log"].contiguous(), t["dt_bias"].contiguous(), t["norm"].contiguous()
 
     def kernel_units(self):
-        return kernels.gemm_units(self.compute) + [("recurrent", ())]
+        return kernels.gemm_units(self.compute) + kernels.recurrent_units(self.compute, self.dim)
 
     def cache_needs(self):
         return [StateNeed((self.taps - 1, self.channels)), StateNeed((self.heads, kernels.recurrent_state_floats(self.dim, self.vdim)))]
@@ -83,7 +83,8 @@ class GatedDeltaRule(Part):
         y = torch.empty((t, hv), dtype=torch.float32, device=p.device)
         kernels.delta_rule(f[:, :qk], f[:, qk:2 * qk], f[:, 2 * qk:], p[:, c + hv:c + hv + nh], p[:, c + hv + nh:],
                            self.a_log, self.dt_bias, state, ctx.cu_seqlens, ctx.seq_slot, y, nh, self.kv_heads, self.dim,
-                           self.vdim, float(self.dim) ** -0.5)
+                           self.vdim, float(self.dim) ** -0.5,
+                           chunked=kernels.chunk_scan_usable(self.compute, ctx.max_new, self.dim))
         out = torch.empty((t, hv), dtype=self.act_dtype, device=p.device)
         kernels.gated_group_norm(y, p[:, c:c + hv], self.norm, out, self.vdim, self.eps, False, self.out_scale)
         self.o.add_into(out, residual)

@@ -57,7 +57,7 @@ class GatedLinearAttention(Part):
         self.a2, self.a2_bias, self.norm = t["a2"].contiguous(), t["a2_bias"].contiguous(), t["norm"].contiguous()
 
     def kernel_units(self):
-        return kernels.gemm_units(self.compute) + [("recurrent", ())]
+        return kernels.gemm_units(self.compute) + kernels.recurrent_units(self.compute, self.dim)
 
     def cache_needs(self):
         return [StateNeed((self.heads, kernels.recurrent_state_floats(self.dim, self.vdim)))]
@@ -77,7 +77,8 @@ class GatedLinearAttention(Part):
         alpha = kernels.lowrank_map(p[:, 2 * hd + hv:], self.a2, self.a2_bias, "sigmoid_root", tau=self.tau)
         y = torch.empty((t, hv), dtype=torch.float32, device=p.device)
         kernels.wkv_scan(p[:, :hd], p[:, hd:2 * hd], alpha, p[:, 2 * hd:2 * hd + hv], None, state, ctx.cu_seqlens,
-                         ctx.seq_slot, y, self.heads, self.dim, self.vdim, out_scale=float(self.dim) ** -0.5)
+                         ctx.seq_slot, y, self.heads, self.dim, self.vdim, out_scale=float(self.dim) ** -0.5,
+                         chunked=kernels.chunk_scan_usable(self.compute, ctx.max_new, self.dim))
         gate = self.g(h, out_dtype=torch.float32)
         out = torch.empty((t, hv), dtype=self.act_dtype, device=p.device)
         kernels.gated_group_norm(y, gate, self.norm, out, self.vdim, self.eps, False, self.out_scale)

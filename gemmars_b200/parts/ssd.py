@@ -60,7 +60,7 @@ class StateSpaceDual(Part):
         self.skip, self.norm = t["D"].contiguous(), t["norm"].contiguous()
 
     def kernel_units(self):
-        return kernels.gemm_units(self.compute) + [("recurrent", ())]
+        return kernels.gemm_units(self.compute) + kernels.recurrent_units(self.compute, self.n_state)
 
     def cache_needs(self):
         return [StateNeed((self.taps - 1, self.channels)), StateNeed((self.heads, kernels.recurrent_state_floats(self.n_state, self.vdim)))]
@@ -82,7 +82,8 @@ class StateSpaceDual(Part):
                              ctx.seq_slot, f, act=True)
         y = torch.empty((t, inner), dtype=torch.float32, device=p.device)
         kernels.ssd_scan(f[:, :inner], f[:, inner:inner + gn], f[:, inner + gn:], p[:, inner + c:], self.a_log, self.dt_bias,
-                         self.skip, state, ctx.cu_seqlens, ctx.seq_slot, y, self.heads, self.groups, self.n_state, self.vdim)
+                         self.skip, state, ctx.cu_seqlens, ctx.seq_slot, y, self.heads, self.groups, self.n_state, self.vdim,
+                         chunked=kernels.chunk_scan_usable(self.compute, ctx.max_new, self.n_state))
         out = torch.empty((t, inner), dtype=self.act_dtype, device=p.device)
         kernels.gated_group_norm(y, p[:, :inner], self.norm, out, inner // self.norm_groups, self.eps, True, self.out_scale)
         self.o.add_into(out, residual)

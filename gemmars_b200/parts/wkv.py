@@ -62,7 +62,7 @@ class DecayedLinearAttention(Part):
         self.o = Linear(t["o"])
 
     def kernel_units(self):
-        return kernels.gemm_units(self.compute) + [("recurrent", ())]
+        return kernels.gemm_units(self.compute) + kernels.recurrent_units(self.compute, self.dim)
 
     def cache_needs(self):
         return [StateNeed((self.hidden_size,)),
@@ -81,7 +81,8 @@ class DecayedLinearAttention(Part):
         r, k, v, gate = (m(mixes[i], out_dtype=torch.float32) for i, m in enumerate((self.r, self.k, self.v, self.g)))
         decay = kernels.lowrank_decay(self.w1(mixes[4], out_dtype=torch.float32), self.w2, self.w0)
         y = torch.empty((h.shape[0], self.inner), dtype=torch.float32, device=h.device)
-        kernels.wkv_scan(r, k, decay, v, self.u, state, ctx.cu_seqlens, ctx.seq_slot, y, self.heads, self.dim, self.dim)
+        kernels.wkv_scan(r, k, decay, v, self.u, state, ctx.cu_seqlens, ctx.seq_slot, y, self.heads, self.dim, self.dim,
+                         chunked=kernels.chunk_scan_usable(self.compute, ctx.max_new, self.dim))
         out = torch.empty((h.shape[0], self.inner), dtype=self.act_dtype, device=h.device)
         kernels.gated_group_norm(y, gate, self.norm, out, self.dim, self.eps, False, self.out_scale)
         self.o.add_into(out, residual)

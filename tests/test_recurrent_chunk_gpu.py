@@ -1,0 +1,102 @@
+"""The recurrences of a prompt taken in chunks of 16 tokens against plain sums in 64 bits, token by token, and against the
+kernels that walk token by token: borders of chunks, sequences shorter than one, sizes that fill no tile, decays of zero,
+states carried in and out, and heads taken in turns."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+LENS = [100, 1, 16, 33, 15, 64, 17]
+SLOTS = [3, 1, 6, 0, 7, 2, 5]
+
+
+def _plain(q, k, v, g, new, bonus, S):
+    """(outputs, state) of one head: q, k, g [n, dim], v [n, vdim]; ``new`` [n] the delta rule's beta, or None."""
+    out = []
+    for t in range(q.shape[0]):
+        if bonus is not None:
+            out.append(q[t] @ S + (q[t] * bonus * k[t]).sum() * v[t])
+            S = g[t][:, None] * S + torch.outer(k[t], v[t])
+            continue
+        S = g[t][:, None] * S
+        S = S + torch.outer(k[t], v[t] if new is None else new[t] * (v[t] - k[t] @ S))
+        out.append(q[t] @ S)
+    return torch.stack(out), S
+
+
+@pytest.mark.parametrize("turns", [False, True])
+@pytest.mark.parametrize("heads,groups,dim,vdim", [(4, 2, 128, 128), (2, 1, 64, 64), (3, 3, 12, 33), (6, 2, 100, 20), (40, 20, 128, 40)])
+@pytest.mark.parametrize("form", ["delta", "channel_delta", "ssd", "before", "after"])
+def test_chunks_of_a_prompt(form, heads, groups, dim, vdim, turns, monkeypatch):
+    from gemmars_b200 import kernels as k
+    if turns and heads > 8:
+        pytest.skip("the small sizes show it")
+    if turns:
+        monkeypatch.setattr(k, "CHUNK_SCAN_SCRATCH", 1)         # one head at a time
+    gen = torch.Generator().manual_seed(heads * 1000 + dim + vdim)
+    ntok, gh = sum(LENS), groups if form in ("delta", "channel_delta", "ssd") else heads
+    rand = lambda *s: torch.randn(s, generator=gen)      # noqa: E731
+    x = rand(ntok, 2 * gh * dim + heads * vdim + 4)
+    gates = rand(ntok, 2 * heads + 1) * 2
+    a_log, dt_bias, skip, bonus = rand(heads) * 0.5, rand(heads) * 0.5, rand(heads), rand(heads, dim)
+    decay = torch.exp(-torch.exp(rand(ntok, heads * dim) * 2 - 2))
+    decay[5, :] = 0.0
+    decay[40, ::2] = 0.0
+    start = rand(len(LENS), heads, dim, vdim)
+    lanes = 1 if dim <= 32 else 2 if dim <= 64 else 4
+    full = torch.zeros(len(LENS), heads, 32 * lanes, vdim)
+    full[:, :, :dim] = start
+    stored = full.view(-1, heads, lanes, 8, 4, vdim).permute(0, 1, 3, 5, 2, 4).reshape(len(LENS), heads, -1)
+    state = torch.zeros(9, heads, k.recurrent_state_floats(dim, vdim))
+    for i, s in enumerate(SLOTS):
+        state[s] = stored[i]
+    q, kk, v = (t.double() for t in (x[:, :gh * dim], x[:, gh * dim:2 * gh * dim], x[:, 2 * gh * dim:2 * gh * dim + heads * vdim]))
+    q, kk, v = q.view(ntok, gh, dim), kk.view(ntok, gh, dim), v.view(ntok, heads, vdim)
+    z, rate, new = gates.double(), torch.exp(a_log.double()), None
+    soft = torch.nn.functional.softplus
+    if form in ("delta", "channel_delta"):
+        q, kk = (t / torch.sqrt(t.square().sum(-1, keepdim=True) + 1e-6) for t in (q, kk))
+        q, new = q * dim ** -0.5, torch.sigmoid(z[:, :heads])
+    g = decay.double().view(ntok, heads, dim)
+    if form == "delta":
+        g = torch.exp(-rate * soft(z[:, heads:2 * heads] + dt_bias.double()))[..., None].expand(ntok, heads, dim)
+    if form == "ssd":
+        dt = soft(z[:, :heads] + dt_bias.double())
+        g, new = torch.exp(-rate * dt)[..., None].expand(ntok, heads, dim), None
+    rep = heads // gh
+    want, final, at = torch.zeros(ntok, heads, vdim, dtype=torch.float64), torch.zeros(len(LENS), heads, dim, vdim, dtype=torch.float64), 0
+    for i, n in enumerate(LENS):
+        for h in range(heads):
+            r = slice(at, at + n)
+            kh = kk[r, h // rep] * (dt[r, h, None] if form == "ssd" else 1.0)
+            o, final[i, h] = _plain(q[r, h // rep], kh, v[r, h], g[r, h], None if new is None else new[r, h],
+                                    bonus[h].double() if form == "before" else None, start[i, h].double())
+            want[r, h] = o + (skip[h].double() * v[r, h] if form == "ssd" else 0.0)
+        at += n
+    dev = lambda t: t.to(DEV)      # noqa: E731
+    xd, gd, cu = dev(x), dev(gates), dev(torch.tensor([0] + LENS).cumsum(0).int())
+    slots, dd = dev(torch.tensor(SLOTS, dtype=torch.int32)), dev(decay)
+    a, b, c = xd[:, :gh * dim], xd[:, gh * dim:2 * gh * dim], xd[:, 2 * gh * dim:2 * gh * dim + heads * vdim]
+
+    def run(chunked):
+        st, y = dev(state).clone(), torch.empty(ntok, heads * vdim, device=DEV)
+        if form == "delta":
+            k.delta_rule(a, b, c, gd[:, :heads], gd[:, heads:2 * heads], dev(a_log), dev(dt_bias), st, cu, slots, y, heads, groups, dim,
+                         vdim, dim ** -0.5, chunked=chunked)
+        elif form == "channel_delta":
+            k.channel_delta_rule(a, b, c, gd[:, :heads], dd, st, cu, slots, y, heads, groups, dim, vdim, dim ** -0.5, chunked=chunked)
+        elif form == "ssd":
+            k.ssd_scan(c, b, a, gd[:, :heads], dev(a_log), dev(dt_bias), dev(skip), st, cu, slots, y, heads, groups, dim, vdim,
+                       chunked=chunked)
+        else:
+            k.wkv_scan(a, b, dd, c, dev(bonus) if form == "before" else None, st, cu, slots, y, heads, dim, vdim, 0.5, chunked=chunked)
+        held = st[slots.long()].cpu().view(len(LENS), heads, 8, vdim, lanes, 4).permute(0, 1, 4, 2, 5, 3).reshape(len(LENS), heads, -1, vdim)
+        assert not st[4].any() and not st[8].any()          # slots of no sequence of the step
+        assert not held[:, :, dim:].any()
+        scale = 0.5 if form in ("before", "after") else 1.0
+        off = lambda u, w: ((u.double() - w).norm() / w.norm()).item()      # noqa: E731
+        return off(y.cpu().view(ntok, heads, vdim), want * scale), off(held[:, :, :dim], final)
+
+    (y_err, s_err), (y_walk, s_walk) = run(True), run(False)
+    # a few roundings of 2^-24 an element, and what the split products leave out (2^-22 of a product)
+    assert y_err < 1.5e-6 and s_err < 1.5e-6, (y_err, s_err, y_walk, s_walk)
