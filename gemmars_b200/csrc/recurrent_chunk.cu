@@ -19,9 +19,10 @@
 // index may be taken in any order, and lane t's two neighbouring columns of an accumulator stand for inner
 // indexes t and t + 4).
 //
-// Numbers: everything is float32.  A product's operands are split into two tf32 halves, hi + lo (hi rounded to
-// nearest, so lo is at most 2^-12 of the number), and hi hi + hi lo + lo hi is summed in float32: what is left out
-// is 2^-22 of a product, as much as float32 rounding itself.  The state's own sum, S <- G S + (chunk's part), is a
+// Numbers: everything is float32.  A product's operands are split into two tf32 halves, hi + lo, and hi hi + hi lo +
+// lo hi is summed in float32.  The left operand's hi is rounded to nearest (lo at most 2^-12 of the number, of either
+// sign), the right one's is what the instruction reads of it (the upper 11 bits: lo at most 2^-10); what is left out,
+// lo lo, is at most 2^-22 of a product and has no sign of its own.  The state's own sum, S <- G S + (chunk's part), is a
 // float32 fused multiply-add outside the tensor cores.  A value that is not finite reaches the outputs of its whole
 // chunk (zero times infinity), not only of the tokens from its own on.
 #include "common.cuh"
@@ -54,11 +55,9 @@ __device__ __forceinline__ void mma(float (&d)[4], const uint32_t (&a)[4], uint3
 }
 // d += a b in three parts: hi hi into d, the two cross parts into x.
 __device__ __forceinline__ void mma3(float (&d)[4], float (&x)[4], const uint32_t (&ahi)[4], const uint32_t (&alo)[4], float b0, float b1) {
-  uint32_t h0, l0, h1, l1;
-  split(b0, h0, l0);
-  split(b1, h1, l1);
+  const uint32_t h0 = __float_as_uint(b0), h1 = __float_as_uint(b1);
   mma(d, ahi, h0, h1);
-  mma(x, ahi, l0, l1);
+  mma(x, ahi, __float_as_uint(b0 - __uint_as_float(h0 & 0xffffe000u)), __float_as_uint(b1 - __uint_as_float(h1 & 0xffffe000u)));
   mma(x, alo, h0, h1);
 }
 
@@ -78,16 +77,17 @@ struct Prepare {
   int nseq, H, G, D, head0;
   float qscale;
   float* blocks;
-  int slots;
+  int slots, wide;
 };
 
 template <int DP, int MODE>
-__global__ void __launch_bounds__(128) chunk_prepare_kernel(const Prepare a) {
+__global__ void __launch_bounds__(128, DP == 64 ? 8 : 6) chunk_prepare_kernel(const Prepare a) {
   constexpr bool HAS_W = is_delta(MODE), CH = per_channel(MODE);
   using B = Block<DP, HAS_W>;
   constexpr int LD = DP + 4;
-  __shared__ float ks[CT][LD], qs[CT][LD], extra[HAS_W || CH ? CT : 1][LD];    // extra: the decays, then W
-  __shared__ float kk[CT][CT + 1], qk[CT][CT + 1], tb[HAS_W ? CT : 1][CT + 1];
+  __shared__ __align__(16) float ks[CT][LD], qs[CT][LD], extra[HAS_W || CH ? CT : 1][LD];    // extra: the decays, then W
+  __shared__ __align__(16) float at[CT][CT + 4];        // A transposed: what row i takes of w_j, at [j][i]
+  __shared__ float qk[CT][CT + 1], tb[HAS_W ? CT : 1][CT + 1];
   __shared__ float gate[CT], beta[CT];
   pdl_release_next();
   pdl_wait_prior();
@@ -97,13 +97,30 @@ __global__ void __launch_bounds__(128) chunk_prepare_kernel(const Prepare a) {
     if (b + step < a.nseq && a.cu[b + step] / CT + b + step <= slot) b += step;
   const int first = a.cu[b] + (slot - (a.cu[b] / CT + b)) * CT, n = min(CT, a.cu[b + 1] - first);
   if (n <= 0) return;
-  for (int e = tid; e < CT * DP; e += 128) {
-    const int i = e / DP, d = e % DP;
-    const bool in = i < n && d < D;
-    ks[i][d] = in ? a.k[(size_t)(first + i) * a.ldqk + (size_t)g * D + d] : 0.f;
-    qs[i][d] = in ? a.q[(size_t)(first + i) * a.ldqk + (size_t)g * D + d] : 0.f;
-    if (CH) extra[i][d] = in ? a.decay[(size_t)(first + i) * a.ldd + (size_t)head * D + d] : 1.f;
-  }
+  auto load = [&](const float* base, long long ld, float (*to)[LD], float beyond) {
+    if (a.wide) {                       // D fills the block's columns and rows start at 16-byte boundaries
+      float4 v[DP * CT / 512];
+#pragma unroll
+      for (int u = 0; u < DP * CT / 512; ++u) {
+        const int e = tid + 128 * u, i = e / (DP / 4), d = e % (DP / 4) * 4;
+        v[u] = i < n ? *(const float4*)(base + (size_t)(first + i) * ld + d) : make_float4(beyond, beyond, beyond, beyond);
+      }
+#pragma unroll
+      for (int u = 0; u < DP * CT / 512; ++u) {
+        const int e = tid + 128 * u;
+        *(float4*)&to[e / (DP / 4)][e % (DP / 4) * 4] = v[u];
+      }
+      return;
+    }
+#pragma unroll 8
+    for (int e = tid; e < CT * DP; e += 128) {
+      const int i = e / DP, d = e % DP;
+      to[i][d] = i < n && d < D ? base[(size_t)(first + i) * ld + d] : beyond;
+    }
+  };
+  load(a.k + (size_t)g * D, a.ldqk, ks, 0.f);
+  load(a.q + (size_t)g * D, a.ldqk, qs, 0.f);
+  if (CH) load(a.decay + (size_t)head * D, a.ldd, extra, 1.f);
   if (tid < CT) {          // tokens beyond the end write nothing and keep everything
     float bt = 0.f, gt = 1.f;
     if (tid < n) {
@@ -137,7 +154,7 @@ __global__ void __launch_bounds__(128) chunk_prepare_kernel(const Prepare a) {
     if (which == 0 || HAS_W) {
       const float(*rows)[LD] = which ? ks : qs;
       float d[4] = {}, x[4] = {};
-#pragma unroll
+#pragma unroll 4
       for (int s = 0; s < DP / 8; ++s) {
         uint32_t hi[4], lo[4];
         split(rows[gr][8 * s + t], hi[0], lo[0]);
@@ -146,11 +163,12 @@ __global__ void __launch_bounds__(128) chunk_prepare_kernel(const Prepare a) {
         split(rows[gr + 8][8 * s + t + 4], hi[3], lo[3]);
         mma3(d, x, hi, lo, ks[8 * nt + gr][8 * s + t], ks[8 * nt + gr][8 * s + t + 4]);
       }
-      float(*out)[CT + 1] = which ? kk : qk;
-      out[gr][8 * nt + 2 * t] = d[0] + x[0];
-      out[gr][8 * nt + 2 * t + 1] = d[1] + x[1];
-      out[gr + 8][8 * nt + 2 * t] = d[2] + x[2];
-      out[gr + 8][8 * nt + 2 * t + 1] = d[3] + x[3];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int i = gr + 8 * (e >> 1), j = 8 * nt + 2 * t + (e & 1);
+        if (which) at[j][i] = d[e] + x[e];
+        else qk[i][j] = d[e] + x[e];
+      }
     }
     __syncthreads();
     const int j = tid >> 3, i0 = (tid & 7) * 2;       // two neighbouring rows of a column
@@ -165,50 +183,78 @@ __global__ void __launch_bounds__(128) chunk_prepare_kernel(const Prepare a) {
       float p = i >= j ? qk[i][j] * r : 0.f;
       if (MODE == STATE_SPACE) p = p * beta[j] + (i == j ? a.skip[head] : 0.f);
       qk[i][j] = p;
-      if (HAS_W) kk[i][j] = i > j ? beta[i] * (kk[i][j] * r) : 0.f;
+      if (HAS_W) at[j][i] = i > j ? beta[i] * (at[j][i] * r) : 0.f;
     }
   } else {
-    // a decay per channel stands inside the sums: 16 lanes take a column's sums, DP / 16 channels each, and carry
-    // k_j times the decays since j from row to row; columns j and 15 - j together have 17 rows
-    const int pair = tid >> 4, part = tid & 15;
-    const unsigned mine = 0xffffu << (lane & 16);       // the halves of a warp walk columns of unequal length
+    // a decay per channel stands inside the sums: eight lanes take a column j's sums, DP / 8 channels each, and carry
+    // k_j times the decays since j from row to row; a warp's four columns walk the rows together
+    constexpr int E = DP / 8;
+    const int j = tid >> 3, part = (tid & 7) * 4;      // four channels of every 32: eight lanes' 16 bytes side by side
+    auto dim = [&](int e) { return part + (e & 3) + 8 * (e & ~3); };
+    float kr[E];
+#pragma unroll
+    for (int e = 0; e < E; ++e) kr[e] = ks[j][dim(e)];
+    if (MODE == READ_BEFORE) {            // a token's own write, which it reads through the bonus
+      float s = 0.f;
+#pragma unroll
+      for (int e = 0; e < E; ++e)
+        if (dim(e) < D) s = fmaf(qs[j][dim(e)] * a.bonus[(size_t)head * D + dim(e)], kr[e], s);
+#pragma unroll
+      for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      if ((tid & 7) == 0) qk[j][j] = s;
+    }
 #pragma unroll 1
-    for (int half = 0; half < 2; ++half) {
-      const int j = half ? CT - 1 - pair : pair;
-      float kr[DP / 16];
+    for (int i = warp * 4; i < CT; ++i) {
+      float sq = 0.f, sk = 0.f;
 #pragma unroll
-      for (int e = 0; e < DP / 16; ++e) kr[e] = ks[j][part + 16 * e];
-      for (int i = j; i < CT; ++i) {
-        float sq = 0.f, sk = 0.f;
+      for (int e = 0; e < E; e += 4) {
+        const float4 q4 = *(const float4*)&qs[i][dim(e)], g4 = *(const float4*)&extra[i][dim(e)];
+        const float qv[4] = {q4.x, q4.y, q4.z, q4.w}, gv[4] = {g4.x, g4.y, g4.z, g4.w};
+        float4 k4;
+        if (HAS_W) k4 = *(const float4*)&ks[i][dim(e)];
+        const float kv[4] = {HAS_W ? k4.x : 0.f, HAS_W ? k4.y : 0.f, HAS_W ? k4.z : 0.f, HAS_W ? k4.w : 0.f};
 #pragma unroll
-        for (int e = 0; e < DP / 16; ++e) {
-          const int d = part + 16 * e;
-          if (MODE == READ_BEFORE) {                  // token i reads before its own decay and write
-            sq = fmaf(qs[i][d], i == j ? (d < D ? a.bonus[(size_t)head * D + d] : 0.f) * kr[e] : kr[e], sq);
-            if (i > j) kr[e] *= extra[i][d];
-          } else {
-            if (i > j) kr[e] *= extra[i][d];
-            sq = fmaf(qs[i][d], kr[e], sq);
-            if (HAS_W) sk = fmaf(ks[i][d], kr[e], sk);
-          }
-        }
-#pragma unroll
-        for (int o = 8; o > 0; o >>= 1) {
-          sq += __shfl_xor_sync(mine, sq, o, 16);
-          if (HAS_W) sk += __shfl_xor_sync(mine, sk, o, 16);
-        }
-        if (part == 0) {
-          qk[i][j] = sq;
-          if (HAS_W) kk[i][j] = i > j ? beta[i] * sk : 0.f;
+        for (int u = 0; u < 4; ++u) {
+          if (MODE == READ_BEFORE) sq = fmaf(qv[u], kr[e + u], sq);     // token i reads before its own decay
+          if (i > j) kr[e + u] *= gv[u];
+          if (MODE != READ_BEFORE) sq = fmaf(qv[u], kr[e + u], sq);
+          if (HAS_W) sk = fmaf(kv[u], kr[e + u], sk);
         }
       }
-      if (part < j) qk[part][j] = 0.f;
+#pragma unroll
+      for (int o = 4; o > 0; o >>= 1) {
+        sq += __shfl_xor_sync(0xffffffffu, sq, o);
+        if (HAS_W) sk += __shfl_xor_sync(0xffffffffu, sk, o);
+      }
+      if ((tid & 7) == 0) {
+        if (MODE != READ_BEFORE || i != j) qk[i][j] = i >= j ? sq : 0.f;
+        if (HAS_W) at[j][i] = i > j ? beta[i] * sk : 0.f;
+      }
+    }
+    for (int i = tid & 7; i < warp * 4; i += 8) {        // the rows that no column of this warp reaches
+      qk[i][j] = 0.f;
+      if (HAS_W) at[j][i] = 0.f;
     }
   }
   __syncthreads();
   // a thread a channel: Q~, Kd and G, and W by forward substitution; then T's columns in the same way
+  auto solve = [&](float (&w)[CT]) {        // w <- (1 + A)^-1 w, a column at a time
+#pragma unroll
+    for (int j = 0; j < CT - 1; ++j) {
+      asm volatile("" ::: "memory");        // A is read a column at a time: all of it at once would not fit the registers
+#pragma unroll
+      for (int i4 = (j + 1) / 4 * 4; i4 < CT; i4 += 4) {
+        const float4 c = *(const float4*)&at[j][i4];
+        if (i4 > j) w[i4] = fmaf(-c.x, w[j], w[i4]);
+        if (i4 + 1 > j) w[i4 + 1] = fmaf(-c.y, w[j], w[i4 + 1]);
+        if (i4 + 2 > j) w[i4 + 2] = fmaf(-c.z, w[j], w[i4 + 2]);
+        if (i4 + 3 > j) w[i4 + 3] = fmaf(-c.w, w[j], w[i4 + 3]);
+      }
+    }
+  };
+  constexpr bool APART = !HAS_W && DP == 64;       // Kd by the other 64 threads
   if (tid < DP) {
-    float c = 1.f, w[HAS_W ? CT : 1];
+    float c = 1.f, w[CT];
 #pragma unroll
     for (int i = 0; i < CT; ++i) {
       const float gi = CH ? extra[i][tid] : gate[i];
@@ -219,36 +265,45 @@ __global__ void __launch_bounds__(128) chunk_prepare_kernel(const Prepare a) {
         c *= gi;
         qs[i][tid] *= c;
       }
-      if (HAS_W) {
-        float v = beta[i] * (c * ks[i][tid]);
-#pragma unroll
-        for (int j = 0; j < i; ++j) v = fmaf(-kk[i][j], w[j], v);
-        w[HAS_W ? i : 0] = v;
-      }
+      if (HAS_W) w[i] = beta[i] * (c * ks[i][tid]);
     }
     a.blocks[((size_t)blockIdx.y * a.slots + slot) * B::FLOATS + B::G + tid] = c;
+    if (HAS_W) {
+      solve(w);
+#pragma unroll
+      for (int i = 0; i < CT; ++i)
+        if (!CH) extra[i][tid] = w[i];
+    }
+    if (HAS_W || !APART) {
+      float r = 1.f;
+#pragma unroll
+      for (int i = CT - 1; i >= 0; --i) {
+        const float gi = CH ? extra[i][tid] : gate[i];
+        ks[i][tid] *= MODE == STATE_SPACE ? r * beta[i] : r;
+        r *= gi;
+      }
+    }
+    if (HAS_W && CH) {
+#pragma unroll
+      for (int i = 0; i < CT; ++i) extra[i][tid] = w[i];
+    }
+  } else if (APART) {
     float r = 1.f;
 #pragma unroll
     for (int i = CT - 1; i >= 0; --i) {
-      const float gi = CH ? extra[i][tid] : gate[i];
-      ks[i][tid] *= MODE == STATE_SPACE ? r * beta[i] : r;
+      const float gi = CH ? extra[i][tid - 64] : gate[i];
+      ks[i][tid - 64] *= MODE == STATE_SPACE ? r * beta[i] : r;
       r *= gi;
-    }
-    if (HAS_W) {
-#pragma unroll
-      for (int i = 0; i < CT; ++i) extra[i][tid] = w[HAS_W ? i : 0];
     }
   }
   if (HAS_W && tid >= 128 - CT) {
     const int c = tid - (128 - CT);
     float t[CT];
 #pragma unroll
-    for (int i = 0; i < CT; ++i) {
-      float v = i == c ? beta[i] : 0.f;
+    for (int i = 0; i < CT; ++i) t[i] = i == c ? beta[i] : 0.f;
+    solve(t);
 #pragma unroll
-      for (int j = 0; j < i; ++j) v = fmaf(-kk[i][j], t[j], v);
-      tb[HAS_W ? i : 0][c] = t[i] = v;
-    }
+    for (int i = 0; i < CT; ++i) tb[HAS_W ? i : 0][c] = t[i];
   }
   __syncthreads();
   float4* out = (float4*)(a.blocks + ((size_t)blockIdx.y * a.slots + slot) * B::FLOATS);
@@ -277,46 +332,68 @@ struct Scan {
   float* y;                             // [ntok, H * V]
   int H, head0, V, lanes;               // lanes: 32 channels of a column each, as the state lies in memory
   float yscale;
+  int wide;
 };
 
 // NV groups of 16 columns a CTA; a group's channels are shared by DS warps (their parts of U and Y meet in shared
-// memory, added in one order).  Blocks of coming chunks arrive by asynchronous copies, STAGES - 1 ahead.
+// memory, added in one order).  One more warp brings the blocks of coming chunks by asynchronous copies, STAGES - 1
+// ahead.
 template <int DP, int DS, int NV, bool HAS_W, int STAGES>
-__global__ void __launch_bounds__(32 * DS * NV) chunk_scan_kernel(const Scan a) {
+__global__ void __launch_bounds__(32 * DS * NV + 32) chunk_scan_kernel(const Scan a) {
   using B = Block<DP, HAS_W>;
-  constexpr int NT = 32 * DS * NV, DW = DP / DS, NJ = DW / 8;
+  constexpr int DW = DP / DS, NJ = DW / 8;
+  constexpr int LV = 16 * NV + 4, STAGE = B::FLOATS + CT * LV;      // a chunk's block, then its rows of V
   extern __shared__ __align__(16) float smem[];
-  float* exch = smem + STAGES * B::FLOATS;             // [2][warps][12][32], with DS 2
+  float* exch = smem + STAGES * STAGE;             // [2][warps][16][32], with DS over 1
   pdl_wait_prior();
   const int b = blockIdx.x, head = a.head0 + blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int gr = lane >> 2, t = lane & 3, part = warp % DS, V = a.V;
   const int col0 = (blockIdx.z * NV + warp / DS) * 16, d0 = part * DW;
   const int t0 = a.cu[b], t1 = a.cu[b + 1], chunks = (t1 - t0 + CT - 1) / CT;
   const float* blocks = a.blocks + ((size_t)blockIdx.y * a.slots + t0 / CT + b) * B::FLOATS;
-  auto bring = [&](int c) {
-    if (c < chunks) {
-      const float* src = blocks + (size_t)c * B::FLOATS;
-      const uint32_t dst = (uint32_t)__cvta_generic_to_shared(smem + (c % STAGES) * B::FLOATS);
-      for (int e = tid; e < B::FLOATS / 4; e += NT)
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16 * e), "l"(src + 4 * e) : "memory");
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  };
-#pragma unroll
-  for (int c = 0; c < STAGES - 1; ++c) bring(c);
-  const bool in0 = col0 + gr < V, in1 = col0 + gr + 8 < V;
-  const float* vcol = a.v + (size_t)head * V + col0 + gr;
-  float vn[2][4];
-  auto fetch_v = [&](int c) {          // V transposed as a left operand: columns gr, gr + 8; tokens 2 t, 2 t + 1 of each half
-#pragma unroll
-    for (int h = 0; h < 2; ++h)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int tok = t0 + c * CT + 8 * h + 2 * t + (e >> 1);
-        vn[h][e] = tok < t1 && ((e & 1) ? in1 : in0) ? vcol[(size_t)tok * a.ldv + 8 * (e & 1)] : 0.f;
+  const int vcol0 = blockIdx.z * NV * 16;
+  const float* vbase = a.v + (size_t)t0 * a.ldv + (size_t)head * V + vcol0;
+  if (warp == DS * NV) {
+    auto bring = [&](int c) {
+      if (c < chunks) {
+        const float* src = blocks + (size_t)c * B::FLOATS + 4 * lane;
+        const uint32_t dst = (uint32_t)__cvta_generic_to_shared(smem + (c % STAGES) * STAGE);
+#pragma unroll 8
+        for (int e = lane; e < B::FLOATS / 4; e += 32)
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16 * e), "l"(src + 4 * (e - lane)) : "memory");
+        if (a.wide) {                     // rows of V at 16-byte boundaries, whole groups of 16 columns; zeros beyond the end
+          for (int e = lane; e < CT * NV * 4; e += 32) {
+            const int i = e / (NV * 4), col = e % (NV * 4) * 4, in = c * CT + i < t1 - t0 && vcol0 + col < V;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + 4 * (B::FLOATS + i * LV + col)),
+                         "l"(in ? vbase + (size_t)(c * CT + i) * a.ldv + col : a.v), "r"(in ? 16 : 0)
+                         : "memory");
+          }
+        } else {
+          for (int e = lane; e < CT * NV * 16; e += 32) {
+            const int i = e / (NV * 16), col = e % (NV * 16), in = c * CT + i < t1 - t0 && vcol0 + col < V;
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst + 4 * (B::FLOATS + i * LV + col)),
+                         "l"(in ? vbase + (size_t)(c * CT + i) * a.ldv + col : a.v), "r"(in ? 4 : 0)
+                         : "memory");
+          }
+        }
       }
-  };
-  if (chunks > 0) fetch_v(0);
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+#pragma unroll
+    for (int c = 0; c < STAGES - 1; ++c) bring(c);
+    asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
+    asm volatile("bar.sync 0;" ::: "memory");             // block 0 is there
+#pragma unroll 1
+    for (int c = 0; c < chunks; ++c) {
+      asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 3) : "memory");
+      asm volatile("bar.sync 0;" ::: "memory");           // block c + 1 is there; all have left block c - 1
+      bring(c + STAGES - 1);
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    pdl_release_next();
+    return;
+  }
+  const bool in0 = col0 + gr < V, in1 = col0 + gr + 8 < V;
   float* st = a.state + ((size_t)a.seq_slot[b] * a.H + head) * 32 * V * a.lanes;
   auto place = [&](int j, int col) {   // of channels d0 + 8 j + 2 t and the next
     const int d = d0 + 8 * j + 2 * t;
@@ -330,17 +407,18 @@ __global__ void __launch_bounds__(32 * DS * NV) chunk_scan_kernel(const Scan a) 
     const float2 z = in && in1 ? *(const float2*)(st + place(j, col0 + gr + 8)) : make_float2(0.f, 0.f);
     S[j][0] = x.x; S[j][1] = x.y; S[j][2] = z.x; S[j][3] = z.y;
   }
-  asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
-  __syncthreads();
+  float* yrow = a.y + ((size_t)t0 * a.H + head) * V + col0 + gr;
+  asm volatile("bar.sync 0;" ::: "memory");
 #pragma unroll 1
-  for (int c = 0; c < chunks; ++c) {
-    const float4* blk = (const float4*)(smem + (c % STAGES) * B::FLOATS);
+  for (int c = 0; c < chunks; ++c, yrow += (size_t)CT * a.H * V) {
+    const float4* blk = (const float4*)(smem + (c % STAGES) * STAGE);
+    const float* vs = (const float*)blk + B::FLOATS + 2 * t * LV + warp / DS * 16 + gr;
     uint32_t vhi[2][4], vlo[2][4];
 #pragma unroll
     for (int h = 0; h < 2; ++h)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) split(vn[h][e], vhi[h][e], vlo[h][e]);
-    if (c + 1 < chunks) fetch_v(c + 1);
+      for (int e = 0; e < 4; ++e)        // a left operand: columns gr, gr + 8 of tokens 2 t, 2 t + 1 of each half
+        split(vs[(8 * h + (e >> 1)) * LV + 8 * (e & 1)], vhi[h][e], vlo[h][e]);
     // W S and Q~ S over this warp's channels, transposed: 16 columns by 16 tokens
     float y[2][4] = {}, yx[2][4] = {}, u[2][4] = {}, ux[2][4] = {};
 #pragma unroll
@@ -374,9 +452,11 @@ __global__ void __launch_bounds__(32 * DS * NV) chunk_scan_kernel(const Scan a) 
         y[nt][e] += yx[nt][e];
         if (HAS_W) u[nt][e] = -(u[nt][e] + ux[nt][e]);
       }
-    if (HAS_W && part == 0) {           // + T V
+    // + T V: the last warp's work, or the last two's, a half of the tokens each
+    if (HAS_W && part >= DS - (DS == 4 ? 2 : 1)) {
 #pragma unroll
       for (int nt = 0; nt < 2; ++nt) {
+        if (DS == 4 && nt != (part & 1)) continue;
         const float4 tf = blk[B::T / 4 + 32 * nt + lane];
         float d[4] = {}, x[4] = {};
         mma3(d, x, vhi[0], vlo[0], tf.x, tf.y);
@@ -385,23 +465,28 @@ __global__ void __launch_bounds__(32 * DS * NV) chunk_scan_kernel(const Scan a) 
         for (int e = 0; e < 4; ++e) u[nt][e] += d[e] + x[e];
       }
     }
-    if (DS == 2) {
-      float* mine = exch + ((c & 1) * DS * NV + warp) * 384 + lane;
+    if (DS > 1) {
+      float* mine = exch + ((c & 1) * DS * NV + warp) * 512 + lane;
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         if (HAS_W) mine[32 * e] = u[0][e], mine[32 * (4 + e)] = u[1][e];
-        mine[32 * (8 + e)] = part ? y[0][e] : y[1][e];         // the half of the tokens that the other warp finishes
+        mine[32 * (8 + e)] = y[0][e];
+        mine[32 * (12 + e)] = y[1][e];
       }
     }
-    asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2 > 0 ? STAGES - 3 : 0) : "memory");
-    __syncthreads();                    // block c + 1 is there; all have left block c - 1
-    bring(c + STAGES - 1);
-    if (DS == 2) {
-      const float* other = exch + ((c & 1) * DS * NV + (warp ^ 1)) * 384 + lane;
+    asm volatile("bar.sync 0;" ::: "memory");     // the warps' parts are there, and block c + 1; block c - 1 may go
+    const bool finishes = DS == 1 || part < 2;     // warp 0 the first half of the tokens, warp 1 the second
+    if (DS > 1) {                                  // the warps' parts, in their order
+      const float* group = exch + ((c & 1) * DS * NV + warp - part) * 512 + lane;
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        if (HAS_W) u[0][e] += other[32 * e], u[1][e] += other[32 * (4 + e)];
-        y[0][e] = (part ? y[1][e] : y[0][e]) + other[32 * (8 + e)];
+        if (HAS_W) u[0][e] = group[32 * e], u[1][e] = group[32 * (4 + e)];
+        if (finishes) y[0][e] = group[32 * (8 + 4 * part + e)];
+#pragma unroll
+        for (int o = 1; o < DS; ++o) {
+          if (HAS_W) u[0][e] += group[512 * o + 32 * e], u[1][e] += group[512 * o + 32 * (4 + e)];
+          if (finishes) y[0][e] += group[512 * o + 32 * (8 + 4 * part + e)];
+        }
       }
     }
     uint32_t uhi[2][4], ulo[2][4];
@@ -433,19 +518,19 @@ __global__ void __launch_bounds__(32 * DS * NV) chunk_scan_kernel(const Scan a) 
     }
     // Y = Q~ S + P U, of the tokens that this warp finishes
 #pragma unroll
-    for (int i = 0; i < 2 / DS; ++i) {
-      const int nt = DS == 2 ? part : i;
+    for (int i = 0; i < (DS == 1 ? 2 : 1); ++i) {
+      if (!finishes) break;
+      const int nt = DS == 1 ? i : part;
       const float4 pf = blk[B::P / 4 + 32 * nt + lane];
       float d[4] = {}, x[4] = {};
       mma3(d, x, uhi[0], ulo[0], pf.x, pf.y);
       mma3(d, x, uhi[1], ulo[1], pf.z, pf.w);
-      const int tok = t0 + c * CT + 8 * nt + 2 * t;
+      const int row = 8 * nt + 2 * t, rows = t1 - t0 - c * CT;
+      float* to = yrow + (size_t)row * a.H * V;
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int to = tok + (e & 1);
-        if (to < t1 && (e < 2 ? in0 : in1))
-          a.y[(size_t)to * a.H * V + (size_t)head * V + col0 + gr + 8 * (e >> 1)] = (y[i][e] + (d[e] + x[e])) * a.yscale;
-      }
+      for (int e = 0; e < 4; ++e)
+        if (row + (e & 1) < rows && (e < 2 ? in0 : in1))
+          to[(size_t)(e & 1) * a.H * V + 8 * (e >> 1)] = (y[i][e] + (d[e] + x[e])) * a.yscale;
     }
   }
   pdl_release_next();
@@ -457,10 +542,10 @@ __global__ void __launch_bounds__(32 * DS * NV) chunk_scan_kernel(const Scan a) 
   }
 }
 
-template <int DP, int DS, int NV, bool HAS_W>
+template <int DP, int DS, int NV, bool HAS_W, int STAGES>
 static void launch_scan(const Scan& s, int nseq, int heads, cudaStream_t stream) {
-  constexpr int STAGES = 3;
-  constexpr size_t smem = (STAGES * Block<DP, HAS_W>::FLOATS + (DS == 2 ? 2 * DS * NV * 384 : 0)) * sizeof(float);
+  static_assert(STAGES >= 3, "a chunk's block is asked for before the one ahead of it is read");
+  constexpr size_t smem = (STAGES * (Block<DP, HAS_W>::FLOATS + CT * (16 * NV + 4)) + (DS > 1 ? 2 * DS * NV * 512 : 0)) * sizeof(float);
   auto kernel = chunk_scan_kernel<DP, DS, NV, HAS_W, STAGES>;
   cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   const dim3 grid(nseq, heads, (s.V + 16 * NV - 1) / (16 * NV));
@@ -468,7 +553,7 @@ static void launch_scan(const Scan& s, int nseq, int heads, cudaStream_t stream)
   // an SM (see launch_scan in recurrent.cu)
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
-  cfg.blockDim = 32 * DS * NV;
+  cfg.blockDim = 32 * DS * NV + 32;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
   cudaLaunchKernelEx(&cfg, kernel, s);
@@ -478,19 +563,27 @@ template <int DP, int MODE>
 static int run(Prepare p, Scan s, int ntok, int heads_at_once, cudaStream_t stream) {
   constexpr bool HAS_W = is_delta(MODE);
   p.slots = s.slots = chunk_slots(ntok, p.nseq);
+  const bool ch = per_channel(MODE);
+  p.wide = p.D == DP && p.ldqk % 4 == 0 && (!ch || p.ldd % 4 == 0) &&
+           !(((uintptr_t)p.q | (uintptr_t)p.k | (ch ? (uintptr_t)p.decay : 0)) & 15);
+  s.wide = s.V % 4 == 0 && s.ldv % 4 == 0 && ((uintptr_t)s.v & 15) == 0;
   for (int h = 0; h < p.H; h += heads_at_once) {
     const int heads = p.H - h < heads_at_once ? p.H - h : heads_at_once;
     p.head0 = s.head0 = h;
     gb_launch(chunk_prepare_kernel<DP, MODE>, dim3(p.slots, heads), 128, 0, stream, p);
+    // us for a delta rule at heads of 128 x 128, preparation and all, by (DS, NV): 64 groups of 16 columns, 1,218 tokens:
+    // (4, 1) 93, (2, 2) 121, (1, 4) 206; 256 groups, 2,048 tokens: 267, 236, 379; 2,048 groups of 512: 522, 491, 421.
+    // Few groups leave the chain to itself and want it short (more warps a group); many fill the SMs either way and
+    // want the least that a group costs.
     const long long groups = (long long)p.nseq * heads * ((s.V + 15) / 16);
-    if (groups <= 2 * 148) {
-      if constexpr (DP == 128)
-        launch_scan<DP, 2, 2, HAS_W>(s, p.nseq, heads, stream);
-      else
-        launch_scan<DP, 1, 2, HAS_W>(s, p.nseq, heads, stream);
-    } else {
-      launch_scan<DP, 1, 4, HAS_W>(s, p.nseq, heads, stream);
-    }
+    if constexpr (DP == 64)
+      launch_scan<DP, 2, 1, HAS_W, 4>(s, p.nseq, heads, stream);
+    else if (groups <= 148)
+      launch_scan<DP, 4, 1, HAS_W, 3>(s, p.nseq, heads, stream);
+    else if (!HAS_W || groups <= 8 * 148)
+      launch_scan<DP, 2, 2, HAS_W, 4>(s, p.nseq, heads, stream);
+    else
+      launch_scan<DP, 1, 4, HAS_W, 3>(s, p.nseq, heads, stream);
   }
   return gb_launch_status();
 }
@@ -527,8 +620,8 @@ GB_EXPORT int gb_chunk_delta_rule(const float* q, const float* k, const float* v
                                   const float* a_logit, long long ldg, const float* A_log, const float* dt_bias, const float* decay,
                                   long long ldd, float* state, const int* cu, const int* seq_slot, float* y, int ntok, int nseq, int H,
                                   int G, int D, int V, float qscale, float* scratch, long long scratch_floats, cudaStream_t stream) {
-  Prepare p = {q, k, ld, beta_logit, a_logit, ldg, decay, ldd, A_log, dt_bias, nullptr, nullptr, cu, nseq, H, G, D, 0, qscale, scratch, 0};
-  Scan s = {scratch, 0, v, ld, state, cu, seq_slot, y, H, 0, V, lanes_for(D), 1.0f};
+  Prepare p = {q, k, ld, beta_logit, a_logit, ldg, decay, ldd, A_log, dt_bias, nullptr, nullptr, cu, nseq, H, G, D, 0, qscale, scratch, 0, 0};
+  Scan s = {scratch, 0, v, ld, state, cu, seq_slot, y, H, 0, V, lanes_for(D), 1.0f, 0};
   return decay ? run_any<CHANNEL_DELTA>(p, s, ntok, scratch_floats, stream) : run_any<DELTA>(p, s, ntok, scratch_floats, stream);
 }
 
@@ -536,15 +629,15 @@ GB_EXPORT int gb_chunk_ssd_scan(const float* x, const float* Bm, const float* Cm
                                 const float* A_log, const float* dt_bias, const float* skip, float* state, const int* cu,
                                 const int* seq_slot, float* y, int ntok, int nseq, int H, int G, int N, int V, float* scratch,
                                 long long scratch_floats, cudaStream_t stream) {
-  Prepare p = {Cm, Bm, ld, dt_raw, nullptr, ldd, nullptr, 0, A_log, dt_bias, skip, nullptr, cu, nseq, H, G, N, 0, 1.0f, scratch, 0};
-  Scan s = {scratch, 0, x, ld, state, cu, seq_slot, y, H, 0, V, lanes_for(N), 1.0f};
+  Prepare p = {Cm, Bm, ld, dt_raw, nullptr, ldd, nullptr, 0, A_log, dt_bias, skip, nullptr, cu, nseq, H, G, N, 0, 1.0f, scratch, 0, 0};
+  Scan s = {scratch, 0, x, ld, state, cu, seq_slot, y, H, 0, V, lanes_for(N), 1.0f, 0};
   return run_any<STATE_SPACE>(p, s, ntok, scratch_floats, stream);
 }
 
 GB_EXPORT int gb_chunk_wkv_scan(const float* r, const float* k, const float* w, long long ld, long long ldw, const float* v, long long ldv,
                                 const float* bonus, float* state, const int* cu, const int* seq_slot, float* y, int ntok, int nseq,
                                 int H, int D, int V, float yscale, float* scratch, long long scratch_floats, cudaStream_t stream) {
-  Prepare p = {r, k, ld, nullptr, nullptr, 0, w, ldw, nullptr, nullptr, nullptr, bonus, cu, nseq, H, H, D, 0, 1.0f, scratch, 0};
-  Scan s = {scratch, 0, v, ldv, state, cu, seq_slot, y, H, 0, V, lanes_for(D), yscale};
+  Prepare p = {r, k, ld, nullptr, nullptr, 0, w, ldw, nullptr, nullptr, nullptr, bonus, cu, nseq, H, H, D, 0, 1.0f, scratch, 0, 0};
+  Scan s = {scratch, 0, v, ldv, state, cu, seq_slot, y, H, 0, V, lanes_for(D), yscale, 0};
   return bonus ? run_any<READ_BEFORE>(p, s, ntok, scratch_floats, stream) : run_any<READ_AFTER>(p, s, ntok, scratch_floats, stream);
 }
