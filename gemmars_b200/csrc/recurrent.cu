@@ -81,6 +81,72 @@ __global__ void __launch_bounds__(256) short_filter_kernel(const T* __restrict__
   }
 }
 
+// The same for float32 rows at 16-byte boundaries and up to four taps: a thread works four neighbouring channels, rows
+// asked for four at a time (a second four in flight took 49 us: fewer threads fit).  A row and channel costs a quarter of the instructions of addresses and loop; a row's sums
+// keep their order.  Bound by the instructions of the exact SiLU and by memory: 2,048 rows of 8,192 channels, four
+// taps: 60 us with a channel a thread, 42 so.
+__global__ void __launch_bounds__(128) short_filter_wide_kernel(const float* __restrict__ u, long long ldu, const float* __restrict__ taps,
+                                                               const float* __restrict__ bias, const float* __restrict__ state,
+                                                               const int* __restrict__ cu, const int* __restrict__ tok_seq,
+                                                               const int* __restrict__ seq_slot, float* __restrict__ out, long long ldo,
+                                                               int ntok, int per, int C, int K, int act) {
+  constexpr int AHEAD = 4, TAPS = 4;
+  pdl_release_next();
+  pdl_wait_prior();
+  const int c = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
+  if (c >= C) return;
+  // the window and its taps end with the row at hand: win[TAPS - 2] is the row before it, leading taps are zeros
+  float4 w[TAPS], win[TAPS - 1];
+#pragma unroll
+  for (int j = 0; j < TAPS; ++j) {
+    const int tap = j - (TAPS - K);
+    w[j] = tap >= 0 ? make_float4(taps[(size_t)c * K + tap], taps[(size_t)(c + 1) * K + tap], taps[(size_t)(c + 2) * K + tap],
+                                  taps[(size_t)(c + 3) * K + tap])
+                    : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  const float4 b0 = bias ? make_float4(bias[c], bias[c + 1], bias[c + 2], bias[c + 3]) : make_float4(0.f, 0.f, 0.f, 0.f);
+  const int first = blockIdx.x * per, end = min(first + per, ntok);
+  int b = tok_seq[first], row0 = cu[b], next_start = cu[b + 1];
+  auto before = [&](int local, int j) {      // the input of row `local` (negative: kept from earlier steps) of sequence b
+    const int tap = j - (TAPS - K);
+    if (tap < 0) return make_float4(0.f, 0.f, 0.f, 0.f);
+    return local >= 0 ? *(const float4*)(u + (size_t)(row0 + local) * ldu + c)
+                      : *(const float4*)(state + ((size_t)seq_slot[b] * (K - 1) + K - 1 + local) * C + c);
+  };
+#pragma unroll
+  for (int j = 0; j < TAPS - 1; ++j) win[j] = before(first - row0 - (TAPS - 1) + j, j);
+  const float* in = u + (size_t)first * ldu + c;
+  float* o = out + (size_t)first * ldo + c;
+  for (int t0 = first; t0 < end; t0 += AHEAD, in += AHEAD * ldu, o += AHEAD * ldo) {
+    float4 now[AHEAD];
+#pragma unroll
+    for (int r = 0; r < AHEAD; ++r) now[r] = t0 + r < end ? *(const float4*)(in + r * ldu) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int r = 0; r < AHEAD; ++r) {
+      if (t0 + r >= end) break;
+      while (t0 + r == next_start) {                      // the next sequence of the step starts here
+        ++b;
+        row0 = next_start;
+        next_start = cu[b + 1];
+#pragma unroll
+        for (int j = 0; j < TAPS - 1; ++j) win[j] = before(j - (TAPS - 1), j);
+      }
+      float4 a = b0;
+#pragma unroll
+      for (int j = 0; j < TAPS; ++j) {
+        if (j < TAPS - K) continue;
+        const float4 x = j < TAPS - 1 ? win[j < TAPS - 1 ? j : 0] : now[r];
+        a.x = fmaf(w[j].x, x.x, a.x); a.y = fmaf(w[j].y, x.y, a.y);
+        a.z = fmaf(w[j].z, x.z, a.z); a.w = fmaf(w[j].w, x.w, a.w);
+      }
+#pragma unroll
+      for (int j = 0; j < TAPS - 1; ++j) win[j] = j + 1 < TAPS - 1 ? win[j + 1 < TAPS - 1 ? j + 1 : 0] : now[r];
+      if (act == ACT_SILU) a = make_float4(silu_f(a.x), silu_f(a.y), silu_f(a.z), silu_f(a.w));
+      *(float4*)(o + r * ldo) = a;
+    }
+  }
+}
+
 // The state after the step: the last K-1 inputs of the sequence, old rows shifted where the step
 // brought fewer than K-1.
 template <typename T>
@@ -151,10 +217,15 @@ GB_EXPORT int gb_short_filter(const void* u, int in_dtype, long long ldu, const 
 #undef GB_SINGLE
     return gb_launch_status();
   }
+  const bool wide = in_dtype == GB_F32 && out_dtype == GB_F32 && K >= 2 && K <= 4 && C % 4 == 0 && ldu % 4 == 0 && ldo % 4 == 0 &&
+                    !(((uintptr_t)u | (uintptr_t)out | (uintptr_t)state) & 15);
 #define GB_FILTER(T, O)                                                                                                   \
   gb_launch(short_filter_kernel<T, O>, grid, 256, 0, stream, (const T*)u, ldu, taps, bias, (const float*)state, cu, tok_seq, \
             seq_slot, (O*)out, ldo, ntok, per, C, K, act)
-  if (in_dtype == GB_F32 && out_dtype == GB_F32) GB_FILTER(float, float);
+  if (wide)
+    gb_launch(short_filter_wide_kernel, dim3((ntok + per - 1) / per, (C / 4 + 127) / 128), 128, 0, stream, (const float*)u, ldu, taps,
+              bias, (const float*)state, cu, tok_seq, seq_slot, (float*)out, ldo, ntok, per, C, K, act);
+  else if (in_dtype == GB_F32 && out_dtype == GB_F32) GB_FILTER(float, float);
   else if (in_dtype == GB_F32 && out_dtype == GB_BF16) GB_FILTER(float, bf16);
   else if (in_dtype == GB_BF16 && out_dtype == GB_BF16) GB_FILTER(bf16, bf16);
   else if (in_dtype == GB_BF16 && out_dtype == GB_F32) GB_FILTER(bf16, float);
@@ -572,12 +643,99 @@ __global__ void __launch_bounds__(256) gated_group_norm_warp_kernel(const float*
   }
 }
 
+// The same for groups of 64, 128, 256, 512 or 1,024 channels whose rows lie at 16-byte boundaries: a lane holds four channels
+// of two rows; the warps of a wider group meet in shared memory.  Bound by memory and by the exact SiLU: 2,048 rows of 4,096
+// channels in groups of 128: 35 us with single channels, 18 so.
+template <typename O>
+__device__ __forceinline__ void store4(O* to, float4 v);
+template <>
+__device__ __forceinline__ void store4<float>(float* to, float4 v) { *(float4*)to = v; }
+template <>
+__device__ __forceinline__ void store4<bf16>(bf16* to, float4 v) {
+  const __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
+  *(uint2*)to = make_uint2(*(const uint32_t*)&a, *(const uint32_t*)&b);
+}
+template <typename O, int LANES>
+__global__ void __launch_bounds__(256) gated_group_norm_wide_kernel(const float* __restrict__ y, const float* __restrict__ gate,
+                                                                   long long ldgate, const float* __restrict__ w, int wn,
+                                                                   O* __restrict__ out, int ntok, int n, float eps, int gate_first,
+                                                                   float out_scale, int gate_act) {
+  constexpr int GS = LANES * 4, ROWS = 2;
+  pdl_release_next();
+  pdl_wait_prior();
+  const int t0 = blockIdx.x * ROWS, c = (blockIdx.y * 256 + threadIdx.x) * 4;
+  __shared__ float part[LANES > 32 ? ROWS : 1][8];
+  const bool live = c < n;            // whole groups
+  if (LANES <= 32 && !live) return;
+  const unsigned mine = LANES >= 32 ? 0xffffffffu : 0xffffu << (threadIdx.x & 16);
+  float4 v[ROWS], g[ROWS];
+  float ss[ROWS];
+#pragma unroll
+  for (int r = 0; r < ROWS; ++r) {
+    const int t = min(t0 + r, ntok - 1);
+    v[r] = live ? *(const float4*)(y + (size_t)t * n + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    g[r] = live ? *(const float4*)(gate + (size_t)t * ldgate + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+#pragma unroll
+  for (int r = 0; r < ROWS; ++r) {
+    g[r] = make_float4(gate_f(g[r].x, gate_act), gate_f(g[r].y, gate_act), gate_f(g[r].z, gate_act), gate_f(g[r].w, gate_act));
+    if (gate_first) v[r] = make_float4(v[r].x * g[r].x, v[r].y * g[r].y, v[r].z * g[r].z, v[r].w * g[r].w);
+    ss[r] = fmaf(v[r].w, v[r].w, fmaf(v[r].z, v[r].z, fmaf(v[r].y, v[r].y, v[r].x * v[r].x)));
+#pragma unroll
+    for (int o = (LANES < 32 ? LANES : 32) / 2; o > 0; o >>= 1) ss[r] += __shfl_xor_sync(mine, ss[r], o);
+  }
+  if (LANES > 32) {
+    constexpr int WARPS = LANES / 32;
+    const int warp = threadIdx.x >> 5;
+    if ((threadIdx.x & 31) == 0)
+#pragma unroll
+      for (int r = 0; r < ROWS; ++r) part[LANES > 32 ? r : 0][warp] = ss[r];
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) {
+      ss[r] = 0.f;
+#pragma unroll
+      for (int i = 0; i < WARPS; ++i) ss[r] += part[LANES > 32 ? r : 0][warp / WARPS * WARPS + i];
+    }
+    if (!live) return;
+  }
+  const int wc = c % wn;              // wn is a multiple of the group
+  const float4 ww = make_float4(w[wc], w[wc + 1], w[wc + 2], w[wc + 3]);
+#pragma unroll
+  for (int r = 0; r < ROWS; ++r) {
+    if (t0 + r >= ntok) break;
+    const float inv = 1.0f / sqrtf(ss[r] / (float)GS + eps);
+    float4 res = make_float4(v[r].x * inv * ww.x, v[r].y * inv * ww.y, v[r].z * inv * ww.z, v[r].w * inv * ww.w);
+    if (!gate_first) res = make_float4(res.x * g[r].x, res.y * g[r].y, res.z * g[r].z, res.w * g[r].w);
+    store4(out + (size_t)(t0 + r) * n + c, make_float4(res.x * out_scale, res.y * out_scale, res.z * out_scale, res.w * out_scale));
+  }
+}
+
 GB_EXPORT int gb_gated_group_norm_act(const float* y, const float* gate, long long ldgate, const float* w, int wn, void* out,
                                       int out_dtype, int ntok, int n, int gs, float eps, int gate_first, float out_scale,
                                       int gate_act, cudaStream_t stream) {
   if (ntok <= 0) return 0;
   if (gs <= 0 || n % gs || wn <= 0) return GB_ERR_SIZE;
   if (out_dtype != GB_F32 && out_dtype != GB_BF16) return GB_ERR_DTYPE;
+  if ((gs == 64 || gs == 128 || gs == 256 || gs == 512 || gs == 1024) && wn % gs == 0 && ldgate % 4 == 0 && !(((uintptr_t)y | (uintptr_t)gate | (uintptr_t)out) & 15)) {
+    const dim3 grid4((ntok + 1) / 2, (n / 4 + 255) / 256);
+#define GB_NORM_WIDE(O, L)                                                                                              \
+  gb_launch(gated_group_norm_wide_kernel<O, L>, grid4, 256, 0, stream, y, gate, ldgate, w, wn, (O*)out, ntok, n, eps, gate_first, \
+            out_scale, gate_act)
+#define GB_NORM_WIDTHS(O)                                                                                               \
+  switch (gs) {                                                                                                         \
+    case 64: GB_NORM_WIDE(O, 16); break;                                                                                \
+    case 128: GB_NORM_WIDE(O, 32); break;                                                                               \
+    case 256: GB_NORM_WIDE(O, 64); break;                                                                               \
+    case 512: GB_NORM_WIDE(O, 128); break;                                                                              \
+    default: GB_NORM_WIDE(O, 256);                                                                                      \
+  }
+    if (out_dtype == GB_F32) GB_NORM_WIDTHS(float)
+    else GB_NORM_WIDTHS(bf16)
+#undef GB_NORM_WIDTHS
+#undef GB_NORM_WIDE
+    return gb_launch_status();
+  }
   if (gs <= 128) {
     dim3 wgrid(ntok, (n / gs + 7) / 8);
 #define GB_NORM_WARP(O, E)                                                                                              \
@@ -632,6 +790,63 @@ __global__ void __launch_bounds__(256) shift_mix_kernel(const T* __restrict__ x,
   }
 }
 
+// Prompts in bfloat16 with rows at 16-byte boundaries: a thread works eight channels over SHIFT_ROWS rows, their factors in
+// registers and the row before at hand.  Bound by memory (a row in, n_mix rows out): 2,048 rows of 4,096 channels, five
+// mixes: 58 us with a channel and row a thread, 26 so.
+constexpr int SHIFT_ROWS = 8;
+__device__ __forceinline__ void unpack8(uint4 v, float (&f)[8]) {
+  const unsigned u[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {      // a bfloat16 is the upper half of the float32 of the same value
+    f[2 * e] = __uint_as_float(u[e] << 16);
+    f[2 * e + 1] = __uint_as_float(u[e] & 0xffff0000u);
+  }
+}
+__global__ void __launch_bounds__(128) shift_mix_wide_kernel(const bf16* __restrict__ x, long long ldx, const float* __restrict__ mu,
+                                                            const float* __restrict__ state, const int* __restrict__ cu,
+                                                            const int* __restrict__ tok_seq, const int* __restrict__ seq_slot,
+                                                            bf16* __restrict__ out, int ntok, int C, int n_mix) {
+  pdl_release_next();
+  pdl_wait_prior();
+  const int c = (blockIdx.y * 128 + threadIdx.x) * 8, t0 = blockIdx.x * SHIFT_ROWS, end = min(t0 + SHIFT_ROWS, ntok);
+  if (c >= C) return;
+  uint4 rows[SHIFT_ROWS + 1];
+#pragma unroll
+  for (int r = 0; r <= SHIFT_ROWS; ++r) {
+    const int t = min(max(t0 + r - 1, 0), ntok - 1);
+    rows[r] = *(const uint4*)(x + (size_t)t * ldx + c);
+  }
+  float prev[8];
+  unpack8(rows[0], prev);
+#pragma unroll
+  for (int r = 0; r < SHIFT_ROWS; ++r) {
+    const int t = t0 + r;
+    if (t >= end) break;
+    const int b = tok_seq[t];
+    if (t == cu[b]) {                 // the row before is an earlier step's
+      const float* st = state + (size_t)seq_slot[b] * C + c;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) prev[e] = st[e];
+    }
+    float cur[8];
+    unpack8(rows[r + 1], cur);
+    for (int s = 0; s < n_mix; ++s) {
+      const float4 m0 = *(const float4*)(mu + (size_t)s * C + c), m1 = *(const float4*)(mu + (size_t)s * C + c + 4);
+      const float m[8] = {m0.x, m0.y, m0.z, m0.w, m1.x, m1.y, m1.z, m1.w};
+      uint32_t o[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const __nv_bfloat162 p = __floats2bfloat162_rn(fmaf(prev[2 * e] - cur[2 * e], m[2 * e], cur[2 * e]),
+                                                       fmaf(prev[2 * e + 1] - cur[2 * e + 1], m[2 * e + 1], cur[2 * e + 1]));
+        o[e] = *(const uint32_t*)&p;
+      }
+      *(uint4*)(out + ((size_t)s * ntok + t) * C + c) = make_uint4(o[0], o[1], o[2], o[3]);
+    }
+#pragma unroll
+    for (int e = 0; e < 8; ++e) prev[e] = cur[e];
+  }
+}
+
 template <typename T>
 __global__ void __launch_bounds__(256) shift_state_kernel(const T* __restrict__ x, long long ldx, float* __restrict__ state,
                                                          const int* __restrict__ cu, const int* __restrict__ seq_slot, int C) {
@@ -655,6 +870,11 @@ GB_EXPORT int gb_shift_mix(const void* x, int dtype, long long ldx, const float*
     gb_launch(shift_mix_kernel<float>, grid, 256, 0, stream, (const float*)x, ldx, mu, state, cu, tok_seq, seq_slot, (float*)out,
               ntok, C, n_mix, single);
     if (!single) gb_launch(shift_state_kernel<float>, sgrid, 256, 0, stream, (const float*)x, ldx, state, cu, seq_slot, C);
+  } else if (dtype == GB_BF16 && !single && ntok >= 64 && C % 8 == 0 && ldx % 8 == 0 &&
+             !(((uintptr_t)x | (uintptr_t)out | (uintptr_t)mu) & 15)) {
+    gb_launch(shift_mix_wide_kernel, dim3((ntok + SHIFT_ROWS - 1) / SHIFT_ROWS, (C / 8 + 127) / 128), 128, 0, stream, (const bf16*)x, ldx,
+              mu, (const float*)state, cu, tok_seq, seq_slot, (bf16*)out, ntok, C, n_mix);
+    gb_launch(shift_state_kernel<bf16>, sgrid, 256, 0, stream, (const bf16*)x, ldx, state, cu, seq_slot, C);
   } else if (dtype == GB_BF16) {
     gb_launch(shift_mix_kernel<bf16>, grid, 256, 0, stream, (const bf16*)x, ldx, mu, state, cu, tok_seq, seq_slot, (bf16*)out,
               ntok, C, n_mix, single);
@@ -754,6 +974,98 @@ __global__ void __launch_bounds__(128) lowrank_decay_kernel(const float* __restr
     }
 }
 
+// Prompts with a bfloat16 W: the sums on the tensor cores.  A CTA is 64 rows by four times 64 channels, a warp 16 rows; z (or tanh z) is
+// split into two tf32 halves, hi + lo, whose products with the bfloat16 numbers of W are exact in float32, so a sum is as
+// good as one of float32 products.  (lo is cut at 2^-21 of z.)  The inner index is taken in pairs: lane t's two neighbouring
+// k stand for the instruction's t and t + 4.  Bound by the exponentials of the results: 2,048 rows, 4,096 channels, rank 64,
+// two exponentials: 70 us with FFMA, 47 so.
+constexpr int LR_ROWS = 64, LR_COLS = 64, LR_K = 64, LR_TILES = 4;
+__device__ __forceinline__ void mma_tf32(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__global__ void __launch_bounds__(128) lowrank_mma_kernel(const float* __restrict__ z, long long ldz, int rank, const bf16* __restrict__ W,
+                                                         const float* __restrict__ base, float* __restrict__ w, int ntok, int C,
+                                                         int mode, const float* __restrict__ rate, int rate_group, float inv_tau) {
+  constexpr int LD = LR_K + 8;
+  __shared__ __align__(16) float hi[LR_ROWS][LD], lo[LR_ROWS][LD];
+  pdl_release_next();
+  pdl_wait_prior();
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const int t0 = blockIdx.y * LR_ROWS;
+  auto bring = [&](int k0) {
+    __syncthreads();
+#pragma unroll 8
+    for (int e = tid; e < LR_ROWS * LR_K; e += 128) {
+      const int r = e / LR_K, k = e % LR_K;
+      float v = t0 + r < ntok && k0 + k < rank ? z[(size_t)(t0 + r) * ldz + k0 + k] : 0.f;
+      if (mode == LR_TANH_EXPEXP) v = tanhf(v);
+      const float h = __uint_as_float((__float_as_uint(v) + 0x1000u) & 0xffffe000u);
+      hi[r][k] = h;
+      lo[r][k] = v - h;
+    }
+    __syncthreads();
+  };
+  if (rank <= LR_K) bring(0);
+#pragma unroll 1
+  for (int tile = 0; tile < LR_TILES; ++tile) {
+    const int c0 = (blockIdx.x * LR_TILES + tile) * LR_COLS;
+    if (c0 >= C) return;
+    float acc[LR_COLS / 8][4] = {};
+    for (int k0 = 0; k0 < rank; k0 += LR_K) {
+      if (rank > LR_K) bring(k0);
+      const int steps = min(LR_K, rank - k0 + 7) / 8;
+      for (int s = 0; s < steps; ++s) {
+        const float *h0 = &hi[warp * 16 + g][8 * s + 2 * t], *l0 = &lo[warp * 16 + g][8 * s + 2 * t];
+        const float2 ha = *(const float2*)h0, hb = *(const float2*)(h0 + 8 * LD), la = *(const float2*)l0, lb = *(const float2*)(l0 + 8 * LD);
+        const uint32_t ah[4] = {__float_as_uint(ha.x), __float_as_uint(hb.x), __float_as_uint(ha.y), __float_as_uint(hb.y)};
+        const uint32_t al[4] = {__float_as_uint(la.x), __float_as_uint(lb.x), __float_as_uint(la.y), __float_as_uint(lb.y)};
+        const int k = k0 + 8 * s + 2 * t;
+#pragma unroll
+        for (int n = 0; n < LR_COLS / 8; ++n) {
+          const int c = c0 + 8 * n + g;
+          const uint32_t p = c < C && k < rank ? *(const uint32_t*)(W + (size_t)c * rank + k) : 0u;
+          mma_tf32(acc[n], ah, p << 16, p & 0xffff0000u);
+          mma_tf32(acc[n], al, p << 16, p & 0xffff0000u);
+        }
+      }
+    }
+#pragma unroll
+    for (int n = 0; n < LR_COLS / 8; ++n) {
+      const int c = c0 + 8 * n + 2 * t;
+      float bs[2], rt[2];
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int ce = min(c + e, C - 1);
+        bs[e] = base ? base[ce] : 0.f;
+        rt[e] = mode == LR_RATE ? expf(rate[ce / rate_group]) : 0.f;
+      }
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int row = t0 + warp * 16 + g + 8 * h;
+        if (row >= ntok) continue;
+        float r[2];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const float a = acc[n][2 * h + e] + bs[e];
+          if (mode == LR_TANH_EXPEXP) r[e] = expf(-expf(a));
+          else if (mode == LR_RATE) r[e] = expf(-rt[e] * softplus_f(a));
+          else if (mode == LR_SIGMOID_ROOT) r[e] = expf(-softplus_f(-a) * inv_tau);
+          else r[e] = a;
+        }
+        float* to = w + (size_t)row * C + c;
+        if (c + 1 < C && C % 2 == 0) {
+          *(float2*)to = make_float2(r[0], r[1]);
+        } else {
+          if (c < C) to[0] = r[0];
+          if (c + 1 < C) to[1] = r[1];
+        }
+      }
+    }
+  }
+}
+
 // z: [ntok, rank] float32; W: [C, rank] float32 or bfloat16; base: [C]; w: [ntok, C] float32.
 // The general form (see the modes above): z rows of ldz floats; rate [C / rate_group] for LR_RATE;
 // tau for LR_SIGMOID_ROOT.
@@ -770,6 +1082,9 @@ GB_EXPORT int gb_lowrank_map(const float* z, long long ldz, int rank, const void
   if (w_dtype == GB_F32)
     gb_launch(lowrank_decay_kernel<float>, grid, 128, 0, stream, z, ldz, rank, (const float*)W, base, w, ntok, C, mode, rate,
               rate_group, inv_tau);
+  else if (w_dtype == GB_BF16 && ntok >= 128 && rank % 2 == 0 && !((uintptr_t)W & 3) && !((uintptr_t)w & 7))
+    gb_launch(lowrank_mma_kernel, dim3((C + LR_TILES * LR_COLS - 1) / (LR_TILES * LR_COLS), (ntok + LR_ROWS - 1) / LR_ROWS), 128, 0, stream, z, ldz, rank,
+              (const bf16*)W, base, w, ntok, C, mode, rate, rate_group, inv_tau);
   else if (w_dtype == GB_BF16)
     gb_launch(lowrank_decay_kernel<bf16>, grid, 128, 0, stream, z, ldz, rank, (const bf16*)W, base, w, ntok, C, mode, rate,
               rate_group, inv_tau);
