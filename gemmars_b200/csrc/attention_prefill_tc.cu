@@ -23,6 +23,13 @@
 // Two CTAs fit an SM (112 KB of shared memory, 256 columns of tensor memory each), so one CTA's
 // softmax overlaps the other's MMAs.  Every mbarrier wait is bounded; a wait that runs out sets
 // the status word and an abort flag that ends the CTA's other loops, and tensor memory is freed.
+//
+// A third build (-DGB_ROT_DIM=..., up to 64) is for latent attention over a prompt's own tokens: the keys of a head are
+// its expanded part, HD - ROT dims (a multiple of 64), beside a rotated part that all heads share, and keys and values
+// lie token by token in buffers of the step instead of in pages: keys [tokens, heads (HD - ROT)], the shared parts
+// [tokens, ROT], values transposed [heads VD, tokens], sequence b from token (cu[b] / 8 + b) * 8 on.  With keys of 192 the
+// tiles of two CTAs an SM leave room for one stage each of keys and values: the other CTA's softmax covers the wait.
+// 2,048 tokens, 16 heads of 128 + 64 and 128: 47 us; the mma.sync kernel over rows [v | k] took 169.
 #include "tc_common.cuh"
 
 #ifndef GB_HEAD_DIM
@@ -35,12 +42,18 @@
 namespace {
 
 constexpr int HD = GB_HEAD_DIM, VD = GB_VALUE_DIM;
+#ifdef GB_ROT_DIM
+constexpr int ROT = GB_ROT_DIM, NOPE = HD - ROT;
+static_assert(NOPE > 0 && NOPE % 64 == 0 && ROT % 8 == 0 && ROT >= 8 && ROT <= 64 && HD <= 192, "keys: whole boxes and a shared part");
+#else
 static_assert(HD % 8 == 0 && HD >= 8 && HD <= 128, "keys: a multiple of 8 up to 128 (a head starts on a 16-byte boundary)");
+#endif
 static_assert(VD % 16 == 0 && VD >= 16 && VD <= 128, "values: a multiple of 16 up to 128");
 constexpr int ROWS = 128, KEYS = 64, QH = (HD + 63) / 64, HDP = QH * 64;     // HDP: a key's row in shared memory
 constexpr uint32_t Q_BYTES = ROWS * HDP * 2, K_BYTES = KEYS * HDP * 2, V_BYTES = VD * KEYS * 2, P_BYTES = ROWS * KEYS * 2;
 constexpr int OC = VD % 32 == 0 ? 32 : 16;                                    // columns of O a thread handles at a time
-constexpr uint32_t SMEM_TILES = Q_BYTES + 2 * K_BYTES + 2 * V_BYTES + P_BYTES;
+constexpr int ST = Q_BYTES + 2 * K_BYTES + 2 * V_BYTES + P_BYTES <= 112 * 1024 ? 2 : 1;   // stages: two CTAs share an SM
+constexpr uint32_t SMEM_TILES = Q_BYTES + ST * K_BYTES + ST * V_BYTES + P_BYTES;
 constexpr uint32_t TMEM_COLS = 256, S_COL0 = 0, S_COL1 = 64, O_COL = 128;
 constexpr uint32_t IDESC_S = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(KEYS >> 3) << 17) | ((uint32_t)(ROWS >> 4) << 24);
 constexpr uint32_t IDESC_PV = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(VD >> 3) << 17) | ((uint32_t)(ROWS >> 4) << 24);
@@ -123,6 +136,8 @@ struct Extras {
   float mul = LOG2E, pre = 0.f;
   const float* sink = nullptr;                                        // per head, natural units
   const bf16* gate = nullptr; long long gate_stride = 0; int gate_per_head = 0;
+  const float* row_scale = nullptr;                                   // [tokens, heads], multiplied into the result
+  const float* gate32 = nullptr; long long gate32_stride = 0;         // float32 logits, a number per output
   float out_scale = 1.f;
 };
 
@@ -130,16 +145,19 @@ struct Extras {
 template <bool CAP>
 __global__ void __launch_bounds__(192, 2)
 attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
-                            const __grid_constant__ CUtensorMap map_v, bf16* __restrict__ out, long long out_stride,
-                            const int* __restrict__ page_table, int table_width, int nkv,
+                            const __grid_constant__ CUtensorMap map_v,
+#ifdef GB_ROT_DIM
+                            const __grid_constant__ CUtensorMap map_r,
+#endif
+                            bf16* __restrict__ out, long long out_stride, const int* __restrict__ page_table, int table_width, int nkv,
                             const int* __restrict__ cu_seqlens, const int* __restrict__ seq_start,
                             const int* __restrict__ seq_slot, int n_seqs, int nh, int window,
                             const __grid_constant__ Extras ex) {
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* q_smem = smem;
-  uint8_t* k_smem = q_smem + Q_BYTES;          // two stages
-  uint8_t* v_smem = k_smem + 2 * K_BYTES;      // two stages
-  uint8_t* p_smem = v_smem + 2 * V_BYTES;
+  uint8_t* k_smem = q_smem + Q_BYTES;          // ST stages
+  uint8_t* v_smem = k_smem + ST * K_BYTES;     // ST stages
+  uint8_t* p_smem = v_smem + ST * V_BYTES;
   uint64_t* bars = (uint64_t*)(smem + SMEM_TILES);
   uint64_t* q_full = bars;            // 1
   uint64_t* k_full = bars + 1;        // 2: a page of keys has arrived
@@ -170,7 +188,8 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
   const int seq_len = cu_seqlens[b + 1] - cu_seqlens[b];
   const int first = tile * ROWS;
   const int rows_valid = min(ROWS, seq_len - first);
-  const int slot = seq_slot[b], start = seq_start[b];
+  [[maybe_unused]] const int slot = seq_slot[b];
+  const int start = seq_start[b];
   const int tok0 = cu_seqlens[b] + first;
   const int pos_last = start + first + rows_valid - 1;
   const int lo_first = window > 0 ? max(0, start + first + 1 - window) : 0;
@@ -223,22 +242,33 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
       uint32_t spins = 0;
       while ((jk < n_tiles || jv < n_tiles) && !*abort) {
         bool moved = false;
-        if (jk < n_tiles && (jk < 2 || mbar_try_wait(&k_empty[jk & 1], ((jk >> 1) - 1) & 1))) {
-          const int sidx = jk & 1;
+        if (jk < n_tiles && (jk < ST || mbar_try_wait(&k_empty[jk % ST], (jk / ST - 1) & 1))) {
+          const int sidx = jk % ST;
+          mbar_expect_tx(&k_full[sidx], K_BYTES);
+#ifdef GB_ROT_DIM
+          const int row = (cu_seqlens[b] / 8 + b) * 8 + (kt_begin + jk) * KEYS;
+          for (int h = 0; h < NOPE / 64; ++h)
+            tma_load_2d(k_smem + sidx * K_BYTES + h * (KEYS * 128), &map_k, kvh * NOPE + h * 64, row, &k_full[sidx]);
+          tma_load_2d(k_smem + sidx * K_BYTES + NOPE / 64 * (KEYS * 128), &map_r, 0, row, &k_full[sidx]);
+#else
           const int page = page_table[(size_t)slot * table_width + (kt_begin + jk) % table_width];
           const int row = page * nkv + kvh;
-          mbar_expect_tx(&k_full[sidx], K_BYTES);
           for (int h = 0; h < QH; ++h)
             tma_load_2d(k_smem + sidx * K_BYTES + h * (KEYS * 128), &map_k, h * 64, row * KEYS, &k_full[sidx]);
+#endif
           ++jk;
           moved = true;
         }
-        if (jv < n_tiles && jv < jk && (jv < 2 || mbar_try_wait(&v_empty[jv & 1], ((jv >> 1) - 1) & 1))) {
-          const int sidx = jv & 1;
+        if (jv < n_tiles && jv < jk && (jv < ST || mbar_try_wait(&v_empty[jv % ST], (jv / ST - 1) & 1))) {
+          const int sidx = jv % ST;
+          mbar_expect_tx(&v_full[sidx], V_BYTES);
+#ifdef GB_ROT_DIM
+          tma_load_2d(v_smem + sidx * V_BYTES, &map_v, (cu_seqlens[b] / 8 + b) * 8 + (kt_begin + jv) * KEYS, kvh * VD, &v_full[sidx]);
+#else
           const int page = page_table[(size_t)slot * table_width + (kt_begin + jv) % table_width];
           const int row = page * nkv + kvh;
-          mbar_expect_tx(&v_full[sidx], V_BYTES);
           tma_load_2d(v_smem + sidx * V_BYTES, &map_v, 0, row * VD, &v_full[sidx]);
+#endif
           ++jv;
           moved = true;
         }
@@ -261,7 +291,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
       uint32_t spins = 0;
       while (jp < n_tiles && !*abort) {
         bool moved = false;
-        if (js < n_tiles && mbar_try_wait(&k_full[js & 1], (js >> 1) & 1) &&
+        if (js < n_tiles && mbar_try_wait(&k_full[js % ST], (js / ST) & 1) &&
             (js < 2 || mbar_try_wait(&s_empty[js & 1], ((js >> 1) - 1) & 1))) {
           const int sidx = js & 1;
           tc_fence_after();
@@ -269,23 +299,23 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
 #pragma unroll
           for (int h = 0; h < QH; ++h) {
             const uint64_t qd = smem_desc(smem_u32(q_smem + h * (ROWS * 128)));
-            const uint64_t kd = smem_desc(smem_u32(k_smem + sidx * K_BYTES + h * (KEYS * 128)));
+            const uint64_t kd = smem_desc(smem_u32(k_smem + js % ST * K_BYTES + h * (KEYS * 128)));
 #pragma unroll
             for (int k = 0; k < 4; ++k) tc_mma(d, qd + (uint64_t)(k * 2), kd + (uint64_t)(k * 2), IDESC_S, (h > 0 || k > 0) ? 1u : 0u);
           }
           tc_commit(&s_full[sidx]);
-          tc_commit(&k_empty[sidx]);
+          tc_commit(&k_empty[js % ST]);
           ++js;
           moved = true;
         }
-        if (jp < js && mbar_try_wait(p_full, jp & 1) && mbar_try_wait(&v_full[jp & 1], (jp >> 1) & 1)) {
+        if (jp < js && mbar_try_wait(p_full, jp & 1) && mbar_try_wait(&v_full[jp % ST], (jp / ST) & 1)) {
           tc_fence_after();
           const uint64_t pd = smem_desc(smem_u32(p_smem));
-          const uint64_t vd = smem_desc(smem_u32(v_smem + (jp & 1) * V_BYTES));
+          const uint64_t vd = smem_desc(smem_u32(v_smem + jp % ST * V_BYTES));
 #pragma unroll
           for (int k = 0; k < 4; ++k) tc_mma(tmem + O_COL, pd + (uint64_t)(k * 2), vd + (uint64_t)(k * 2), IDESC_PV, (jp > 0 || k > 0) ? 1u : 0u);
           tc_commit(o_done);
-          tc_commit(&v_empty[jp & 1]);
+          tc_commit(&v_empty[jp % ST]);
           ++jp;
           moved = true;
         }
@@ -405,6 +435,8 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
       }
       float inv = l > 0.f ? keep / l : 0.f;
       const bf16* gt = ex.gate && valid ? ex.gate + (size_t)(tok0 + r) * ex.gate_stride : nullptr;
+      if (ex.row_scale && valid) inv *= ex.row_scale[(size_t)(tok0 + r) * nh + head];
+      const float* g32 = ex.gate32 && valid ? ex.gate32 + (size_t)(tok0 + r) * ex.gate32_stride + (size_t)head * VD : nullptr;
       if (gt && ex.gate_per_head) inv *= 1.0f / (1.0f + __expf(-__bfloat162float(gt[head])));
       bf16* dst = out + (size_t)(tok0 + r) * out_stride + (size_t)head * VD;
 #pragma unroll 1
@@ -417,6 +449,10 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
 #pragma unroll
             for (int i = 0; i < OC; ++i)
               ov[i] = __float_as_uint(__uint_as_float(ov[i]) / (1.0f + __expf(-__bfloat162float(gt[head * VD + c + i]))));
+          }
+          if (g32) {
+#pragma unroll
+            for (int i = 0; i < OC; ++i) ov[i] = __float_as_uint(__uint_as_float(ov[i]) / (1.0f + __expf(-g32[c + i])));
           }
 #pragma unroll
           for (int i = 0; i < OC / 8; ++i) {
@@ -439,6 +475,48 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
 
 }  // namespace
 
+static int configure() {
+  constexpr size_t SMEM = SMEM_TILES + 15 * 8 + 16;
+  static bool configured = false;
+  if (!configured) {
+    if (cudaFuncSetAttribute(attention_prefill_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM) != cudaSuccess ||
+        cudaFuncSetAttribute(attention_prefill_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM) != cudaSuccess)
+      return (int)cudaGetLastError();
+    configured = true;
+  }
+  return 0;
+}
+
+#ifdef GB_ROT_DIM
+// q: [ntok, nh * HD] (scaled), out: [ntok, nh * VD] bfloat16, tokens of all sequences packed (cu_seqlens: [n_seqs + 1]),
+// every sequence from position 0.  keys: [rows, nh * (HD - ROT)], shared: [rows, ROT], values: [nh * VD, rows], where
+// sequence b's rows are (cu[b] / 8 + b) * 8 and those after it; rows a multiple of 8 and at least (ntok / 8 + n_seqs) * 8;
+// every row finite.  seq_zeros: n_seqs zeros (the sequences' starts).  row_scale: float32 [ntok, nh] or null; gate32:
+// float32 logits [ntok, nh * VD], rows gate32_stride apart, or null.
+GB_EXPORT int gb_attention_prefill_latent(const void* q, long long q_stride, void* out, long long out_stride, const void* keys,
+                                          const void* shared, const void* values, long long rows, int hd, int vd, int rot,
+                                          const int* cu_seqlens, const int* seq_zeros, int n_seqs, int ntok, int nh, int window,
+                                          const float* row_scale, const float* gate32, long long gate32_stride, cudaStream_t stream) {
+  if (ntok <= 0 || n_seqs <= 0) return 0;
+  if (hd != HD || vd != VD || rot != ROT || nh <= 0 || rows % 8 || rows < ((long long)ntok / 8 + n_seqs) * 8) return GB_ERR_SIZE;
+  if (((uintptr_t)q & 15) || (q_stride % 8) || ((uintptr_t)out & 15) || (out_stride % 8) || ((uintptr_t)keys & 15) ||
+      ((uintptr_t)shared & 15) || ((uintptr_t)values & 15))
+    return GB_ERR_SIZE;
+  CUtensorMap mq, mk, mr, mv;
+  if (!tensor_map(&mq, q, (uint64_t)ntok, (uint64_t)nh * HD, (uint64_t)q_stride * 2, ROWS)) return GB_ERR_ARG;
+  if (!tensor_map(&mk, keys, (uint64_t)rows, (uint64_t)nh * NOPE, (uint64_t)nh * NOPE * 2, KEYS)) return GB_ERR_ARG;
+  if (!tensor_map(&mr, shared, (uint64_t)rows, (uint64_t)ROT, (uint64_t)ROT * 2, KEYS)) return GB_ERR_ARG;
+  if (!tensor_map(&mv, values, (uint64_t)nh * VD, (uint64_t)rows, (uint64_t)rows * 2, VD)) return GB_ERR_ARG;
+  if (const int rc = configure()) return rc;
+  Extras ex;
+  ex.row_scale = row_scale;
+  ex.gate32 = gate32; ex.gate32_stride = gate32_stride;
+  const dim3 grid(nh, (ntok + ROWS - 1) / ROWS + n_seqs);
+  gb_launch(attention_prefill_tc_kernel<false>, grid, 192, SMEM_TILES + 15 * 8 + 16, stream, mq, mk, mv, mr, (bf16*)out, out_stride,
+            (const int*)nullptr, 1, nh, cu_seqlens, seq_zeros, seq_zeros, n_seqs, nh, window, ex);
+  return gb_launch_status();
+}
+#else
 // q: [ntok, nh * HD], out: [ntok, nh * VD] bfloat16, tokens of all sequences packed (cu_seqlens: [n_seqs +
 // 1]); q rows q_stride elements apart.  kcache: [pages, nkv, 64, HD]; vcache: [pages, nkv, VD, 64] (pages
 // counts every page of the layer, the spare one included).  seq_start: cache length of each sequence
@@ -462,13 +540,7 @@ GB_EXPORT int gb_attention_prefill_tc_ext(const void* q, long long q_stride, voi
   if (!tensor_map(&mk, kcache, (uint64_t)pages * nkv * KEYS, (uint64_t)HD, (uint64_t)HD * 2, KEYS)) return GB_ERR_ARG;
   if (!tensor_map(&mv, vcache, (uint64_t)pages * nkv * VD, (uint64_t)KEYS, (uint64_t)KEYS * 2, VD)) return GB_ERR_ARG;
   constexpr size_t SMEM = SMEM_TILES + 15 * 8 + 16;
-  static bool configured = false;
-  if (!configured) {
-    if (cudaFuncSetAttribute(attention_prefill_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM) != cudaSuccess ||
-        cudaFuncSetAttribute(attention_prefill_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM) != cudaSuccess)
-      return (int)cudaGetLastError();
-    configured = true;
-  }
+  if (const int rc = configure()) return rc;
   Extras ex;
   ex.mul = (cap > 0.f ? cap : scale) * LOG2E;
   ex.pre = cap > 0.f ? scale / cap : 0.f;
@@ -495,6 +567,7 @@ GB_EXPORT int gb_attention_prefill_tc(const void* q, long long q_stride, void* o
                                      nkv, hd, hd, cu_seqlens, seq_start, seq_slot, n_seqs, ntok, nh, window, 1.0f, 0.f,
                                      nullptr, nullptr, 0, 0, 1.0f, stream);
 }
+#endif
 
 // 0, or the code of the first bounded wait that ran out (synchronizes the device).
 

@@ -22,16 +22,30 @@
 
 // Rotation of a pair (u, v) -> (u cos - v sin, v cos + u sin), angle = float(pos) * inv_freq[i], all in
 // float32, cosine and sine times `mag`.  Pair i < rot/2 is dims (2i, 2i+1), or with the half layout (i, i + rot/2).
-__device__ __forceinline__ void rotate_pair(float u, float v, float angle, float mag, float& ou, float& ov) {
+__device__ __forceinline__ float2 cos_sin(float angle, float mag) {
   float s, c;
   sincosf(angle, &s, &c);
-  s *= mag;
-  c *= mag;
-  ou = u * c - v * s;
-  ov = v * c + u * s;
+  return make_float2(c * mag, s * mag);
+}
+__device__ __forceinline__ void rotate_pair(float u, float v, float2 cs, float& ou, float& ov) {
+  ou = u * cs.x - v * cs.y;
+  ov = v * cs.x + u * cs.y;
 }
 
-// One block per token.  Inputs are the float32 results of the layer's projections.
+// A second copy of the cache rows (latents null: not wanted): latents and rotated key parts, rows ldl and ldr apart, token
+// by token.  With `cu` it is for keys and values that a prompt expands per head: sequence b's rows then start at
+// (cu[b] / 8 + b) * 8 (a multiple of 8, with room for every sequence's last, partly filled eight), and the queries lie
+// head by head as [dim | rd].
+template <typename T>
+struct Copy {
+  T *latents, *rotated;
+  long long ldl, ldr;
+  const int* cu;
+};
+
+// One block per token.  Inputs are the float32 results of the layer's projections.  A token's angles are taken once
+// into shared memory, for the key part and all heads (16 heads of 64 rotated dims, 2,048 tokens: 22 us with a sine and
+// cosine for every pair of every head).
 template <typename T>
 __global__ void __launch_bounds__(256) latent_prepare_kernel(
     const float* __restrict__ q_in, long long ldq, const float* __restrict__ kv_in, long long ldkv,
@@ -40,7 +54,8 @@ __global__ void __launch_bounds__(256) latent_prepare_kernel(
     T* __restrict__ q_lat, long long ldql, float* __restrict__ gate, T* __restrict__ cache,
     const int* __restrict__ page_table, int table_width, int page_size, const int* __restrict__ tok_pos,
     const int* __restrict__ tok_seq, const int* __restrict__ seq_slot, int H, int dim, int rd, int rank,
-    T* __restrict__ dense, long long ldd, int half_layout, float rot_mag) {
+    Copy<T> ex, int half_layout, float rot_mag) {
+  extern __shared__ float2 turn[];          // [rot / 2] cosine and sine
   __shared__ float scratch[34];
   pdl_release_next();
   pdl_wait_prior();
@@ -48,81 +63,88 @@ __global__ void __launch_bounds__(256) latent_prepare_kernel(
   const int pos = tok_pos[t];
   const float fpos = (float)pos;
   const float* kv = kv_in + (size_t)t * ldkv;
+  for (int i = tid; i < rot / 2; i += blockDim.x) turn[i] = cos_sin(fpos * inv_freq[i], rot_mag);
   // the latent: x / sqrt(mean(x^2) + eps) * w
   float ss = 0.f;
   for (int i = tid; i < rank; i += blockDim.x) ss = fmaf(kv[i], kv[i], ss);
-  ss = block_sum(ss, scratch);
+  ss = block_sum(ss, scratch);              // also: the angles are there
   const float rstd = 1.0f / sqrtf(ss / (float)rank + eps);
-  // the row goes into the paged cache and, when asked for, into a dense copy [ntok, rank + rd] as well
-  for (int copy = 0; copy < 2; ++copy) {
-    T* row;
-    if (copy == 0) {
-      if (cache == nullptr) continue;
-      const int slot = seq_slot[tok_seq[t]];
-      const int page = page_table[(size_t)slot * table_width + (pos / page_size) % table_width];
-      row = cache + ((size_t)page * page_size + pos % page_size) * (size_t)(rank + rd);
-    } else {
-      if (dense == nullptr) continue;
-      row = dense + (size_t)t * ldd;
+  // the row goes into the paged cache and, when asked for, into the rows to be expanded as well
+  T *lat0 = nullptr, *lat1 = nullptr, *key0 = nullptr, *key1 = nullptr;
+  if (cache != nullptr) {
+    const int slot = seq_slot[tok_seq[t]];
+    const int page = page_table[(size_t)slot * table_width + (pos / page_size) % table_width];
+    lat0 = cache + ((size_t)page * page_size + pos % page_size) * (size_t)(rank + rd);
+    key0 = lat0 + rank;
+  }
+  if (ex.latents != nullptr) {
+    size_t row = t;
+    if (ex.cu) {
+      const int b = tok_seq[t];
+      row = (size_t)(ex.cu[b] / 8 + b) * 8 + (t - ex.cu[b]);
     }
-    for (int i = tid; i < rank; i += blockDim.x) row[i] = from_f32<T>(kv[i] * rstd * norm_w[i]);
-    // the shared rotated key part: pairs below `rot` turn, the rest passes
-    for (int i = tid; i < rd / 2 + (rd & 1); i += blockDim.x) {
-      const bool turns = 2 * i < rot;
-      const int a = turns && half_layout ? i : 2 * i, b = turns && half_layout ? i + rot / 2 : 2 * i + 1;
-      if (turns) {
-        float u, v;
-        rotate_pair(kv[rank + a], kv[rank + b], fpos * inv_freq[i], rot_mag, u, v);
-        row[rank + a] = from_f32<T>(u);
-        row[rank + b] = from_f32<T>(v);
-      } else {
-        row[rank + a] = from_f32<T>(kv[rank + a]);
-        if (b < rd) row[rank + b] = from_f32<T>(kv[rank + b]);
-      }
+    lat1 = ex.latents + row * ex.ldl;
+    key1 = ex.rotated + row * ex.ldr;
+  }
+  for (int i = tid; i < rank; i += blockDim.x) {
+    const T v = from_f32<T>(kv[i] * rstd * norm_w[i]);
+    if (lat0) lat0[i] = v;
+    if (lat1) lat1[i] = v;
+  }
+  // the shared rotated key part: pairs below `rot` turn, the rest passes
+  const int halves = rd / 2 + (rd & 1);
+  for (int i = tid; i < halves; i += blockDim.x) {
+    const bool turns = 2 * i < rot;
+    const int a = turns && half_layout ? i : 2 * i, b = turns && half_layout ? i + rot / 2 : 2 * i + 1;
+    float u = kv[rank + a], v = b < rd ? kv[rank + b] : 0.f;
+    if (turns) rotate_pair(u, v, turn[i], u, v);
+    for (int copy = 0; copy < 2; ++copy) {
+      T* key = copy ? key1 : key0;
+      if (!key) continue;
+      key[a] = from_f32<T>(u);
+      if (b < rd) key[b] = from_f32<T>(v);
     }
   }
-  // queries: the unrotated dims go to the absorbing product, the rotated ones straight into qa
+  // queries: the unrotated dims go to the absorbing product and the rotated ones straight into qa, or both into the
+  // head's own row
   const float* q = q_in + (size_t)t * ldq;
-  const int qd = dim + rd;
+  const int qd = dim + rd, rot_at = ex.cu ? dim : rank, nope_head = ex.cu ? qd : dim, lat_head = rot_at + rd;
   for (int e = tid; e < H * dim; e += blockDim.x) {
     const int h = e / dim, d = e % dim;
-    q_nope[(size_t)t * ldqn + e] = from_f32<T>(q[h * qd + d] * q_scale);
+    q_nope[(size_t)t * ldqn + (size_t)h * nope_head + d] = from_f32<T>(q[h * qd + d] * q_scale);
   }
-  const int halves = rd / 2 + (rd & 1);
   for (int e = tid; e < H * halves; e += blockDim.x) {
     const int h = e / halves, i = e % halves;
     const bool turns = 2 * i < rot;
     const int a = turns && half_layout ? i : 2 * i, b = turns && half_layout ? i + rot / 2 : 2 * i + 1;
     const float* src = q + h * qd + dim;
-    T* dst = q_lat + (size_t)t * ldql + (size_t)h * (rank + rd) + rank;
-    if (turns) {
-      float u, v;
-      rotate_pair(src[a], src[b], fpos * inv_freq[i], rot_mag, u, v);
-      dst[a] = from_f32<T>(u * q_scale);
-      dst[b] = from_f32<T>(v * q_scale);
-    } else {
-      dst[a] = from_f32<T>(src[a] * q_scale);
-      if (b < rd) dst[b] = from_f32<T>(src[b] * q_scale);
-    }
+    T* dst = q_lat + (size_t)t * ldql + (size_t)h * lat_head + rot_at;
+    float u = src[a], v = b < rd ? src[b] : 0.f;
+    if (turns) rotate_pair(u, v, turn[i], u, v);
+    dst[a] = from_f32<T>(u * q_scale);
+    if (b < rd) dst[b] = from_f32<T>(v * q_scale);
   }
   if (g_in != nullptr)
     for (int h = tid; h < H; h += blockDim.x) gate[(size_t)t * H + h] = 1.0f / (1.0f + expf(-g_in[(size_t)t * ldg + h]));
 }
 
+// latents, rotated, cu: see Copy; with cu, q_nope and q_lat are one buffer of rows [H, dim + rd].
 GB_EXPORT int gb_latent_prepare(const float* q_in, long long ldq, const float* kv_in, long long ldkv, const float* g_in,
                                 long long ldg, const float* norm_w, float eps, const float* inv_freq, int rot,
                                 float q_scale, void* q_nope, long long ldqn, void* q_lat, long long ldql, float* gate,
                                 void* cache, int dtype, const int* page_table, int table_width, int page_size,
                                 const int* tok_pos, const int* tok_seq, const int* seq_slot, int ntok, int H, int dim,
-                                int rd, int rank, void* dense, long long ldd, int half_layout, float rot_mag,
-                                cudaStream_t stream) {
+                                int rd, int rank, void* latents, long long ldl, void* rotated, long long ldr, const int* cu,
+                                int half_layout, float rot_mag, cudaStream_t stream) {
   if (ntok <= 0) return 0;
-  if (H <= 0 || dim < 0 || rd < 0 || rank <= 0 || rot < 0 || rot > rd || (rot & 1)) return GB_ERR_SIZE;
+  if (H <= 0 || dim < 0 || rd < 0 || rank <= 0 || rot < 0 || rot > rd || (rot & 1) || rot > 8192) return GB_ERR_SIZE;
   if (rot > 0 && inv_freq == nullptr) return GB_ERR_ARG;
+  if (cu != nullptr && latents == nullptr) return GB_ERR_ARG;
 #define LAUNCH(T)                                                                                                     \
-  gb_launch(latent_prepare_kernel<T>, dim3(ntok), dim3(256), 0, stream, q_in, ldq, kv_in, ldkv, g_in, ldg, norm_w, eps, \
-            inv_freq, rot, q_scale, (T*)q_nope, ldqn, (T*)q_lat, ldql, gate, (T*)cache, page_table, table_width,       \
-            page_size, tok_pos, tok_seq, seq_slot, H, dim, rd, rank, (T*)dense, ldd, half_layout, rot_mag)
+  gb_launch(latent_prepare_kernel<T>, dim3(ntok), dim3(256), (size_t)(rot / 2) * sizeof(float2), stream, q_in, ldq, kv_in, ldkv, \
+            g_in, ldg, norm_w, eps, inv_freq, rot, q_scale, (T*)q_nope, ldqn, (T*)q_lat, ldql, gate, (T*)cache, page_table, \
+            table_width, page_size, tok_pos, tok_seq, seq_slot, H, dim, rd, rank, Copy<T>{(T*)latents, (T*)rotated, ldl, ldr, cu}, \
+            half_layout, rot_mag)
   if (dtype == GB_F32) LAUNCH(float);
   else if (dtype == GB_BF16) LAUNCH(bf16);
   else return GB_ERR_DTYPE;
@@ -310,7 +332,7 @@ __global__ void rope_pairs_kernel(T* __restrict__ x, long long ldx, const int* _
     const int h = e / half, i = e % half;
     T* v = x + (size_t)t * ldx + (size_t)h * hd + 2 * i;
     float a, b;
-    rotate_pair(to_f32(v[0]), to_f32(v[1]), fpos * inv_freq[i], mag, a, b);
+    rotate_pair(to_f32(v[0]), to_f32(v[1]), cos_sin(fpos * inv_freq[i], mag), a, b);
     v[0] = from_f32<T>(a);
     v[1] = from_f32<T>(b);
   }

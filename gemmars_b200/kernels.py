@@ -868,7 +868,7 @@ def attention_prefill_tc_status(head_dim: int = 0, reset: bool = True) -> int:
 
 def latent_prepare(q_in, kv_in, g_in, norm_w, eps, inv_freq, rot, q_scale, q_nope, q_lat, gate, cache, page_table,
                    page_size, tok_pos, tok_seq, seq_slot, heads, dim, rd, rank, dense=None, half_layout=False,
-                   rot_magnitude: float = 1.0):
+                   rot_magnitude: float = 1.0, expand=None):
     """From the float32 projections of a latent attention layer: the cache row of every token
     (RMS-normed latent ``kv_in[:, :rank]``, then the key part ``kv_in[:, rank:]`` with its first
     ``rot`` dims rotated, as interleaved pairs or with ``half_layout`` as pairs (i, i + rot/2), cosines
@@ -876,12 +876,28 @@ def latent_prepare(q_in, kv_in, g_in, norm_w, eps, inv_freq, rot, q_scale, q_nop
     the queries' unrotated dims times ``q_scale`` into ``q_nope`` [T, heads * dim], their rotated
     dims (rotated, scaled) into the last ``rd`` columns of each head of ``q_lat``
     [T, heads * (rank + rd)]; ``gate`` [T, heads] = sigmoid(g_in) (float32; None: no gate).  ``dense``
-    [T, rank + rd] (None: not wanted) receives the same rows as the cache, token by token."""
+    [T, rank + rd] (None: not wanted) receives the same rows as the cache, token by token.  ``expand``
+    (latents [R, rank], key parts [R, rd], cu_seqlens), R = latent_expand_rows(T, sequences), instead of
+    ``dense``: the rows of sequence b from (cu_seqlens[b] // 8 + b) * 8 on, and the queries head by head as
+    [dim | rd]: ``q_nope`` and ``q_lat`` are then one [T, heads * (dim + rd)]."""
     _cuda(q_in, kv_in, g_in, norm_w, inv_freq, q_nope, q_lat, gate, cache, page_table, tok_pos, tok_seq, seq_slot)
     t = q_in.shape[0]
     assert q_in.dtype == torch.float32 and kv_in.dtype == torch.float32 and q_in.stride(1) == 1 and kv_in.stride(1) == 1
     assert q_in.shape[1] == heads * (dim + rd) and kv_in.shape == (t, rank + rd) and norm_w.numel() == rank
-    assert q_nope.shape == (t, heads * dim) and q_lat.shape == (t, heads * (rank + rd)) and q_nope.dtype == q_lat.dtype
+    if expand is not None:
+        assert dense is None and q_nope.data_ptr() == q_lat.data_ptr() and q_lat.shape == (t, heads * (dim + rd))
+        lat, keys, cu = expand
+        rows = latent_expand_rows(t, cu.numel() - 1)
+        assert lat.shape == (rows, rank) and keys.shape == (rows, rd) and lat.is_contiguous() and keys.is_contiguous()
+        assert lat.dtype == keys.dtype == q_lat.dtype
+        copy = (lat.data_ptr(), rank, keys.data_ptr(), rd, cu.data_ptr())
+    else:
+        assert q_nope.shape == (t, heads * dim) and q_lat.shape == (t, heads * (rank + rd))
+        copy = (None, 0, None, 0, None)
+        if dense is not None:
+            assert dense.dtype == q_lat.dtype and dense.shape == (t, rank + rd) and dense.stride(1) == 1
+            copy = (dense.data_ptr(), dense.stride(0), dense[:, rank:].data_ptr(), dense.stride(0), None)
+    assert q_nope.dtype == q_lat.dtype
     assert q_nope.stride(1) == 1 and q_lat.stride(1) == 1 and norm_w.dtype == torch.float32
     if g_in is not None:
         assert g_in.dtype == torch.float32 and g_in.shape == (t, heads) and g_in.stride(1) == 1
@@ -893,15 +909,14 @@ def latent_prepare(q_in, kv_in, g_in, norm_w, eps, inv_freq, rot, q_scale, q_nop
     f = _fn("latent_attention", "gb_latent_prepare",
             [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_float, c_void_p, c_int, c_float,
              c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p,
-             c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_longlong, c_int, c_float, c_void_p])
-    if dense is not None:
-        assert dense.dtype == q_lat.dtype and dense.shape == (t, rank + rd) and dense.stride(1) == 1
+             c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_int,
+             c_float, c_void_p])
     _check(f(q_in.data_ptr(), q_in.stride(0), kv_in.data_ptr(), kv_in.stride(0), _ptr(g_in),
              g_in.stride(0) if g_in is not None else 0, norm_w.data_ptr(), eps, _ptr(inv_freq), rot, q_scale,
              q_nope.data_ptr(), q_nope.stride(0), q_lat.data_ptr(), q_lat.stride(0), _ptr(gate), _ptr(cache),
              dtype_code(q_lat.dtype), _ptr(page_table), page_table.shape[1] if page_table is not None else 1, page_size,
-             tok_pos.data_ptr(), tok_seq.data_ptr(), seq_slot.data_ptr(), t, heads, dim, rd, rank, _ptr(dense),
-             dense.stride(0) if dense is not None else 0, 1 if half_layout else 0, float(rot_magnitude), _stream()),
+             tok_pos.data_ptr(), tok_seq.data_ptr(), seq_slot.data_ptr(), t, heads, dim, rd, rank, *copy,
+             1 if half_layout else 0, float(rot_magnitude), _stream()),
            "latent_prepare", "elementwise", _nbytes(q_in, kv_in, q_nope) + t * (rank + 2 * rd) * q_lat.element_size())
 
 
@@ -1082,11 +1097,50 @@ def latent_expand_usable(dtype, rank: int, dim: int, rd: int, vd: int) -> bool:
             and 2 * vd + dim + rd < 2 * rank + rd)
 
 
+def latent_expand_rows(ntok: int, nseq: int) -> int:
+    """Rows that a step's latents take when every sequence starts at a multiple of 8."""
+    return (ntok // 8 + nseq) * 8
+
+
+def latent_prefill_tc_usable(dtype, rank: int, dim: int, rd: int, vd: int) -> bool:
+    """Whether attention over expanded heads runs on the tcgen05 kernel: a head's own key dims in whole boxes of 64,
+    shared ones that fill at most one, values and keys that its tiles hold.  Other sizes take the mma.sync kernel over
+    rows [v | k_nope | k_rot]."""
+    return (dtype == torch.bfloat16 and rank % 8 == 0 and dim % 64 == 0 and dim > 0 and rd % 8 == 0 and 8 <= rd <= 64
+            and dim + rd <= 192 and vd % 16 == 0 and 16 <= vd <= 128)
+
+
+def attention_prefill_latent(q, out, nh, keys, shared, values, rot, cu_seqlens, seq_start, window=None, row_scale=None, gate=None):
+    """Causal attention of packed prompts (every sequence from position 0: ``seq_start`` is zeros) over keys and values
+    expanded per head: q [T, nh * (dim + rot)], scaled; keys [R, nh * dim], the key part all heads share [R, rot], values
+    transposed [nh * vd, R], R = latent_expand_rows(T, sequences), sequence b's rows from (cu_seqlens[b] // 8 + b) * 8 on,
+    all of them finite.  out [T, nh * vd] times ``row_scale`` (float32 [T, nh]) and sigmoid(``gate``) (float32 [T, nh * vd],
+    rows may be wider) where given."""
+    _cuda(q, out, keys, shared, values, cu_seqlens, seq_start, row_scale, gate)
+    rows, vd, hd = keys.shape[0], out.shape[1] // nh, q.shape[1] // nh
+    assert rows == latent_expand_rows(q.shape[0], cu_seqlens.numel() - 1) and q.stride(1) == 1 and out.stride(1) == 1
+    assert keys.shape == (rows, nh * (hd - rot)) and shared.shape == (rows, rot) and values.shape == (nh * vd, rows)
+    assert keys.is_contiguous() and shared.is_contiguous() and values.is_contiguous()
+    assert q.dtype == out.dtype == keys.dtype == shared.dtype == values.dtype == torch.bfloat16
+    assert row_scale is None or (row_scale.dtype == torch.float32 and row_scale.shape == (q.shape[0], nh) and row_scale.is_contiguous())
+    assert gate is None or (gate.dtype == torch.float32 and gate.shape == (q.shape[0], nh * vd) and gate.stride(1) == 1)
+    f = _fn("attention_prefill_tc", "gb_attention_prefill_latent",
+            [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_longlong, c_int, c_int, c_int, c_void_p,
+             c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_longlong, c_void_p],
+            defines=(("GB_HEAD_DIM", hd), ("GB_VALUE_DIM", vd), ("GB_ROT_DIM", rot)))
+    _check(f(q.data_ptr(), q.stride(0), out.data_ptr(), out.stride(0), keys.data_ptr(), shared.data_ptr(), values.data_ptr(), rows,
+             hd, vd, rot, cu_seqlens.data_ptr(), seq_start.data_ptr(), cu_seqlens.numel() - 1, q.shape[0], nh, window or 0,
+             _ptr(row_scale), _ptr(gate), gate.stride(0) if gate is not None else 0, _stream()), "attention_prefill_latent",
+           "attention", _nbytes(q, out, keys, shared, values))
+
+
 def latent_attention_units(compute: str, rank: int, rd: int, dim: int = 0, vd: int = 0):
     units = [("latent_attention", ())]
     if compute != "float32" and latent_attention_mma_usable(torch.bfloat16, rank, rd, 64):
         units.append(("latent_attention_mma", (("GB_LATENT_RANK", rank), ("GB_LATENT_ROT", rd))))
-    if compute != "float32" and vd and latent_expand_usable(torch.bfloat16, rank, dim, rd, vd):
+    if compute != "float32" and vd and latent_prefill_tc_usable(torch.bfloat16, rank, dim, rd, vd) and 2 * vd + dim + rd < 2 * rank + rd:
+        units.append(("attention_prefill_tc", (("GB_HEAD_DIM", dim + rd), ("GB_VALUE_DIM", vd), ("GB_ROT_DIM", rd))))
+    elif compute != "float32" and vd and latent_expand_usable(torch.bfloat16, rank, dim, rd, vd):
         units.append(("latent_attention_mma", (("GB_LATENT_RANK", vd), ("GB_LATENT_ROT", dim + rd))))
     return units
 

@@ -149,8 +149,6 @@ class LatentAttention(Part):
             cq = torch.empty((t, nq), dtype=self.act_dtype, device=h.device)
             kernels.norm_cols(q, self.q_norm_w, cq, self.eps)
             q = self.uq(cq, out_dtype=torch.float32)
-        q_nope = torch.empty((t, nh * dim), dtype=self.act_dtype, device=h.device)
-        qa = torch.empty((t, nh * (r + rd)), dtype=self.act_dtype, device=h.device)
         logits = proj[:, nq + r + rd:nq + r + rd + self.gate_rows] if self.gated else None
         # one gate per head is made beside the queries and scales the heads' results; one per number is
         # taken from its logits where the results are written
@@ -159,15 +157,29 @@ class LatentAttention(Part):
         rot = self.position.rotary_dim if self.position is not None else 0
         # a prompt step whose sequences all start at position 0 (no cached prefix) may expand keys and
         # values per head, which is less arithmetic than attention over the latent rows
-        expand = (t >= kernels.LATENT_EXPAND_MIN_TOKENS and ctx.host is not None
-                  and not any(ctx.host["seq_start"]) and kernels.latent_expand_usable(h.dtype, r, dim, rd, vd))
+        expand = (t >= kernels.LATENT_EXPAND_MIN_TOKENS and ctx.host is not None and not any(ctx.host["seq_start"])
+                  and 2 * vd + dim + rd < 2 * r + rd)
+        on_tc = expand and kernels.latent_prefill_tc_usable(h.dtype, r, dim, rd, vd)
+        expand = expand and not on_tc and kernels.latent_expand_usable(h.dtype, r, dim, rd, vd)
         dense = torch.empty((t, r + rd), dtype=self.act_dtype, device=h.device) if expand else None
+        rows = None
+        if on_tc:
+            # rows between two sequences, which no token fills, have to be finite
+            n = kernels.latent_expand_rows(t, ctx.n_seqs)
+            rows = (torch.zeros((n, r), dtype=self.act_dtype, device=h.device),
+                    torch.zeros((n, rd), dtype=self.act_dtype, device=h.device), ctx.cu_seqlens)
+            q_nope = qa = torch.empty((t, nh * (dim + rd)), dtype=self.act_dtype, device=h.device)
+        else:
+            q_nope = torch.empty((t, nh * dim), dtype=self.act_dtype, device=h.device)
+            qa = torch.empty((t, nh * (r + rd)), dtype=self.act_dtype, device=h.device)
         kernels.latent_prepare(q, proj[:, nq:nq + r + rd], logits if self.gate_per_head else None,
                                self.norm_w, self.eps, self.position.inv_freq(h.device) if rot else None, rot, self.scale,
                                q_nope, qa, gate, kc.view(-1, group.page_size, r + rd) if writes_cache else None,
                                group.page_table, group.page_size, ctx.tok_pos, ctx.tok_seq, ctx.seq_slot, nh, dim, rd, r,
                                dense=dense, half_layout=self.position is not None and self.position.layout == "half",
-                               rot_magnitude=self.position.magnitude if rot else 1.0)
+                               rot_magnitude=self.position.magnitude if rot else 1.0, expand=rows)
+        if on_tc:
+            return self._expanded_tc(ctx, qa, gate, channel, rows, residual)
         if expand:
             return self._expanded(ctx, q_nope, qa, gate, channel, dense, residual)
         if dim:
@@ -180,6 +192,20 @@ class LatentAttention(Part):
         o = torch.empty((t, nh * vd), dtype=self.act_dtype, device=h.device)
         kernels.heads_gemm(lat.view(t, nh, r), self.uv, o.view(t, nh, vd), nh, scale=gate, gate=channel)
         return self.o.add_into(o, residual, then_norm)
+
+    def _expanded_tc(self, ctx, q, gate, channel, rows, residual):
+        """Attention of a prompt step over keys and values expanded per head, on the tcgen05 kernel: two plain
+        products over the step's latents make every head's keys token by token and every head's values transposed."""
+        nh, dim, rd, r, vd = self.num_heads, self.dim, self.rot_dim, self.rank, self.vdim
+        latents, shared, cu = rows
+        t, n = q.shape[0], latents.shape[0]
+        keys = torch.empty((n, nh * dim), dtype=self.act_dtype, device=q.device)
+        kernels.gemm(latents, self.uk.view(nh * dim, r), keys)
+        values = torch.empty((nh * vd, n), dtype=self.act_dtype, device=q.device)
+        kernels.gemm(self.uv.view(nh * vd, r), latents, values)
+        o = torch.empty((t, nh * vd), dtype=self.act_dtype, device=q.device)
+        kernels.attention_prefill_latent(q, o, nh, keys, shared, values, rd, cu, ctx.seq_start, self.window, gate, channel)
+        self.o.add_into(o, residual)
 
     def _expanded(self, ctx, q_nope, qa, gate, channel, dense, residual):
         """Attention of a prompt step over keys and values expanded per head.  Every head gets rows
