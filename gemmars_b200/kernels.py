@@ -673,7 +673,8 @@ def gated_units(compute: str, act: str):
     return units
 
 
-_STATUS_ENTRIES = ("gb_gemm_tc_status", "gb_attention_prefill_tc_status", "gb_attention_decode_stream_status")
+_STATUS_ENTRIES = ("gb_gemm_tc_status", "gb_attention_prefill_tc_status", "gb_attention_decode_stream_status",
+                   "gb_latent_decode_status")
 
 
 def _status(entry: str, reset: bool) -> int:
@@ -1018,11 +1019,9 @@ _latent_scratch = {}
 
 
 def latent_attention_mma(qa, out, heads, rank, rd, cache, page_table, page_size, cu_seqlens, seq_start, seq_slot,
-                         max_new: int, window=None, ksplits: int = 1, cache_bytes: int = 0, head_stride: int = 0,
-                         out_scale=None, out_gate=None):
+                         max_new: int, window=None, cache_bytes: int = 0, head_stride: int = 0, out_scale=None, out_gate=None):
     """bfloat16 latent attention on the tensor cores (mma.sync) for packed sequences that bring any
-    number of tokens each; with ``ksplits`` > 1 the keys of a tile of rows are dealt to that many
-    CTAs and a second kernel adds their parts.  ``head_stride`` > 0: every head has rows of its own,
+    number of tokens each.  ``head_stride`` > 0: every head has rows of its own,
     ``cache`` [heads, packed tokens + 64, rank + rd] (elements ``head_stride`` apart), a sequence's rows
     from its first packed token on, every sequence from position 0, no page table; ``out_scale``
     float32 [T, heads] multiplies the output, sigmoid(``out_gate``) too (float32 [T, heads * rank], rows may be wider)."""
@@ -1034,35 +1033,49 @@ def latent_attention_mma(qa, out, heads, rank, rd, cache, page_table, page_size,
     assert qa.shape[1] == heads * (rank + rd) and out.shape[1] == heads * rank and cache.shape[-1] == rank + rd
     ntok = qa.shape[0]
     if head_stride:
-        assert ksplits == 1 and cache.shape[0] == heads and cache.shape[1] >= ntok + 64 and head_stride == cache.stride(0)
+        assert cache.shape[0] == heads and cache.shape[1] >= ntok + 64 and head_stride == cache.stride(0)
     defines = (("GB_LATENT_RANK", rank), ("GB_LATENT_ROT", rd))
-    part = None
-    if ksplits > 1:
-        need = ntok * heads * ksplits * (rank + 4)
-        part = _latent_scratch.get(qa.device.index)
-        if part is None or part.numel() < need:
-            if part is not None:
-                _outgrown.append(part)        # a captured step may still point at it: never freed
-            part = _latent_scratch[qa.device.index] = torch.empty(max(need, 1 << 20), dtype=torch.float32, device=qa.device)
     f = _fn("latent_attention_mma", "gb_latent_attention_mma",
-            [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p,
-             c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_longlong, c_void_p, c_void_p, c_longlong,
+            [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p,
+             c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_longlong, c_void_p, c_void_p, c_longlong,
              c_void_p], defines=defines)
-    _check(f(qa.data_ptr(), qa.stride(0), out.data_ptr(), out.stride(0), _ptr(part), cache.data_ptr(), _ptr(page_table),
+    _check(f(qa.data_ptr(), qa.stride(0), out.data_ptr(), out.stride(0), cache.data_ptr(), _ptr(page_table),
              page_table.shape[1] if page_table is not None else 1, page_size, cu_seqlens.data_ptr(), seq_start.data_ptr(),
              seq_slot.data_ptr(), seq_slot.numel(), ntok, heads, rank, rd, max_new * (1 if head_stride else heads),
-             window or 0, ksplits, head_stride, _ptr(out_scale), _ptr(out_gate), out_gate.stride(0) if out_gate is not None else 0,
+             window or 0, head_stride, _ptr(out_scale), _ptr(out_gate), out_gate.stride(0) if out_gate is not None else 0,
              _stream()),
            "latent_attention_mma", "attention", _nbytes(qa, out) + cache_bytes)
-    if ksplits > 1:
-        count_launches(1)   # the merge kernel
 
 
-def latent_decode_splits(n_seqs: int, heads: int) -> int:
-    """CTAs along the keys for each sequence of a decode step: about two CTAs per SM in all (a CTA is
-    one group of 16 rows, few warps; two to an SM hide each other's waits)."""
-    tiles = n_seqs * -(-heads // 32)
-    return max(1, min(64, (2 * sm_count()) // max(tiles, 1)))
+#: sequences a step of single tokens may have for the streaming kernel
+LATENT_DECODE_MAX_SEQS = 1024
+
+
+def latent_decode(qa, out, heads, rank, rd, cache, page_table, page_size, seq_start, seq_slot, window=None, cache_bytes: int = 0):
+    """bfloat16 latent attention of single tokens: row b of ``qa`` [B, heads * (rank + rd)] at position seq_start[b] of
+    the sequence in slot seq_slot[b], over the paged rows streamed through shared memory by one CTA an SM."""
+    _cuda(qa, out, cache, page_table, seq_start, seq_slot)
+    if not latent_attention_mma_usable(qa.dtype, rank, rd, page_size):
+        raise KernelError(f"latent_decode: latent {rank} + {rd}, pages of {page_size} or {qa.dtype} not supported")
+    n = qa.shape[0]
+    assert qa.stride(-1) == 1 and out.stride(-1) == 1 and out.dtype == cache.dtype == torch.bfloat16 and cache.is_contiguous()
+    assert qa.shape[1] == heads * (rank + rd) and out.shape == (n, heads * rank) and cache.shape[-1] == rank + rd
+    assert seq_start.numel() == seq_slot.numel() == n
+    ctas, defines = sm_count(), (("GB_LATENT_RANK", rank), ("GB_LATENT_ROT", rd))
+    # parts of a CTA's first and last list (gb_latent_decode_scratch)
+    need = ctas * 2 * (32 if heads > 16 else 16) * (rank + 4)
+    part = _latent_scratch.get(qa.device.index)
+    if part is None or part.numel() < need:
+        if part is not None:
+            _outgrown.append(part)        # a captured step may still point at it: never freed
+        part = _latent_scratch[qa.device.index] = torch.empty(max(need, 1 << 20), dtype=torch.float32, device=qa.device)
+    f = _fn("latent_attention_mma", "gb_latent_decode",
+            [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p, c_int, c_int,
+             c_int, c_int, c_int, c_int, c_void_p], defines=defines)
+    _check(f(qa.data_ptr(), qa.stride(0), out.data_ptr(), out.stride(0), part.data_ptr(), cache.data_ptr(), page_table.data_ptr(),
+             page_table.shape[1], page_size, seq_start.data_ptr(), seq_slot.data_ptr(), n, heads, rank, rd, window or 0, ctas,
+             _stream()), "latent_decode", "attention", _nbytes(qa, out) + cache_bytes)
+    count_launches(1)   # the merge kernel
 
 
 def latent_attention(ctx, qa, out, heads, rank, rd, cache, page_table, page_size, window=None):
@@ -1075,9 +1088,11 @@ def latent_attention(ctx, qa, out, heads, rank, rd, cache, page_table, page_size
         for start, n in zip(ctx.host["seq_start"], ctx.host["seq_len"]):
             cached += per_pos * (min(start + n, window + n - 1) if window else start + n)
     if latent_attention_mma_usable(qa.dtype, rank, rd, page_size) and qa.stride(0) % 8 == 0:
-        ksplits = latent_decode_splits(ctx.n_seqs, heads) if ctx.max_new <= 1 else 1
+        if ctx.max_new <= 1 and ctx.n_seqs == qa.shape[0] <= LATENT_DECODE_MAX_SEQS:
+            latent_decode(qa, out, heads, rank, rd, cache, page_table, page_size, ctx.seq_start, ctx.seq_slot, window, cached)
+            return
         latent_attention_mma(qa, out, heads, rank, rd, cache, page_table, page_size, ctx.cu_seqlens, ctx.seq_start,
-                             ctx.seq_slot, ctx.max_new, window, ksplits, cache_bytes=cached)
+                             ctx.seq_slot, ctx.max_new, window, cache_bytes=cached)
         return
     latent_attention_ref(qa, out, heads, rank, rd, cache, page_table, page_size, ctx.tok_pos, ctx.tok_seq, ctx.seq_slot,
                          window, cache_bytes=cached)

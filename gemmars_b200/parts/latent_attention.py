@@ -230,7 +230,7 @@ class LatentAttention(Part):
         q[:, :, vd + dim:] = qa.view(t, nh, r + rd)[:, :, r:]
         o = torch.empty((t, nh * vd), dtype=self.act_dtype, device=q_nope.device)
         kernels.latent_attention_mma(q.view(t, nh * kd), o, nh, vd, dim + rd, rows, None, 64, ctx.cu_seqlens, ctx.seq_start,
-                                     ctx.seq_slot, ctx.max_new, self.window, 1, head_stride=hs, out_scale=gate, out_gate=channel)
+                                     ctx.seq_slot, ctx.max_new, self.window, head_stride=hs, out_scale=gate, out_gate=channel)
         self.o.add_into(o, residual)
 
 
