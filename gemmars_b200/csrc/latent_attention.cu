@@ -18,7 +18,7 @@
 // attention itself one (token, head) per block (gb_latent_attention_ref), and the stand-alone
 // rotation of interleaved pairs (gb_rope_pairs).  The arithmetic for one (token, head) depends on
 // its position and the cache alone, so prompts, single tokens and any batch give the same bits.
-#include "common.cuh"
+#include "mma.cuh"
 
 // Rotation of a pair (u, v) -> (u cos - v sin, v cos + u sin), angle = float(pos) * inv_freq[i], all in
 // float32, cosine and sine times `mag`.  Pair i < rot/2 is dims (2i, 2i+1), or with the half layout (i, i + rot/2).
@@ -43,9 +43,16 @@ struct Copy {
   const int* cu;
 };
 
+template <typename T> __device__ __forceinline__ void store4(T* to, float a, float b, float c, float d);
+template <> __device__ __forceinline__ void store4<float>(float* to, float a, float b, float c, float d) { *(float4*)to = make_float4(a, b, c, d); }
+template <> __device__ __forceinline__ void store4<bf16>(bf16* to, float a, float b, float c, float d) {
+  const __nv_bfloat162 p = __floats2bfloat162_rn(a, b), q = __floats2bfloat162_rn(c, d);
+  *(uint2*)to = make_uint2(*(const uint32_t*)&p, *(const uint32_t*)&q);
+}
+
 // One block per token.  Inputs are the float32 results of the layer's projections.  A token's angles are taken once
-// into shared memory, for the key part and all heads (16 heads of 64 rotated dims, 2,048 tokens: 22 us with a sine and
-// cosine for every pair of every head).
+// into shared memory, for the key part and all heads.  `wide` (interleaved pairs, everything in fours): a head a warp, four
+// dims a lane (16 heads of 64 rotated dims: 2,048 tokens 22 -> 20.9 us, 16 tokens 8.5 -> 7.3 us).
 template <typename T>
 __global__ void __launch_bounds__(256) latent_prepare_kernel(
     const float* __restrict__ q_in, long long ldq, const float* __restrict__ kv_in, long long ldkv,
@@ -54,7 +61,7 @@ __global__ void __launch_bounds__(256) latent_prepare_kernel(
     T* __restrict__ q_lat, long long ldql, float* __restrict__ gate, T* __restrict__ cache,
     const int* __restrict__ page_table, int table_width, int page_size, const int* __restrict__ tok_pos,
     const int* __restrict__ tok_seq, const int* __restrict__ seq_slot, int H, int dim, int rd, int rank,
-    Copy<T> ex, int half_layout, float rot_mag) {
+    Copy<T> ex, int half_layout, float rot_mag, int wide) {
   extern __shared__ float2 turn[];          // [rot / 2] cosine and sine
   __shared__ float scratch[34];
   pdl_release_next();
@@ -109,6 +116,26 @@ __global__ void __launch_bounds__(256) latent_prepare_kernel(
   // head's own row
   const float* q = q_in + (size_t)t * ldq;
   const int qd = dim + rd, rot_at = ex.cu ? dim : rank, nope_head = ex.cu ? qd : dim, lat_head = rot_at + rd;
+  if (wide) {       // four neighbouring dims a lane, a head a warp
+    for (int h = tid >> 5; h < H; h += 8)
+      for (int d = (tid & 31) * 4; d < qd; d += 128) {
+        const float4 v = *(const float4*)(q + h * qd + d);
+        float o[4] = {v.x, v.y, v.z, v.w};
+        const bool turned = d >= dim;
+        if (turned) {
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const int i = (d - dim) / 2 + e;
+            if (2 * i < rot) rotate_pair(o[2 * e], o[2 * e + 1], turn[i], o[2 * e], o[2 * e + 1]);
+          }
+        }
+        T* dst = turned ? q_lat + (size_t)t * ldql + (size_t)h * lat_head + rot_at + d - dim : q_nope + (size_t)t * ldqn + (size_t)h * nope_head + d;
+        store4(dst, o[0] * q_scale, o[1] * q_scale, o[2] * q_scale, o[3] * q_scale);
+      }
+    if (g_in != nullptr)
+      for (int h = tid; h < H; h += blockDim.x) gate[(size_t)t * H + h] = 1.0f / (1.0f + expf(-g_in[(size_t)t * ldg + h]));
+    return;
+  }
   for (int e = tid; e < H * dim; e += blockDim.x) {
     const int h = e / dim, d = e % dim;
     q_nope[(size_t)t * ldqn + (size_t)h * nope_head + d] = from_f32<T>(q[h * qd + d] * q_scale);
@@ -140,11 +167,16 @@ GB_EXPORT int gb_latent_prepare(const float* q_in, long long ldq, const float* k
   if (H <= 0 || dim < 0 || rd < 0 || rank <= 0 || rot < 0 || rot > rd || (rot & 1) || rot > 8192) return GB_ERR_SIZE;
   if (rot > 0 && inv_freq == nullptr) return GB_ERR_ARG;
   if (cu != nullptr && latents == nullptr) return GB_ERR_ARG;
+  const int qd = dim + rd, head_end = (cu ? dim : rank) + rd;
+  const int elem = dtype == GB_F32 ? 16 : 8;          // bytes of four results
+  const int wide = (rot == 0 || !half_layout) && dim % 4 == 0 && rd % 4 == 0 && rank % 4 == 0 && ldq % 4 == 0 && ldqn % 4 == 0 &&
+                   ldql % 4 == 0 && head_end % 4 == 0 && ((uintptr_t)q_in & 15) == 0 &&
+                   ((uintptr_t)q_nope % elem) == 0 && ((uintptr_t)q_lat % elem) == 0 && qd > 0;
 #define LAUNCH(T)                                                                                                     \
   gb_launch(latent_prepare_kernel<T>, dim3(ntok), dim3(256), (size_t)(rot / 2) * sizeof(float2), stream, q_in, ldq, kv_in, ldkv, \
             g_in, ldg, norm_w, eps, inv_freq, rot, q_scale, (T*)q_nope, ldqn, (T*)q_lat, ldql, gate, (T*)cache, page_table, \
             table_width, page_size, tok_pos, tok_seq, seq_slot, H, dim, rd, rank, Copy<T>{(T*)latents, (T*)rotated, ldl, ldr, cu}, \
-            half_layout, rot_mag)
+            half_layout, rot_mag, wide)
   if (dtype == GB_F32) LAUNCH(float);
   else if (dtype == GB_BF16) LAUNCH(bf16);
   else return GB_ERR_DTYPE;
@@ -208,6 +240,87 @@ __global__ void __launch_bounds__(256) heads_gemm_kernel(const TI* __restrict__ 
       y[(size_t)gm * ldy_t + (size_t)h * ldy_h + gn] = from_f32<TO>(acc[i][j] * s * open);
     }
   }
+}
+
+// The same in bfloat16 for a few rows (a step of single tokens): mma.sync on operands straight from memory.  A CTA is one
+// head and 16 NSP columns; its eight warps deal the inner dimension, in blocks of 32, to KSP of them (a lane's 16 bytes are
+// its share of a block in both operands), and their sums meet in shared memory in warp order.  The first blocks of the
+// matrices are asked for before the kernel before this one has ended.  Bound by one round trip for the matrices and one for
+// the rows: 16 tokens, 16 heads, 128 -> 512 and 512 -> 128: 8.3 us each on the grouped product's tiles of 128 rows, 2.8 and 2.6 so.
+template <int KSP>
+__global__ void __launch_bounds__(256) heads_few_kernel(const bf16* __restrict__ x, long long ldx_t, long long ldx_h,
+                                                        const bf16* __restrict__ w, bf16* __restrict__ y, long long ldy_t, long long ldy_h,
+                                                        const float* __restrict__ scale, int M, int H, int N, int K,
+                                                        const float* __restrict__ gate, long long ldg) {
+  constexpr int NSP = 8 / KSP, AHEAD = 2;
+  __shared__ float sums[8][16][17];
+  pdl_release_next();
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, c = lane & 3;
+  const int h = blockIdx.y, n0 = (blockIdx.x * NSP + warp / KSP) * 16, kw = warp % KSP, blocks = K / 32;
+  const bf16* wrow = w + ((size_t)h * N + n0 + g) * K + 8 * c;
+  const bool in0 = n0 + g < N, in1 = n0 + 8 + g < N;
+  auto weights = [&](int kb, uint4 (&v)[2]) {
+    const uint4 zero = make_uint4(0, 0, 0, 0);
+    v[0] = in0 && kb < blocks ? *(const uint4*)(wrow + kb * 32) : zero;
+    v[1] = in1 && kb < blocks ? *(const uint4*)(wrow + (size_t)8 * K + kb * 32) : zero;
+  };
+  uint4 first[AHEAD][2];
+#pragma unroll
+  for (int i = 0; i < AHEAD; ++i) weights(kw + i * KSP, first[i]);
+  pdl_wait_prior();
+  for (int m0 = 0; m0 < M; m0 += 16) {
+    const bool a0 = m0 + g < M, a1 = m0 + g + 8 < M;
+    const bf16* r0 = x + (size_t)(a0 ? m0 + g : 0) * ldx_t + (size_t)h * ldx_h + 8 * c;
+    const bf16* r1 = x + (size_t)(a1 ? m0 + g + 8 : 0) * ldx_t + (size_t)h * ldx_h + 8 * c;
+    float acc[2][4] = {};
+    auto block = [&](int kb, const uint4 (&v)[2]) {
+      const uint4 p = *(const uint4*)(r0 + kb * 32), q = *(const uint4*)(r1 + kb * 32);     // rows beyond M are not stored
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        mma16816(acc[j], p.x, q.x, p.y, q.y, v[j].x, v[j].y);
+        mma16816(acc[j], p.z, q.z, p.w, q.w, v[j].z, v[j].w);
+      }
+    };
+#pragma unroll
+    for (int i = 0; i < AHEAD; ++i)
+      if (kw + i * KSP < blocks) block(kw + i * KSP, first[i]);
+    for (int kb = kw + AHEAD * KSP; kb < blocks; kb += KSP) {
+      uint4 v[2];
+      weights(kb, v);
+      block(kb, v);
+    }
+    __syncthreads();                    // the rows before have left
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) sums[warp][g + 8 * (e >> 1)][8 * j + 2 * c + (e & 1)] = acc[j][e];
+    __syncthreads();
+    for (int e = tid; e < 256 * NSP; e += 256) {
+      const int part = e >> 8, r = (e >> 4) & 15, col = e & 15, m = m0 + r, n = (blockIdx.x * NSP + part) * 16 + col;
+      if (m >= M || n >= N) continue;
+      float v = 0.f;
+#pragma unroll
+      for (int k = 0; k < KSP; ++k) v += sums[part * KSP + k][r][col];
+      if (scale) v *= scale[(size_t)m * H + h];
+      if (gate) v *= 1.0f / (1.0f + expf(-gate[(size_t)m * ldg + (size_t)h * N + n]));
+      y[(size_t)m * ldy_t + (size_t)h * ldy_h + n] = __float2bfloat16_rn(v);
+    }
+  }
+}
+
+// x: [M, H, K], w: [H, N, K], y: [M, H, N] bfloat16; K a multiple of 32, x and w rows at 16-byte boundaries.
+GB_EXPORT int gb_heads_few(const void* x, long long ldx_t, long long ldx_h, const void* w, void* y, long long ldy_t, long long ldy_h,
+                           const float* scale, int M, int H, int N, int K, const float* gate, long long ldg, cudaStream_t stream) {
+  if (M <= 0 || H <= 0 || N <= 0) return 0;
+  if (K <= 0 || K % 32 || H > 65535 || ldx_t % 8 || ldx_h % 8 || (((uintptr_t)x | (uintptr_t)w) & 15)) return GB_ERR_SIZE;
+#define HEADS_FEW(KSP)                                                                                                \
+  gb_launch(heads_few_kernel<KSP>, dim3((N + 16 * (8 / KSP) - 1) / (16 * (8 / KSP)), H), dim3(256), 0, stream, (const bf16*)x, ldx_t, \
+            ldx_h, (const bf16*)w, (bf16*)y, ldy_t, ldy_h, scale, M, H, N, K, gate, ldg)
+  if (K >= 256) HEADS_FEW(8);
+  else if (K >= 128) HEADS_FEW(4);
+  else HEADS_FEW(2);
+#undef HEADS_FEW
+  return gb_launch_status();
 }
 
 GB_EXPORT int gb_heads_gemm(const void* x, long long ldx_t, long long ldx_h, const void* w, void* y, long long ldy_t,

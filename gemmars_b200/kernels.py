@@ -937,6 +937,14 @@ def heads_gemm(x, w, y, heads, scale=None, gate=None):
         assert gate.dtype == torch.float32 and gate.shape == (t, heads * n) and gate.stride(1) == 1
     if (x.dtype == torch.bfloat16 and k % 8 == 0 and x.stride(0) % 8 == 0 and x.stride(1) % 8 == 0
             and x.data_ptr() % 16 == 0 and t >= HEADS_GEMM_TC_MIN_TOKENS):
+        if t <= HEADS_FEW_MAX_TOKENS and k % 32 == 0 and w.data_ptr() % 16 == 0:
+            f = _fn("latent_attention", "gb_heads_few",
+                    [c_void_p, c_longlong, c_longlong, c_void_p, c_void_p, c_longlong, c_longlong, c_void_p, c_int, c_int, c_int, c_int,
+                     c_void_p, c_longlong, c_void_p])
+            _check(f(x.data_ptr(), x.stride(0), x.stride(1), w.data_ptr(), y.data_ptr(), y.stride(0), y.stride(1), _ptr(scale), t, heads,
+                     n, k, _ptr(gate), gate.stride(0) if gate is not None else 0, _stream()), "heads_few", "matmul",
+                   _nbytes(w) + t * heads * (n + k) * 2)
+            return
         grouped_gemm(x, x.stride(0), x.stride(1), None, 1, w, n * k, y, y.stride(0), y.stride(1), scale, None, heads, 1,
                      None, heads, t, t, n, k, gate=gate, gate_gstride=n, what="heads_gemm_tc", nbytes=_nbytes(w) + t * heads * (n + k) * 2)
         return
@@ -952,6 +960,8 @@ def heads_gemm(x, w, y, heads, scale=None, gate=None):
 # kernel took 20 and 58 us for the two products of a layer (16 heads, 128 -> 512 and 512 -> 128), one
 # scalar load per element and 64 x 16 blocks in turn; a nearly empty 128-row tile costs nothing here
 HEADS_GEMM_TC_MIN_TOKENS = 1
+#: rows up to which the matrices are read straight from memory, 16 rows at a time
+HEADS_FEW_MAX_TOKENS = 64
 
 
 def grouped_gemm(a, lda, a_gstride, a_rows, a_div, w, w_gstride, c, ldc, c_gstride, scale, scale_rows, s_rstride, s_gstride,

@@ -47,3 +47,22 @@ def test_single_tokens_over_streamed_rows(rank, rot, heads, lens, window):
         want = p @ seen[:, :rank]
         # weights rounded to 8 bits before their product, the result once more
         assert (out[i].double().view(heads, rank) - want).abs().max() <= 2.0 ** -7 * max(1.0, want.abs().max().item())
+
+
+@pytest.mark.parametrize("tokens", [1, 16, 17, 40, 64, 65])
+@pytest.mark.parametrize("heads,n,kk", [(3, 64, 128), (16, 40, 512), (2, 512, 32), (5, 8, 96), (4, 100, 64)])
+@pytest.mark.parametrize("gated", [False, True])
+def test_products_of_few_rows_per_head(tokens, heads, n, kk, gated):
+    from gemmars_b200 import kernels as k
+    torch.manual_seed(tokens + n)
+    x = torch.randn(tokens, heads, kk + 16, device=DEV).bfloat16()[:, :, 8:8 + kk]
+    w = (torch.randn(heads, n, kk, device=DEV) * kk ** -0.5).bfloat16()
+    y = torch.zeros(tokens, heads, n + 24, device=DEV, dtype=torch.bfloat16)
+    scale = torch.rand(tokens, heads, device=DEV)
+    gate = torch.randn(tokens, heads * n + 4, device=DEV)[:, 4:] if gated else None
+    k.heads_gemm(x, w, y[:, :, :n], heads, scale=scale, gate=gate)
+    want = torch.einsum("thk,hnk->thn", x.double(), w.double()) * scale.double()[..., None]
+    if gated:
+        want = want * torch.sigmoid(gate.double()).view(tokens, heads, n)
+    assert (y[:, :, :n].double() - want).abs().max() <= 2.0 ** -8 * want.abs().max() + 1e-5
+    assert not y[:, :, n:].any()
