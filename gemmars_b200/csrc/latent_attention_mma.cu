@@ -311,9 +311,11 @@ struct Decode {
   static constexpr int MEET = (KG - 1) * NSPLIT * GROUPS * (DW / 2 + 4) * 32;          // floats: the teams' results
   static constexpr int FLOATS = KG * GROUPS * SX > MEET ? KG * GROUPS * SX : MEET;
   static constexpr int FIT = (227 * 1024 - FLOATS * 4 - 512 - MAX_SEQS * 4) / STAGE_BYTES;
-  static constexpr int STAGES = FIT > 16 ? 16 : FIT;
+  // A place in the ring belongs to one team: whoever waits for a tile has then had the tile before it in that place, so
+  // that a parity never stands for the phase before the last (copies may arrive out of their order).
+  static constexpr int STAGES = (FIT > 16 ? 16 : FIT) / KG * KG;
   static constexpr size_t SMEM = (size_t)STAGES * STAGE_BYTES + FLOATS * 4 + 2 * STAGES * 8 + 16 + (size_t)(MAX_SEQS + 1) * 4;
-  static_assert(STAGES > KG, "a tile ahead of the teams");
+  static_assert(STAGES > KG && STAGES % KG == 0, "a tile ahead of the teams");
 };
 
 __device__ int g_latent_status;   // 0, or the first wait that ran out (1 free stage, 2 tile)
@@ -461,7 +463,7 @@ latent_decode_kernel(const bf16* __restrict__ qa, long long ldq, bf16* __restric
     float o[DW / 8][4];
 #pragma unroll
     for (int d = 0; d < DW / 8; ++d) o[d][0] = o[d][1] = o[d][2] = o[d][3] = 0.f;
-    for (int i = team; i < n; i += KG) {
+    for (int i = (team + KG - it0 % KG) % KG; i < n; i += KG) {          // tile it0 + i of the CTA: team (it0 + i) % KG
       const int st = (it0 + i) % STAGES;
       // a wait that gives up ends no loop: the warps of a team go on to meet at their barriers
       if (ok) ok = wait_or_abort(&full[st], ((it0 + i) / STAGES) & 1, abort, 2);
