@@ -847,10 +847,13 @@ constexpr int PERSISTENT_QKV_THREADS = 320, QKV_STAGING_BYTES = 65 * 1024;   // 
 // tile's rows of W are the group's (W stacks the groups' matrices, rows_per_expert each).  The gated
 // mode then applies g = min(g, limit), u = clamp(u, -limit, limit), g * sigmoid(alpha g) * (u + shift)
 // when limit > 0, and multiplies row r of the result by row_scale[r], or with `scale_in` row r of both sums
-// before the activation (an expert of the weighted input).  `act` (bfloat16 results of a
+// before the activation (an expert of the weighted input).  tile_rows[m tile] (null: all) says how many of the tile's
+// rows exist: the MMAs are as wide as those (a multiple of 16) and only those leave; what the others hold, which the
+// loads still bring, counts nothing.  `act` (bfloat16 results of a
 // product without a gate, grouped or not): an activation of every result (out_act), then the row's scale.
 struct Grouped {
   const int* tile_expert = nullptr;
+  const int* tile_rows = nullptr;
   const float* row_scale = nullptr;
   int rows_per_expert = 0;
   float limit = 0.f, alpha = 0.f, shift = 0.f;
@@ -886,7 +889,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
   constexpr uint32_t ACC_COLS = BN, TMEM_COLS = 2 * ACC_COLS;
   static_assert(TMEM_COLS == 256 || TMEM_COLS == 512, "two accumulator buffers: 256 or 512 columns");
   // bn: tokens per tile, a multiple of 16 up to BN (BN sizes the stages and the accumulators)
-  const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+  const uint32_t idesc_rest = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BM >> 4) << 24);
   const uint32_t stage_tx = A_BYTES + (uint32_t)bn * BK * 2;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -981,6 +984,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
       // that is never filled
       if (grp.tile_expert) pdl_wait_prior();
       for (TileWalk w(tiles, kb_total, split); w.more() && ok; w.next(), ++i) {
+        uint32_t width = (uint32_t)bn;
         if (grp.tile_expert) {                         // a tile no group uses: not counted, as in the other roles
           int m0, n0;
           tile_origin(w.t, tiles_m, tiles_n, bn, TILE_F, m0, n0);
@@ -988,7 +992,9 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
             --i;
             continue;
           }
+          if (grp.tile_rows) width = (uint32_t)(grp.tile_rows[m0 / bn] + 15) & ~15u;
         }
+        const uint32_t idesc = idesc_rest | (width >> 3 << 17);
         const uint32_t b = i & 1;
         if (i >= 2 && !mbar_wait(&acc_empty[b], ((i >> 1) - 1) & 1)) {   // the epilogue has read this buffer out
           atomicCAS(&g_status, ST_OK, ST_TIMEOUT_TMEM);
@@ -1036,6 +1042,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
       }
       const uint32_t b = i & 1;
       const int n = n0 + f;
+      const int m_end = grp.tile_rows ? min(M, m0 + grp.tile_rows[m0 / bn]) : M;     // the tile's rows that exist
       bool have = __all_sync(0xffffffffu, mbar_wait(&acc_full[b], (i >> 1) & 1));
       if (!have && lane == 0) atomicCAS(&g_status, ST_OK, ST_TIMEOUT_TMEM);
       if (GATED || QKV) {   // the warps meet at barriers below: they leave together or not at all
@@ -1072,7 +1079,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
       const uint32_t acc = tmem + ((uint32_t)(quarter * 32) << 16) + b * ACC_COLS;
 #pragma unroll 1
       for (int c = QKV ? 32 * group : 0; c < bn; c += QKV ? 64 : (both ? 32 : 16)) {
-        if (m0 + c >= M) break;
+        if (m0 + c >= m_end) break;
         uint32_t v[16], v2[16];
         tc_ld16(acc + c, v);
         if (both) tc_ld16(acc + c + 16, v2);
@@ -1090,7 +1097,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
             if (grp.scale_in) {
 #pragma unroll
               for (int j = 0; j < 16; ++j) {
-                const float sc = row + j < M ? grp.row_scale[row + j] : 0.f;
+                const float sc = row + j < m_end ? grp.row_scale[row + j] : 0.f;
                 const float gs = __uint_as_float(g[j]) * sc, us = __uint_as_float(u[j]) * sc;
                 r[j] = grp.limit > 0.f ? clamped_gate(gs, us, grp) : silu_mul(gs, us);
               }
@@ -1104,7 +1111,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
             }
             if (grp.row_scale && !grp.scale_in) {
 #pragma unroll
-              for (int j = 0; j < 16; ++j) r[j] *= row + j < M ? grp.row_scale[row + j] : 0.f;
+              for (int j = 0; j < 16; ++j) r[j] *= row + j < m_end ? grp.row_scale[row + j] : 0.f;
             }
             if (y_tma) {
               uint8_t* p = tile_out.next(lane);
@@ -1114,7 +1121,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
             } else if (n < N) {
 #pragma unroll
               for (int j = 0; j < 16; ++j)
-                if (row + j < M) emit<MODE>(y, (size_t)(row + j) * ldy + n, r[j]);
+                if (row + j < m_end) emit<MODE>(y, (size_t)(row + j) * ldy + n, r[j]);
             }
           }
         } else if (QKV) {
@@ -1128,8 +1135,8 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
         } else {
           float b_out = bv;
           if (MODE == EPI_STORE_BF16 && grp.act) {
-            act_rows(v, bv, grp.act, grp.row_scale, m0 + c, M);
-            if (both) act_rows(v2, bv, grp.act, grp.row_scale, m0 + c + 16, M);
+            act_rows(v, bv, grp.act, grp.row_scale, m0 + c, m_end);
+            if (both) act_rows(v2, bv, grp.act, grp.row_scale, m0 + c + 16, m_end);
             b_out = 0.f;
           }
           if (MODE == EPI_ACCUMULATE_F32 && tail.col_scale) {
@@ -1139,8 +1146,8 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
           if (y_tma) {
             tile_out.send(v, v2, both, b_out, lane, n0 + warp * 32, m0 + c, N);
           } else {
-            store_direct<MODE>(y, ldy, v, b_out, m0 + c, M, n, N);
-            if (both) store_direct<MODE>(y, ldy, v2, b_out, m0 + c + 16, M, n, N);
+            store_direct<MODE>(y, ldy, v, b_out, m0 + c, m_end, n, N);
+            if (both) store_direct<MODE>(y, ldy, v2, b_out, m0 + c + 16, m_end, n, N);
           }
         }
       }
@@ -1489,10 +1496,11 @@ GB_EXPORT int gb_gemm_tc_persistent(const void* x, const void* w, const float* b
 // w stacks `experts` matrices of N rows (2 N gated: gate rows, then up rows); tile_expert [M / bn].
 // mode 1: y float32 [M, N] = x W_g^T; mode 3: y bfloat16 [M, N] = row_scale * act(gate, up), act the
 // clamped form when limit > 0, or with scale_in act(row_scale * gate, row_scale * up); mode 0: y bfloat16 [M, N] = row_scale * act(x W_g^T) (no gate rows in w;
-// act 1: the exact GELU, 2: the square of relu).  bn: 128 or 256.
+// act 1: the exact GELU, 2: the square of relu).  bn: 128 or 256.  tile_rows [M / bn]: how many of a tile's rows exist
+// (null: all); the others' results are not written, or not to be read.
 GB_EXPORT int gb_gemm_tc_grouped(const void* x, const void* w, void* y, int mode, int M, int N, int K, long long ldx,
-                                 long long ldy, int bn, int ctas, int experts, const int* tile_expert, const float* row_scale,
-                                 float limit, float alpha, float shift, int act, int scale_in, cudaStream_t stream) {
+                                 long long ldy, int bn, int ctas, int experts, const int* tile_expert, const int* tile_rows,
+                                 const float* row_scale, float limit, float alpha, float shift, int act, int scale_in, cudaStream_t stream) {
   if (M <= 0 || N <= 0 || experts <= 0) return 0;
   if (act < OUT_ACT_NONE || act > OUT_ACT_RELU2) return GB_ERR_ARG;
   if (K <= 0 || (K % 8) || (ldx % 8) || ((uintptr_t)x & 15) || ((uintptr_t)w & 15) || ctas <= 0) return GB_ERR_SIZE;
@@ -1501,6 +1509,7 @@ GB_EXPORT int gb_gemm_tc_grouped(const void* x, const void* w, void* y, int mode
   if (!gated && mode != EPI_STORE_F32 && mode != EPI_STORE_BF16) return GB_ERR_ARG;
   Grouped grp;
   grp.tile_expert = tile_expert;
+  grp.tile_rows = tile_rows;
   grp.row_scale = (gated || mode == EPI_STORE_BF16) ? row_scale : nullptr;
   grp.rows_per_expert = N * (gated ? 2 : 1);
   grp.limit = limit; grp.alpha = alpha; grp.shift = shift;

@@ -1295,24 +1295,12 @@ def moe_experts_plain_tc(h, idx, wts, w_up, w_down, residual, act="gelu", col_sc
     _cuda(h, idx, wts, w_up, w_down, residual)
     t, width = h.shape
     e, ff, _ = w_up.shape
-    top, bn = idx.shape[1], MOE_TC_TILE
-    entries = t * top
-    rows = (-(-entries // bn) + e) * bn
-    meta = torch.empty(rows // bn + entries + rows, dtype=torch.int32, device=h.device)
-    tile_expert, place, row_entry = meta[:rows // bn], meta[rows // bn:rows // bn + entries], meta[rows // bn + entries:]
-    f = _fn("grouped_gemm", "gb_moe_sort_padded", [c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p])
-    _check(f(idx.data_ptr(), entries, e, bn, rows, tile_expert.data_ptr(), place.data_ptr(), row_entry.data_ptr(), _stream()),
-           "moe_sort", "elementwise", 3 * entries * 4)
-    xp = torch.empty((rows, width), dtype=torch.bfloat16, device=h.device)
-    scale = torch.empty((rows,), dtype=torch.float32, device=h.device)
-    f = _fn("grouped_gemm", "gb_moe_permute", [c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int,
-                                               c_int, c_int, c_int, c_void_p])
-    _check(f(h.data_ptr(), h.stride(0), row_entry.data_ptr(), tile_expert.data_ptr(), wts.data_ptr(), xp.data_ptr(),
-             scale.data_ptr(), rows, width, top, bn, _stream()), "moe_permute", "elementwise", 2 * entries * width * 2)
+    top = idx.shape[1]
+    entries, bn, rows, tile_expert, tile_rows, place, xp, scale = _moe_order(h, idx, wts, e)
     y = torch.empty((rows, ff), dtype=torch.bfloat16, device=h.device)
-    gemm_tc_grouped(xp, w_up.view(e * ff, width), y, ff, e, tile_expert, scale, act=act)
+    gemm_tc_grouped(xp, w_up.view(e * ff, width), y, ff, e, tile_expert, scale, act=act, bn=bn, tile_rows=tile_rows)
     out = torch.empty((rows, width), dtype=torch.float32, device=h.device)
-    gemm_tc_grouped(y, w_down.view(e * width, ff), out, width, e, tile_expert)
+    gemm_tc_grouped(y, w_down.view(e * width, ff), out, width, e, tile_expert, bn=bn, tile_rows=tile_rows)
     _check_col_scale(col_scale, width)
     f = _fn("grouped_gemm", "gb_moe_combine", [c_void_p, c_void_p, c_void_p, c_longlong, c_int, c_int, c_int, c_void_p, c_int,
                                                 c_void_p])
@@ -1368,6 +1356,33 @@ def moe_experts_grouped(h, idx, wts, sg, w_gate_up, w_down, shared_gate_up, shar
 
 MOE_TC_MIN_TOKENS = 256
 MOE_TC_TILE = 128
+#: rows an expert has on average from which its tiles are of 256 rows instead of 128 (us, 128 / 256): 64 experts with 96 rows
+#: 326 / 343, with 192 rows 490 / 413; 128 experts with 64 rows 286 / 310, with 128 rows 382 / 351; 8 experts with 128 rows
+#: 155 / 134 (and with 64 rows 136 / 126: few tiles either way)
+MOE_WIDE_TILE_ROWS = 112
+
+
+def _moe_order(h, idx, wts, experts: int):
+    """(entries, rows a tile, rows, the tiles' experts and rows in use, every entry's row, the activations in that order, the
+    rows' weights): a prompt's (token, slot) entries ordered by expert, every expert's rows from a multiple of the tile's
+    rows on.  Rows without an entry hold whatever was there."""
+    t, width = h.shape
+    entries = idx.numel()
+    bn = 256 if entries >= MOE_WIDE_TILE_ROWS * experts else MOE_TC_TILE
+    rows = (-(-entries // bn) + experts) * bn
+    tiles = rows // bn
+    meta = torch.empty(2 * tiles + entries, dtype=torch.int32, device=h.device)
+    tile_expert, tile_rows, place = meta[:tiles], meta[tiles:2 * tiles], meta[2 * tiles:]
+    f = _fn("grouped_gemm", "gb_moe_sort_padded", [c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p])
+    _check(f(idx.data_ptr(), entries, experts, bn, rows, tile_expert.data_ptr(), tile_rows.data_ptr(), place.data_ptr(), _stream()),
+           "moe_sort", "elementwise", 3 * entries * 4)
+    xp = torch.empty((rows, width), dtype=torch.bfloat16, device=h.device)
+    scale = torch.empty((rows,), dtype=torch.float32, device=h.device)
+    f = _fn("grouped_gemm", "gb_moe_permute", [c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
+                                               c_void_p])
+    _check(f(h.data_ptr(), h.stride(0), place.data_ptr(), wts.data_ptr(), xp.data_ptr(), scale.data_ptr(), t, width, idx.shape[1],
+             _stream()), "moe_permute", "elementwise", (entries + t) * width * 2)
+    return entries, bn, rows, tile_expert, tile_rows, place, xp, scale
 
 
 def moe_tc_usable(h, w_gate_up, w_down) -> bool:
@@ -1378,14 +1393,16 @@ def moe_tc_usable(h, w_gate_up, w_down) -> bool:
 
 
 def gemm_tc_grouped(x, w, y, n, experts, tile_expert, row_scale=None, gated=False, limit=0.0, alpha=0.0, shift=0.0,
-                    bn=MOE_TC_TILE, act=None, scale_in=False):
+                    bn=MOE_TC_TILE, act=None, scale_in=False, tile_rows=None):
     """The tcgen05 product over groups of rows: x [rows, K] holds the groups one after the other, each
     starting at a multiple of ``bn`` rows; w stacks the groups' matrices ([experts * n, K], or
     [experts * 2 n, K] gated); tile_expert names the group of every tile of ``bn`` rows (-1: none).
     y float32 [rows, n], or with ``gated`` bfloat16 [rows, n] = row_scale * act(gate, up), or with
     ``act`` (one of PLAIN_ACTS) bfloat16 [rows, n] = row_scale * act(x w^T) (no gate rows).  ``scale_in``
-    (gated): act(row_scale * gate, row_scale * up)."""
-    _cuda(x, w, y, tile_expert, row_scale)
+    (gated): act(row_scale * gate, row_scale * up).  ``tile_rows`` [rows / bn] (None: all): how many of a tile's rows
+    exist; what y holds in the others is not to be read."""
+    _cuda(x, w, y, tile_expert, row_scale, tile_rows)
+    assert tile_rows is None or (tile_rows.dtype == torch.int32 and tile_rows.numel() == tile_expert.numel())
     rows, k = x.shape
     assert x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and x.stride(1) == 1 and w.is_contiguous()
     assert not (gated and act)
@@ -1393,9 +1410,9 @@ def gemm_tc_grouped(x, w, y, n, experts, tile_expert, row_scale=None, gated=Fals
     assert tile_expert.dtype == torch.int32 and tile_expert.numel() == rows // bn and rows % bn == 0
     f = _fn("gemm_tc", "gb_gemm_tc_grouped",
             [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_longlong, c_longlong, c_int, c_int, c_int, c_void_p,
-             c_void_p, c_float, c_float, c_float, c_int, c_int, c_void_p])
+             c_void_p, c_void_p, c_float, c_float, c_float, c_int, c_int, c_void_p])
     _check(f(x.data_ptr(), w.data_ptr(), y.data_ptr(), 3 if gated else (0 if act else 1), rows, n, k, x.stride(0), y.stride(0), bn,
-             sm_count(x.device), experts, tile_expert.data_ptr(), _ptr(row_scale), limit, alpha, shift, PLAIN_ACTS[act],
+             sm_count(x.device), experts, tile_expert.data_ptr(), _ptr(tile_rows), _ptr(row_scale), limit, alpha, shift, PLAIN_ACTS[act],
              1 if scale_in else 0, _stream()),
            "gemm_tc_grouped", "matmul", _nbytes(x, w, y))
 
@@ -1404,30 +1421,18 @@ def moe_experts_tc(h, idx, wts, sg, w_gate_up, w_down, shared_gate_up, shared_do
                    shift, col_scale=None, weigh_input=False, store=False):
     """As moe_experts_grouped for a prompt step, the experts' two products on the tcgen05 kernel: the
     activations are copied into an order in which every expert's rows start at a multiple of the
-    tile's tokens (zeros between), the routing weight multiplies the activation's rows, and a token's
+    tile's tokens (anything between), the routing weight multiplies the activation's rows, and a token's
     float32 rows are added into the residual in slot order."""
     _cuda(h, idx, wts, sg, w_gate_up, w_down, shared_gate_up, shared_down, residual)
     t, width = h.shape
     e, ff2, _ = w_gate_up.shape
-    ff, top, bn = ff2 // 2, idx.shape[1], MOE_TC_TILE
-    entries = t * top
-    rows = (-(-entries // bn) + e) * bn
-    meta = torch.empty(rows // bn + entries + rows, dtype=torch.int32, device=h.device)
-    tile_expert, place, row_entry = meta[:rows // bn], meta[rows // bn:rows // bn + entries], meta[rows // bn + entries:]
-    f = _fn("grouped_gemm", "gb_moe_sort_padded", [c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p])
-    _check(f(idx.data_ptr(), entries, e, bn, rows, tile_expert.data_ptr(), place.data_ptr(), row_entry.data_ptr(), _stream()),
-           "moe_sort", "elementwise", 3 * entries * 4)
-    xp = torch.empty((rows, width), dtype=torch.bfloat16, device=h.device)
-    scale = torch.empty((rows,), dtype=torch.float32, device=h.device)
-    f = _fn("grouped_gemm", "gb_moe_permute", [c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int,
-                                               c_int, c_int, c_int, c_void_p])
-    _check(f(h.data_ptr(), h.stride(0), row_entry.data_ptr(), tile_expert.data_ptr(), wts.data_ptr(), xp.data_ptr(),
-             scale.data_ptr(), rows, width, top, bn, _stream()), "moe_permute", "elementwise", 2 * entries * width * 2)
+    ff, top = ff2 // 2, idx.shape[1]
+    entries, bn, rows, tile_expert, tile_rows, place, xp, scale = _moe_order(h, idx, wts, e)
     y = torch.empty((rows, ff), dtype=torch.bfloat16, device=h.device)
     gemm_tc_grouped(xp, w_gate_up.view(e * ff2, width), y, ff, e, tile_expert, scale, gated=True, limit=limit, alpha=alpha,
-                    shift=shift, scale_in=weigh_input)
+                    shift=shift, scale_in=weigh_input, bn=bn, tile_rows=tile_rows)
     out = torch.empty((rows, width), dtype=torch.float32, device=h.device)
-    gemm_tc_grouped(y, w_down.view(e * width, ff), out, width, e, tile_expert)
+    gemm_tc_grouped(y, w_down.view(e * width, ff), out, width, e, tile_expert, bn=bn, tile_rows=tile_rows)
     _check_col_scale(col_scale, width)
     f = _fn("grouped_gemm", "gb_moe_combine", [c_void_p, c_void_p, c_void_p, c_longlong, c_int, c_int, c_int, c_void_p, c_int,
                                                 c_void_p])
