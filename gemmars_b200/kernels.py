@@ -937,7 +937,7 @@ def heads_gemm(x, w, y, heads, scale=None, gate=None):
         assert gate.dtype == torch.float32 and gate.shape == (t, heads * n) and gate.stride(1) == 1
     if (x.dtype == torch.bfloat16 and k % 8 == 0 and x.stride(0) % 8 == 0 and x.stride(1) % 8 == 0
             and x.data_ptr() % 16 == 0 and t >= HEADS_GEMM_TC_MIN_TOKENS):
-        if t <= HEADS_FEW_MAX_TOKENS and k % 32 == 0 and w.data_ptr() % 16 == 0:
+        if t <= HEADS_FEW_MAX_TOKENS and t * heads <= HEADS_FEW_MAX_ROWS and k % 32 == 0 and w.data_ptr() % 16 == 0:
             f = _fn("latent_attention", "gb_heads_few",
                     [c_void_p, c_longlong, c_longlong, c_void_p, c_void_p, c_longlong, c_longlong, c_void_p, c_int, c_int, c_int, c_int,
                      c_void_p, c_longlong, c_void_p])
@@ -960,8 +960,12 @@ def heads_gemm(x, w, y, heads, scale=None, gate=None):
 # kernel took 20 and 58 us for the two products of a layer (16 heads, 128 -> 512 and 512 -> 128), one
 # scalar load per element and 64 x 16 blocks in turn; a nearly empty 128-row tile costs nothing here
 HEADS_GEMM_TC_MIN_TOKENS = 1
-#: rows up to which the matrices are read straight from memory, 16 rows at a time
-HEADS_FEW_MAX_TOKENS = 64
+#: tokens and rows up to which matrices and rows are read straight from memory, 16 tokens at a time: against the grouped
+#: product's tiles (us, 128 -> 512 / 512 -> 128) 16 heads 8.2 / 8.2 against 10.2 / 14.3 at 16 tokens, 12.3 / 12.3 against
+#: 18.4 / 24.6 at 64, 16.4 / 16.4 against 18.4 / 24.6 at 128; 128 heads 16.4 / 14.4 against 16.4 / 16.4 at 16 tokens, but
+#: 22.5 / 18.4 against 20.5 / 18.5 at 32
+HEADS_FEW_MAX_TOKENS = 128
+HEADS_FEW_MAX_ROWS = 2048
 
 
 def grouped_gemm(a, lda, a_gstride, a_rows, a_div, w, w_gstride, c, ldc, c_gstride, scale, scale_rows, s_rstride, s_gstride,

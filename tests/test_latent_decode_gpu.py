@@ -49,7 +49,7 @@ def test_single_tokens_over_streamed_rows(rank, rot, heads, lens, window):
         assert (out[i].double().view(heads, rank) - want).abs().max() <= 2.0 ** -7 * max(1.0, want.abs().max().item())
 
 
-@pytest.mark.parametrize("tokens", [1, 16, 17, 40, 64, 65])
+@pytest.mark.parametrize("tokens", [1, 16, 17, 40, 128, 129])
 @pytest.mark.parametrize("heads,n,kk", [(3, 64, 128), (16, 40, 512), (2, 512, 32), (5, 8, 96), (4, 100, 64)])
 @pytest.mark.parametrize("gated", [False, True])
 def test_products_of_few_rows_per_head(tokens, heads, n, kk, gated):
