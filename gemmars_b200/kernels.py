@@ -1203,7 +1203,7 @@ def moe_topk(z, bias, experts, top, has_gate=False, routing="softmax_top", scale
 def moe_experts(h, idx, wts, sg, w_gate_up, w_down, shared_gate_up, shared_down, residual, limit, shared_limit, alpha,
                 shift, col_scale=None, weigh_input=False, store=False):
     """residual[t] += sum_k wts[t, k] * expert_{idx[t, k]}(h[t]) + sg[t] * shared(h[t]), token-major
-    (two kernels: gate/up with the activation, then down).  w_gate_up [E, 2 ff, width] (gate rows,
+    (two kernels: gate/up with the activation, then down; in bfloat16 by expert).  w_gate_up [E, 2 ff, width] (gate rows,
     then up rows), w_down [E, width, ff]; the shared expert's [2 ffs, width] and [width, ffs], or None.
     ``col_scale`` (float32 [width]) multiplies what is added.  ``weigh_input``: the weights multiply the
     experts' inputs, expert(wts[t, k] * h[t]).  ``store``: the result replaces the rows of ``residual``."""
@@ -1222,16 +1222,16 @@ def moe_experts(h, idx, wts, sg, w_gate_up, w_down, shared_gate_up, shared_down,
     slots = top + (1 if shared_down is not None else 0)
     y = torch.empty((t, slots, max(ff, ffs)), dtype=h.dtype, device=h.device)
     f = _fn("moe", "gb_moe_gate_up", [c_void_p, c_longlong, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int,
-                                      c_int, c_int, c_int, c_float, c_float, c_float, c_float, c_void_p, c_void_p])
+                                      c_int, c_int, c_int, c_int, c_float, c_float, c_float, c_float, c_void_p, c_void_p])
     _check(f(h.data_ptr(), h.stride(0), dtype_code(h.dtype), idx.data_ptr(), w_gate_up.data_ptr(), _ptr(shared_gate_up),
-             y.data_ptr(), t, width, ff, ffs, top, limit, shared_limit, alpha, shift, wts.data_ptr() if weigh_input else None,
-             _stream()), "moe_gate_up", "matmul",
+             y.data_ptr(), t, e, width, ff, ffs, top, limit, shared_limit, alpha, shift,
+             wts.data_ptr() if weigh_input else None, _stream()), "moe_gate_up", "matmul",
            _nbytes(h, y) + t * slots * 2 * ff * width * h.element_size())
     rows = torch.empty((t, slots, width), dtype=torch.float32, device=h.device)
     f = _fn("moe", "gb_moe_down", [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
-                                   c_longlong, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p])
+                                   c_longlong, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p])
     _check(f(y.data_ptr(), dtype_code(h.dtype), idx.data_ptr(), None if weigh_input else wts.data_ptr(), _ptr(sg),
-             w_down.data_ptr(), _ptr(shared_down), rows.data_ptr(), residual.data_ptr(), residual.stride(0), t, width, ff, ffs,
+             w_down.data_ptr(), _ptr(shared_down), rows.data_ptr(), residual.data_ptr(), residual.stride(0), t, e, width, ff, ffs,
              top, _ptr(col_scale), 1 if store else 0, _stream()),
            "moe_down", "matmul", _nbytes(y) + 2 * _nbytes(rows) + 2 * t * width * 4 + t * slots * ff * width * h.element_size())
     count_launches(1)   # the kernel that adds a token's rows
@@ -1250,14 +1250,15 @@ def moe_experts_plain(h, idx, wts, w_up, w_down, residual, act="gelu", col_scale
     assert w_up.is_contiguous() and w_down.is_contiguous() and w_down.shape == (e, width, ff) and w_up.shape[2] == width
     assert w_up.dtype == h.dtype == w_down.dtype and residual.dtype == torch.float32 and residual.stride(1) == 1
     y = torch.empty((t, top, ff), dtype=h.dtype, device=h.device)
-    f = _fn("moe", "gb_moe_up", [c_void_p, c_longlong, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p])
-    _check(f(h.data_ptr(), h.stride(0), dtype_code(h.dtype), idx.data_ptr(), w_up.data_ptr(), y.data_ptr(), t, width, ff, top,
+    f = _fn("moe", "gb_moe_up", [c_void_p, c_longlong, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int,
+                                c_void_p])
+    _check(f(h.data_ptr(), h.stride(0), dtype_code(h.dtype), idx.data_ptr(), w_up.data_ptr(), y.data_ptr(), t, e, width, ff, top,
              PLAIN_ACTS[act], _stream()), "moe_up", "matmul", _nbytes(h, y) + t * top * ff * width * h.element_size())
     rows = torch.empty((t, top, width), dtype=torch.float32, device=h.device)
     f = _fn("moe", "gb_moe_down", [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
-                                   c_longlong, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p])
+                                   c_longlong, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p])
     _check(f(y.data_ptr(), dtype_code(h.dtype), idx.data_ptr(), wts.data_ptr(), None, w_down.data_ptr(), None,
-             rows.data_ptr(), residual.data_ptr(), residual.stride(0), t, width, ff, 0, top, _ptr(col_scale),
+             rows.data_ptr(), residual.data_ptr(), residual.stride(0), t, e, width, ff, 0, top, _ptr(col_scale),
              1 if store else 0, _stream()),
            "moe_down", "matmul", _nbytes(y) + 2 * _nbytes(rows) + 2 * t * width * 4 + t * top * ff * width * h.element_size())
     count_launches(1)   # the kernel that adds a token's rows
@@ -1313,6 +1314,22 @@ def moe_experts_plain_tc(h, idx, wts, w_up, w_down, residual, act="gelu", col_sc
            "moe_combine", "elementwise", entries * width * 4 + 2 * t * width * 4)
 
 
+#: tokens up to which moe_experts takes bfloat16 experts by moe_few_kernel rather than ordered by expert on the tcgen05
+#: product (us, both products and all around them, L2 flushed; 6 of 64 experts of 1,408 and a shared one / 2 of 8 of 4,096 /
+#: 8 of 128 of 768, width 2,048): 16 tokens 198 / 97 / 171 against 245 / 118 / 196, 32 tokens 249 / 101 / 239 against
+#: 261 / 118 / 247, 48 tokens 280 / 103 / 273 against 265 / 116 / 251, 64 tokens 316 / 130 / 300 against 269 / 116 / 253
+MOE_FEW_MAX_TOKENS = 32
+
+
+def moe_few_usable(h, w_down, shared_down=None) -> bool:
+    """Whether moe_experts and moe_experts_plain work a step's bfloat16 experts by expert (see csrc/moe.cu) and should."""
+    dims = [h.shape[1], w_down.shape[2]] + ([shared_down.shape[1]] if shared_down is not None else [])
+    return (h.dtype == torch.bfloat16 and h.shape[0] <= MOE_FEW_MAX_TOKENS and all(d % 32 == 0 for d in dims)
+            and h.stride(0) % 8 == 0 and h.data_ptr() % 16 == 0)
+
+
+#: against the token-major kernels; where the tcgen05 product can be used too that is faster at every step size (6 of 64
+#: experts, us: 16 tokens 245 against 362, 64 tokens 269 against 429, 255 tokens 288 against 470)
 MOE_GROUPED_MIN_TOKENS = 16
 
 
@@ -1358,7 +1375,10 @@ def moe_experts_grouped(h, idx, wts, sg, w_gate_up, w_down, shared_gate_up, shar
     _shared_expert(h, sg, shared_gate_up, shared_down, residual, shared_limit, alpha, shift, col_scale)
 
 
+#: below MOE_TC_MIN_TOKENS tokens (steps that may be captured, each with scratch of its own) a step's padded float32 rows
+#: may take this many bytes on the tcgen05 product; the grouped product needs no padding
 MOE_TC_MIN_TOKENS = 256
+MOE_TC_SMALL_BYTES = 256 << 20
 MOE_TC_TILE = 128
 #: rows an expert has on average from which its tiles are of 256 rows instead of 128 (us, 128 / 256): 64 experts with 96 rows
 #: 326 / 343, with 192 rows 490 / 413; 128 experts with 64 rows 286 / 310, with 128 rows 382 / 351; 8 experts with 128 rows
@@ -1390,9 +1410,11 @@ def _moe_order(h, idx, wts, experts: int):
 
 
 def moe_tc_usable(h, w_gate_up, w_down) -> bool:
-    """Whether a step's experts run on the tcgen05 product: a prompt's worth of tokens, operands the
-    product's TMA loads can address."""
-    return (moe_grouped_usable(h, w_gate_up, w_down) and h.shape[0] >= MOE_TC_MIN_TOKENS
+    """Whether a step's experts run on the tcgen05 product: more than a few tokens, operands the product's TMA loads can
+    address, padded rows (of at most 32 entries a token) that are not out of all proportion to the step."""
+    t, width = h.shape
+    return (moe_grouped_usable(h, w_gate_up, w_down)
+            and (t >= MOE_TC_MIN_TOKENS or (32 * t + MOE_TC_TILE * w_down.shape[0]) * width * 4 <= MOE_TC_SMALL_BYTES)
             and w_gate_up.data_ptr() % 16 == 0 and w_down.data_ptr() % 16 == 0)
 
 

@@ -143,7 +143,9 @@ class RoutedExperts(Part):
     def forward(self, ctx, h, residual):
         idx, wts, sg = self._route(h)
         if not self.gated:
-            if kernels.moe_tc_usable(h, self.gate_up, self.down):
+            if kernels.moe_few_usable(h, self.down):
+                run = kernels.moe_experts_plain
+            elif kernels.moe_tc_usable(h, self.gate_up, self.down):
                 run = kernels.moe_experts_plain_tc
             elif kernels.moe_grouped_usable(h, self.gate_up, self.down):
                 run = kernels.moe_experts_plain_grouped
@@ -154,7 +156,9 @@ class RoutedExperts(Part):
             return
         if self.shared_ff and sg is None:
             sg = torch.ones((h.shape[0],), dtype=torch.float32, device=h.device)
-        if kernels.moe_tc_usable(h, self.gate_up, self.down):
+        if kernels.moe_few_usable(h, self.down, self.shared_down):
+            run = kernels.moe_experts
+        elif kernels.moe_tc_usable(h, self.gate_up, self.down):
             run = kernels.moe_experts_tc
         elif kernels.moe_grouped_usable(h, self.gate_up, self.down):
             run = kernels.moe_experts_grouped

@@ -63,7 +63,34 @@ def _run(kernels, idx, wts, m, base, lim, weigh_input, run, rows=slice(None)):
     return res
 
 
-@pytest.mark.parametrize("tokens", [256, 331, 1030])
+@pytest.mark.parametrize("tokens", [1, 2, 8, 9, 15, 40])
+@pytest.mark.parametrize("e,top,width,ff,ffs,skew", [(8, 2, 64, 32, 0, 0.), (5, 5, 96, 160, 96, 0.), (64, 6, 256, 96, 64, 8.), (9, 1, 544, 40, 24, 0.),
+                                                     (3, 2, 72, 64, 0, 4.)])
+def test_few_tokens(tokens, e, top, width, ff, ffs, skew):
+    from gemmars_b200 import kernels
+    idx, wts, m, base = _case(tokens, e, top, width, ff, ffs, skew, tokens + e)
+    for weigh in (False, True):
+        got = _run(kernels, idx, wts, m, base, 1.5, weigh, kernels.moe_experts)
+        want, room = _want(idx, wts, m, 1.5, weigh)
+        assert ((got.double() - base.double() - want).abs() <= room).all()
+        for t in (0, tokens - 1):          # alone as in the batch
+            assert torch.equal(_run(kernels, idx, wts, m, base, 1.5, weigh, kernels.moe_experts, slice(t, t + 1))[0], got[t])
+
+
+@pytest.mark.parametrize("tokens", [1, 7, 12])
+@pytest.mark.parametrize("act", ["gelu", "relu2"])
+@pytest.mark.parametrize("width,ff", [(96, 64), (64, 72), (256, 200)])
+def test_few_tokens_without_a_gate(tokens, act, width, ff):
+    from gemmars_b200 import kernels
+    idx, wts, m, base = _case(tokens, 6, 3, width, ff, 0, 1.0, tokens + ff)
+    m["gu"] = m["gu"][:, :ff].contiguous()
+    got = base.clone()
+    kernels.moe_experts_plain(m["h"], idx, wts, m["gu"], m["d"], got, act=act)
+    want, room = _want(idx, wts, m, 1.0, False, act)
+    assert ((got.double() - base.double() - want).abs() <= room).all()
+
+
+@pytest.mark.parametrize("tokens", [16, 33, 100, 256, 331, 1030])
 @pytest.mark.parametrize("e,top,width,ff,ffs,skew", [(2, 2, 128, 64, 64, 0.), (64, 6, 256, 128, 0, 0.), (40, 2, 136, 64, 0, 9.), (7, 3, 128, 192, 128, 3.)])
 @pytest.mark.parametrize("weigh", [False, True])
 def test_prompts_in_padded_tiles(tokens, e, top, width, ff, ffs, skew, weigh):
