@@ -291,15 +291,16 @@ latent_attention_mma_kernel(const bf16* __restrict__ qa, long long ldq, bf16* __
 // Decoding reads every cached row once for all heads, so it is a stream of key tiles, and its time is how steadily
 // every SM pulls its share.  The tiles to read (KT keys of one sequence, for 16 GROUPS of its heads) are one flat list,
 // sequence by sequence; CTA i of G takes the tiles [i P / G, (i + 1) P / G) whatever the lengths.  A producer warp asks
-// for a tile a row a lane (one bulk copy a row, into rows pitched against bank conflicts) up to STAGES tiles ahead of
+// for a tile in TMA boxes of KT rows x 128 bytes (swizzled, against bank conflicts) up to STAGES tiles ahead of
 // KG teams of warps that take the tiles in turn, each with a softmax of its own; the teams meet at the end of a
 // segment (the part of one sequence's list in the CTA's range), in their order.  A whole list is written out, a part
 // goes to one of the CTA's two scratch places and latent_decode_merge_kernel adds the parts in key order: the same
 // bits every run.  Every wait is bounded; one that runs out sets the status word and the CTA's abort flag.
 // 16 sequences of 5,330 to 8,000 keys, 16 heads, rows of 512 + 64 (121 MB): 49 + 6 us with the keys dealt to 18 CTAs a
-// sequence by the kernel above, two tiles in flight and a barrier of the block a tile; 37.5 + 6.5 us so.
+// sequence by the kernel above, two tiles in flight and a barrier of the block a tile; 37.5 + 6.5 us with a bulk copy a row,
+// 30 + 6.5 us so (boxes of 32 rows x 128 bytes: 9 requests a tile instead of 32).
 constexpr int KT = 32;
-constexpr int ROW_BYTES = KD * 2, STAGE_BYTES = KT * LDS * 2;
+constexpr int BOXES = (KD + 63) / 64, BOX_BYTES = KT * 128, STAGE_BYTES = BOXES * BOX_BYTES;
 constexpr int MAX_SEQS = 1024;
 template <int GROUPS>
 struct Decode {
@@ -310,11 +311,11 @@ struct Decode {
   static constexpr int SX = NSPLIT > 1 ? NSPLIT * 16 * SXP + NSPLIT * 16 + 16 * PP / 2 : 0;
   static constexpr int MEET = (KG - 1) * NSPLIT * GROUPS * (DW / 2 + 4) * 32;          // floats: the teams' results
   static constexpr int FLOATS = KG * GROUPS * SX > MEET ? KG * GROUPS * SX : MEET;
-  static constexpr int FIT = (227 * 1024 - FLOATS * 4 - 512 - MAX_SEQS * 4) / STAGE_BYTES;
+  static constexpr int FIT = (227 * 1024 - FLOATS * 4 - 512 - MAX_SEQS * 4 - 1024) / STAGE_BYTES;
   // A place in the ring belongs to one team: whoever waits for a tile has then had the tile before it in that place, so
   // that a parity never stands for the phase before the last (copies may arrive out of their order).
   static constexpr int STAGES = (FIT > 16 ? 16 : FIT) / KG * KG;
-  static constexpr size_t SMEM = (size_t)STAGES * STAGE_BYTES + FLOATS * 4 + 2 * STAGES * 8 + 16 + (size_t)(MAX_SEQS + 1) * 4;
+  static constexpr size_t SMEM = 1024 + (size_t)STAGES * STAGE_BYTES + FLOATS * 4 + 2 * STAGES * 8 + 16 + (size_t)(MAX_SEQS + 1) * 4;
   static_assert(STAGES > KG && STAGES % KG == 0, "a tile ahead of the teams");
 };
 
@@ -356,12 +357,13 @@ __device__ __forceinline__ int seq_of(const int* prefix, int n, int p) {      //
 // part: [G * 2][ROWS][PART].
 template <int GROUPS>
 __global__ void __launch_bounds__(Decode<GROUPS>::WARPS * 32 + 32, 1)
-latent_decode_kernel(const bf16* __restrict__ qa, long long ldq, bf16* __restrict__ out, long long ldo, float* __restrict__ part,
-                     const bf16* __restrict__ cache, const int* __restrict__ page_table, int table_width, int page_size,
+latent_decode_kernel(const __grid_constant__ CUtensorMap rows, const bf16* __restrict__ qa, long long ldq, bf16* __restrict__ out,
+                     long long ldo, float* __restrict__ part, const int* __restrict__ page_table, int table_width, int page_size,
                      const int* __restrict__ seq_start, const int* __restrict__ seq_slot, int n_seqs, int H, int window) {
   using D = Decode<GROUPS>;
   constexpr int KG = D::KG, SXP = D::SXP, NB = KT / 8, STAGES = D::STAGES;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
+  extern __shared__ __align__(16) unsigned char smem_any[];
+  unsigned char* smem_raw = smem_any + ((1024 - (smem_u32(smem_any) & 1023)) & 1023);      // the boxes' swizzle counts from there
   float* shared = (float*)(smem_raw + (size_t)STAGES * STAGE_BYTES);
   uint64_t* full = (uint64_t*)(shared + D::FLOATS);
   uint64_t* empty = full + STAGES;
@@ -418,12 +420,10 @@ latent_decode_kernel(const bf16* __restrict__ qa, long long ldq, bf16* __restric
         const int st = it % STAGES;
         if (it >= STAGES) ok = __all_sync(0xffffffffu, wait_or_abort(&empty[st], (it / STAGES - 1) & 1, abort, 1));
         if (!ok) break;
-        if (lane == 0) mbar_expect_tx(&full[st], KT * ROW_BYTES);
+        if (lane == 0) mbar_expect_tx(&full[st], STAGE_BYTES);
         __syncwarp();
-        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                         smem_u32(smem_raw + (size_t)st * STAGE_BYTES + (size_t)lane * LDS * 2)),
-                     "l"(cache + (row + lane) * KD), "r"(ROW_BYTES), "r"(smem_u32(&full[st]))
-                     : "memory");
+        for (int x = lane; x < BOXES; x += 32)
+          tma_load_2d(smem_raw + (size_t)st * STAGE_BYTES + (size_t)x * BOX_BYTES, &rows, x * 64, (int)row, &full[st]);
       }
     }
     pdl_release_next();
@@ -436,6 +436,9 @@ latent_decode_kernel(const bf16* __restrict__ qa, long long ldq, bf16* __restric
   float* tops = mine + NSPLIT * 16 * SXP;
   bf16* weights = (bf16*)(tops + NSPLIT * 16);
   const int bar = 2 + team * GROUPS + rg;
+  // Where in a tile (boxes of KT rows x 128 bytes, their 16-byte pieces swizzled by the row) this lane's share of a piece lies
+  auto piece = [&](int row, int at) { return (at >> 3) * BOX_BYTES + row * 128 + (((at & 7) ^ (row & 7)) << 4); };
+  const int k_row = (lane & 7) + 8 * (lane >> 4), v_row = (lane & 7) + 8 * ((lane >> 3) & 1);
   bool ok = true;
   int it0 = 0, seg = 0;
   for (int p = p0; p < p1;) {
@@ -468,11 +471,10 @@ latent_decode_kernel(const bf16* __restrict__ qa, long long ldq, bf16* __restric
       // a wait that gives up ends no loop: the warps of a team go on to meet at their barriers
       if (ok) ok = wait_or_abort(&full[st], ((it0 + i) / STAGES) & 1, abort, 2);
       ok = __all_sync(0xffffffffu, ok);
-      const bf16* kt = (const bf16*)(smem_raw + (size_t)st * STAGE_BYTES);
+      const unsigned char* kt = smem_raw + (size_t)st * STAGE_BYTES;
       float s[NB][4];
 #pragma unroll
       for (int j = 0; j < NB; ++j) s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.f;
-      const bf16* k_lane = kt + (size_t)((lane & 7) + 8 * (lane >> 4)) * LDS + 8 * ((lane >> 3) & 1);
 #pragma unroll
       for (int x = 0; x < KSW; ++x) {
         const int ks = w * KSW + x;
@@ -480,7 +482,7 @@ latent_decode_kernel(const bf16* __restrict__ qa, long long ldq, bf16* __restric
 #pragma unroll
           for (int j = 0; j < NB; j += 2) {
             uint32_t kb[4];
-            ldsm_x4(kb, k_lane + (size_t)j * 8 * LDS + ks * 16);
+            ldsm_x4(kb, (const bf16*)(kt + j * 8 * 128 + piece(k_row, 2 * ks + ((lane >> 3) & 1))));
             mma16816(s[j], qf[x][0], qf[x][1], qf[x][2], qf[x][3], kb[0], kb[1]);
             mma16816(s[j + 1], qf[x][0], qf[x][1], qf[x][2], qf[x][3], kb[2], kb[3]);
           }
@@ -566,13 +568,12 @@ latent_decode_kernel(const bf16* __restrict__ qa, long long ldq, bf16* __restric
 #pragma unroll
         for (int d = 0; d < DW / 8; ++d) { o[d][0] *= alpha0; o[d][1] *= alpha0; o[d][2] *= alpha1; o[d][3] *= alpha1; }
       }
-      const bf16* v_lane = kt + (size_t)((lane & 7) + 8 * ((lane >> 3) & 1)) * LDS + w * DW + 8 * (lane >> 4);
 #pragma unroll
       for (int kk = 0; kk < KT / 16; ++kk) {
 #pragma unroll
         for (int db = 0; db < DW / 16; ++db) {
           uint32_t vb[4];
-          ldsm_x4_t(vb, v_lane + (size_t)kk * 16 * LDS + db * 16);
+          ldsm_x4_t(vb, (const bf16*)(kt + kk * 16 * 128 + piece(v_row, w * (DW / 8) + 2 * db + (lane >> 4))));
           mma16816(o[2 * db], pk[2 * kk][0], pk[2 * kk][1], pk[2 * kk + 1][0], pk[2 * kk + 1][1], vb[0], vb[1]);
           mma16816(o[2 * db + 1], pk[2 * kk][0], pk[2 * kk][1], pk[2 * kk + 1][0], pk[2 * kk + 1][1], vb[2], vb[3]);
         }
@@ -752,7 +753,7 @@ __global__ void __launch_bounds__(128) latent_decode_merge_kernel(const float* _
 }
 
 template <int GROUPS>
-int launch_decode(const bf16* qa, long long ldq, bf16* out, long long ldo, float* scratch, const bf16* cache, const int* page_table,
+int launch_decode(const CUtensorMap& rows, const bf16* qa, long long ldq, bf16* out, long long ldo, float* scratch, const int* page_table,
                   int table_width, int page_size, const int* seq_start, const int* seq_slot, int n_seqs, int H, int window, int ctas,
                   cudaStream_t stream) {
   using D = Decode<GROUPS>;
@@ -763,7 +764,7 @@ int launch_decode(const bf16* qa, long long ldq, bf16* out, long long ldo, float
       return GB_ERR_SIZE;
     allowed = true;
   }
-  gb_launch(latent_decode_kernel<GROUPS>, dim3(ctas), dim3(D::WARPS * 32 + 32), D::SMEM, stream, qa, ldq, out, ldo, scratch, cache,
+  gb_launch(latent_decode_kernel<GROUPS>, dim3(ctas), dim3(D::WARPS * 32 + 32), D::SMEM, stream, rows, qa, ldq, out, ldo, scratch,
             page_table, table_width, page_size, seq_start, seq_slot, n_seqs, H, window);
   gb_launch(latent_decode_merge_kernel, dim3(n_seqs * H), dim3(128), 0, stream, (const float*)scratch, seq_start, out, ldo, n_seqs,
             H, D::ROWS, window, (unsigned)ctas);
@@ -824,19 +825,21 @@ GB_EXPORT long long gb_latent_decode_scratch(int H, int ctas) {
   return (long long)ctas * 2 * (H > 16 ? 32 : 16) * PART;
 }
 
-// Every sequence brings one token: row b of qa and out is sequence b's.  scratch: gb_latent_decode_scratch() floats,
+// Every sequence brings one token: row b of qa and out is sequence b's.  cache: cache_rows rows.  scratch: gb_latent_decode_scratch() floats,
 // 16-byte aligned.
 GB_EXPORT int gb_latent_decode(const void* qa, long long ldq, void* out, long long ldo, float* scratch, const void* cache,
-                               const int* page_table, int table_width, int page_size, const int* seq_start, const int* seq_slot,
+                               long long cache_rows, const int* page_table, int table_width, int page_size, const int* seq_start, const int* seq_slot,
                                int n_seqs, int H, int rank, int rot, int window, int ctas, cudaStream_t stream) {
   if (n_seqs <= 0) return 0;
   if (rank != RANK || rot != ROT || H <= 0 || page_size % 64 || n_seqs > MAX_SEQS || ctas < 1) return GB_ERR_SIZE;
   if (((uintptr_t)qa & 15) || (ldq % 8) || ((uintptr_t)out & 3) || (ldo % 2) || ((uintptr_t)cache & 15) || ((uintptr_t)scratch & 15) || !scratch)
     return GB_ERR_SIZE;
-  return H > 16 ? launch_decode<2>((const bf16*)qa, ldq, (bf16*)out, ldo, scratch, (const bf16*)cache, page_table, table_width, page_size,
-                                   seq_start, seq_slot, n_seqs, H, window, ctas, stream)
-                : launch_decode<1>((const bf16*)qa, ldq, (bf16*)out, ldo, scratch, (const bf16*)cache, page_table, table_width, page_size,
-                                   seq_start, seq_slot, n_seqs, H, window, ctas, stream);
+  CUtensorMap rows;
+  if (cache_rows < KT || cache_rows > INT_MAX || !tensor_map(&rows, cache, (uint64_t)cache_rows, KD, KD * 2, KT)) return GB_ERR_ARG;
+  return H > 16 ? launch_decode<2>(rows, (const bf16*)qa, ldq, (bf16*)out, ldo, scratch, page_table, table_width, page_size, seq_start,
+                                   seq_slot, n_seqs, H, window, ctas, stream)
+                : launch_decode<1>(rows, (const bf16*)qa, ldq, (bf16*)out, ldo, scratch, page_table, table_width, page_size, seq_start,
+                                   seq_slot, n_seqs, H, window, ctas, stream);
 }
 
 // 0, or the code of the first bounded wait that ran out (synchronizes the device).

@@ -1084,10 +1084,10 @@ def latent_decode(qa, out, heads, rank, rd, cache, page_table, page_size, seq_st
             _outgrown.append(part)        # a captured step may still point at it: never freed
         part = _latent_scratch[qa.device.index] = torch.empty(max(need, 1 << 20), dtype=torch.float32, device=qa.device)
     f = _fn("latent_attention_mma", "gb_latent_decode",
-            [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p, c_int, c_int,
+            [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_void_p, c_longlong, c_void_p, c_int, c_int, c_void_p, c_void_p, c_int, c_int,
              c_int, c_int, c_int, c_int, c_void_p], defines=defines)
-    _check(f(qa.data_ptr(), qa.stride(0), out.data_ptr(), out.stride(0), part.data_ptr(), cache.data_ptr(), page_table.data_ptr(),
-             page_table.shape[1], page_size, seq_start.data_ptr(), seq_slot.data_ptr(), n, heads, rank, rd, window or 0, ctas,
+    _check(f(qa.data_ptr(), qa.stride(0), out.data_ptr(), out.stride(0), part.data_ptr(), cache.data_ptr(), cache.numel() // (rank + rd),
+             page_table.data_ptr(), page_table.shape[1], page_size, seq_start.data_ptr(), seq_slot.data_ptr(), n, heads, rank, rd, window or 0, ctas,
              _stream()), "latent_decode", "attention", _nbytes(qa, out) + cache_bytes)
     count_launches(1)   # the merge kernel
 
