@@ -226,7 +226,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
 
   if (warp == 4) {
     // ---------------- TMA: the query tile once, then one page of keys and values per step
-    if (lane == 0 && !*abort) {
+    if (elect_one() && !*abort) {
       asm volatile("prefetch.tensormap [%0];" ::"l"(&map_q) : "memory");
       asm volatile("prefetch.tensormap [%0];" ::"l"(&map_k) : "memory");
       asm volatile("prefetch.tensormap [%0];" ::"l"(&map_v) : "memory");
@@ -286,7 +286,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
   } else if (warp == 5) {
     // ---------------- MMA issue: S up to two pages ahead of the softmax, and O += P V as soon as a
     // P is there; whichever can go next (neither waits for the other's operands)
-    if (lane == 0 && !*abort && wait_or_abort(q_full, 0, abort, 2)) {
+    if (elect_one() && !*abort && wait_or_abort(q_full, 0, abort, 2)) {
       int js = 0, jp = 0;   // next S, next P V
       uint32_t spins = 0;
       while (jp < n_tiles && !*abort) {

@@ -501,7 +501,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
 
   if (warp == 4) {
     // ---------------- TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       asm volatile("prefetch.tensormap [%0];" ::"l"(&map_w) : "memory");
       asm volatile("prefetch.tensormap [%0];" ::"l"(&map_x) : "memory");
       // the weights do not depend on the kernel before this one: the first stages' W tiles are
@@ -545,7 +545,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     __syncwarp();
   } else if (warp == 5) {
     // ---------------- MMA issue
-    if (lane == 0) {
+    if (elect_one()) {
       bool ok = true;
       for (int i = 0; i < kb_count && ok; ++i) {
         const int s = i % STAGES;
@@ -936,7 +936,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
 
   if (warp == 4) {
     // ---------------- TMA producer: all of this CTA's tiles, one stream of stages
-    if (lane == 0) {
+    if (elect_one()) {
       asm volatile("prefetch.tensormap [%0];" ::"l"(&map_w) : "memory");
       asm volatile("prefetch.tensormap [%0];" ::"l"(&map_x) : "memory");
       pdl_wait_prior();
@@ -976,7 +976,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
     __syncwarp();
   } else if (warp == 5) {
     // ---------------- MMA issue
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t it = 0, i = 0;
       bool ok = true;
       // which tiles are used is written by a kernel before this one: it must have ended before the
