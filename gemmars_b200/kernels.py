@@ -483,6 +483,14 @@ def gemm_tc_persistent(x, w, out, bias=None, accumulate=False, swiglu=False, bn=
         # SMs; a 2,048-token prompt of a 4B-shaped model took 20.5 ms against 18.4, of a 32B-shaped one
         # 35.3 ms against 30.9 over 16 layers)
         bn = 128 if m <= 128 else 256
+        # Where those leave two SMs in five without a tile (a router, a low-rank factor, few tokens), the narrowest tiles that
+        # still are one round; a block of the inner dimension takes less time the narrower they are (us, 256 tokens a
+        # tile / so; 2,048 inner): 65 features of 2,048 tokens (8 tiles) 23.8 / 11.5, 576 of 2,048 (40) 17.7 / 13.1, 1,024
+        # of 2,048 (64) 17.7 / 13.6, 576 of 4,096 (80) 17.7 / 15.6, but 1,024 of 4,096 (128 tiles) 19.2 / 19.7.
+        # A product that adds cuts its tiles along the inner dimension instead.
+        tiles_n, sms = -(-n // (64 if swiglu else 128)), ctas or sm_count(x.device)
+        if not accumulate and 5 * tiles_n * -(-m // bn) <= 3 * sms:
+            bn = min(bn, (-(-m // (sms // tiles_n)) + 15) // 16 * 16)
     ctas = ctas or sm_count(x.device)
     flags = None
     if accumulate and split_last:

@@ -100,3 +100,34 @@ def test_prompts_in_padded_tiles(tokens, e, top, width, ff, ffs, skew, weigh):
     got = _run(kernels, idx, wts, m, base, 1.5, weigh, kernels.moe_experts_tc)
     want, room = _want(idx, wts, m, 1.5, weigh)
     assert ((got.double() - base.double() - want).abs() <= room).all()
+
+
+@pytest.mark.parametrize("rows", [65, 100, 300, 2048])
+@pytest.mark.parametrize("n", [1, 65, 130, 576, 1000])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_products_of_few_features_in_narrow_tiles(rows, n, dtype):
+    """The tile's width changes nothing: the same bits as in tiles of 256 rows."""
+    from gemmars_b200 import kernels
+    torch.manual_seed(rows + n)
+    x, w = torch.randn(rows, 328, device=DEV).bfloat16(), torch.randn(n, 328, device=DEV).bfloat16()
+    got, wide = torch.full((rows, n), 7.0, device=DEV, dtype=dtype), torch.full((rows, n), 7.0, device=DEV, dtype=dtype)
+    kernels.gemm_tc_persistent(x, w, got)
+    kernels.gemm_tc_persistent(x, w, wide, bn=256)
+    kernels.check_status()
+    assert torch.equal(got, wide)
+    want = x.double() @ w.double().T       # float32 sums of 328 products, then the result's own rounding
+    assert (got.double() - want).abs().max() <= (2.0 ** -8 if dtype is torch.bfloat16 else 1e-5) * want.abs().max()
+
+
+@pytest.mark.parametrize("features", [8, 24, 100, 2056])
+def test_the_shared_experts_activation(features):
+    from gemmars_b200 import kernels
+    torch.manual_seed(features)
+    gu, scale = torch.randn(33, 2 * features, device=DEV).bfloat16() * 3, torch.rand(33, device=DEV)
+    y = torch.empty(33, features, device=DEV, dtype=torch.bfloat16)
+    f = kernels._fn("grouped_gemm", "gb_gated_act", [kernels.c_void_p] * 3 + [kernels.c_int] * 2 + [kernels.c_float] * 3 + [kernels.c_void_p])
+    assert f(gu.data_ptr(), y.data_ptr(), scale.data_ptr(), 33, features, 2.0, 1.7, 0.5, kernels._stream()) == 0
+    g, u = gu.double().chunk(2, 1)
+    g, u = g.clamp(max=2.0), u.clamp(-2.0, 2.0)
+    want = g * torch.sigmoid(1.7 * g) * (u + 0.5) * scale.double()[:, None]
+    assert ((y.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-6).all()
