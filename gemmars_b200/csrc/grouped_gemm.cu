@@ -352,7 +352,15 @@ __global__ void __launch_bounds__(256) moe_combine_wide_kernel(const float* __re
   }
 }
 
-// y[t, f] = act(gu[t, f], gu[t, F + f]) * scale[t]: the activation of a dense (shared) expert
+// y[t, f] = act(gu[t, f], gu[t, F + f]) * scale[t]: the activation of a dense (shared) expert.  Bound by memory; eight features a
+// thread where rows of both lie at 16-byte boundaries: 2,048 tokens of 2,816 features (35 MB) 13 us a feature a thread, 9.7
+// so.  (In the epilogue of the product before it, which then has tiles of 64 + 64 rows: the shared expert as a whole 89 us
+// against 83.)
+__device__ __forceinline__ float gated_value(float g, float u, float sc, float limit, float alpha, float shift) {
+  g = fminf(g, limit);
+  u = fminf(fmaxf(u, -limit), limit);
+  return g / (1.0f + expf(-alpha * g)) * (u + shift) * sc;
+}
 __global__ void __launch_bounds__(256) gated_act_kernel(const bf16* __restrict__ gu, bf16* __restrict__ y,
                                                         const float* __restrict__ scale, int F, float limit, float alpha,
                                                         float shift) {
@@ -360,11 +368,24 @@ __global__ void __launch_bounds__(256) gated_act_kernel(const bf16* __restrict__
   pdl_wait_prior();
   const int t = blockIdx.x;
   const float sc = scale ? scale[t] : 1.f;
-  for (int f = threadIdx.x; f < F; f += 256) {
-    const float gt = fminf(__bfloat162float(gu[(size_t)t * 2 * F + f]), limit);
-    const float up = fminf(fmaxf(__bfloat162float(gu[(size_t)t * 2 * F + F + f]), -limit), limit);
-    y[(size_t)t * F + f] = __float2bfloat16_rn(gt / (1.0f + expf(-alpha * gt)) * (up + shift) * sc);
+  const bf16 *g = gu + (size_t)t * 2 * F, *u = g + F;
+  if (F % 8 == 0 && !(((uintptr_t)gu | (uintptr_t)y) & 15)) {
+    for (int f = threadIdx.x * 8; f < F; f += 2048) {
+      const uint4 gv = *(const uint4*)(g + f), uv = *(const uint4*)(u + f);
+      const __nv_bfloat162 *gp = (const __nv_bfloat162*)&gv, *up = (const __nv_bfloat162*)&uv;
+      uint4 o;
+      uint32_t* op = (uint32_t*)&o;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float2 a = __bfloat1622float2(gp[i]), b = __bfloat1622float2(up[i]);
+        op[i] = pack_bf16(gated_value(a.x, b.x, sc, limit, alpha, shift), gated_value(a.y, b.y, sc, limit, alpha, shift));
+      }
+      *(uint4*)(y + (size_t)t * F + f) = o;
+    }
+    return;
   }
+  for (int f = threadIdx.x; f < F; f += 256)
+    y[(size_t)t * F + f] = __float2bfloat16_rn(gated_value(__bfloat162float(g[f]), __bfloat162float(u[f]), sc, limit, alpha, shift));
 }
 
 template <int MODE, typename TO>
