@@ -24,6 +24,7 @@
 // the output.
 //
 // A step of single tokens has a kernel of its own (latent_decode_kernel), the same arithmetic over a stream of keys.
+#include "latent_decode_ring.h"
 #include "mma.cuh"
 #include "tc_common.cuh"
 
@@ -299,24 +300,18 @@ latent_attention_mma_kernel(const bf16* __restrict__ qa, long long ldq, bf16* __
 // 16 sequences of 5,330 to 8,000 keys, 16 heads, rows of 512 + 64 (121 MB): 49 + 6 us with the keys dealt to 18 CTAs a
 // sequence by the kernel above, two tiles in flight and a barrier of the block a tile; 37.5 + 6.5 us with a bulk copy a row,
 // 30 + 6.5 us so (boxes of 32 rows x 128 bytes: 9 requests a tile instead of 32).
-constexpr int KT = 32;
+constexpr int KT = latent_ring::KT, MAX_SEQS = latent_ring::MAX_SEQS;
 constexpr int BOXES = (KD + 63) / 64, BOX_BYTES = KT * 128, STAGE_BYTES = BOXES * BOX_BYTES;
-constexpr int MAX_SEQS = 1024;
+static_assert(NSPLIT == latent_ring::warps_of(RANK), "the ring counts with as many warps");
 template <int GROUPS>
 struct Decode {
-  static constexpr int KG = NSPLIT * GROUPS == 1 ? 4 : 8 / (NSPLIT * GROUPS);      // teams
+  static constexpr latent_ring::Ring R = latent_ring::ring(RANK, ROT, GROUPS);
+  static constexpr bool FITS = R.stages > 0;
+  static constexpr int KG = FITS ? R.teams : 1, STAGES = FITS ? R.stages : 2;
   static constexpr int WARPS = KG * NSPLIT * GROUPS, ROWS = 16 * GROUPS;
   static constexpr int SXP = KT + 8, PP = KT + 8;                // pitches of the scores' parts and of the weights
-  // floats that 16 rows of a team share: the scores' parts, the warps' maxima (and sums), the weights (bfloat16)
-  static constexpr int SX = NSPLIT > 1 ? NSPLIT * 16 * SXP + NSPLIT * 16 + 16 * PP / 2 : 0;
-  static constexpr int MEET = (KG - 1) * NSPLIT * GROUPS * (DW / 2 + 4) * 32;          // floats: the teams' results
-  static constexpr int FLOATS = KG * GROUPS * SX > MEET ? KG * GROUPS * SX : MEET;
-  static constexpr int FIT = (227 * 1024 - FLOATS * 4 - 512 - MAX_SEQS * 4 - 1024) / STAGE_BYTES;
-  // A place in the ring belongs to one team: whoever waits for a tile has then had the tile before it in that place, so
-  // that a parity never stands for the phase before the last (copies may arrive out of their order).
-  static constexpr int STAGES = (FIT > 16 ? 16 : FIT) / KG * KG;
-  static constexpr size_t SMEM = 1024 + (size_t)STAGES * STAGE_BYTES + FLOATS * 4 + 2 * STAGES * 8 + 16 + (size_t)(MAX_SEQS + 1) * 4;
-  static_assert(STAGES > KG && STAGES % KG == 0, "a tile ahead of the teams");
+  static constexpr int SX = R.share, FLOATS = R.floats;
+  static constexpr size_t SMEM = R.smem;
 };
 
 __device__ int g_latent_status;   // 0, or the first wait that ran out (1 free stage, 2 tile)
@@ -757,7 +752,7 @@ int launch_decode(const CUtensorMap& rows, const bf16* qa, long long ldq, bf16* 
                   int table_width, int page_size, const int* seq_start, const int* seq_slot, int n_seqs, int H, int window, int ctas,
                   cudaStream_t stream) {
   using D = Decode<GROUPS>;
-  static_assert(D::SMEM <= 227 * 1024, "shared memory");
+  static_assert(D::SMEM <= latent_ring::ROOM, "shared memory");
   static bool allowed = false;
   if (!allowed) {
     if (cudaFuncSetAttribute(latent_decode_kernel<GROUPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)D::SMEM) != cudaSuccess)
@@ -820,8 +815,10 @@ GB_EXPORT int gb_latent_attention_mma(const void* qa, long long ldq, void* out, 
                            cu_seqlens, seq_start, seq_slot, n_seqs, ntok, H, groups, window, head_stride, out_scale, out_gate, ldg, stream);
 }
 
-// Floats of scratch for a step of single tokens on `ctas` CTAs.
+// Floats of scratch for a step of single tokens on `ctas` CTAs; 0: the rows are too wide for the stream (such steps run on
+// the kernel of the prompts).
 GB_EXPORT long long gb_latent_decode_scratch(int H, int ctas) {
+  if (!(H > 16 ? Decode<2>::FITS : Decode<1>::FITS)) return 0;
   return (long long)ctas * 2 * (H > 16 ? 32 : 16) * PART;
 }
 
@@ -836,10 +833,16 @@ GB_EXPORT int gb_latent_decode(const void* qa, long long ldq, void* out, long lo
     return GB_ERR_SIZE;
   CUtensorMap rows;
   if (cache_rows < KT || cache_rows > INT_MAX || !tensor_map(&rows, cache, (uint64_t)cache_rows, KD, KD * 2, KT)) return GB_ERR_ARG;
-  return H > 16 ? launch_decode<2>(rows, (const bf16*)qa, ldq, (bf16*)out, ldo, scratch, page_table, table_width, page_size, seq_start,
-                                   seq_slot, n_seqs, H, window, ctas, stream)
-                : launch_decode<1>(rows, (const bf16*)qa, ldq, (bf16*)out, ldo, scratch, page_table, table_width, page_size, seq_start,
-                                   seq_slot, n_seqs, H, window, ctas, stream);
+  if (H > 16) {
+    if constexpr (Decode<2>::FITS)
+      return launch_decode<2>(rows, (const bf16*)qa, ldq, (bf16*)out, ldo, scratch, page_table, table_width, page_size, seq_start, seq_slot,
+                              n_seqs, H, window, ctas, stream);
+  } else {
+    if constexpr (Decode<1>::FITS)
+      return launch_decode<1>(rows, (const bf16*)qa, ldq, (bf16*)out, ldo, scratch, page_table, table_width, page_size, seq_start, seq_slot,
+                              n_seqs, H, window, ctas, stream);
+  }
+  return GB_ERR_SIZE;
 }
 
 // 0, or the code of the first bounded wait that ran out (synchronizes the device).

@@ -8,7 +8,7 @@ pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
 
 
-@pytest.mark.parametrize("rank,rot", [(64, 32), (112, 16), (256, 32), (512, 64)])
+@pytest.mark.parametrize("rank,rot", [(64, 32), (112, 16), (256, 32), (256, 96), (512, 64)])
 @pytest.mark.parametrize("heads,lens,window", [(16, [3000, 1, 32, 33, 64, 65, 700], None), (1, [20], None), (9, [5000], None),
                                                (40, [31, 2048, 97], None), (32, [200] * 70, None), (17, [900, 150, 64], 100),
                                                (5, [1] * 300, None)])

@@ -47,6 +47,20 @@ def _plain(w, h, lens, nh, dim, rot, vd, rank, window, gate):
                                                             (2, 64, 64, 48, 256, None, False), (2, 128, 8, 16, 256, 70, True)])
 def test_prompts_over_expanded_heads(lens, nh, dim, rot, vd, rank, window, gate, monkeypatch):
     from gemmars_b200 import kernels
+    assert kernels.latent_prefill_tc_usable(torch.bfloat16, rank, dim, rot, vd)
+    _compare(lens, nh, dim, rot, vd, rank, window, gate, monkeypatch)
+
+
+@pytest.mark.parametrize("nh,dim,rot,vd,rank,window,gate", [(2, 192, 64, 128, 512, None, True), (3, 192, 64, 128, 256, 90, "channel")])
+def test_prompts_over_expanded_heads_that_the_tcgen05_kernel_does_not_take(nh, dim, rot, vd, rank, window, gate, monkeypatch):
+    """Heads of 192 + 64: rows [v | k_nope | k_rot] on mma.sync."""
+    from gemmars_b200 import kernels
+    assert not kernels.latent_prefill_tc_usable(torch.bfloat16, rank, dim, rot, vd)
+    _compare([257, 1, 130, 66], nh, dim, rot, vd, rank, window, gate, monkeypatch)
+
+
+def _compare(lens, nh, dim, rot, vd, rank, window, gate, monkeypatch):
+    from gemmars_b200 import kernels
     from gemmars_b200.cache.pool import SequenceCache
     from gemmars_b200.parts.base import StepContext, build_part
     from gemmars_b200.parts.plan import PartSpec
@@ -62,7 +76,6 @@ def test_prompts_over_expanded_heads(lens, nh, dim, rot, vd, rank, window, gate,
         "norm_eps": EPS, "gate": gate, "window": window,
         "position": PartSpec("rotary", {"head_dim": rot, "rotary_dim": rot, "theta": 1e4, "layout": "interleaved"})}), "bfloat16")
     part.load(w)
-    assert kernels.latent_prefill_tc_usable(torch.bfloat16, rank, dim, rot, vd)
     h = torch.randn(t, hid, device=DEV).bfloat16()
     ints = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)      # noqa: E731
 
