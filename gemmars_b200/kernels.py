@@ -1071,6 +1071,17 @@ def latent_attention_mma(qa, out, heads, rank, rd, cache, page_table, page_size,
 
 #: sequences a step of single tokens may have for the streaming kernel
 LATENT_DECODE_MAX_SEQS = 1024
+_latent_decode_floats = {}
+
+
+def latent_decode_scratch(heads: int, rank: int, rd: int, ctas: int) -> int:
+    """Floats of scratch that latent_decode needs; 0: cached rows too wide for it (latent_attention_mma takes such steps)."""
+    key = (heads > 16, rank, rd, ctas)
+    if key not in _latent_decode_floats:
+        f = _fn("latent_attention_mma", "gb_latent_decode_scratch", [c_int, c_int], defines=(("GB_LATENT_RANK", rank), ("GB_LATENT_ROT", rd)))
+        f.restype = c_longlong
+        _latent_decode_floats[key] = f(heads, ctas)
+    return _latent_decode_floats[key]
 
 
 def latent_decode(qa, out, heads, rank, rd, cache, page_table, page_size, seq_start, seq_slot, window=None, cache_bytes: int = 0):
@@ -1084,8 +1095,9 @@ def latent_decode(qa, out, heads, rank, rd, cache, page_table, page_size, seq_st
     assert qa.shape[1] == heads * (rank + rd) and out.shape == (n, heads * rank) and cache.shape[-1] == rank + rd
     assert seq_start.numel() == seq_slot.numel() == n
     ctas, defines = sm_count(), (("GB_LATENT_RANK", rank), ("GB_LATENT_ROT", rd))
-    # parts of a CTA's first and last list (gb_latent_decode_scratch)
-    need = ctas * 2 * (32 if heads > 16 else 16) * (rank + 4)
+    need = latent_decode_scratch(heads, rank, rd, ctas)      # parts of a CTA's first and last list
+    if not need:
+        raise KernelError(f"latent_decode: rows of {rank} + {rd} are too wide")
     part = _latent_scratch.get(qa.device.index)
     if part is None or part.numel() < need:
         if part is not None:
@@ -1110,7 +1122,8 @@ def latent_attention(ctx, qa, out, heads, rank, rd, cache, page_table, page_size
         for start, n in zip(ctx.host["seq_start"], ctx.host["seq_len"]):
             cached += per_pos * (min(start + n, window + n - 1) if window else start + n)
     if latent_attention_mma_usable(qa.dtype, rank, rd, page_size) and qa.stride(0) % 8 == 0:
-        if ctx.max_new <= 1 and ctx.n_seqs == qa.shape[0] <= LATENT_DECODE_MAX_SEQS:
+        if (ctx.max_new <= 1 and ctx.n_seqs == qa.shape[0] <= LATENT_DECODE_MAX_SEQS
+                and latent_decode_scratch(heads, rank, rd, sm_count())):
             latent_decode(qa, out, heads, rank, rd, cache, page_table, page_size, ctx.seq_start, ctx.seq_slot, window, cached)
             return
         latent_attention_mma(qa, out, heads, rank, rd, cache, page_table, page_size, ctx.cu_seqlens, ctx.seq_start,
