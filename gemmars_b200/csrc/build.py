@@ -60,13 +60,26 @@ def build_dir() -> str:
         return d
 
 
+_read: Dict[str, Tuple[Tuple, "hashlib._Hash"]] = {}
+
+
+def _hash_of(paths: Sequence[str], label: bool) -> "hashlib._Hash":
+    """SHA-256 over the files (``label``: each after its name), read again only where a size or a time has changed: a
+    program that sets up many layers asks for the same few units over and over."""
+    key = "\0".join(paths)
+    stamp = tuple((st.st_mtime_ns, st.st_size) for st in map(os.stat, paths))
+    known = _read.get(key)
+    if known is None or known[0] != stamp:
+        h = hashlib.sha256()
+        for path in paths:
+            with open(path, "rb") as f:
+                h.update((os.path.basename(path).encode() + b"\0" if label else b"") + f.read())
+        known = _read[key] = (stamp, h)
+    return known[1].copy()
+
+
 def _headers_digest() -> str:
-    h = hashlib.sha256()
-    for name in sorted(os.listdir(HERE)):
-        if name.endswith((".cuh", ".h")):
-            with open(os.path.join(HERE, name), "rb") as f:
-                h.update(name.encode() + b"\0" + f.read())
-    return h.hexdigest()
+    return _hash_of([os.path.join(HERE, name) for name in sorted(os.listdir(HERE)) if name.endswith((".cuh", ".h"))], True).hexdigest()
 
 
 def library_path(unit: str, defines: Sequence[Tuple[str, object]] = ()) -> Tuple[str, list]:
@@ -74,9 +87,7 @@ def library_path(unit: str, defines: Sequence[Tuple[str, object]] = ()) -> Tuple
     if not os.path.exists(src):
         raise KernelBuildError(f"no CUDA source {src}")
     flags = ARCH_FLAGS + BASE_FLAGS + [f"-D{k}={v}" for k, v in defines]
-    h = hashlib.sha256()
-    with open(src, "rb") as f:
-        h.update(f.read())
+    h = _hash_of([src], False)
     h.update(_headers_digest().encode())
     h.update(" ".join(flags).encode())
     tag = "_".join(f"{k.lower()}{v}" for k, v in defines)
