@@ -1563,7 +1563,7 @@ def gemm_units(compute: str):
 NORM_LINKS = True
 
 
-def gemm(x, w, out, bias=None, accumulate=False, then_norm=None, act=None, col_scale=None):
+def gemm(x, w, out, bias=None, accumulate=False, then_norm=None, act=None, col_scale=None, w_made=False):
     """out = x @ w.T (+ bias) or, with ``accumulate``, out += ...; picks the kernel for the
     precision and the shape: float32 runs on the CUDA cores in a fixed order; bfloat16 runs on the
     tensor cores, except for operands whose rows TMA cannot address (an inner size that is not
@@ -1572,7 +1572,10 @@ def gemm(x, w, out, bias=None, accumulate=False, then_norm=None, act=None, col_s
     product: where the kernel can, it leaves that norm's input as UnscaledRows, which is returned
     (None: the norm has to run by itself).  ``act`` (one of PLAIN_ACTS): an activation of the results,
     in the product's epilogue, before they are rounded.  ``col_scale`` (float32 [N]): with
-    ``accumulate``, multiplies what is added, per output feature."""
+    ``accumulate``, multiplies what is added, per output feature.  ``w_made`` (bfloat16): ``w`` is the work of
+    a kernel of this step.  The kernels for few rows ask for ``w`` before the kernel ahead of them has ended (a
+    weight does not depend on it); such a ``w`` goes to those that wait first."""
+    assert not w_made or x.dtype == torch.bfloat16
     link = x if isinstance(x, UnscaledRows) else None
     if link is not None:
         if norm_link_usable(link.rows, w, link.rows.shape[0]):
@@ -1581,7 +1584,7 @@ def gemm(x, w, out, bias=None, accumulate=False, then_norm=None, act=None, col_s
             x, link = link.materialize(), None
     if x.dtype == torch.bfloat16 and gemm_tc_usable(x, w):
         m, n, k = x.shape[0], w.shape[0], x.shape[1]
-        if m > 64:
+        if m > 64 or w_made:
             gemm_tc_persistent(x, w, out, bias, accumulate, plain_act=act, col_scale=col_scale)
             return None
         if then_norm is not None and not (accumulate and gemm_tc_tiling(m, n, k)[1] >= 2):

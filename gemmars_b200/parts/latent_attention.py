@@ -202,7 +202,7 @@ class LatentAttention(Part):
         keys = torch.empty((n, nh * dim), dtype=self.act_dtype, device=q.device)
         kernels.gemm(latents, self.uk.view(nh * dim, r), keys)
         values = torch.empty((nh * vd, n), dtype=self.act_dtype, device=q.device)
-        kernels.gemm(self.uv.view(nh * vd, r), latents, values)
+        kernels.gemm(self.uv.view(nh * vd, r), latents, values, w_made=True)
         o = torch.empty((t, nh * vd), dtype=self.act_dtype, device=q.device)
         kernels.attention_prefill_latent(q, o, nh, keys, shared, values, rd, cu, ctx.seq_start, self.window, gate, channel)
         self.o.add_into(o, residual)

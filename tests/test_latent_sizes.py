@@ -67,3 +67,38 @@ def test_expanded_heads_ask_for_a_size_that_fits(rings):
         sizes = [(dict(d)["GB_LATENT_RANK"], dict(d)["GB_LATENT_ROT"]) for u, d in units if u == "latent_attention_mma"]
         assert (vd, dim + rd) in sizes
         assert all(rings[r, t, g][1] for r, t in sizes for g in (1, 2))
+
+
+@pytest.mark.parametrize("heads,vdim", [(4, 16), (1, 32), (3, 32)])
+def test_latents_of_the_step_go_to_no_product_that_asks_for_its_weights_early(heads, vdim, monkeypatch):
+    """The values' product over a prompt's latents has the latents in the weights' place.  The kernel for up to 64 rows reads
+    weights before the kernel ahead of it has ended, so latents that this step made must not go there."""
+    from gemmars_b200 import kernels
+    from gemmars_b200.parts.base import build_part
+    from gemmars_b200.parts.plan import PartSpec
+    dim, rot, rank, hidden, t = 64, 8, 64, 32, 300
+    part = build_part("mixer", PartSpec("latent_attention", {
+        "hidden_size": hidden, "num_heads": heads, "dim": dim, "rot_dim": rot, "vdim": vdim, "rank": rank, "scale": 0.1, "norm_eps": 1e-6,
+        "gate": False, "window": None}), "bfloat16")
+    made = {n: torch.randn(w.shape).to(torch.bfloat16 if w.role == "matrix" else torch.float32) for n, w in part.wants().items()}
+    part.load(made)
+    latents, shared = torch.randn(kernels.latent_expand_rows(t, 1), rank).bfloat16(), torch.randn(kernels.latent_expand_rows(t, 1), rot).bfloat16()
+    early, results = [], {}
+
+    def product(x, w, out, *args, **kwargs):
+        out.copy_(x.float() @ w.float().T)
+
+    def few(x, w, out, *args, **kwargs):
+        early.append(w.data_ptr())
+        product(x, w, out)
+
+    monkeypatch.setattr(kernels, "gemm_tc", few)
+    monkeypatch.setattr(kernels, "gemm_tc_persistent", product)
+    monkeypatch.setattr(kernels, "attention_prefill_latent", lambda q, o, nh, keys, shared, values, *a: results.update(keys=keys, values=values))
+    part.o = type("O", (), {"add_into": lambda self, *a: None})()
+    q = torch.zeros(t, heads * (dim + rot), dtype=torch.bfloat16)
+    ctx = type("Ctx", (), {"seq_start": torch.zeros(1, dtype=torch.int32)})()
+    part._expanded_tc(ctx, q, None, None, (latents, shared, torch.tensor([0, t], dtype=torch.int32)), torch.zeros(t, hidden))
+    assert latents.data_ptr() not in early
+    assert torch.equal(results["values"], (made["uv"].float() @ latents.float().T).bfloat16())
+    assert torch.equal(results["keys"], (latents.float() @ made["uk"].float().T).bfloat16())
