@@ -210,17 +210,20 @@ static int launch_ref(int ntok, int rep, const PagedKV& kv, cudaStream_t stream,
   return gb_launch_status();
 }
 
-// q: [ntok, nh, hd] rows q_stride apart (already normed, rotated, scaled); out likewise.
+// q: [ntok, nh, hd] rows q_stride apart (already normed, rotated, scaled); out likewise.  apart: tokens seldom share their
+// sequence and first key (single tokens, or most of a prompt past its window), so that a block would work its four one after
+// the other: one token a block then.  The same bits either way.
 GB_EXPORT int gb_attention_ref(const void* q, long long q_stride, void* out, long long out_stride, int dtype,
                                const void* kcache, const void* vcache, const int* page_table, int table_width,
                                int page_size, int nkv, int hd, const int* tok_pos, const int* tok_seq,
-                               const int* seq_slot, int ntok, int nh, int window, cudaStream_t stream) {
+                               const int* seq_slot, int ntok, int nh, int window, int apart, cudaStream_t stream) {
   if (ntok <= 0) return 0;
   if (hd <= 0 || hd > 2 * CHUNK || nkv <= 0 || nh % nkv) return GB_ERR_SIZE;
   PagedKV kv{page_table, table_width, page_size, nkv, hd};
   const int rep = nh / nkv, heads = rep >= 3 ? 4 : rep;
-  // Positions of a prompt share their keys: four tokens a block, once that leaves two blocks an SM
-  const bool four = (long long)ntok * nkv * ((rep + heads - 1) / heads) >= 4 * 2 * 148;
+  // Positions of a prompt share their keys: four tokens a block, once that leaves two blocks an SM (us, one / four; 16 heads of
+  // 128 over 8: 1,024 tokens 869 / 554, but in a window of 128 278 / 569, and 2,048 in one of 512 1,818 / 3,465)
+  const bool four = !apart && (long long)ntok * nkv * ((rep + heads - 1) / heads) >= 4 * 2 * 148;
   const int wide = hd % 4 == 0 && (((uintptr_t)kcache | (uintptr_t)vcache) & 15) == 0;
 #define REF(T, TOKENS, HEADS)                                                                                              \
   launch_ref<T, TOKENS, HEADS>(ntok, rep, kv, stream, (const T*)q, q_stride, (T*)out, out_stride, (const T*)kcache, (const T*)vcache, \

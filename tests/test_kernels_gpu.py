@@ -292,6 +292,10 @@ def test_attention_ref_of_prompts_gives_the_bits_of_single_tokens(k, hd, nh, nkv
         s = int(tok_seq[i])
         ref = _attn_ref(q[i].float().view(nh, hd), *dense[s], int(tok_pos[i]), nh, window).view(-1)
         assert (out[i].float() - ref).abs().max().item() <= tol * max(1.0, ref.abs().max().item())
+    for apart in (False, True):                              # four tokens a block, and one
+        again = torch.zeros_like(out)
+        k.attention_ref(q, again, nh, kc, vc, table, 64, tok_pos, tok_seq, slots, window, apart=apart)
+        assert torch.equal(again, out)
     alone = torch.zeros_like(out)
     for i in range(0, t, 7):
         k.attention_ref(q[i:i + 1], alone[i:i + 1], nh, kc, vc, table, 64, tok_pos[i:i + 1], tok_seq[i:i + 1], slots, window)
