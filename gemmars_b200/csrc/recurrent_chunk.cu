@@ -27,7 +27,7 @@
 // outputs and state, 1e-7): delta rule 2.2 / 2.5 and 3.6 / 3.5, with a decay per channel 1.9 / 1.8 and 2.2 / 1.9, state space
 // 1.0 / 1.4 and 1.8 / 1.8, read before 2.4 / 2.2 and 2.5 / 2.0, read after 1.9 / 1.9 and 1.7 / 1.6; of a layer's states,
 // whose inputs come from bfloat16 products, 54 / 54, 67 / 66 and 80 / 79 (delta rule, state space, read before).
-// A value that is not finite reaches the outputs of its whole chunk (zero times infinity), not only of the tokens from its own on.
+// A number that is not finite reaches what it reaches token by token: see mma_lower().
 #include <type_traits>
 #include "common.cuh"
 
@@ -79,14 +79,48 @@ __device__ __forceinline__ void mma3_apart(float (&d)[4], float (&x)[4], const u
 // where roundings do not.  That mean is given back, for partial sums that on the mean grow evenly.
 __device__ __forceinline__ float whole(float d, float x, float links) { return d + fmaf(d, 4.3e-8f * (0.5f * (links + 1.f)), x); }
 
-// Over a chunk's tokens, by weights below a diagonal (T, P): d = (columns of V or U) x (weights of the eight tokens 8 nt ..).
-__device__ __forceinline__ void mma_lower(float (&d)[4], const uint32_t (&hi)[2][4], const uint32_t (&lo)[2][4], float4 w, int nt) {
+// Over a chunk's tokens, by weights below a diagonal (T, P): d = (columns of V or U) x (weights of the eight tokens 8 nt ..), token i
+// from tokens up to i.  Above the diagonal the weights are zeros, and what they multiply must not reach the result where it is
+// not finite: without `clean`, a column's tokens before the first such one take the product without it.
+__device__ __forceinline__ void mma_lower(float (&d)[4], const uint32_t (&hi)[2][4], const uint32_t (&lo)[2][4], float4 w, int nt, bool clean,
+                                          int lane) {
   float x[4] = {};
   d[0] = d[1] = d[2] = d[3] = 0.f;
   mma3(d, x, hi[0], lo[0], w.x, w.y);
   if (nt) mma3(d, x, hi[1], lo[1], w.z, w.w);
 #pragma unroll
   for (int e = 0; e < 4; ++e) d[e] = whole(d[e], x[e], nt ? 2.f : 1.f);
+  if (clean) return;
+  uint32_t h[2][4], l[2][4];
+  int first[2] = {CT, CT};                      // of columns gr and gr + 8
+#pragma unroll
+  for (int half = 1; half >= 0; --half)
+#pragma unroll
+    for (int e = 3; e >= 0; --e) {              // entry e: column e & 1, token 2 t + (e >> 1) of the half
+      const bool bad = !isfinite(__uint_as_float(lo[half][e]));
+      h[half][e] = bad ? 0u : hi[half][e];
+      l[half][e] = bad ? 0u : lo[half][e];
+      if (bad) first[e & 1] = 8 * half + 2 * (lane & 3) + (e >> 1);
+    }
+#pragma unroll
+  for (int o = 1; o <= 2; o <<= 1)
+#pragma unroll
+    for (int c = 0; c < 2; ++c) first[c] = min(first[c], __shfl_xor_sync(0xffffffffu, first[c], o));
+  float f[4] = {}, fx[4] = {};
+  mma3(f, fx, h[0], l[0], w.x, w.y);
+  if (nt) mma3(f, fx, h[1], l[1], w.z, w.w);
+#pragma unroll
+  for (int e = 0; e < 4; ++e)                   // result e: column e >> 1, token 2 t + (e & 1)
+    if (8 * nt + 2 * (lane & 3) + (e & 1) < first[e >> 1]) d[e] = whole(f[e], fx[e], nt ? 2.f : 1.f);
+}
+// Whether all of a warp's numbers in such an operand are finite (a low half is not finite where its number, or the high half, is not).
+__device__ __forceinline__ bool all_finite(const uint32_t (&lo)[2][4]) {
+  float z = 0.f;
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) z = fmaf(__uint_as_float(lo[h][e]), 0.f, z);
+  return __all_sync(0xffffffffu, z == 0.f);
 }
 
 // Chunks are numbered over the whole step: sequence b's are cu[b] / 16 + b and those after it, which leaves room
@@ -212,7 +246,7 @@ __global__ void __launch_bounds__(128, DP == 64 ? 8 : 6) chunk_prepare_kernel(co
       if (u && i > j) between *= gate[i];
       const float r = (float)between;
       float p = i >= j ? qk[i][j] * r : 0.f;
-      if (MODE == STATE_SPACE) p = p * beta[j] + (i == j ? a.skip[head] : 0.f);
+      if (MODE == STATE_SPACE && i >= j) p = p * beta[j] + (i == j ? a.skip[head] : 0.f);
       qk[i][j] = p;
       if (HAS_W) at[j][i] = i > j ? beta[i] * (at[j][i] * r) : 0.f;
     }
@@ -486,11 +520,12 @@ __global__ void __launch_bounds__(32 * DS * NV + 32) chunk_scan_kernel(const Sca
       }
     // + T V: the last warp's work, or the last two's, a half of the tokens each
     if (HAS_W && part >= DS - (DS == 4 ? 2 : 1)) {
+      const bool v_clean = all_finite(vlo);
 #pragma unroll
       for (int nt = 0; nt < 2; ++nt) {
         if (DS == 4 && nt != (part & 1)) continue;
         float d[4];
-        mma_lower(d, vhi, vlo, blk[B::T / 4 + 32 * nt + lane], nt);
+        mma_lower(d, vhi, vlo, blk[B::T / 4 + 32 * nt + lane], nt, v_clean, lane);
 #pragma unroll
         for (int e = 0; e < 4; ++e) u[nt][e] += d[e];
       }
@@ -547,12 +582,13 @@ __global__ void __launch_bounds__(32 * DS * NV + 32) chunk_scan_kernel(const Sca
       S[j][3] = fmaf(gf.y, S[j][3], whole(d[3], x[3], 2.f));
     }
     // Y = Q~ S + P U, of the tokens that this warp finishes
+    const bool u_clean = !finishes || all_finite(ulo);
 #pragma unroll
     for (int i = 0; i < (DS == 1 ? 2 : 1); ++i) {
       if (!finishes) break;
       const int nt = DS == 1 ? i : part;
       float d[4];
-      mma_lower(d, uhi, ulo, blk[B::P / 4 + 32 * nt + lane], nt);
+      mma_lower(d, uhi, ulo, blk[B::P / 4 + 32 * nt + lane], nt, u_clean, lane);
       const int row = 8 * nt + 2 * t, rows = t1 - t0 - c * CT;
       float* to = yrow + (size_t)row * a.H * V;
 #pragma unroll

@@ -103,3 +103,51 @@ def test_chunks_of_a_prompt(form, heads, groups, dim, vdim, turns, monkeypatch):
     assert y_err < 1.5e-6 and s_err < 1.5e-6, (y_err, s_err, y_walk, s_walk)
     # no less exact than token by token: the state; and the outputs but for a decay or a head's gates that stand before whole rows
     assert s_err < 1.15 * s_walk + 2e-8 and y_err < 1.5 * y_walk + 2e-8, (y_err, s_err, y_walk, s_walk)
+
+
+@pytest.mark.parametrize("heads,groups,dim,vdim", [(4, 2, 128, 128), (2, 1, 64, 64), (3, 3, 12, 33), (40, 20, 128, 40), (24, 12, 128, 128)])
+@pytest.mark.parametrize("form", ["delta", "channel_delta", "ssd", "before", "after"])
+@pytest.mark.parametrize("what", ["q", "k", "v", "gate"])
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+def test_a_number_that_is_not_finite_reaches_what_it_reaches_token_by_token(form, heads, groups, dim, vdim, what, value):
+    """Tokens before it keep their bits, and what is not finite afterwards is what is not finite token by token."""
+    from gemmars_b200 import kernels as k
+    torch.manual_seed(heads + dim)
+    lens, bad = [100, 40, 3, 1, 17, 20, 33, 16], (37, 104, 175)       # inside a chunk, near a sequence's start, near the end of one
+    ntok, gh = sum(lens), groups if form in ("delta", "channel_delta", "ssd") else heads
+    x = torch.randn(ntok, 2 * gh * dim + heads * vdim + 4, device=DEV)
+    gates, decay = torch.randn(ntok, 2 * heads, device=DEV), torch.exp(-torch.exp(torch.randn(ntok, heads * dim, device=DEV) - 1))
+    a_log, dt_bias, skip, bonus = (torch.randn(s, device=DEV) * 0.5 for s in ((heads,), (heads,), (heads,), (heads, dim)))
+    cu = torch.tensor([0] + lens, device=DEV).cumsum(0).int()
+    slots = torch.arange(len(lens), dtype=torch.int32, device=DEV)
+    start = torch.zeros(len(lens), heads, k.recurrent_state_floats(dim, vdim), device=DEV)
+
+    def run(x, gates, decay, chunked):
+        a, b, c = x[:, :gh * dim], x[:, gh * dim:2 * gh * dim], x[:, 2 * gh * dim:2 * gh * dim + heads * vdim]
+        st, y = start.clone(), torch.empty(ntok, heads * vdim, device=DEV)
+        if form == "delta":
+            k.delta_rule(a, b, c, gates[:, :heads], gates[:, heads:], a_log, dt_bias, st, cu, slots, y, heads, groups, dim, vdim,
+                         dim ** -0.5, chunked=chunked)
+        elif form == "channel_delta":
+            k.channel_delta_rule(a, b, c, gates[:, :heads], decay, st, cu, slots, y, heads, groups, dim, vdim, dim ** -0.5, chunked=chunked)
+        elif form == "ssd":
+            k.ssd_scan(c, b, a, gates[:, :heads], a_log, dt_bias, skip, st, cu, slots, y, heads, groups, dim, vdim, chunked=chunked)
+        else:
+            k.wkv_scan(a, b, decay, c, bonus if form == "before" else None, st, cu, slots, y, heads, dim, vdim, 1.0, chunked=chunked)
+        return y, st
+
+    clean, _ = run(x, gates, decay, True)
+    assert clean.isfinite().all()
+    x, gates, decay = x.clone(), gates.clone(), decay.clone()
+    for t in bad:
+        if what == "gate":
+            gates[t, 0] = gates[t, heads] = float("nan")
+            decay[t, 1] = float("nan")
+        else:
+            x[t, {"q": 0, "k": gh * dim, "v": 2 * gh * dim}[what] + 2] = value
+    (y, st), (y_walk, st_walk) = run(x, gates, decay, True), run(x, gates, decay, False)
+    for i, at in enumerate(cu[:-1].tolist()):
+        first = min([t for t in bad if at <= t < at + lens[i]], default=at + lens[i])
+        assert torch.equal(y[at:first], clean[at:first]), i
+    assert torch.equal(y.isfinite(), y_walk.isfinite()) and torch.equal(st.isfinite(), st_walk.isfinite())
+    assert not y.isfinite().all()
