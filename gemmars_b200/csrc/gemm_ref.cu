@@ -257,6 +257,9 @@ static int launch_f32(int tile, const F32Call& c, int mode, cudaStream_t stream)
   }
 }
 
+// Which of F32_TILES a float32 product of these sizes takes (-1: none).
+GB_EXPORT int gb_gemm_ref_tile(int M, int N) { return pick_f32_tile(M, N); }
+
 // x: [M, K] rows ldx apart; w: [N, K]; y: [M, N] rows ldy apart.
 // mode OUT_STORE writes y in out_dtype; OUT_ACCUMULATE_F32 adds into a float32 y.  act: an activation of
 // product + bias; col_scale (null: ones): [N], multiplied in after it, before the store or the add.

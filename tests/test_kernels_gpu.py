@@ -106,8 +106,17 @@ def test_gemm_ref_float32_rows_do_not_depend_on_the_batch(k):
         assert torch.equal(part, full[13:13 + rows])
 
 
-@pytest.mark.parametrize("m,n,kk", [(1, 31, 4), (4, 32, 64), (5, 1033, 1023), (8, 4100, 128), (17, 9000, 36), (33, 4096, 260),
-                                    (100, 6144, 68), (301, 6144, 100), (129, 19000, 33), (700, 4000, 16)])
+F32_SIZES = [(1, 31, 4), (4, 32, 64), (5, 1033, 1023), (8, 4100, 128), (17, 9000, 36), (33, 4096, 260), (12, 16001, 100), (32, 9000, 68),
+             (100, 6144, 68), (301, 6144, 100), (129, 19000, 33), (700, 4000, 16)]
+
+
+def test_the_float32_sizes_reach_every_tile(k):
+    from gemmars_b200.csrc import build
+    tile = build.load("gemm_ref").gb_gemm_ref_tile
+    assert {tile(m, n) for m, n, _ in F32_SIZES} == set(range(6))
+
+
+@pytest.mark.parametrize("m,n,kk", F32_SIZES)
 def test_gemm_ref_float32_gives_the_same_bits_on_every_tile(k, m, n, kk):
     """Sizes that reach each tile, with remainders in every direction; rows that start at 16-byte boundaries and rows that
     do not.  A row alone runs on the smallest tile: its bits must be those of the row among the others."""
