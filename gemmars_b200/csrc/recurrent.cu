@@ -912,6 +912,12 @@ __device__ __forceinline__ void load8(const bf16* p, float (&v)[8]) {
 //   LR_PLAIN:    a + base[c]
 // with a = sum_j W[c, j] z[t, j]; base may be null (zeros).
 enum { LR_TANH_EXPEXP = 0, LR_RATE = 1, LR_SIGMOID_ROOT = 2, LR_PLAIN = 3 };
+__device__ __forceinline__ float lowrank_result(float a, int mode, float rt, float inv_tau) {
+  if (mode == LR_TANH_EXPEXP) return expf(-expf(a));
+  if (mode == LR_RATE) return expf(-rt * softplus_f(a));
+  if (mode == LR_SIGMOID_ROOT) return expf(-softplus_f(-a) * inv_tau);
+  return a;
+}
 template <typename T>
 __global__ void __launch_bounds__(128) lowrank_decay_kernel(const float* __restrict__ z, long long ldz, int rank,
                                                            const T* __restrict__ W, const float* __restrict__ base,
@@ -964,106 +970,101 @@ __global__ void __launch_bounds__(128) lowrank_decay_kernel(const float* __restr
 #pragma unroll
   for (int tt = 0; tt < DEC_TOK; ++tt)
     if (tt < n) {
-      const float a = acc[tt] + b;
-      float r;
-      if (mode == LR_TANH_EXPEXP) r = expf(-expf(a));
-      else if (mode == LR_RATE) r = expf(-rt * softplus_f(a));
-      else if (mode == LR_SIGMOID_ROOT) r = expf(-softplus_f(-a) * inv_tau);
-      else r = a;
-      w[(size_t)(t0 + tt) * C + c] = r;
+      w[(size_t)(t0 + tt) * C + c] = lowrank_result(acc[tt] + b, mode, rt, inv_tau);
     }
 }
 
-// Prompts with a bfloat16 W: the sums on the tensor cores.  A CTA is 64 rows by four times 64 channels, a warp 16 rows; z (or tanh z) is
-// split into two tf32 halves, hi + lo, whose products with the bfloat16 numbers of W are exact in float32, so a sum is as
-// good as one of float32 products.  (lo is cut at 2^-21 of z.)  The inner index is taken in pairs: lane t's two neighbouring
-// k stand for the instruction's t and t + 4.  Bound by the exponentials of the results: 2,048 rows, 4,096 channels, rank 64,
-// two exponentials: 70 us with FFMA, 47 so.
-constexpr int LR_ROWS = 64, LR_COLS = 64, LR_K = 64, LR_TILES = 4;
-__device__ __forceinline__ void mma_tf32(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-__global__ void __launch_bounds__(128) lowrank_mma_kernel(const float* __restrict__ z, long long ldz, int rank, const bf16* __restrict__ W,
-                                                         const float* __restrict__ base, float* __restrict__ w, int ntok, int C,
-                                                         int mode, const float* __restrict__ rate, int rate_group, float inv_tau) {
-  constexpr int LD = LR_K + 8;
-  __shared__ __align__(16) float hi[LR_ROWS][LD], lo[LR_ROWS][LD];
+// Prompts with a bfloat16 W: a CTA is LT_TOK tokens by LT_CH channels, a thread 8 x 8 of them; LT_K entries of the rank of both lie
+// in shared memory, a channel or token side by side, so that a thread's 16-byte reads (four an entry) feed 64 multiply-adds.  Every
+// sum is that of the kernel above, product by product: the same bits.  Bound by the multiply-adds and the results'
+// exponentials.  (The kernel above is bound by its shared-memory reads, two for eight multiply-adds.  On the tensor cores, z in two tf32
+// halves, the sums were cut towards zero by up to 1e-6 at a rank of 192, and few wide CTAs left most SMs idle.)
+constexpr int LT_TOK = 64, LT_CH = 128, LT_K = 16;
+__global__ void __launch_bounds__(128) lowrank_tile_kernel(const float* __restrict__ z, long long ldz, int rank, const bf16* __restrict__ W,
+                                                          const float* __restrict__ base, float* __restrict__ w, int ntok, int C,
+                                                          int mode, const float* __restrict__ rate, int rate_group, float inv_tau) {
+  __shared__ __align__(16) float zs[LT_K][LT_TOK + 4], ws[LT_K][LT_CH + 4];
   pdl_release_next();
   pdl_wait_prior();
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-  const int t0 = blockIdx.y * LR_ROWS;
-  auto bring = [&](int k0) {
-    __syncthreads();
-#pragma unroll 8
-    for (int e = tid; e < LR_ROWS * LR_K; e += 128) {
-      const int r = e / LR_K, k = e % LR_K;
-      float v = t0 + r < ntok && k0 + k < rank ? z[(size_t)(t0 + r) * ldz + k0 + k] : 0.f;
-      if (mode == LR_TANH_EXPEXP) v = tanhf(v);
-      const float h = __uint_as_float((__float_as_uint(v) + 0x1000u) & 0xffffe000u);
-      hi[r][k] = h;
-      lo[r][k] = v - h;
-    }
-    __syncthreads();
-  };
-  if (rank <= LR_K) bring(0);
-#pragma unroll 1
-  for (int tile = 0; tile < LR_TILES; ++tile) {
-    const int c0 = (blockIdx.x * LR_TILES + tile) * LR_COLS;
-    if (c0 >= C) return;
-    float acc[LR_COLS / 8][4] = {};
-    for (int k0 = 0; k0 < rank; k0 += LR_K) {
-      if (rank > LR_K) bring(k0);
-      const int steps = min(LR_K, rank - k0 + 7) / 8;
-      for (int s = 0; s < steps; ++s) {
-        const float *h0 = &hi[warp * 16 + g][8 * s + 2 * t], *l0 = &lo[warp * 16 + g][8 * s + 2 * t];
-        const float2 ha = *(const float2*)h0, hb = *(const float2*)(h0 + 8 * LD), la = *(const float2*)l0, lb = *(const float2*)(l0 + 8 * LD);
-        const uint32_t ah[4] = {__float_as_uint(ha.x), __float_as_uint(hb.x), __float_as_uint(ha.y), __float_as_uint(hb.y)};
-        const uint32_t al[4] = {__float_as_uint(la.x), __float_as_uint(lb.x), __float_as_uint(la.y), __float_as_uint(lb.y)};
-        const int k = k0 + 8 * s + 2 * t;
+  const int tid = threadIdx.x, c0 = blockIdx.x * LT_CH, t0 = blockIdx.y * LT_TOK;
+  const int tx = tid & 15, ty = tid >> 4;            // channels tx * 4 and 64 + tx * 4, tokens ty * 4 and 32 + ty * 4, four each
+  const bf16* wrow = W + (size_t)min(c0 + tid, C - 1) * rank;
+  const int zt = tid & 63, zk = (tid >> 6) * (LT_K / 2);
+  const float* zrow = z + (size_t)min(t0 + zt, ntok - 1) * ldz;
+  const bool vec = rank % 8 == 0 && ((uintptr_t)W & 15) == 0;
+  float acc[8][8] = {};                              // [token][channel]
+  for (int k0 = 0; k0 < rank; k0 += LT_K) {
+    float wv[LT_K], zv[LT_K / 2];
 #pragma unroll
-        for (int n = 0; n < LR_COLS / 8; ++n) {
-          const int c = c0 + 8 * n + g;
-          const uint32_t p = c < C && k < rank ? *(const uint32_t*)(W + (size_t)c * rank + k) : 0u;
-          mma_tf32(acc[n], ah, p << 16, p & 0xffff0000u);
-          mma_tf32(acc[n], al, p << 16, p & 0xffff0000u);
-        }
+    for (int k = 0; k < LT_K; k += 8) {
+      if (vec && k0 + k < rank) {                    // whole eights
+        float v[8];
+        load8(wrow + k0 + k, v);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) wv[k + e] = v[e];
+      } else {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) wv[k + e] = k0 + k + e < rank ? to_f32(wrow[k0 + k + e]) : 0.f;
       }
     }
 #pragma unroll
-    for (int n = 0; n < LR_COLS / 8; ++n) {
-      const int c = c0 + 8 * n + 2 * t;
-      float bs[2], rt[2];
+    for (int k = 0; k < LT_K / 2; ++k) {
+      const float v = k0 + zk + k < rank ? zrow[k0 + zk + k] : 0.f;
+      zv[k] = mode == LR_TANH_EXPEXP ? tanhf(v) : v;
+    }
+    __syncthreads();                                 // the entries before have been read
 #pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const int ce = min(c + e, C - 1);
-        bs[e] = base ? base[ce] : 0.f;
-        rt[e] = mode == LR_RATE ? expf(rate[ce / rate_group]) : 0.f;
-      }
+    for (int k = 0; k < LT_K; ++k) ws[k][tid] = wv[k];
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int row = t0 + warp * 16 + g + 8 * h;
-        if (row >= ntok) continue;
-        float r[2];
+    for (int k = 0; k < LT_K / 2; ++k) zs[zk + k][zt] = zv[k];
+    __syncthreads();
+    const int n = min(LT_K, rank - k0);
+#pragma unroll 4
+    for (int k = 0; k < n; ++k) {
+      const float4 z0 = *(const float4*)&zs[k][ty * 4], z1 = *(const float4*)&zs[k][32 + ty * 4];
+      const float4 w0 = *(const float4*)&ws[k][tx * 4], w1 = *(const float4*)&ws[k][64 + tx * 4];
+      const float a[8] = {z0.x, z0.y, z0.z, z0.w, z1.x, z1.y, z1.z, z1.w}, b[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
 #pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const float a = acc[n][2 * h + e] + bs[e];
-          if (mode == LR_TANH_EXPEXP) r[e] = expf(-expf(a));
-          else if (mode == LR_RATE) r[e] = expf(-rt[e] * softplus_f(a));
-          else if (mode == LR_SIGMOID_ROOT) r[e] = expf(-softplus_f(-a) * inv_tau);
-          else r[e] = a;
-        }
-        float* to = w + (size_t)row * C + c;
-        if (c + 1 < C && C % 2 == 0) {
-          *(float2*)to = make_float2(r[0], r[1]);
-        } else {
-          if (c < C) to[0] = r[0];
-          if (c + 1 < C) to[1] = r[1];
-        }
+      for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(b[j], a[i], acc[i][j]);
+    }
+  }
+  const bool wide = C % 4 == 0 && ((uintptr_t)w & 15) == 0;
+#pragma unroll
+  for (int jq = 0; jq < 2; ++jq) {
+    const int c = c0 + 64 * jq + tx * 4;
+    float bs[4], rt[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int cj = min(c + j, C - 1);
+      bs[j] = base ? base[cj] : 0.f;
+      rt[j] = mode == LR_RATE ? expf(rate[cj / rate_group]) : 0.f;
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int t = t0 + 32 * (i >> 2) + ty * 4 + (i & 3);
+      if (t >= ntok) continue;
+      float r[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) r[j] = lowrank_result(acc[i][4 * jq + j] + bs[j], mode, rt[j], inv_tau);
+      float* to = w + (size_t)t * C + c;
+      if (wide && c + 3 < C) {
+        *(float4*)to = make_float4(r[0], r[1], r[2], r[3]);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (c + j < C) to[j] = r[j];
       }
     }
   }
+}
+
+// Tiles are wide: they want three an SM and a rank that is worth laying out (us, the kernel of rows / of tiles, plain: 1,024
+// tokens of 1,024 channels, rank 64, 10.8 / 13.0; of 4,096 35.7 / 25.5; 2,048 of 4,096 66.9 / 50.7, two exponentials 68.6 / 53.9,
+// a rate 74 / 68; rank 16 20.0 / 16.7, but a rate 33.8 / 37.5).
+static bool lowrank_tiles(int ntok, int C, int rank) {
+  return rank >= 32 && (long long)((C + LT_CH - 1) / LT_CH) * ((ntok + LT_TOK - 1) / LT_TOK) >= 3 * 148;
 }
 
 // z: [ntok, rank] float32; W: [C, rank] float32 or bfloat16; base: [C]; w: [ntok, C] float32.
@@ -1082,8 +1083,8 @@ GB_EXPORT int gb_lowrank_map(const float* z, long long ldz, int rank, const void
   if (w_dtype == GB_F32)
     gb_launch(lowrank_decay_kernel<float>, grid, 128, 0, stream, z, ldz, rank, (const float*)W, base, w, ntok, C, mode, rate,
               rate_group, inv_tau);
-  else if (w_dtype == GB_BF16 && ntok >= 128 && rank % 2 == 0 && !((uintptr_t)W & 3) && !((uintptr_t)w & 7))
-    gb_launch(lowrank_mma_kernel, dim3((C + LR_TILES * LR_COLS - 1) / (LR_TILES * LR_COLS), (ntok + LR_ROWS - 1) / LR_ROWS), 128, 0, stream, z, ldz, rank,
+  else if (w_dtype == GB_BF16 && lowrank_tiles(ntok, C, rank))
+    gb_launch(lowrank_tile_kernel, dim3((C + LT_CH - 1) / LT_CH, (ntok + LT_TOK - 1) / LT_TOK), 128, 0, stream, z, ldz, rank,
               (const bf16*)W, base, w, ntok, C, mode, rate, rate_group, inv_tau);
   else if (w_dtype == GB_BF16)
     gb_launch(lowrank_decay_kernel<bf16>, grid, 128, 0, stream, z, ldz, rank, (const bf16*)W, base, w, ntok, C, mode, rate,

@@ -101,8 +101,6 @@ def test_chunks_of_a_prompt(form, heads, groups, dim, vdim, turns, monkeypatch):
     (y_err, s_err), (y_walk, s_walk) = run(True), run(False)
     # a few roundings of 2^-24 an element, and what the split products leave out (2^-21 of a product at most, of either sign)
     assert y_err < 1.5e-6 and s_err < 1.5e-6, (y_err, s_err, y_walk, s_walk)
-    # no less exact than token by token: the state; and the outputs but for a decay or a head's gates that stand before whole rows
-    assert s_err < 1.15 * s_walk + 2e-8 and y_err < 1.5 * y_walk + 2e-8, (y_err, s_err, y_walk, s_walk)
 
 
 @pytest.mark.parametrize("heads,groups,dim,vdim", [(4, 2, 128, 128), (2, 1, 64, 64), (3, 3, 12, 33), (40, 20, 128, 40), (24, 12, 128, 128)])
@@ -151,3 +149,44 @@ def test_a_number_that_is_not_finite_reaches_what_it_reaches_token_by_token(form
         assert torch.equal(y[at:first], clean[at:first]), i
     assert torch.equal(y.isfinite(), y_walk.isfinite()) and torch.equal(st.isfinite(), st_walk.isfinite())
     assert not y.isfinite().all()
+
+
+@pytest.mark.parametrize("ntok,nseq,dims", [(1, 1, 1), (16, 1, 64), (17, 3, 65), (2048, 1, 128), (1000, 40, 100)])
+@pytest.mark.parametrize("delta", [False, True])
+def test_scratch_of_a_step(ntok, nseq, dims, delta):
+    """The size that the step works out is the library's."""
+    import ctypes
+    from gemmars_b200 import kernels as k
+    from gemmars_b200.csrc import build
+    f = build.load("recurrent_chunk").gb_chunk_floats
+    f.restype = ctypes.c_longlong
+    assert f(ntok, nseq, dims, int(delta)) == k.chunk_floats(ntok, nseq, dims, delta)
+
+
+@pytest.mark.parametrize("heads,dim,vdim", [(4, 128, 128), (3, 64, 64), (2, 100, 40)])
+@pytest.mark.parametrize("form", ["ssd", "before", "after"])
+def test_sums_of_one_sign_are_not_cut(form, heads, dim, vdim):
+    """A state that 1,000 tokens only add to: its numbers are off by roundings of either sign.  The tensor core's cut of every sum
+    would make them 0.72 x 2^-24 (4.3e-8) and more too small on the mean, a cut operand 2^-24; token by token the mean is below 1e-8."""
+    from gemmars_b200 import kernels as k
+    torch.manual_seed(dim)
+    ntok, lanes = 1000, 2 if dim <= 64 else 4
+    x = torch.rand(ntok, heads * (2 * dim + vdim), device=DEV) + 0.5
+    a, b, c = x[:, :heads * dim], x[:, heads * dim:2 * heads * dim], x[:, 2 * heads * dim:]
+    cu, slots = torch.tensor([0, ntok], dtype=torch.int32, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+    one = torch.ones(ntok, heads * dim, device=DEV)
+    steps, a_log = torch.rand(ntok, heads, device=DEV), torch.full((heads,), -60.0, device=DEV)      # exp(-e^-60 dt) is 1
+    for chunked in (True, False):
+        st, y = torch.zeros(1, heads, k.recurrent_state_floats(dim, vdim), device=DEV), torch.empty(ntok, heads * vdim, device=DEV)
+        scale = 1.0
+        if form == "ssd":
+            zero = torch.zeros(heads, device=DEV)
+            k.ssd_scan(c, b, a, steps, a_log, zero, zero, st, cu, slots, y, heads, heads, dim, vdim, chunked=chunked)
+            scale = torch.nn.functional.softplus(steps).double()[:, :, None]       # as the kernel has them, in float32
+        else:
+            k.wkv_scan(a, b, one, c, torch.ones(heads, dim, device=DEV) if form == "before" else None, st, cu, slots, y, heads, dim, vdim,
+                       1.0, chunked=chunked)
+        held = st[0].view(heads, 8, vdim, lanes, 4).permute(0, 3, 1, 4, 2).reshape(heads, -1, vdim)[:, :dim]
+        want = torch.einsum("thd,thv->hdv", b.double().reshape(ntok, heads, dim) * scale, c.double().reshape(ntok, heads, vdim))
+        off = (held.double() / want - 1.0).mean().item()
+        assert abs(off) < 2e-8, (chunked, off)

@@ -100,3 +100,25 @@ def test_low_rank_maps_of_prompts(rows, channels, rank, mode):
         out, want = k.lowrank_map(z, w, base, "plain"), a
     # a sum of `rank` products rounded to 24 bits each, through functions of slope at most 1 (2.3 for the rates drawn)
     assert (out.double() - want).abs().max() <= 4e-6
+
+
+@pytest.mark.parametrize("rows,channels,rank", [(2048, 2048, 64), (2011, 2050, 40), (1999, 2003, 33), (1700, 2200, 200)])
+@pytest.mark.parametrize("mode", ["tanh_expexp", "rate", "sigmoid_root", "plain"])
+def test_low_rank_maps_of_long_prompts_give_the_bits_of_few_tokens(rows, channels, rank, mode):
+    """Many tokens by many channels run in tiles, a few tokens by rows: the same sums, infinities included."""
+    from gemmars_b200 import kernels as k
+    torch.manual_seed(rows + rank)
+    z = torch.randn(rows, rank + 3, device=DEV)[:, 1:1 + rank]
+    z[rows // 3, 5], z[rows // 2, 7] = float("inf"), float("-inf")
+    w, base = (torch.randn(channels, rank, device=DEV) * rank ** -0.5).bfloat16(), torch.randn(channels, device=DEV)
+    more = {"rate": torch.randn(channels, device=DEV) * 0.5} if mode == "rate" else {}
+    out = k.lowrank_map(z, w, base, mode, tau=4.0, **more)
+    for at in (0, rows // 3 - 1, rows // 2 - 2, rows - 3):
+        assert torch.equal(k.lowrank_map(z[at:at + 3], w, base, mode, tau=4.0, **more).nan_to_num(7.0), out[at:at + 3].nan_to_num(7.0))
+    keep = torch.ones(rows, dtype=torch.bool, device=DEV)
+    keep[rows // 3] = keep[rows // 2] = False
+    a = (torch.tanh(z.double()) if mode == "tanh_expexp" else z.double()) @ w.double().T + base.double()
+    want = {"tanh_expexp": lambda: torch.exp(-torch.exp(a)), "sigmoid_root": lambda: torch.sigmoid(a) ** 0.25, "plain": lambda: a,
+            "rate": lambda: torch.exp(-torch.exp(more["rate"].double()) * torch.nn.functional.softplus(a))}[mode]()
+    # a sum of `rank` products rounded to 24 bits each, through functions of slope at most 1 (2.3 for the rates drawn)
+    assert (out.double() - want)[keep].abs().max() <= 6e-6
