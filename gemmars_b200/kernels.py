@@ -1811,12 +1811,9 @@ def recurrent_state_matrix(head_state: torch.Tensor, dims: int, vdim: int) -> to
     return head_state.reshape(8, vdim, lanes, 4).permute(2, 0, 3, 1).reshape(32 * lanes, vdim)[:dims]
 
 
-# A prompt step takes the recurrences in chunks of 16 tokens (recurrent_chunk.cu) where a sequence brings at least
-# this many, in the bfloat16 engine only: the float32 engine's results must not depend on how a prompt is cut into
-# steps, bit for bit, and a chunk's sums are grouped by where the step begins.
-# Both sides (us, token by token / in chunks; one sequence): delta rule, 32 heads: 24 tokens 20 / 24, 32 24 / 24, 48
-# 34 / 25, 64 43 / 25; wkv, 64 heads: 32 21 / 26, 48 26 / 26, 64 34 / 26; state space: 32 18 / 21, 48 24 / 21, 64 30 / 21;
-# four sequences of 32: 41 / 33, 24 / 26 and 22 / 21.
+# A prompt step takes the recurrences in chunks of 16 tokens (recurrent_chunk.cu) in the bfloat16 engine only: the float32
+# engine's results must not depend on how a prompt is cut into steps, bit for bit, and a chunk's sums are grouped by where the
+# step begins.
 CHUNK_SCAN_MIN_TOKENS = 32
 CHUNK_SCAN_MAX_DIM = 128
 #: bytes of scratch a step's chunks may take (a block a chunk and head); the kernels take the heads in turns beyond it
@@ -1828,15 +1825,52 @@ def chunk_scan_usable(compute: str, max_new: int, dim: int) -> bool:
     return compute != "float32" and max_new >= CHUNK_SCAN_MIN_TOKENS and dim <= CHUNK_SCAN_MAX_DIM
 
 
+# Which steps.  A layer launched from Python is bound by its launches for short prompts, and a chunk's form has one more; the
+# walk's time grows with the longest sequence, and beyond about 80 pairs of a sequence and a head with the pairs.  So the line is on
+# longest x (80 + pairs), by form (us a layer, walk / chunks, widths 2,048 and 4,096; one sequence, then four):
+#   delta rule          64 tokens 99 / 106 and 109 / 104, 96 107 / 108 and 135 / 106, 128 131 / 109 and 162 / 105; 4 x 64 107 / 111 and 182 / 156
+#   decay per channel   96 124 / 130 and 132 / 132, 128 131 / 131 and 157 / 133; 4 x 64 124 / 132 and 185 / 141
+#   state space         128 96 / 104 and 115 / 103, 192 117 / 104 and 155 / 114; 4 x 64 96 / 104 and 172 / 131
+#   read before (wkv)   128 163 / 170 and 181 / 171, 256 193 / 171 and 250 / 175; 4 x 128 163 / 169 and 304 / 217
+#   read after          128 101 / 108 and 113 / 110, 256 131 / 109 and 162 / 113; 4 x 128 102 / 110 and 211 / 134
+CHUNK_SCAN_LINES = {"delta": 9500, "channel_delta": 13000, "ssd": 19500, "before": 20500, "after": 15500}
+# A single token beside a prompt costs a chunk's work in every head, which only a long prompt makes up for: heads x places for
+# tokens that stay empty in the step's chunks, per token of the longest sequence (delta rule, 16 heads: 128 single tokens and a prompt of
+# 64 159 / 217, of 128 217 / 235, of 512 569 / 335; 32 single tokens and one of 128 166 / 118).
+CHUNK_SCAN_EMPTY_PLACES = 96
+
+
+def chunk_scan_pays(form: str, max_new: int, heads: int, ntok: int, nseq: int, chunks: int) -> bool:
+    """Whether a step of ``nseq`` sequences (the longest of ``max_new`` tokens, ``ntok`` and ``chunks`` in all) is faster chunk by
+    chunk, as a layer launched from Python."""
+    return (max_new * (80 + nseq * heads) >= CHUNK_SCAN_LINES[form]
+            and heads * (16 * chunks - ntok) <= CHUNK_SCAN_EMPTY_PLACES * max_new)
+
+
+def chunk_scan(form: str, compute: str, dim: int, heads: int, ctx) -> bool:
+    """Whether a recurrent mixer walks the step's recurrences chunk by chunk."""
+    if not chunk_scan_usable(compute, ctx.max_new, dim):
+        return False
+    chunks = ctx.extras.get("recurrent_chunks")
+    if chunks is None:
+        chunks = ctx.n_tokens // 16 + ctx.n_seqs if ctx.host is None else sum(-(-int(n) // 16) for n in ctx.host["seq_len"])
+        ctx.extras["recurrent_chunks"] = chunks
+    return chunk_scan_pays(form, ctx.max_new, heads, ctx.n_tokens, ctx.n_seqs, chunks)
+
+
 def recurrent_units(compute: str, dim: int):
     """The units a recurrent mixer with keys of ``dim`` launches."""
     return [("recurrent", ())] + ([("recurrent_chunk", ())] if chunk_scan_usable(compute, CHUNK_SCAN_MIN_TOKENS, dim) else [])
 
 
+def chunk_floats(ntok: int, nseq: int, dims: int, delta: bool) -> int:
+    """Floats of scratch that one head of a step's chunks needs (gb_chunk_floats, without a call into the library)."""
+    dp = 64 if dims <= 64 else 128
+    return (ntok // 16 + nseq) * ((3 if delta else 2) * dp * 16 + (2 if delta else 1) * 256 + dp)
+
+
 def _chunk_scratch(ntok: int, nseq: int, heads: int, dim: int, delta: bool, device) -> torch.Tensor:
-    f = _fn("recurrent_chunk", "gb_chunk_floats", [c_int, c_int, c_int, c_int])
-    f.restype = c_longlong
-    per = f(ntok, nseq, dim, int(delta))
+    per = chunk_floats(ntok, nseq, dim, delta)
     at_once = max(1, min(heads, CHUNK_SCAN_SCRATCH // (4 * per)))
     turns = -(-heads // at_once)
     return torch.empty(per * -(-heads // turns), dtype=torch.float32, device=device)

@@ -96,7 +96,7 @@ class ChannelDeltaRule(Part):
         y = torch.empty((t, hv), dtype=torch.float32, device=p.device)
         kernels.channel_delta_rule(f[:, :qk], f[:, qk:2 * qk], f[:, 2 * qk:], p[:, c:c + nh], decay, state, ctx.cu_seqlens,
                                    ctx.seq_slot, y, nh, self.kv_heads, self.dim, self.vdim, float(self.dim) ** -0.5,
-                                   chunked=kernels.chunk_scan_usable(self.compute, ctx.max_new, self.dim))
+                                   chunked=kernels.chunk_scan("channel_delta", self.compute, self.dim, self.heads, ctx))
         out = torch.empty((t, hv), dtype=self.act_dtype, device=p.device)
         kernels.gated_group_norm(y, gate, self.norm, out, self.vdim, self.eps, False, self.out_scale, gate_act="sigmoid")
         self.o.add_into(out, residual)

@@ -84,7 +84,7 @@ class GatedDeltaRule(Part):
         kernels.delta_rule(f[:, :qk], f[:, qk:2 * qk], f[:, 2 * qk:], p[:, c + hv:c + hv + nh], p[:, c + hv + nh:],
                            self.a_log, self.dt_bias, state, ctx.cu_seqlens, ctx.seq_slot, y, nh, self.kv_heads, self.dim,
                            self.vdim, float(self.dim) ** -0.5,
-                           chunked=kernels.chunk_scan_usable(self.compute, ctx.max_new, self.dim))
+                           chunked=kernels.chunk_scan("delta", self.compute, self.dim, self.heads, ctx))
         out = torch.empty((t, hv), dtype=self.act_dtype, device=p.device)
         kernels.gated_group_norm(y, p[:, c:c + hv], self.norm, out, self.vdim, self.eps, False, self.out_scale)
         self.o.add_into(out, residual)

@@ -78,7 +78,7 @@ class GatedLinearAttention(Part):
         y = torch.empty((t, hv), dtype=torch.float32, device=p.device)
         kernels.wkv_scan(p[:, :hd], p[:, hd:2 * hd], alpha, p[:, 2 * hd:2 * hd + hv], None, state, ctx.cu_seqlens,
                          ctx.seq_slot, y, self.heads, self.dim, self.vdim, out_scale=float(self.dim) ** -0.5,
-                         chunked=kernels.chunk_scan_usable(self.compute, ctx.max_new, self.dim))
+                         chunked=kernels.chunk_scan("after", self.compute, self.dim, self.heads, ctx))
         gate = self.g(h, out_dtype=torch.float32)
         out = torch.empty((t, hv), dtype=self.act_dtype, device=p.device)
         kernels.gated_group_norm(y, gate, self.norm, out, self.vdim, self.eps, False, self.out_scale)

@@ -83,7 +83,7 @@ class StateSpaceDual(Part):
         y = torch.empty((t, inner), dtype=torch.float32, device=p.device)
         kernels.ssd_scan(f[:, :inner], f[:, inner:inner + gn], f[:, inner + gn:], p[:, inner + c:], self.a_log, self.dt_bias,
                          self.skip, state, ctx.cu_seqlens, ctx.seq_slot, y, self.heads, self.groups, self.n_state, self.vdim,
-                         chunked=kernels.chunk_scan_usable(self.compute, ctx.max_new, self.n_state))
+                         chunked=kernels.chunk_scan("ssd", self.compute, self.n_state, self.heads, ctx))
         out = torch.empty((t, inner), dtype=self.act_dtype, device=p.device)
         kernels.gated_group_norm(y, p[:, :inner], self.norm, out, inner // self.norm_groups, self.eps, True, self.out_scale)
         self.o.add_into(out, residual)

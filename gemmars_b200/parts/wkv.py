@@ -82,7 +82,7 @@ class DecayedLinearAttention(Part):
         decay = kernels.lowrank_decay(self.w1(mixes[4], out_dtype=torch.float32), self.w2, self.w0)
         y = torch.empty((h.shape[0], self.inner), dtype=torch.float32, device=h.device)
         kernels.wkv_scan(r, k, decay, v, self.u, state, ctx.cu_seqlens, ctx.seq_slot, y, self.heads, self.dim, self.dim,
-                         chunked=kernels.chunk_scan_usable(self.compute, ctx.max_new, self.dim))
+                         chunked=kernels.chunk_scan("before", self.compute, self.dim, self.heads, ctx))
         out = torch.empty((h.shape[0], self.inner), dtype=self.act_dtype, device=h.device)
         kernels.gated_group_norm(y, gate, self.norm, out, self.dim, self.eps, False, self.out_scale)
         self.o.add_into(out, residual)
