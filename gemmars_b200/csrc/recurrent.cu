@@ -217,13 +217,16 @@ GB_EXPORT int gb_short_filter(const void* u, int in_dtype, long long ldu, const 
 #undef GB_SINGLE
     return gb_launch_status();
   }
+  // four channels a thread want prompts whose blocks still fill the chip (us, one channel a thread / four: 300 tokens of 8,192 24 / 31,
+  // 1,000 of 1,024 8.5 / 9.8, of 2,048 10.8 / 10.9, of 8,192 27 / 22.5)
+  const dim3 grid4((ntok + per - 1) / per, (C / 4 + 127) / 128);
   const bool wide = in_dtype == GB_F32 && out_dtype == GB_F32 && K >= 2 && K <= 4 && C % 4 == 0 && ldu % 4 == 0 && ldo % 4 == 0 &&
-                    !(((uintptr_t)u | (uintptr_t)out | (uintptr_t)state) & 15);
+                    per > 1 && grid4.x * grid4.y >= 2 * 148 && !(((uintptr_t)u | (uintptr_t)out | (uintptr_t)state) & 15);
 #define GB_FILTER(T, O)                                                                                                   \
   gb_launch(short_filter_kernel<T, O>, grid, 256, 0, stream, (const T*)u, ldu, taps, bias, (const float*)state, cu, tok_seq, \
             seq_slot, (O*)out, ldo, ntok, per, C, K, act)
   if (wide)
-    gb_launch(short_filter_wide_kernel, dim3((ntok + per - 1) / per, (C / 4 + 127) / 128), 128, 0, stream, (const float*)u, ldu, taps,
+    gb_launch(short_filter_wide_kernel, grid4, 128, 0, stream, (const float*)u, ldu, taps,
               bias, (const float*)state, cu, tok_seq, seq_slot, (float*)out, ldo, ntok, per, C, K, act);
   else if (in_dtype == GB_F32 && out_dtype == GB_F32) GB_FILTER(float, float);
   else if (in_dtype == GB_F32 && out_dtype == GB_BF16) GB_FILTER(float, bf16);
@@ -870,7 +873,9 @@ GB_EXPORT int gb_shift_mix(const void* x, int dtype, long long ldx, const float*
     gb_launch(shift_mix_kernel<float>, grid, 256, 0, stream, (const float*)x, ldx, mu, state, cu, tok_seq, seq_slot, (float*)out,
               ntok, C, n_mix, single);
     if (!single) gb_launch(shift_state_kernel<float>, sgrid, 256, 0, stream, (const float*)x, ldx, state, cu, seq_slot, C);
-  } else if (dtype == GB_BF16 && !single && ntok >= 64 && C % 8 == 0 && ldx % 8 == 0 &&
+  // eight rows and channels a thread leave few blocks (us, one of each / eight: 128 tokens of 2,048 channels 6.8 / 8.0, 96 of 6,144 in 33
+  // sequences 9.1 / 11.1, 300 of 1,024 6.8 / 7.7)
+  } else if (dtype == GB_BF16 && !single && (long long)((ntok + SHIFT_ROWS - 1) / SHIFT_ROWS) * ((C / 8 + 127) / 128) >= 148 && C % 8 == 0 && ldx % 8 == 0 &&
              !(((uintptr_t)x | (uintptr_t)out | (uintptr_t)mu) & 15)) {
     gb_launch(shift_mix_wide_kernel, dim3((ntok + SHIFT_ROWS - 1) / SHIFT_ROWS, (C / 8 + 127) / 128), 128, 0, stream, (const bf16*)x, ldx,
               mu, (const float*)state, cu, tok_seq, seq_slot, (bf16*)out, ntok, C, n_mix);

@@ -14,7 +14,7 @@ def _packed(lens, slots):
 
 
 @pytest.mark.parametrize("lens", [[600], [1, 2, 513, 3, 16, 1], [40, 2, 1]])
-@pytest.mark.parametrize("channels", [64, 516, 67])
+@pytest.mark.parametrize("channels", [64, 516, 67, 5124])
 @pytest.mark.parametrize("taps,bias,act", [(2, True, True), (3, False, False), (4, True, True), (5, False, True)])
 def test_short_filter_of_prompts(lens, channels, taps, bias, act):
     from gemmars_b200 import kernels as k
@@ -60,7 +60,7 @@ def test_gated_norm_of_whole_groups(rows, n, group, wn, first, act, dtype):
         assert ((out.double() - want).abs() <= tol * want.abs() + 1e-6).all()
 
 
-@pytest.mark.parametrize("lens", [[64], [1, 70, 2, 9, 1], [3, 2], [1, 1]])
+@pytest.mark.parametrize("lens", [[64], [1, 70, 2, 9, 1], [3, 2], [1, 1], [900, 1, 400, 2, 5]])
 @pytest.mark.parametrize("channels", [64, 1032, 1100])
 def test_mixes_of_prompts(lens, channels):
     from gemmars_b200 import kernels as k
