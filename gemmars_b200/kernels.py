@@ -477,11 +477,12 @@ def gemm_tc_persistent(x, w, out, bias=None, accumulate=False, swiglu=False, bn=
     if bias is not None:
         assert bias.dtype == torch.float32 and bias.numel() == n
     if bn is None:
-        # 256 tokens a tile.  Narrower tiles that fill the last round of tiles better were measured and
-        # are slower: 240 tokens for 2,048 x 4,096 (1.5 % faster alone, 4 % slower inside a prompt step),
-        # and 128 tokens where 256 leave the last round nearly empty (2,048 x 2,560 is 160 tiles on 148
-        # SMs; a 2,048-token prompt of a 4B-shaped model took 20.5 ms against 18.4, of a 32B-shaped one
-        # 35.3 ms against 30.9 over 16 layers)
+        # 256 tokens a tile.  Narrower tiles that fill the last round of tiles better were slower while a block
+        # of 64 inner elements took some 310 ns whatever its tokens: 240 tokens for 2,048 x 4,096 (1.5 % faster
+        # alone, 4 % slower inside a prompt step), and 128 tokens where 256 leave the last round nearly empty
+        # (2,048 x 2,560 is 160 tiles on 148 SMs; a 2,048-token prompt of a 4B-shaped model took 20.5 ms against
+        # 18.4, of a 32B-shaped one 35.3 ms against 30.9 over 16 layers).  With an elected issuing thread a block
+        # of 128 tokens takes 190 ns; the comparison has not been made again since.
         bn = 128 if m <= 128 else 256
         # Where those leave two SMs in five without a tile (a router, a low-rank factor, few tokens), the narrowest tiles that
         # still are one round; a block of the inner dimension takes less time the narrower they are (us, 256 tokens a
@@ -1408,8 +1409,10 @@ def moe_experts_grouped(h, idx, wts, sg, w_gate_up, w_down, shared_gate_up, shar
     _shared_expert(h, sg, shared_gate_up, shared_down, residual, shared_limit, alpha, shift, col_scale)
 
 
-#: below MOE_TC_MIN_TOKENS tokens (steps that may be captured, each with scratch of its own) a step's padded float32 rows
-#: may take this many bytes on the tcgen05 product; the grouped product needs no padding
+#: below MOE_TC_MIN_TOKENS tokens (steps that may be captured) a step's padded float32 rows may take this many bytes on the
+#: tcgen05 product, its activations half of that and the experts' middle ff / (2 width) of it; the grouped product needs no
+#: padding.  Captured steps of one runner share a pool, so it holds this once, for the largest of them: 128 tokens, 6 of 64
+#: experts of 1,408 at a width of 2,048 are 8,960 rows, 73 + 37 + 25 MB where the grouped product holds 768 rows, 12 MB in all.
 MOE_TC_MIN_TOKENS = 256
 MOE_TC_SMALL_BYTES = 256 << 20
 MOE_TC_TILE = 128
