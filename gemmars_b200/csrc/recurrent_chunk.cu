@@ -636,7 +636,9 @@ static int run(Prepare p, Scan s, int ntok, int heads_at_once, cudaStream_t stre
     p.head0 = s.head0 = h;
     gb_launch(chunk_prepare_kernel<DP, MODE>, dim3(p.slots, heads), 128, 0, stream, p);
     // us for a delta rule at heads of 128 x 128, preparation and all, by (DS, NV): 64 groups of 16 columns, 1,218 tokens:
-    // (4, 1) 93, (2, 2) 121, (1, 4) 206; 256 groups, 2,048 tokens: 267, 236, 379; 2,048 groups of 512: 522, 491, 421.
+    // (4, 1) 96, (2, 2) 137, (1, 4) 236; 256 groups, 2,048 tokens: 287, 278, 434; eight sequences of 113 to 910 tokens in two
+    // launches of 1,024 groups: 609, 632, 684.  2,048 groups of 512 tokens took 522, 491, 421 before both operands' halves were
+    // rounded and the cut given back (256 groups then: 267, 236, 379); the line to (1, 4) is from then.
     // Few groups leave the chain to itself and want it short (more warps a group); many fill the SMs either way and
     // want the least that a group costs.
     const long long groups = (long long)p.nseq * heads * ((s.V + 15) / 16);
