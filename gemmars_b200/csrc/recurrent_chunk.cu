@@ -637,8 +637,8 @@ static int run(Prepare p, Scan s, int ntok, int heads_at_once, cudaStream_t stre
     gb_launch(chunk_prepare_kernel<DP, MODE>, dim3(p.slots, heads), 128, 0, stream, p);
     // us for a delta rule at heads of 128 x 128, preparation and all, by (DS, NV): 64 groups of 16 columns, 1,218 tokens:
     // (4, 1) 96, (2, 2) 137, (1, 4) 236; 256 groups, 2,048 tokens: 287, 278, 434; eight sequences of 113 to 910 tokens in two
-    // launches of 1,024 groups: 609, 632, 684.  2,048 groups of 512 tokens took 522, 491, 421 before both operands' halves were
-    // rounded and the cut given back (256 groups then: 267, 236, 379); the line to (1, 4) is from then.
+    // launches of 1,024 groups: 609, 632, 684; sixteen of 3,200 tokens in all, 2,048 groups a launch: 473, 491, 451; twelve of
+    // 1,500, 3,072 groups: 232, 242, 203.
     // Few groups leave the chain to itself and want it short (more warps a group); many fill the SMs either way and
     // want the least that a group costs.
     const long long groups = (long long)p.nseq * heads * ((s.V + 15) / 16);
