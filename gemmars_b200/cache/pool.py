@@ -21,6 +21,7 @@ from __future__ import annotations
 import dataclasses
 from typing import Dict, List, Optional, Sequence, Tuple
 
+import numpy as np
 import torch
 
 PAGE_SIZE = 64
@@ -138,6 +139,7 @@ class KVGroup:
         self.v = torch.zeros(shape[:3] + (vdim, page_size) if vdim else (n_layers, 0), dtype=dtype, device=device)
         # row n_slots stays all zero: padded rows of a batch use it and land in page 0
         self.table_host = torch.zeros((n_slots + 1, self.table_width), dtype=torch.int32)
+        self._table = self.table_host.numpy()     # the same memory: a page number is read and written without a tensor's call
         self.page_table = torch.zeros((n_slots + 1, self.table_width), dtype=torch.int32, device=device)
         self._dirty = set()
         self._mapped: Dict[int, int] = {}   # slot -> logical pages mapped so far
@@ -150,7 +152,7 @@ class KVGroup:
             col = lp % self.table_width
             if lp >= self.table_width:
                 continue  # a ring: the page of logical page lp - width is written over
-            self.table_host[slot, col] = self.pages.take()
+            self._table[slot, col] = self.pages.take()
             self._dirty.add(slot)
         self._mapped[slot] = max(have, need_pages)
 
@@ -161,8 +163,8 @@ class KVGroup:
 
     def release(self, slot: int) -> None:
         for col in range(min(self._mapped.pop(slot, 0), self.table_width)):
-            self.pages.give_back(int(self.table_host[slot, col]))
-            self.table_host[slot, col] = 0
+            self.pages.give_back(int(self._table[slot, col]))
+            self._table[slot, col] = 0
         self._dirty.add(slot)
 
     def truncate(self, slot: int, new_len: int) -> None:
@@ -171,13 +173,30 @@ class KVGroup:
             raise CacheError("a windowed group cannot be truncated")
         keep = (new_len + self.page_size - 1) // self.page_size
         for lp in range(keep, self._mapped.get(slot, 0)):
-            self.pages.give_back(int(self.table_host[slot, lp]))
-            self.table_host[slot, lp] = 0
+            self.pages.give_back(int(self._table[slot, lp]))
+            self._table[slot, lp] = 0
             self._dirty.add(slot)
         self._mapped[slot] = min(self._mapped.get(slot, 0), keep)
 
+    def changed_rows(self) -> np.ndarray:
+        """The rows of the page table that changed since they were last sent."""
+        return np.array(sorted(self._dirty), dtype=np.int64)
+
+    def table_rows(self, rows: np.ndarray) -> np.ndarray:
+        return self._table[rows]
+
+    def put_rows(self, rows: np.ndarray, rows_dev: torch.Tensor, values: torch.Tensor) -> None:
+        """Sends rows of the page table that a step's index block has brought to the device: ``rows``, the same numbers there,
+        and ``values`` [rows, width] (``table_rows``)."""
+        if len(rows) <= 2:
+            for i, r in enumerate(rows.tolist()):
+                self.page_table[r].copy_(values[i])
+        else:
+            self.page_table.index_copy_(0, rows_dev.long(), values)
+        self._dirty.difference_update(rows.tolist())
+
     def sync(self) -> None:
-        """Copies the rows of the page table that changed to the device."""
+        """Copies the rows of the page table that changed to the device; the host waits for it."""
         if not self._dirty:
             return
         rows = sorted(self._dirty)
@@ -316,6 +335,10 @@ class SequenceCache:
     def sync(self) -> None:
         for g in self.kv_groups:
             g.sync()
+
+    def changed(self) -> int:
+        """How many numbers the changed rows of the page tables are, each with its row number."""
+        return sum(len(g._dirty) * (1 + g.table_width) for g in self.kv_groups)
 
     def rollback(self, slot: int, old_len: int) -> bool:
         """After a step that failed: takes back the positions from ``old_len`` on that were
