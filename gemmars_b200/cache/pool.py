@@ -185,14 +185,11 @@ class KVGroup:
     def table_rows(self, rows: np.ndarray) -> np.ndarray:
         return self._table[rows]
 
-    def put_rows(self, rows: np.ndarray, rows_dev: torch.Tensor, values: torch.Tensor) -> None:
-        """Sends rows of the page table that a step's index block has brought to the device: ``rows``, the same numbers there,
-        and ``values`` [rows, width] (``table_rows``)."""
-        if len(rows) <= 2:
-            for i, r in enumerate(rows.tolist()):
-                self.page_table[r].copy_(values[i])
-        else:
-            self.page_table.index_copy_(0, rows_dev.long(), values)
+    def put_rows(self, rows: np.ndarray, values: torch.Tensor) -> None:
+        """Puts ``rows`` of the page table in their places from ``values`` [rows, width] (``table_rows``), which a step's
+        index block has brought to the device."""
+        for i, r in enumerate(rows.tolist()):
+            self.page_table[r].copy_(values[i])
         self._dirty.difference_update(rows.tolist())
 
     def sync(self) -> None:
@@ -336,9 +333,9 @@ class SequenceCache:
         for g in self.kv_groups:
             g.sync()
 
-    def changed(self) -> int:
-        """How many numbers the changed rows of the page tables are, each with its row number."""
-        return sum(len(g._dirty) * (1 + g.table_width) for g in self.kv_groups)
+    def changed(self) -> Tuple[int, int]:
+        """How many rows of the page tables have changed since they were last sent, and how many numbers those are."""
+        return (sum(len(g._dirty) for g in self.kv_groups), sum(len(g._dirty) * g.table_width for g in self.kv_groups))
 
     def rollback(self, slot: int, old_len: int) -> bool:
         """After a step that failed: takes back the positions from ``old_len`` on that were

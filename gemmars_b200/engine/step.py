@@ -205,14 +205,15 @@ class Runner:
         # Page table rows that changed go out with the step's index block and are put in their places on the device: a copy
         # of their own out of pageable memory returns only when all steps before have run, so that the device stood idle
         # while the host prepared a prompt's launches (110 us of 1,880 for 2,048 tokens through two layers of 8B sizes, of
-        # 1,550 for 301 float32 tokens).  More of them than a step's tokens take that copy all the same.
+        # 1,550 for 301 float32 tokens).  Each row is a copy on the device, so many rows take that one copy all the same.
         changed = []
-        if 0 < cache.changed() <= self.max_step_tokens:
+        n_rows, n_numbers = cache.changed()
+        if n_rows <= 16 and n_numbers <= self.max_step_tokens:
             changed = [(g, g.changed_rows()) for g in cache.kv_groups]
         else:
             cache.sync()
         block = np.concatenate([tokens, tok_pos, tok_seq, slots, starts, lens, cu, np.asarray(rows, dtype=np.int64)]
-                               + [part for g, r in changed for part in (r, g.table_rows(r).reshape(-1))]).astype(np.int32)
+                               + [g.table_rows(r).reshape(-1) for g, r in changed]).astype(np.int32)
         dev = self._ring.stage(block, self.device)
         o = 0
 
@@ -225,8 +226,7 @@ class Runner:
         d_tokens, d_pos, d_seq = take(t), take(t), take(t)
         d_slot, d_start, d_len, d_cu, d_rows = take(b), take(b), take(b), take(b + 1), take(len(rows))
         for g, r in changed:
-            at = take(len(r))
-            g.put_rows(r, at, take(len(r) * g.table_width).view(len(r), g.table_width))
+            g.put_rows(r, take(len(r) * g.table_width).view(len(r), g.table_width))
         ctx = StepContext(
             compute=self.model.compute, act_dtype=self.model.act_dtype, device=self.device, n_tokens=t, n_seqs=b,
             tok_pos=d_pos, tok_seq=d_seq, seq_slot=d_slot, seq_start=d_start, seq_len=d_len, cu_seqlens=d_cu,

@@ -16,13 +16,14 @@ def test_rows_put_are_the_rows_synced(slots):
         if step == 1:
             cache.close(held[0])
             held[0] = cache.open()
-        assert cache.changed() == sum(len(g.changed_rows()) * (1 + g.table_width) for g in cache.kv_groups)
+        assert cache.changed() == (sum(len(g.changed_rows()) for g in cache.kv_groups),
+                                   sum(g.table_rows(g.changed_rows()).size for g in cache.kv_groups))
         for g in cache.kv_groups:
             rows = g.changed_rows()
             values = torch.from_numpy(g.table_rows(rows).astype(np.int32))
-            g.put_rows(rows, torch.from_numpy(rows.astype(np.int32)), values)
+            g.put_rows(rows, values)
             assert torch.equal(g.page_table, g.table_host)
-        assert cache.changed() == 0
+        assert cache.changed() == (0, 0)
         cache.sync()                       # nothing is left to send
         for g in cache.kv_groups:
             assert torch.equal(g.page_table, g.table_host)
