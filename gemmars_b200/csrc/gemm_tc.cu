@@ -774,6 +774,14 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
 }
 
 // ------------------------------------------------------------------ the persistent kernel for prompts
+// Where it pays (pairs_pay), two CTAs on neighbouring SMs, a cluster, work a tile of twice the features together (PAIR;
+// cta_group::2): each brings its own 128 rows of W and half of the tile's tokens, rank 0 issues MMAs of 256 features that
+// read both CTAs' shared memory, and each CTA's tensor memory gets its own 128 features of all tokens, so the epilogue is
+// the single CTA's.  Loads count on rank 0's full barriers, commits arrive at both CTAs' empty and accumulator barriers,
+// and both CTAs' epilogue warps at rank 0's acc_empty.  What bound the single CTA was bringing 48 KB a block of 64 inner
+// elements from L2 in four stages: 304 to 320 ns a block of 256 tokens, for 260 to 270 of the tensor pipe's work; a pair
+// brings 32 KB in six stages, 275 to 285 ns (2,048 tokens through 8B sizes, us: q/k/v 107 / 80, gated 24,576 x 4,096
+// 308 / 250, 4,096 x 12,288 153 / 137).
 // One CTA per SM walks the output tiles (token tile fastest, so the CTAs that run together
 // share the same rows of W).  The accumulator in tensor memory is double-buffered: while the
 // four epilogue warps read tile i out of one buffer and store it, the MMA warp already fills the
@@ -797,7 +805,7 @@ __device__ __forceinline__ void tile_origin(int t, int tiles_m, int tiles_n, int
 }
 
 
-// The work of one CTA of the persistent kernel: tiles blockIdx.x, + gridDim.x, and so on.  Where
+// The work of one CTA (or pair of CTAs) of the persistent kernel: every `walkers`-th tile from its own on.  Where
 // the last round of tiles would leave SMs idle, a product that adds into its result (`split` > 1)
 // cuts each tile of that round into `split` parts along the inner dimension, and the CTAs walk
 // those parts the same way, part 0 of every tile first: the CTAs stay in step along the inner
@@ -807,9 +815,10 @@ __device__ __forceinline__ void tile_origin(int t, int tiles_m, int tiles_n, int
 // whose 100 MB of W and 50 MB of x in the down product no longer pass through L2 once.)
 struct TileWalk {
   int t, kb0, kb1, part;   // the segment: blocks [kb0, kb1) of tile t; which part of the tile it is
-  int at, whole, last, split, kb_total;
-  __device__ __forceinline__ TileWalk(int tiles, int kb_total_, int split_) : at(blockIdx.x), split(split_), kb_total(kb_total_) {
-    whole = split > 1 ? tiles - tiles % (int)gridDim.x : tiles;   // tiles of the full rounds
+  int at, walkers, whole, last, split, kb_total;
+  __device__ __forceinline__ TileWalk(int tiles, int kb_total_, int split_, int walker, int walkers_)
+      : at(walker), walkers(walkers_), split(split_), kb_total(kb_total_) {
+    whole = split > 1 ? tiles - tiles % walkers : tiles;          // tiles of the full rounds
     last = tiles - whole;                                          // tiles of the round that is cut
     set();
   }
@@ -830,7 +839,7 @@ struct TileWalk {
   __device__ __forceinline__ bool more() const { return at < whole + last * split; }
   __device__ __forceinline__ bool shared() const { return at >= whole; }   // one of several parts of its tile
   __device__ __forceinline__ void next() {
-    at += gridDim.x;
+    at += walkers;
     set();
   }
 };
@@ -872,7 +881,7 @@ __device__ __forceinline__ float clamped_gate(float g, float u, const Grouped& g
   return __fdividef(g, 1.0f + __expf(-grp.alpha * g)) * (u + grp.shift);
 }
 
-template <int BN, int STAGES, int MODE>
+template <int BN, int STAGES, int MODE, bool PAIR>
 __global__ void __launch_bounds__(MODE == EPI_QKV_BF16 ? PERSISTENT_QKV_THREADS : THREADS, 1)
 gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                           const __grid_constant__ CUtensorMap map_y, int y_tma, const float* __restrict__ bias,
@@ -884,13 +893,14 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
   const int split = MODE == EPI_ACCUMULATE_F32 ? max(split_last, 1) : 1;
   constexpr bool QKV = MODE == EPI_QKV_BF16;        // a tile is one head: norm, rotation, cache write (qkv_prompt_round)
   constexpr int TILE_F = GATED ? BM / 2 : BM;       // features of the result per tile
-  constexpr uint32_t A_BYTES = BM * BK * 2, B_BYTES = BN * BK * 2;
+  constexpr int CTAS = PAIR ? 2 : 1;
+  constexpr uint32_t A_BYTES = BM * BK * 2, B_BYTES = BN / CTAS * BK * 2;
   constexpr uint32_t STAGE_BYTES = A_BYTES + B_BYTES;
   constexpr uint32_t ACC_COLS = BN, TMEM_COLS = 2 * ACC_COLS;
   static_assert(TMEM_COLS == 256 || TMEM_COLS == 512, "two accumulator buffers: 256 or 512 columns");
-  // bn: tokens per tile, a multiple of 16 up to BN (BN sizes the stages and the accumulators)
-  const uint32_t idesc_rest = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BM >> 4) << 24);
-  const uint32_t stage_tx = A_BYTES + (uint32_t)bn * BK * 2;
+  // bn: tokens per tile, a multiple of 16 (a pair: of 32) up to BN (BN sizes the stages and the accumulators)
+  const uint32_t idesc_rest = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(CTAS * BM >> 4) << 24);
+  const uint32_t stage_tx = CTAS * A_BYTES + (uint32_t)bn * BK * 2;      // what a pair's stages get counts on rank 0's barrier
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint64_t* full_bar = (uint64_t*)(smem + STAGES * STAGE_BYTES);
@@ -898,6 +908,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
   uint64_t* acc_full = empty_bar + STAGES;     // 2: the MMA warp has finished a tile in that buffer
   uint64_t* acc_empty = acc_full + 2;          // 2: the epilogue warps have read it out
   uint32_t* tmem_slot = (uint32_t*)(acc_empty + 2);
+  volatile int* epilogue_gave_up = (volatile int*)(tmem_slot + 1);
   uint8_t* out_staging = smem + STAGES * STAGE_BYTES + 1024;   // past the barriers; OUT_STAGING_BYTES
   // gated: the pieces are 16 tokens of bfloat16 (1 KB), and the pairs' exchange has the upper half
   constexpr int SLOT = (GATED || QKV) ? OUT_STAGING_BYTES / 2 / (4 * PIECES) : PIECE_BYTES;
@@ -907,10 +918,11 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
   static_assert(!QKV || (SLOT >= PIECE_TOKENS * PIECE_FEATURES * 2 && 8 * PIECES * SLOT == 32 * 1024), "q/k/v staging");
   static_assert((2 * STAGES + 4) * 8 + 16 <= 1024, "the barriers have 1 KB");
   constexpr int EPI_WARPS = QKV ? 8 : 4;
-  __shared__ int epilogue_gave_up;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int tiles_m = (M + bn - 1) / bn, tiles_n = (N + TILE_F - 1) / TILE_F, tiles = tiles_m * tiles_n;
+  const int rank = PAIR ? (int)cluster_rank() : 0, walker = (int)blockIdx.x / CTAS, walkers = (int)gridDim.x / CTAS;
+  constexpr int WALK_F = CTAS * TILE_F;             // features of the result per tile of the walk; rank r has the r-th TILE_F
+  const int tiles_m = (M + bn - 1) / bn, tiles_n = (N + WALK_F - 1) / WALK_F, tiles = tiles_m * tiles_n;
   const int kb_total = (K + BK - 1) / BK;
 
   if (threadIdx.x == 0) {
@@ -920,17 +932,26 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(&acc_full[b], 1);
-      mbar_init(&acc_empty[b], EPI_WARPS);
+      mbar_init(&acc_empty[b], CTAS * EPI_WARPS);
     }
-    epilogue_gave_up = 0;
+    *epilogue_gave_up = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 5) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(TMEM_COLS));
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    if (PAIR) {
+      asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(TMEM_COLS));
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;");
+    } else {
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(TMEM_COLS));
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
   }
   tc_fence_before();
   __syncthreads();
+  if (PAIR) {                  // the other CTA's barriers exist and its tensor memory is there
+    cluster_arrive();
+    cluster_wait();
+  }
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
 
@@ -942,14 +963,16 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
       pdl_wait_prior();
       uint32_t it = 0;
       bool ok = true;
-      for (TileWalk w(tiles, kb_total, split); w.more() && ok; w.next()) {
+      for (TileWalk w(tiles, kb_total, split, walker, walkers); w.more() && ok; w.next()) {
         int m0, n0;
-        tile_origin(w.t, tiles_m, tiles_n, bn, TILE_F, m0, n0);
-        int w0 = n0;                                   // the tile's first row of W
+        tile_origin(w.t, tiles_m, tiles_n, bn, WALK_F, m0, n0);
+        int w0 = n0 + rank * TILE_F;                   // the tile's first row of W
+        int x0 = m0 + rank * bn / 2;                   // a pair: rank 1 brings the second half of the MMA's tokens
         if (grp.tile_expert) {
           const int e = grp.tile_expert[m0 / bn];
           if (e < 0) continue;
           w0 += e * grp.rows_per_expert;
+          if (PAIR && grp.tile_rows) x0 = m0 + rank * (((grp.tile_rows[m0 / bn] + 31) & ~31) / 2);
         }
         for (int kb = w.kb0; kb < w.kb1; ++kb, ++it) {
           const uint32_t s = it % STAGES;
@@ -959,44 +982,50 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
             break;
           }
           uint8_t* a = smem + s * STAGE_BYTES;
-          mbar_expect_tx(&full_bar[s], stage_tx);
+          const uint32_t bar = PAIR ? cluster_addr(&full_bar[s], 0) : 0;
+          auto load = [&](uint8_t* dst, const CUtensorMap* map, int row) {
+            if (PAIR) tma_load_2d_pair(dst, map, kb * BK, row, bar);
+            else tma_load_2d(dst, map, kb * BK, row, &full_bar[s]);
+          };
+          if (rank == 0) mbar_expect_tx(&full_bar[s], stage_tx);
           if (GATED) {   // map_w is cut into boxes of 64 rows: the gate rows, then the same features' up rows
             // (a request costs the issuing thread about 75 cycles: boxes of 16 rows, which would let a
             // warp gate without shared memory, made nine requests a block and the producer the limit)
-            tma_load_2d(a, &map_w, kb * BK, w0, &full_bar[s]);
-            tma_load_2d(a + A_BYTES / 2, &map_w, kb * BK, N + w0, &full_bar[s]);
+            load(a, &map_w, w0);
+            load(a + A_BYTES / 2, &map_w, N + w0);
           } else {
-            tma_load_2d(a, &map_w, kb * BK, w0, &full_bar[s]);
+            load(a, &map_w, w0);
           }
-          tma_load_2d(a + A_BYTES, &map_x, kb * BK, m0, &full_bar[s]);
+          load(a + A_BYTES, &map_x, x0);
         }
       }
       pdl_release_next();   // all loads issued: the next kernel may move in
     }
     __syncwarp();
   } else if (warp == 5) {
-    // ---------------- MMA issue
-    if (elect_one()) {
+    // ---------------- MMA issue (a pair: by rank 0)
+    if (rank == 0 && elect_one()) {
       uint32_t it = 0, i = 0;
       bool ok = true;
       // which tiles are used is written by a kernel before this one: it must have ended before the
       // list is read, or this thread would skip other tiles than the producer and wait for a stage
       // that is never filled
       if (grp.tile_expert) pdl_wait_prior();
-      for (TileWalk w(tiles, kb_total, split); w.more() && ok; w.next(), ++i) {
+      for (TileWalk w(tiles, kb_total, split, walker, walkers); w.more() && ok; w.next(), ++i) {
         uint32_t width = (uint32_t)bn;
         if (grp.tile_expert) {                         // a tile no group uses: not counted, as in the other roles
           int m0, n0;
-          tile_origin(w.t, tiles_m, tiles_n, bn, TILE_F, m0, n0);
+          tile_origin(w.t, tiles_m, tiles_n, bn, WALK_F, m0, n0);
           if (grp.tile_expert[m0 / bn] < 0) {
             --i;
             continue;
           }
-          if (grp.tile_rows) width = (uint32_t)(grp.tile_rows[m0 / bn] + 15) & ~15u;
+          constexpr uint32_t UNIT = 16 * CTAS;
+          if (grp.tile_rows) width = ((uint32_t)grp.tile_rows[m0 / bn] + UNIT - 1) & ~(UNIT - 1);
         }
         const uint32_t idesc = idesc_rest | (width >> 3 << 17);
         const uint32_t b = i & 1;
-        if (i >= 2 && !mbar_wait(&acc_empty[b], ((i >> 1) - 1) & 1)) {   // the epilogue has read this buffer out
+        if (i >= 2 && !(PAIR ? mbar_wait_cluster(&acc_empty[b], ((i >> 1) - 1) & 1) : mbar_wait(&acc_empty[b], ((i >> 1) - 1) & 1))) {   // the epilogue has read this buffer out
           atomicCAS(&g_status, ST_OK, ST_TIMEOUT_TMEM);
           break;
         }
@@ -1004,7 +1033,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
         const uint32_t d = tmem + b * ACC_COLS;
         for (int kb = w.kb0; kb < w.kb1; ++kb, ++it) {
           const uint32_t s = it % STAGES;
-          if (!mbar_wait(&full_bar[s], (it / STAGES) & 1)) {
+          if (!(PAIR ? mbar_wait_cluster(&full_bar[s], (it / STAGES) & 1) : mbar_wait(&full_bar[s], (it / STAGES) & 1))) {
             atomicCAS(&g_status, ST_OK, ST_TIMEOUT_FULL);
             ok = false;
             break;
@@ -1013,11 +1042,16 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
           const uint32_t a = smem_u32(smem + s * STAGE_BYTES);
           const uint64_t adesc = smem_desc(a), bdesc = smem_desc(a + A_BYTES);
 #pragma unroll
-          for (int k = 0; k < BK / UMMA_K; ++k)
-            tc_mma(d, adesc + (uint64_t)(k * 2), bdesc + (uint64_t)(k * 2), idesc, (kb > w.kb0 || k > 0) ? 1u : 0u);
-          tc_commit(&empty_bar[s]);
+          for (int k = 0; k < BK / UMMA_K; ++k) {
+            const uint32_t more = (kb > w.kb0 || k > 0) ? 1u : 0u;
+            if (PAIR) tc_mma_pair(d, adesc + (uint64_t)(k * 2), bdesc + (uint64_t)(k * 2), idesc, more);
+            else tc_mma(d, adesc + (uint64_t)(k * 2), bdesc + (uint64_t)(k * 2), idesc, more);
+          }
+          if (PAIR) tc_commit_pair(&empty_bar[s]);
+          else tc_commit(&empty_bar[s]);
         }
-        tc_commit(&acc_full[b]);
+        if (PAIR) tc_commit_pair(&acc_full[b]);
+        else tc_commit(&acc_full[b]);
       }
     }
     __syncwarp();
@@ -1033,9 +1067,10 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
                                        (float*)(out_staging + 64 * 1024) + group * 4 * 32};
     const bool both = bn % 32 == 0;   // 32 tokens per round; the result's map is cut to match
     uint32_t i = 0;
-    for (TileWalk w(tiles, kb_total, split); w.more(); w.next(), ++i) {
+    for (TileWalk w(tiles, kb_total, split, walker, walkers); w.more(); w.next(), ++i) {
       int m0, n0;
-      tile_origin(w.t, tiles_m, tiles_n, bn, TILE_F, m0, n0);
+      tile_origin(w.t, tiles_m, tiles_n, bn, WALK_F, m0, n0);
+      n0 += rank * TILE_F;
       if (grp.tile_expert && grp.tile_expert[m0 / bn] < 0) {
         --i;
         continue;
@@ -1043,12 +1078,12 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
       const uint32_t b = i & 1;
       const int n = n0 + f;
       const int m_end = grp.tile_rows ? min(M, m0 + grp.tile_rows[m0 / bn]) : M;     // the tile's rows that exist
-      bool have = __all_sync(0xffffffffu, mbar_wait(&acc_full[b], (i >> 1) & 1));
+      bool have = __all_sync(0xffffffffu, PAIR ? mbar_wait_cluster(&acc_full[b], (i >> 1) & 1) : mbar_wait(&acc_full[b], (i >> 1) & 1));
       if (!have && lane == 0) atomicCAS(&g_status, ST_OK, ST_TIMEOUT_TMEM);
       if (GATED || QKV) {   // the warps meet at barriers below: they leave together or not at all
-        if (!have && lane == 0) epilogue_gave_up = 1;
+        if (!have && lane == 0) *epilogue_gave_up = 1;
         asm volatile("bar.sync 3, %0;" ::"n"(EPI_WARPS * 32) : "memory");
-        have = epilogue_gave_up == 0;
+        have = *epilogue_gave_up == 0;
       }
       if (!have) break;
       tc_fence_after();
@@ -1063,7 +1098,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
       // memory, part q adds when it reads q (its predecessors were walked earlier, or at the same
       // time by CTAs that wait for nothing later than this one does), and the last part puts the
       // word back to zero.
-      int* word = w.shared() ? part_flags + (w.t - w.whole) * 4 + warp : nullptr;
+      int* word = w.shared() ? part_flags + ((w.t - w.whole) * CTAS + rank) * 4 + warp : nullptr;
       if (MODE == EPI_ACCUMULATE_F32 && word && w.part > 0) {
         if (lane == 0) {
           bool there = false;
@@ -1079,7 +1114,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
       const uint32_t acc = tmem + ((uint32_t)(quarter * 32) << 16) + b * ACC_COLS;
 #pragma unroll 1
       for (int c = QKV ? 32 * group : 0; c < bn; c += QKV ? 64 : (both ? 32 : 16)) {
-        if (m0 + c >= m_end) break;
+        if (m0 + c >= m_end || n0 >= N) break;     // n0: a pair's last tile may be half beyond the result
         uint32_t v[16], v2[16];
         tc_ld16(acc + c, v);
         if (both) tc_ld16(acc + c + 16, v2);
@@ -1153,7 +1188,10 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&acc_empty[b]);
+      if (lane == 0) {
+        if (PAIR) mbar_arrive_cluster(cluster_addr(&acc_empty[b], 0));
+        else mbar_arrive(&acc_empty[b]);
+      }
       if (MODE == EPI_ACCUMULATE_F32 && word) {
         if (lane == 0) {
           tma_store_wait_all();    // this warp's sums are in memory
@@ -1168,7 +1206,13 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
   tc_fence_before();
   __syncthreads();
   __syncwarp();
-  if (warp == 5) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS));
+  if (PAIR) {                  // neither leaves while the other's MMAs, commits or arrivals may still reach its memory
+    cluster_arrive();
+    cluster_wait();
+    if (warp == 5) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS));
+  } else if (warp == 5) {
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS));
+  }
 }
 
 // cos and sin of every packed token's angles, once per step for all layers: table[t][i] =
@@ -1282,49 +1326,81 @@ int launch_mode(int mode, const CUtensorMap& mw, const CUtensorMap& mx, const Ou
   return GB_ERR_ARG;
 }
 
-template <int BN, int STAGES, int MODE>
+// Whether a pair of CTAs works each tile (see gemm_tc_persistent_kernel).  A pair halves the bytes that an SM fetches of the
+// tokens and has six stages where one CTA has four: a block of 64 inner elements by 256 tokens in 275 to 285 ns where one
+// CTA takes 304 to 320.  It starts and ends with a barrier of the cluster, some 0.8 us a launch, and its tiles are twice as
+// large.  So: not where that makes more rounds of tiles than the faster block gives back, and where there is one round only
+// from 4,096 inner elements on.  Measured (us, one CTA / pairs; 148 SMs): 12,352 x 4,096 by 2,048 tokens 177.8 / 145.4,
+// 4,096 x 4,096 by 2,048 53.8 / 49.7, 3,136 x 1,024 by 1,300 (two rounds) 17.1 / 16.3, 4,096 x 4,096 by 1,000 (one) 27.7 /
+// 26.9; 2,048 x 2,048 by 2,048 (one) 16.2 / 17.2, 4,672 x 2,048 by 2,048 (two rounds against three) 30.6 / 35.9.
+bool pairs_pay(int M, int N, int K, int bn, int ctas, int tile_features) {
+  if (bn <= 128 || ctas < 2) return false;
+  const long long tiles_m = (M + bn - 1) / bn, tiles_n = (N + tile_features - 1) / tile_features;
+  const long long rounds = (tiles_m * tiles_n + ctas - 1) / ctas, pair_rounds = (tiles_m * ((tiles_n + 1) / 2) + ctas / 2 - 1) / (ctas / 2);
+  return 0.92 * pair_rounds < rounds && (rounds > 1 || K >= 4096);
+}
+
+template <int BN, int STAGES, int MODE, bool PAIR = false>
 int launch_persistent(const CUtensorMap& mw, const CUtensorMap& mx, const OutMap& my, const float* bias, void* y, int M,
                       int N, int K, long long ldy, int bn, int ctas, cudaStream_t stream, const QkvTail& tail = QkvTail{},
                       int* part_flags = nullptr, const Grouped& grp = Grouped{}) {
   // stages, 1 KB of barriers, the pieces on their way out, 1 KB to align the base
+  constexpr int CTAS = PAIR ? 2 : 1;
   constexpr size_t STAGING = MODE == EPI_QKV_BF16 ? QKV_STAGING_BYTES : OUT_STAGING_BYTES;
-  constexpr size_t SMEM = (size_t)STAGES * ((size_t)BM * BK * 2 + BN * BK * 2) + 1024 + STAGING + 1024;
+  constexpr size_t SMEM = (size_t)STAGES * ((size_t)BM * BK * 2 + BN / CTAS * BK * 2) + 1024 + STAGING + 1024;
   constexpr int NTHREADS = MODE == EPI_QKV_BF16 ? PERSISTENT_QKV_THREADS : THREADS;
   static_assert(SMEM <= 227 * 1024, "stages do not fit in shared memory");
   static_assert((2 * STAGES + 4) * 8 + 16 <= 1024, "the barriers have 1 KB");
-  constexpr int TILE_F = MODE == EPI_SWIGLU_BF16 ? BM / 2 : BM;
-  auto kernel = gemm_tc_persistent_kernel<BN, STAGES, MODE>;
+  constexpr int WALK_F = CTAS * (MODE == EPI_SWIGLU_BF16 ? BM / 2 : BM);
+  auto kernel = gemm_tc_persistent_kernel<BN, STAGES, MODE, PAIR>;
   static bool configured = false;
   if (!configured) {
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM) != cudaSuccess)
       return (int)cudaGetLastError();
     configured = true;
   }
-  const int tiles = ((M + bn - 1) / bn) * ((N + TILE_F - 1) / TILE_F);
+  const int walkers = ctas / CTAS > 0 ? ctas / CTAS : 1;
+  const int tiles = ((M + bn - 1) / bn) * ((N + WALK_F - 1) / WALK_F);
   // Where the last round of tiles would leave SMs idle and TMA adds the sums into the result: that
   // round's tiles in `split` parts along the inner dimension.  What a split costs, in blocks of the
   // inner dimension: the rounds of parts it makes, and, since the parts of a tile add one after the
   // other, a wait of about one tile's way out (its adds and their completion: about 9 blocks' time
   // at 256 tokens) for every further part of the same tile that is walked in the same round.
-  int split = 1, grid = tiles < ctas ? tiles : ctas;
-  if (MODE == EPI_ACCUMULATE_F32 && part_flags && my.usable && tiles % ctas != 0) {
-    const int last = tiles % ctas, kb_total = (K + BK - 1) / BK;
+  int split = 1, grid = tiles < walkers ? tiles : walkers;
+  if (MODE == EPI_ACCUMULATE_F32 && part_flags && my.usable && tiles % walkers != 0) {
+    const int last = tiles % walkers, kb_total = (K + BK - 1) / BK;
     const double way_out = 9.0 * bn / 256 + 1.0;
     double best = 0.92 * kb_total;
     for (int sp = 2; sp <= 8 && kb_total / sp >= 4; ++sp) {
-      const int rounds = (last * sp + ctas - 1) / ctas;
-      const int together = sp < (ctas + last - 1) / last ? sp : (ctas + last - 1) / last;   // parts of a tile in one round
+      const int rounds = (last * sp + walkers - 1) / walkers;
+      const int together = sp < (walkers + last - 1) / last ? sp : (walkers + last - 1) / last;   // parts of a tile in one round
       const double cost = (double)rounds * kb_total / sp + (together - 1) * way_out + (rounds - 1) * 1.0;
       if (cost < best) {
         best = cost;
         split = sp;
       }
     }
-    if (split > 1) grid = last * split < ctas && tiles < ctas ? last * split : ctas;
+    if (split > 1) grid = last * split < walkers && tiles < walkers ? last * split : walkers;
   }
-  gb_launch(kernel, dim3(grid), dim3(NTHREADS), SMEM, stream, mw, mx, my.map, my.usable, bias, y, M, N, K, ldy, bn, tail,
-            split, part_flags, grp);
-  return gb_launch_status();
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid * CTAS);
+  cfg.blockDim = dim3(NTHREADS);
+  cfg.dynamicSmemBytes = SMEM;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  if (PAIR) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    attr[cfg.numAttrs].val.clusterDim.x = CTAS;
+    attr[cfg.numAttrs].val.clusterDim.y = attr[cfg.numAttrs].val.clusterDim.z = 1;
+    ++cfg.numAttrs;
+  }
+  if (GB_PDL_EARLY_START) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[cfg.numAttrs].val.programmaticStreamSerializationAllowed = 1;
+    ++cfg.numAttrs;
+  }
+  cfg.attrs = attr;
+  return (int)cudaLaunchKernelEx(&cfg, kernel, mw, mx, my.map, my.usable, bias, y, M, N, K, ldy, bn, tail, split, part_flags, grp);
 }
 
 }  // namespace
@@ -1464,16 +1540,26 @@ GB_EXPORT int gb_gemm_tc_persistent(const void* x, const void* w, const float* b
   if (bn < 16 || bn > 256 || (bn % 16)) return GB_ERR_SIZE;
   const bool swiglu = mode == EPI_SWIGLU_BF16;
   if (swiglu && bias) return GB_ERR_ARG;
+  const bool pair = pairs_pay(M, N, K, bn, ctas, swiglu ? BM / 2 : BM);
+  if (pair) bn = (bn + 31) / 32 * 32;          // its MMA is as wide as a multiple of 32 tokens
   CUtensorMap mw, mx;
   // gated: W in boxes of 64 rows; a tile is 64 gate rows and the same features' 64 up rows
   if (!tensor_map(&mw, w, (uint64_t)N * (swiglu ? 2 : 1), (uint64_t)K, (uint64_t)K * 2, swiglu ? BM / 2 : BM)) return GB_ERR_ARG;
-  if (!tensor_map(&mx, x, (uint64_t)M, (uint64_t)K, (uint64_t)ldx * 2, (uint32_t)bn)) return GB_ERR_ARG;
+  if (!tensor_map(&mx, x, (uint64_t)M, (uint64_t)K, (uint64_t)ldx * 2, (uint32_t)(pair ? bn / 2 : bn))) return GB_ERR_ARG;
   const OutMap my = out_map(y, mode, M, N, ldy, swiglu ? 16 : bn);   // gated: a warp sends 16 tokens at a time
   if (swiglu) {
+    if (pair) return launch_persistent<256, 6, EPI_SWIGLU_BF16, true>(mw, mx, my, bias, y, M, N, K, ldy, bn, ctas, stream);
     if (bn > 128) return launch_persistent<256, 4, EPI_SWIGLU_BF16>(mw, mx, my, bias, y, M, N, K, ldy, bn, ctas, stream);
     return launch_persistent<128, 6, EPI_SWIGLU_BF16>(mw, mx, my, bias, y, M, N, K, ldy, bn, ctas, stream);
   }
-  if (bn > 128) {
+  if (pair) {
+    switch (mode) {
+      case EPI_STORE_BF16: return launch_persistent<256, 6, EPI_STORE_BF16, true>(mw, mx, my, bias, y, M, N, K, ldy, bn, ctas, stream, tail, nullptr, grp);
+      case EPI_STORE_F32: return launch_persistent<256, 6, EPI_STORE_F32, true>(mw, mx, my, bias, y, M, N, K, ldy, bn, ctas, stream);
+      case EPI_ACCUMULATE_F32:
+        return launch_persistent<256, 6, EPI_ACCUMULATE_F32, true>(mw, mx, my, bias, y, M, N, K, ldy, bn, ctas, stream, tail, part_flags);
+    }
+  } else if (bn > 128) {
     switch (mode) {
       case EPI_STORE_BF16: return launch_persistent<256, 4, EPI_STORE_BF16>(mw, mx, my, bias, y, M, N, K, ldy, bn, ctas, stream, tail, nullptr, grp);
       case EPI_STORE_F32: return launch_persistent<256, 4, EPI_STORE_F32>(mw, mx, my, bias, y, M, N, K, ldy, bn, ctas, stream);
@@ -1515,20 +1601,29 @@ GB_EXPORT int gb_gemm_tc_grouped(const void* x, const void* w, void* y, int mode
   grp.limit = limit; grp.alpha = alpha; grp.shift = shift;
   grp.act = mode == EPI_STORE_BF16 ? act : OUT_ACT_NONE;
   grp.scale_in = gated && row_scale ? scale_in : 0;
+  const bool pair = pairs_pay(M, N, K, bn, ctas, gated ? BM / 2 : BM);
   CUtensorMap mw, mx;
   if (!tensor_map(&mw, w, (uint64_t)experts * grp.rows_per_expert, (uint64_t)K, (uint64_t)K * 2, gated ? BM / 2 : BM)) return GB_ERR_ARG;
-  if (!tensor_map(&mx, x, (uint64_t)M, (uint64_t)K, (uint64_t)ldx * 2, (uint32_t)bn)) return GB_ERR_ARG;
+  if (!tensor_map(&mx, x, (uint64_t)M, (uint64_t)K, (uint64_t)ldx * 2, (uint32_t)(pair ? bn / 2 : bn))) return GB_ERR_ARG;
   const OutMap my = out_map(y, mode, M, N, ldy, gated ? 16 : bn);
   if (gated) {
+    if (pair) return launch_persistent<256, 6, EPI_SWIGLU_BF16, true>(mw, mx, my, nullptr, y, M, N, K, ldy, bn, ctas, stream, QkvTail{}, nullptr, grp);
     if (bn > 128) return launch_persistent<256, 4, EPI_SWIGLU_BF16>(mw, mx, my, nullptr, y, M, N, K, ldy, bn, ctas, stream, QkvTail{}, nullptr, grp);
     return launch_persistent<128, 6, EPI_SWIGLU_BF16>(mw, mx, my, nullptr, y, M, N, K, ldy, bn, ctas, stream, QkvTail{}, nullptr, grp);
   }
   if (mode == EPI_STORE_BF16) {
+    if (pair) return launch_persistent<256, 6, EPI_STORE_BF16, true>(mw, mx, my, nullptr, y, M, N, K, ldy, bn, ctas, stream, QkvTail{}, nullptr, grp);
     if (bn > 128) return launch_persistent<256, 4, EPI_STORE_BF16>(mw, mx, my, nullptr, y, M, N, K, ldy, bn, ctas, stream, QkvTail{}, nullptr, grp);
     return launch_persistent<128, 6, EPI_STORE_BF16>(mw, mx, my, nullptr, y, M, N, K, ldy, bn, ctas, stream, QkvTail{}, nullptr, grp);
   }
+  if (pair) return launch_persistent<256, 6, EPI_STORE_F32, true>(mw, mx, my, nullptr, y, M, N, K, ldy, bn, ctas, stream, QkvTail{}, nullptr, grp);
   if (bn > 128) return launch_persistent<256, 4, EPI_STORE_F32>(mw, mx, my, nullptr, y, M, N, K, ldy, bn, ctas, stream, QkvTail{}, nullptr, grp);
   return launch_persistent<128, 6, EPI_STORE_F32>(mw, mx, my, nullptr, y, M, N, K, ldy, bn, ctas, stream, QkvTail{}, nullptr, grp);
+}
+
+// Whether the products above take pairs of CTAs at these sizes: N features of the result; gated: mode 3.
+GB_EXPORT int gb_gemm_tc_pairs(int M, int N, int K, int bn, int ctas, int gated) {
+  return pairs_pay(M, N, K, bn, ctas, gated ? BM / 2 : BM) ? 1 : 0;
 }
 
 // (cos, sin) of every packed token's angles: table [ntok][half] float2, for gb_gemm_tc_qkv_prompt.
@@ -1570,13 +1665,15 @@ GB_EXPORT int gb_gemm_tc_qkv_prompt(const void* x, const void* w, const float* b
   if ((q_weight == nullptr) != (k_weight == nullptr)) return GB_ERR_ARG;
   if ((ldy % 8) || ((uintptr_t)y & 15)) return GB_ERR_SIZE;    // the queries leave by TMA
   const int bn = M <= 128 ? 128 : 256;
+  const bool pair = pairs_pay(M, N, K, bn, ctas, BM);
   CUtensorMap mw, mx;
   if (!tensor_map(&mw, w, (uint64_t)N, (uint64_t)K, (uint64_t)K * 2, BM)) return GB_ERR_ARG;
-  if (!tensor_map(&mx, x, (uint64_t)M, (uint64_t)K, (uint64_t)ldx * 2, (uint32_t)bn)) return GB_ERR_ARG;
+  if (!tensor_map(&mx, x, (uint64_t)M, (uint64_t)K, (uint64_t)ldx * 2, (uint32_t)(pair ? bn / 2 : bn))) return GB_ERR_ARG;
   const OutMap my = out_map(y, EPI_STORE_BF16, M, nh * BM, ldy, 32);
   if (!my.usable) return GB_ERR_ARG;
   QkvTail tail{q_weight, k_weight, nullptr, nullptr, nullptr, nullptr, nullptr, (bf16*)kcache, (bf16*)vcache,
                eps, q_scale, nh, nkv, 1, page_size, (const float2*)rope_table, (const int2*)token_place};
+  if (pair) return launch_persistent<256, 5, EPI_QKV_BF16, true>(mw, mx, my, bias, y, M, N, K, ldy, bn, ctas, stream, tail);
   if (bn > 128) return launch_persistent<256, 3, EPI_QKV_BF16>(mw, mx, my, bias, y, M, N, K, ldy, bn, ctas, stream, tail);
   return launch_persistent<128, 4, EPI_QKV_BF16>(mw, mx, my, bias, y, M, N, K, ldy, bn, ctas, stream, tail);
 }
