@@ -38,7 +38,7 @@ constexpr int THREADS = 192;
 // EPI_SWIGLU_BF16: W stacks a gate matrix over an up matrix ([2N, K]) and the kernel writes
 // silu(gate) * up in bfloat16, so the [M, 2N] intermediate never exists.  gemm_tc_kernel keeps two
 // accumulators (gate rows and up rows of the same 128 features against one tile of x);
-// gemm_tc_persistent_kernel one, whose 128 rows are 64 gate rows and the same features' up rows.
+// gemm_tc_persistent_kernel one, whose 128 rows are 8 gate rows, the same features' 8 up rows, and so on.
 enum { EPI_STORE_BF16 = 0, EPI_STORE_F32 = 1, EPI_ACCUMULATE_F32 = 2, EPI_SWIGLU_BF16 = 3, EPI_QKV_BF16 = 4 };
 
 // EPI_QKV_BF16: the q/k/v product of a decode step whose head size is the tile's 128 features: a
@@ -236,32 +236,36 @@ __device__ __forceinline__ void gate(uint32_t (&v)[16], const uint32_t (&u)[16])
   }
 }
 
-// The gated product of the persistent kernel keeps gate and up rows of W in one tile of 128 rows:
-// 64 gate rows, then the up rows of the same 64 features.  Epilogue warps 0 and 1 then hold gate
-// values (32 features each, one per lane), warps 2 and 3 the up values of the same features, and
-// warp w and w + 2 are a pair: of 32 tokens the gate warp finishes the first 16 and the up warp
-// the last 16, each handing the other, through shared memory, the 16 values it lacks (of 16
-// tokens the gate warp finishes all).  GateExchange is one pair's memory: two rounds (a warp
-// writes round r + 2 only after the pair's barrier of round r + 1, which its partner reaches
-// after it has read round r), two directions, 16 tokens x 32 lanes of float32.
-constexpr int EXCHANGE_BYTES = 2 * 2 * 2 * 16 * 32 * 4;   // two pairs
-struct GateExchange {
-  float* base;      // this pair's [round & 1][direction][16][32]
-  uint32_t round;
-  int pair;
-  __device__ __forceinline__ GateExchange(uint8_t* mem, int warp) : base((float*)mem + (warp & 1) * 2 * 2 * 16 * 32), round(0), pair(warp & 1) {}
-  // give: the 16 values of this lane that the partner finishes; returns in `got` the partner's
-  __device__ __forceinline__ void swap(const uint32_t (&give)[16], bool is_up, int lane, uint32_t (&got)[16]) {
-    float* mine = base + ((round & 1) * 2 + (is_up ? 1 : 0)) * 16 * 32;
-    const float* theirs = base + ((round & 1) * 2 + (is_up ? 0 : 1)) * 16 * 32;
+// The gated product of the persistent kernel keeps gate and up rows of W in one tile of 128 rows, 8 gate rows, then the up
+// rows of the same 8 features, and so on: lane l of an epilogue warp holds the gate or the up values of a feature, and lane
+// l ^ 8 the other half.  Of 32 tokens the gate lane finishes the first 16 and the up lane the last 16; each sends the other
+// the 16 values it lacks with a shuffle.  (With 64 gate rows before 64 up rows the halves sat in different warps and went
+// through shared memory and a barrier of two warps a round: 10.5 us a tile of 256 tokens, 15.2 with the clamps and a scale
+// a row that was loaded where it was used, more than the MMAs of a tile take up to 2,560 inner elements.)
+__device__ __forceinline__ void gate_swap(const uint32_t (&lo)[16], const uint32_t (&hi)[16], bool is_up, float (&g)[16], float (&u)[16]) {
 #pragma unroll
-    for (int j = 0; j < 16; ++j) mine[j * 32 + lane] = __uint_as_float(give[j]);
-    asm volatile("bar.sync %0, 64;" ::"r"(1 + pair) : "memory");
-#pragma unroll
-    for (int j = 0; j < 16; ++j) got[j] = __float_as_uint(theirs[j * 32 + lane]);
-    ++round;
+  for (int j = 0; j < 16; ++j) {
+    const float got = __shfl_xor_sync(0xffffffffu, __uint_as_float(is_up ? lo[j] : hi[j]), 8);
+    g[j] = is_up ? got : __uint_as_float(lo[j]);
+    u[j] = is_up ? __uint_as_float(hi[j]) : got;
   }
-};
+}
+
+constexpr int GATED_FEATURES = 16;     // features of the result that a warp holds
+
+// A gated tile's rows of W: [K, 8 rows, gate or up, groups of 8 rows] from group y on.
+__device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %5, %5, %4}], [%2];"
+      ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(0)
+      : "memory");
+}
+__device__ __forceinline__ void tma_load_4d_pair(void* dst, const CUtensorMap* map, int x, int y, uint32_t cluster_bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%3, %5, %5, %4}], [%2];"
+      ::"r"(smem_u32(dst)), "l"(map), "r"(cluster_bar), "r"(x), "r"(y), "r"(0)
+      : "memory");
+}
 
 // One value of one token of one head tile, held by epilogue thread f = feature; all 128 epilogue
 // threads call it together.  red: 4 floats, xs: 128 floats of shared memory.
@@ -844,11 +848,11 @@ struct TileWalk {
   }
 };
 
-// The q/k/v mode has eight epilogue warps, two to each quarter of tensor memory's lanes (a warp
+// The q/k/v and gated modes have eight epilogue warps, two to each quarter of tensor memory's lanes (a warp
 // reaches the quarter warp % 4): warps 0-3 take the even rounds of 32 tokens of a tile, warps 6-9
-// the odd ones.  Its epilogue is work, not stores (a round is 2.9 us for four warps), and at
+// the odd ones.  Their epilogue is work, not stores (q/k/v: a round is 2.9 us for four warps), and at
 // short inner dimensions (2,560: 16 us of MMAs a tile) it, not the MMAs, set the product's time.
-constexpr int PERSISTENT_QKV_THREADS = 320, QKV_STAGING_BYTES = 65 * 1024;   // pieces 32 KB, exchange 2 x 16 KB, sums 1 KB
+constexpr int EIGHT_WARPS_THREADS = 320, QKV_STAGING_BYTES = 65 * 1024;   // pieces 32 KB, exchange 2 x 16 KB, sums 1 KB
 
 // A grouped product (the experts of a routed feed-forward): the rows of x are ordered by group and
 // every group's rows start at a multiple of the tile's tokens, so a tile of tokens belongs to one
@@ -867,6 +871,7 @@ struct Grouped {
   int rows_per_expert = 0;
   float limit = 0.f, alpha = 0.f, shift = 0.f;
   int act = 0, scale_in = 0;
+  int gate_rows_whole = 0;     // gated: map_w brings a tile's gate and up rows in one box (gated_map)
 };
 __device__ __forceinline__ void act_rows(uint32_t (&v)[16], float bias, int act, const float* row_scale, int row, int M) {
 #pragma unroll
@@ -882,13 +887,13 @@ __device__ __forceinline__ float clamped_gate(float g, float u, const Grouped& g
 }
 
 template <int BN, int STAGES, int MODE, bool PAIR>
-__global__ void __launch_bounds__(MODE == EPI_QKV_BF16 ? PERSISTENT_QKV_THREADS : THREADS, 1)
+__global__ void __launch_bounds__(MODE == EPI_QKV_BF16 || MODE == EPI_SWIGLU_BF16 ? EIGHT_WARPS_THREADS : THREADS, 1)
 gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                           const __grid_constant__ CUtensorMap map_y, int y_tma, const float* __restrict__ bias,
                           void* __restrict__ y, int M, int N, int K, long long ldy, int bn,
                           const __grid_constant__ QkvTail tail, int split_last, int* __restrict__ part_flags,
                           const __grid_constant__ Grouped grp) {
-  constexpr bool GATED = MODE == EPI_SWIGLU_BF16;   // rows of a tile: 16 gate, 16 up, ... (see gate_rows)
+  constexpr bool GATED = MODE == EPI_SWIGLU_BF16;   // rows of a tile: 8 gate, 8 up, ... (see gate_swap)
   // the last round's tiles in parts along the inner dimension: only where parts can be added
   const int split = MODE == EPI_ACCUMULATE_F32 ? max(split_last, 1) : 1;
   constexpr bool QKV = MODE == EPI_QKV_BF16;        // a tile is one head: norm, rotation, cache write (qkv_prompt_round)
@@ -910,14 +915,14 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
   uint32_t* tmem_slot = (uint32_t*)(acc_empty + 2);
   volatile int* epilogue_gave_up = (volatile int*)(tmem_slot + 1);
   uint8_t* out_staging = smem + STAGES * STAGE_BYTES + 1024;   // past the barriers; OUT_STAGING_BYTES
-  // gated: the pieces are 16 tokens of bfloat16 (1 KB), and the pairs' exchange has the upper half
-  constexpr int SLOT = (GATED || QKV) ? OUT_STAGING_BYTES / 2 / (4 * PIECES) : PIECE_BYTES;
-  static_assert(!GATED || (SLOT >= 16 * PIECE_FEATURES * 2 && OUT_STAGING_BYTES / 2 >= EXCHANGE_BYTES), "gated staging");
+  // gated: eight warps' pieces of 32 tokens x 16 features of bfloat16 (1 KB)
+  constexpr int SLOT = GATED ? PIECE_TOKENS * GATED_FEATURES * 2 : QKV ? OUT_STAGING_BYTES / 2 / (4 * PIECES) : PIECE_BYTES;
+  static_assert(!GATED || (SLOT >= PIECE_TOKENS * GATED_FEATURES * 2 && 8 * PIECES * SLOT <= OUT_STAGING_BYTES), "gated staging");
   // q/k/v: eight warps' bfloat16 pieces of 32 tokens (32 KB), then each group of four warps' exchange
   // (16 KB each), then their partial sums
   static_assert(!QKV || (SLOT >= PIECE_TOKENS * PIECE_FEATURES * 2 && 8 * PIECES * SLOT == 32 * 1024), "q/k/v staging");
   static_assert((2 * STAGES + 4) * 8 + 16 <= 1024, "the barriers have 1 KB");
-  constexpr int EPI_WARPS = QKV ? 8 : 4;
+  constexpr int EPI_WARPS = QKV || GATED ? 8 : 4;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = PAIR ? (int)cluster_rank() : 0, walker = (int)blockIdx.x / CTAS, walkers = (int)gridDim.x / CTAS;
@@ -988,13 +993,16 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
             else tma_load_2d(dst, map, kb * BK, row, &full_bar[s]);
           };
           if (rank == 0) mbar_expect_tx(&full_bar[s], stage_tx);
-          if (GATED) {   // map_w is cut into boxes of 64 rows: the gate rows, then the same features' up rows
-            // (a request costs the issuing thread about 75 cycles: boxes of 16 rows, which would let a
-            // warp gate without shared memory, made nine requests a block and the producer the limit)
+          if (!GATED) {
             load(a, &map_w, w0);
-            load(a + A_BYTES / 2, &map_w, N + w0);
-          } else {
-            load(a, &map_w, w0);
+          } else if (grp.gate_rows_whole) {      // one box: 8 gate rows, the same features' 8 up rows, and so on
+            if (PAIR) tma_load_4d_pair(a, &map_w, kb * BK, w0 / 8, bar);
+            else tma_load_4d(a, &map_w, kb * BK, w0 / 8, &full_bar[s]);
+          } else {                               // N is not a multiple of 8: a box each (75 cycles of the issuing thread a request)
+            for (int g = 0; g < TILE_F / 8; ++g) {
+              load(a + g * 2048, &map_w, w0 + 8 * g);
+              load(a + g * 2048 + 1024, &map_w, N + w0 + 8 * g);
+            }
           }
           load(a + A_BYTES, &map_x, x0);
         }
@@ -1059,10 +1067,10 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
     // ---------------- epilogue warps: lane = feature, column = token
     pdl_wait_prior();
     const int quarter = warp & 3, group = warp >= 6 ? 1 : 0;          // group 1: the q/k/v mode's second four
-    const int f = GATED ? (warp & 1) * 32 + lane : quarter * 32 + lane;   // this lane's feature of the tile
-    const bool is_up = GATED && warp >= 2;
+    const int piece_f = (lane >> 4) * 8 + (lane & 7);                      // gated: this lane's feature of the warp's 16
+    const int f = GATED ? quarter * GATED_FEATURES + piece_f : quarter * 32 + lane;   // this lane's feature of the tile
+    const bool is_up = GATED && (lane & 8) != 0;
     TileOut<MODE, SLOT> tile_out(&map_y, out_staging, group * 4 + quarter);
-    GateExchange exchange(out_staging + OUT_STAGING_BYTES / 2, warp);
     const PromptTailShared tail_shared{(float*)(out_staging + 32 * 1024 + group * 16 * 1024),
                                        (float*)(out_staging + 64 * 1024) + group * 4 * 32};
     const bool both = bn % 32 == 0;   // 32 tokens per round; the result's map is cut to match
@@ -1080,7 +1088,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
       const int m_end = grp.tile_rows ? min(M, m0 + grp.tile_rows[m0 / bn]) : M;     // the tile's rows that exist
       bool have = __all_sync(0xffffffffu, PAIR ? mbar_wait_cluster(&acc_full[b], (i >> 1) & 1) : mbar_wait(&acc_full[b], (i >> 1) & 1));
       if (!have && lane == 0) atomicCAS(&g_status, ST_OK, ST_TIMEOUT_TMEM);
-      if (GATED || QKV) {   // the warps meet at barriers below: they leave together or not at all
+      if (QKV) {   // the warps meet at barriers below: they leave together or not at all
         if (!have && lane == 0) *epilogue_gave_up = 1;
         asm volatile("bar.sync 3, %0;" ::"n"(EPI_WARPS * 32) : "memory");
         have = *epilogue_gave_up == 0;
@@ -1113,51 +1121,53 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
       }
       const uint32_t acc = tmem + ((uint32_t)(quarter * 32) << 16) + b * ACC_COLS;
 #pragma unroll 1
-      for (int c = QKV ? 32 * group : 0; c < bn; c += QKV ? 64 : (both ? 32 : 16)) {
+      for (int c = QKV || GATED ? 32 * group : 0; c < bn; c += QKV || GATED ? 64 : (both ? 32 : 16)) {
         if (m0 + c >= m_end || n0 >= N) break;     // n0: a pair's last tile may be half beyond the result
         uint32_t v[16], v2[16];
+        // gated: lane l has the row scale of token c + l; asked for before the accumulator is read
+        const float scales = GATED && grp.row_scale && m0 + c + lane < m_end ? grp.row_scale[m0 + c + lane] : 0.f;
         tc_ld16(acc + c, v);
-        if (both) tc_ld16(acc + c + 16, v2);
+        if (both || GATED) tc_ld16(acc + c + 16, v2);     // gated: columns beyond the tile are read and go nowhere
         tc_wait_ld();
         if (GATED) {
-          // 32 tokens: the gate warp gives its last 16 and finishes the first 16, the up warp the other
-          // way round; 16 tokens: the up warp gives, the gate warp finishes
-          uint32_t got[16];
-          exchange.swap((both && !is_up) ? v2 : v, is_up, lane, got);
-          if (both || !is_up) {
-            const uint32_t (&g)[16] = is_up ? got : v;
-            const uint32_t (&u)[16] = is_up ? v2 : got;
-            const int row = m0 + c + (is_up ? 16 : 0);
-            float r[16];
-            if (grp.scale_in) {
+          float g[16], u[16], r[16];
+          gate_swap(v, v2, is_up, g, u);
+          const int row = m0 + c + (is_up ? 16 : 0);
+          if (grp.limit > 0.f || grp.row_scale) {
 #pragma unroll
-              for (int j = 0; j < 16; ++j) {
-                const float sc = row + j < m_end ? grp.row_scale[row + j] : 0.f;
-                const float gs = __uint_as_float(g[j]) * sc, us = __uint_as_float(u[j]) * sc;
-                r[j] = grp.limit > 0.f ? clamped_gate(gs, us, grp) : silu_mul(gs, us);
+            for (int j = 0; j < 16; ++j) {
+              const float sc = __shfl_sync(0xffffffffu, scales, (is_up ? 16 : 0) + j);
+              const float gs = grp.scale_in ? g[j] * sc : g[j], us = grp.scale_in ? u[j] * sc : u[j];
+              r[j] = grp.limit > 0.f ? clamped_gate(gs, us, grp) : silu_mul(gs, us);
+              if (grp.row_scale && !grp.scale_in) r[j] *= sc;
+            }
+          } else {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) r[j] = silu_mul(g[j], u[j]);
+          }
+          if (y_tma) {
+            uint8_t* p = tile_out.next(lane);
+            bf16* to = (bf16*)p + (is_up ? 16 * GATED_FEATURES : 0) + piece_f;
+#pragma unroll
+            for (int j = 0; j < 16; ++j) to[j * GATED_FEATURES] = __float2bfloat16_rn(r[j]);
+            const int x = n0 + quarter * GATED_FEATURES;
+            if (both) {
+              tile_out.post(p, lane, x, m0 + c, N);
+            } else {                              // the map's pieces are 16 tokens; the tile may end after the first
+              fence_smem_to_tma();
+              __syncwarp();
+              if (lane == 0 && x < N) {
+                tma_store_2d(&map_y, p, x, m0 + c);
+                if (c + 16 < bn) tma_store_2d(&map_y, p + 16 * GATED_FEATURES * 2, x, m0 + c + 16);
+                tma_store_commit();
               }
-            } else {
-#pragma unroll
-              for (int j = 0; j < 16; ++j) r[j] = silu_mul(__uint_as_float(g[j]), __uint_as_float(u[j]));
+              ++tile_out.sent;
             }
-            if (grp.limit > 0.f && !grp.scale_in) {
+          } else if (n < N) {
+            const int end = min(m_end, m0 + bn);
 #pragma unroll
-              for (int j = 0; j < 16; ++j) r[j] = clamped_gate(__uint_as_float(g[j]), __uint_as_float(u[j]), grp);
-            }
-            if (grp.row_scale && !grp.scale_in) {
-#pragma unroll
-              for (int j = 0; j < 16; ++j) r[j] *= row + j < m_end ? grp.row_scale[row + j] : 0.f;
-            }
-            if (y_tma) {
-              uint8_t* p = tile_out.next(lane);
-#pragma unroll
-              for (int j = 0; j < 16; ++j) tile_out.put(p, j, lane, r[j]);
-              tile_out.post(p, lane, n0 + (warp & 1) * 32, row, N);
-            } else if (n < N) {
-#pragma unroll
-              for (int j = 0; j < 16; ++j)
-                if (row + j < m_end) emit<MODE>(y, (size_t)(row + j) * ldy + n, r[j]);
-            }
+            for (int j = 0; j < 16; ++j)
+              if (row + j < end) emit<MODE>(y, (size_t)(row + j) * ldy + n, r[j]);
           }
         } else if (QKV) {
           float x[32];
@@ -1249,12 +1259,52 @@ struct OutMap {
   int usable;
 };
 // bn: tokens per tile; the kernels send 32 tokens at a time where a tile has that many.
-OutMap out_map(const void* y, int mode, int M, int N, long long ldy, int bn) {
+OutMap out_map(const void* y, int mode, int M, int N, long long ldy, int bn, int features = PIECE_FEATURES) {
   OutMap o = {};
   const bool f32 = mode == EPI_STORE_F32 || mode == EPI_ACCUMULATE_F32;
   o.usable = mode != EPI_QKV_BF16 && tensor_map_out(&o.map, y, (uint64_t)M, (uint64_t)N, (uint64_t)ldy * (f32 ? 4 : 2),
-                                                    bn % 32 == 0 ? 32 : 16, 32, f32);
+                                                    bn % 32 == 0 ? 32 : 16, (uint32_t)features, f32);
   return o;
+}
+
+// W [experts][gate N rows, up N rows][K] as a gated tile reads it: boxes of 64 inner elements by 8 gate rows, the same
+// features' 8 up rows, 8 times.  Only for N a multiple of 8; group g is rows 8 g .. of all gate and up rows together, so
+// that expert e's first is e N / 4.  The last groups are those whose up rows exist.
+bool gated_map(CUtensorMap* out, const void* w, uint64_t rows, uint64_t N, uint64_t K) {
+  struct Key {
+    const void* w;
+    uint64_t rows, N, K;
+    bool operator==(const Key& o) const { return w == o.w && rows == o.rows && N == o.N && K == o.K; }
+  };
+  struct Hash {
+    size_t operator()(const Key& k) const { return (((size_t)k.w * 1000003u ^ k.rows) * 1000003u ^ k.N) * 1000003u ^ k.K; }
+  };
+  static std::unordered_map<Key, CUtensorMap, Hash> cache;
+  static std::mutex mu;
+  std::lock_guard<std::mutex> lock(mu);
+  const Key key{w, rows, N, K};
+  const auto it = cache.find(key);
+  if (it != cache.end()) {
+    *out = it->second;
+    return true;
+  }
+  const EncodeTiled fn = encode_fn();
+  if (!fn || N % 8 || rows < 2 * N) return false;
+  const cuuint64_t dims[4] = {K, 8, 2, (rows - N) / 8}, strides[3] = {K * 2, N * K * 2, 8 * K * 2};
+  const cuuint32_t box[4] = {BK, 8, 2, BM / 16}, elem[4] = {1, 1, 1, 1};
+  if (fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(w), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+         CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+    return false;
+  if (cache.size() > 65536) cache.clear();
+  cache.emplace(key, *out);
+  return true;
+}
+
+// The rows of W for the persistent kernel: the gated form where there is one, boxes of 8 rows for other N.
+bool persistent_w_map(CUtensorMap* out, const void* w, uint64_t rows, int N, int K, bool gated, Grouped& grp) {
+  grp.gate_rows_whole = gated && N % 8 == 0;
+  return grp.gate_rows_whole ? gated_map(out, w, rows, (uint64_t)N, (uint64_t)K)
+                             : tensor_map(out, w, rows, (uint64_t)K, (uint64_t)K * 2, gated ? 8 : BM);
 }
 
 template <int BN, int STAGES, int MODE>
@@ -1348,7 +1398,7 @@ int launch_persistent(const CUtensorMap& mw, const CUtensorMap& mx, const OutMap
   constexpr int CTAS = PAIR ? 2 : 1;
   constexpr size_t STAGING = MODE == EPI_QKV_BF16 ? QKV_STAGING_BYTES : OUT_STAGING_BYTES;
   constexpr size_t SMEM = (size_t)STAGES * ((size_t)BM * BK * 2 + BN / CTAS * BK * 2) + 1024 + STAGING + 1024;
-  constexpr int NTHREADS = MODE == EPI_QKV_BF16 ? PERSISTENT_QKV_THREADS : THREADS;
+  constexpr int NTHREADS = MODE == EPI_QKV_BF16 || MODE == EPI_SWIGLU_BF16 ? EIGHT_WARPS_THREADS : THREADS;
   static_assert(SMEM <= 227 * 1024, "stages do not fit in shared memory");
   static_assert((2 * STAGES + 4) * 8 + 16 <= 1024, "the barriers have 1 KB");
   constexpr int WALK_F = CTAS * (MODE == EPI_SWIGLU_BF16 ? BM / 2 : BM);
@@ -1543,14 +1593,13 @@ GB_EXPORT int gb_gemm_tc_persistent(const void* x, const void* w, const float* b
   const bool pair = pairs_pay(M, N, K, bn, ctas, swiglu ? BM / 2 : BM);
   if (pair) bn = (bn + 31) / 32 * 32;          // its MMA is as wide as a multiple of 32 tokens
   CUtensorMap mw, mx;
-  // gated: W in boxes of 64 rows; a tile is 64 gate rows and the same features' 64 up rows
-  if (!tensor_map(&mw, w, (uint64_t)N * (swiglu ? 2 : 1), (uint64_t)K, (uint64_t)K * 2, swiglu ? BM / 2 : BM)) return GB_ERR_ARG;
+  if (!persistent_w_map(&mw, w, (uint64_t)N * (swiglu ? 2 : 1), N, K, swiglu, grp)) return GB_ERR_ARG;
   if (!tensor_map(&mx, x, (uint64_t)M, (uint64_t)K, (uint64_t)ldx * 2, (uint32_t)(pair ? bn / 2 : bn))) return GB_ERR_ARG;
-  const OutMap my = out_map(y, mode, M, N, ldy, swiglu ? 16 : bn);   // gated: a warp sends 16 tokens at a time
+  const OutMap my = out_map(y, mode, M, N, ldy, bn, swiglu ? GATED_FEATURES : PIECE_FEATURES);
   if (swiglu) {
-    if (pair) return launch_persistent<256, 6, EPI_SWIGLU_BF16, true>(mw, mx, my, bias, y, M, N, K, ldy, bn, ctas, stream);
-    if (bn > 128) return launch_persistent<256, 4, EPI_SWIGLU_BF16>(mw, mx, my, bias, y, M, N, K, ldy, bn, ctas, stream);
-    return launch_persistent<128, 6, EPI_SWIGLU_BF16>(mw, mx, my, bias, y, M, N, K, ldy, bn, ctas, stream);
+    if (pair) return launch_persistent<256, 6, EPI_SWIGLU_BF16, true>(mw, mx, my, bias, y, M, N, K, ldy, bn, ctas, stream, QkvTail{}, nullptr, grp);
+    if (bn > 128) return launch_persistent<256, 4, EPI_SWIGLU_BF16>(mw, mx, my, bias, y, M, N, K, ldy, bn, ctas, stream, QkvTail{}, nullptr, grp);
+    return launch_persistent<128, 6, EPI_SWIGLU_BF16>(mw, mx, my, bias, y, M, N, K, ldy, bn, ctas, stream, QkvTail{}, nullptr, grp);
   }
   if (pair) {
     switch (mode) {
@@ -1603,9 +1652,9 @@ GB_EXPORT int gb_gemm_tc_grouped(const void* x, const void* w, void* y, int mode
   grp.scale_in = gated && row_scale ? scale_in : 0;
   const bool pair = pairs_pay(M, N, K, bn, ctas, gated ? BM / 2 : BM);
   CUtensorMap mw, mx;
-  if (!tensor_map(&mw, w, (uint64_t)experts * grp.rows_per_expert, (uint64_t)K, (uint64_t)K * 2, gated ? BM / 2 : BM)) return GB_ERR_ARG;
+  if (!persistent_w_map(&mw, w, (uint64_t)experts * grp.rows_per_expert, N, K, gated, grp)) return GB_ERR_ARG;
   if (!tensor_map(&mx, x, (uint64_t)M, (uint64_t)K, (uint64_t)ldx * 2, (uint32_t)(pair ? bn / 2 : bn))) return GB_ERR_ARG;
-  const OutMap my = out_map(y, mode, M, N, ldy, gated ? 16 : bn);
+  const OutMap my = out_map(y, mode, M, N, ldy, bn, gated ? GATED_FEATURES : PIECE_FEATURES);
   if (gated) {
     if (pair) return launch_persistent<256, 6, EPI_SWIGLU_BF16, true>(mw, mx, my, nullptr, y, M, N, K, ldy, bn, ctas, stream, QkvTail{}, nullptr, grp);
     if (bn > 128) return launch_persistent<256, 4, EPI_SWIGLU_BF16>(mw, mx, my, nullptr, y, M, N, K, ldy, bn, ctas, stream, QkvTail{}, nullptr, grp);

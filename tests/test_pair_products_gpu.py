@@ -52,20 +52,23 @@ def test_plain_and_adding_products(k, m, n, kk, bn):
     assert k.gemm_tc_status() == 0
 
 
-@pytest.mark.parametrize("m,n,kk", [(520, 192, 200), (1000, 72, 4104), (300, 960, 64)])
+@pytest.mark.parametrize("m,n,kk", [(520, 192, 200), (1000, 72, 4104), (300, 960, 64), (520, 188, 200), (1000, 1672, 72)])
 def test_gated_product(k, m, n, kk):
+    """Also results whose features are no multiple of 8 (a box of W's rows at a time) or end within a warp's 16."""
     assert pairs(k, m, n, kk, 256, 4, True) == 1
     x, w = operands(m, 2 * n, kk, m + n)
     y = torch.empty(m, n, device="cuda", dtype=torch.bfloat16)
     k.gemm_tc_persistent(x, w, y, swiglu=True, ctas=4)
     one = torch.empty_like(y)
     k.gemm_tc_persistent(x, w, one, swiglu=True, ctas=1)          # one CTA walks all tiles: never a pair
+    narrow = torch.empty_like(y)
+    k.gemm_tc_persistent(x, w, narrow, swiglu=True, bn=112, ctas=4)   # tiles that end after half of a round's tokens
     g, u = (x.double() @ w[:n].double().T), (x.double() @ w[n:].double().T)
     want = g * torch.sigmoid(g) * u
     # bfloat16's half step, and the two sums' float32 errors through a slope of at most 1.1 |u| and 1.1 |g|
     _, bound = exact_and_bound(x, w)
     tol = 2.0 ** -8 * want.abs() + 1.2 * (u.abs() * bound[:, :n] + (g.abs() + 1) * bound[:, n:]) + 2.0 ** -20 * (g.abs() + 1) * (u.abs() + 1)
-    assert ((y.double() - want).abs() <= tol).all() and ((one.double() - want).abs() <= tol).all()
+    assert ((y.double() - want).abs() <= tol).all() and ((one.double() - want).abs() <= tol).all() and ((narrow.double() - want).abs() <= tol).all()
     assert k.gemm_tc_status() == 0
 
 
