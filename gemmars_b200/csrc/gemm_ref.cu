@@ -3,10 +3,11 @@
 // FFMA only: no tensor-core or reduced-precision matrix mode is compiled into this unit.
 //
 // It is the whole matrix path of the float32 engine (gemm_f32_kernel) and the plain reference of the
-// bfloat16 tensor-core kernels (gemm_ref_kernel).  Every output element is accumulated by one thread
-// over i = 0..K-1 in ascending order, so a row's result does not depend on how many rows the call has
-// (the property the reference tests as batch invariance, src/qwen_mtp.rs:748-776), nor on the tile
-// that the launcher picks.
+// bfloat16 tensor-core kernels (gemm_ref_kernel).  The order in which an output element is summed depends
+// on K alone, so a row's result does not depend on how many rows the call has (the property the
+// reference tests as batch invariance, src/qwen_mtp.rs:748-776), nor on the tile that the launcher picks.
+#include <type_traits>
+
 #include "common.cuh"
 
 enum { OUT_STORE = 0, OUT_ACCUMULATE_F32 = 1 };
@@ -72,12 +73,20 @@ __global__ void __launch_bounds__(256) gemm_ref_kernel(const TI* __restrict__ x,
 }
 
 // ------------------------------------------------------------------ float32
-// The float32 product: a CTA works BM rows of x by BN rows of W, a thread TM x TN results in registers.
-// Both operands lie in shared memory as they lie in memory (KB of K side by side, a row 4 floats longer so
-// that the 16-byte reads of eight neighbouring rows touch all banks once), brought by asynchronous copies
-// STAGES - 1 blocks ahead; a thread reads four k of each of its rows at a time: TM + TN 16-byte reads for
-// 4 TM TN multiply-adds.  What bounds it: those reads and the FFMA pipe for prompts, the stream of W for a
-// few rows.  The first blocks of W are asked for before the kernel before this one has ended.
+// The float32 product: four warps, each a part of the inner dimension of one tile of 4 TM rows of x by 8 TN rows of W, TM x TN
+// results a lane.  Every result is the sum of PARTS parts, added in their order; a part's length depends on the inner dimension
+// alone, and in a part the even and the odd inner elements have a sum each (two multiply-adds in one instruction).  So the bits
+// depend neither on the tile nor on the number of rows, and the error is smaller than one long sum's (distance from 64 bits of
+// 1,024 / 4,096 inner elements: 2.1e-7 / 4.1e-7, one sum 5.7e-7 / 1.2e-6).
+// A warp brings its own rows, KB of K side by side and a row 4 floats longer so that the 16-byte reads of eight neighbouring
+// rows touch all banks once, by asynchronous copies STAGES - 1 blocks ahead, and waits for no other warp until the parts are
+// added: no barrier in the main loop, and four warps on a tile where one thread for every result's whole sum would leave an SM
+// two (301 rows by 1,024 features are 2,082 results an SM).  What bounds it: the 16-byte reads, TM + TN for 4 TM TN
+// multiply-adds (2,048 x 4,096 x 4,096 at 45.9 of some 70 TFLOP/s; 43.7 with KB of 16, 40 with a multiply-add an instruction), the last round of tiles, and the stream of W for a few
+// rows.  The first blocks of W are asked for before the kernel before this one has ended.
+constexpr int PARTS = 4;
+__host__ __device__ constexpr int part_length(int K) { return ((K + PARTS - 1) / PARTS + 31) / 32 * 32; }
+
 __device__ __forceinline__ void copy16(float* dst, const float* src, int bytes) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(bytes)
                : "memory");
@@ -86,103 +95,121 @@ __device__ __forceinline__ void copy4(float* dst, const float* src, int bytes) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(bytes)
                : "memory");
 }
+__device__ __forceinline__ void fma2(uint64_t& d, uint64_t a, uint64_t b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ float even_and_odd(uint64_t v) {
+  return __uint_as_float((uint32_t)v) + __uint_as_float((uint32_t)(v >> 32));
+}
 
-template <int BM, int BN, int TM, int TN, int KB, int STAGES>
+template <int TM, int TN, int KB, int STAGES>
 struct F32Tile {
-  static constexpr int TY = BM / TM, TX = BN / TN, THREADS = TY * TX, LD = KB + 4;
-  static constexpr int STAGE_FLOATS = (BM + BN) * LD;
-  static constexpr size_t SMEM = (size_t)STAGES * STAGE_FLOATS * sizeof(float);
+  static constexpr int BM = 4 * TM, BN = 8 * TN, LD = KB + 4;
+  static constexpr int STAGE_FLOATS = (BM + BN) * LD, WARP_FLOATS = STAGES * STAGE_FLOATS;
+  static_assert(WARP_FLOATS >= BM * BN, "a part's results go where its stages were");
+  static_assert(TM * TN % PARTS == 0 && KB == 32, "whole shares; a part is a multiple of KB");
+  static constexpr size_t SMEM = (size_t)PARTS * WARP_FLOATS * sizeof(float);
 };
 
-// VEC: rows of both operands start at 16-byte boundaries and K is a multiple of 4.
-template <int BM, int BN, int TM, int TN, int KB, int STAGES, bool VEC, int MODE>
-__global__ void __launch_bounds__(F32Tile<BM, BN, TM, TN, KB, STAGES>::THREADS)
+// VEC: rows of both operands start at 16-byte boundaries and K is a multiple of 4.  The grid's CTAs run over the rows first.
+template <int TM, int TN, int KB, int STAGES, bool VEC, int MODE>
+__global__ void __launch_bounds__(32 * PARTS)
     gemm_f32_kernel(const float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ bias, float* __restrict__ y,
-                    int M, int N, int K, long long ldx, long long ldy, int act, const float* __restrict__ col_scale) {
-  using T = F32Tile<BM, BN, TM, TN, KB, STAGES>;
-  constexpr int LD = T::LD, NT = T::THREADS, CH = KB / 4;      // 16-byte pieces of a row
-  constexpr int WY = T::TY < 8 ? T::TY : 8, WX = 32 / WY;       // a warp's threads: WY rows by WX columns
-  static_assert(T::TX % WX == 0 && T::TY % WY == 0, "whole warps");
+                    int M, int N, int K, long long ldx, long long ldy, int act, const float* __restrict__ col_scale, int tiles_m) {
+  using T = F32Tile<TM, TN, KB, STAGES>;
+  constexpr int BM = T::BM, BN = T::BN, LD = T::LD, CH = KB / 4, STEP = 32 / CH;      // CH 16-byte pieces of a row, STEP rows a pass
   extern __shared__ __align__(16) float smem[];
-  pdl_release_next();
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-  const int ty = warp / (T::TX / WX) * WY + lane % WY, tx = warp % (T::TX / WX) * WX + lane / WY;
-  const int blocks = (K + KB - 1) / KB;
-  auto bring = [&](int block, const float* base, long long ld, int row0, int rows_have, float* dst, int rows) {
-    for (int e = tid; e < rows * CH; e += NT) {
-      const int r = e / CH, c = (e % CH) * 4, k = block * KB + c;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int m0 = blockIdx.x % tiles_m * BM, n0 = blockIdx.x / tiles_m * BN;
+  const int ty = lane >> 3, tx = lane & 7;
+  const int length = part_length(K), k0 = min(K, warp * length), k1 = min(K, k0 + length);
+  const int blocks = (k1 - k0 + KB - 1) / KB;
+  float* mine = smem + warp * T::WARP_FLOATS;
+  const int r0 = lane / CH, c = lane % CH * 4;
+  auto bring = [&](int block, const float* base, long long ld, int row0, int rows_have, float* dst, auto rows) {
+    constexpr int ROWS = decltype(rows)::value;
+    const int k = k0 + block * KB + c;
+#pragma unroll
+    for (int i = 0; i < (ROWS + STEP - 1) / STEP; ++i) {
+      const int r = r0 + STEP * i;
+      if (ROWS % STEP && r >= ROWS) break;
       float* d = dst + r * LD + c;
       const bool row_in = row0 + r < rows_have;
       const float* src = base + (size_t)(row_in ? row0 + r : 0) * ld;
       if (VEC) {
-        const bool in = row_in && k < K;
+        const bool in = row_in && k < k1;
         copy16(d, in ? src + k : base, in ? 16 : 0);
       } else {
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          const bool in = row_in && k + j < K;
+          const bool in = row_in && k + j < k1;
           copy4(d + j, in ? src + k + j : base, in ? 4 : 0);
         }
       }
     }
   };
-  auto stage_x = [&](int block) { return smem + (block % STAGES) * T::STAGE_FLOATS; };
-  auto stage_w = [&](int block) { return stage_x(block) + BM * LD; };
+  using RowsX = std::integral_constant<int, BM>;
+  using RowsW = std::integral_constant<int, BN>;
 #pragma unroll
   for (int s = 0; s < STAGES - 1; ++s)
-    if (s < blocks) bring(s, w, K, n0, N, stage_w(s), BN);
+    if (s < blocks) bring(s, w, K, n0, N, mine + s * T::STAGE_FLOATS + BM * LD, RowsW());
   pdl_wait_prior();
 #pragma unroll
   for (int s = 0; s < STAGES - 1; ++s) {
-    if (s < blocks) bring(s, x, ldx, m0, M, stage_x(s), BM);
+    if (s < blocks) bring(s, x, ldx, m0, M, mine + s * T::STAGE_FLOATS, RowsX());
     asm volatile("cp.async.commit_group;" ::: "memory");
   }
-  float acc[TM][TN] = {};
+  uint64_t acc[TM][TN] = {};
+  int at = 0, to = STAGES - 1;
+#pragma unroll 1
   for (int b = 0; b < blocks; ++b) {
     asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
-    __syncthreads();                       // block b is there for all, and block b - 1 has been read by all
+    __syncwarp();                          // block b is there for all lanes, and block b - 1 has been read by all
     if (b + STAGES - 1 < blocks) {
-      bring(b + STAGES - 1, x, ldx, m0, M, stage_x(b + STAGES - 1), BM);
-      bring(b + STAGES - 1, w, K, n0, N, stage_w(b + STAGES - 1), BN);
+      bring(b + STAGES - 1, x, ldx, m0, M, mine + to * T::STAGE_FLOATS, RowsX());
+      bring(b + STAGES - 1, w, K, n0, N, mine + to * T::STAGE_FLOATS + BM * LD, RowsW());
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
-    const float *xs = stage_x(b) + ty * LD, *ws = stage_w(b) + tx * LD;
+    const float *xs = mine + at * T::STAGE_FLOATS + ty * LD, *ws = mine + at * T::STAGE_FLOATS + (BM + tx) * LD;
+    at = at + 1 == STAGES ? 0 : at + 1;
+    to = to + 1 == STAGES ? 0 : to + 1;
 #pragma unroll
     for (int kk = 0; kk < KB; kk += 4) {
-      float4 a[TM];
+      ulonglong2 v[TN];
 #pragma unroll
-      for (int i = 0; i < TM; ++i) a[i] = *(const float4*)(xs + i * T::TY * LD + kk);
+      for (int j = 0; j < TN; ++j) v[j] = *(const ulonglong2*)(ws + j * 8 * LD + kk);
 #pragma unroll
-      for (int j = 0; j < TN; ++j) {
-        const float4 v = *(const float4*)(ws + j * T::TX * LD + kk);
+      for (int i = 0; i < TM; ++i) {
+        const ulonglong2 a = *(const ulonglong2*)(xs + i * 4 * LD + kk);
 #pragma unroll
-        for (int i = 0; i < TM; ++i) acc[i][j] = fmaf(a[i].x, v.x, acc[i][j]);
+        for (int j = 0; j < TN; ++j) fma2(acc[i][j], a.x, v[j].x);
 #pragma unroll
-        for (int i = 0; i < TM; ++i) acc[i][j] = fmaf(a[i].y, v.y, acc[i][j]);
-#pragma unroll
-        for (int i = 0; i < TM; ++i) acc[i][j] = fmaf(a[i].z, v.z, acc[i][j]);
-#pragma unroll
-        for (int i = 0; i < TM; ++i) acc[i][j] = fmaf(a[i].w, v.w, acc[i][j]);
+        for (int j = 0; j < TN; ++j) fma2(acc[i][j], a.y, v[j].y);
       }
     }
   }
+  pdl_release_next();
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncwarp();
 #pragma unroll
-  for (int j = 0; j < TN; ++j) {
-    const int gn = n0 + j * T::TX + tx;
-    if (gn >= N) continue;
-    const float b0 = bias ? bias[gn] : 0.f, c0 = col_scale ? col_scale[gn] : 1.f;
+  for (int i = 0; i < TM; ++i)
 #pragma unroll
-    for (int i = 0; i < TM; ++i) {
-      const int gm = m0 + i * T::TY + ty;
-      if (gm >= M) continue;
-      float v = acc[i][j] + b0;
-      if (act == ACT_GELU) v = 0.5f * v * (1.0f + erff(v * 0.70710678118654752f));
-      else if (act == ACT_RELU2) v = fmaxf(v, 0.f) * fmaxf(v, 0.f);
-      if (col_scale) v *= c0;
-      float* dst = y + (size_t)gm * ldy + gn;
-      *dst = MODE == OUT_ACCUMULATE_F32 ? *dst + v : v;
-    }
+    for (int j = 0; j < TN; ++j) mine[(i * TN + j) * 32 + lane] = even_and_odd(acc[i][j]);
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < TM * TN / PARTS; ++q) {      // a warp finishes a quarter of the tile's results
+    const int e = warp * (TM * TN / PARTS) + q, gm = m0 + 4 * (e / TN) + ty, gn = n0 + 8 * (e % TN) + tx;
+    const float* p = smem + e * 32 + lane;
+    float v = p[0];
+#pragma unroll
+    for (int part = 1; part < PARTS; ++part) v += p[part * T::WARP_FLOATS];
+    if (gm >= M || gn >= N) continue;
+    if (bias) v += bias[gn];
+    if (act == ACT_GELU) v = 0.5f * v * (1.0f + erff(v * 0.70710678118654752f));
+    else if (act == ACT_RELU2) v = fmaxf(v, 0.f) * fmaxf(v, 0.f);
+    if (col_scale) v *= col_scale[gn];
+    float* dst = y + (size_t)gm * ldy + gn;
+    *dst = MODE == OUT_ACCUMULATE_F32 ? *dst + v : v;
   }
 }
 
@@ -195,17 +222,19 @@ struct F32Call {
   const float* col_scale;
 };
 
-template <int BM, int BN, int TM, int TN, int KB, int STAGES>
+template <int TM, int TN, int KB, int STAGES>
 static int launch_f32_tile(const F32Call& c, int mode, cudaStream_t stream) {
-  using T = F32Tile<BM, BN, TM, TN, KB, STAGES>;
+  using T = F32Tile<TM, TN, KB, STAGES>;
   const bool vec = c.K % 4 == 0 && c.ldx % 4 == 0 && (((uintptr_t)c.x | (uintptr_t)c.w) & 15) == 0;
-  const dim3 grid((c.N + BN - 1) / BN, (c.M + BM - 1) / BM);
+  const int tiles_m = (c.M + T::BM - 1) / T::BM;
+  const long long tiles = (long long)tiles_m * ((c.N + T::BN - 1) / T::BN);
+  if (tiles > 0x7fffffffLL) return GB_ERR_SIZE;
 #define LAUNCH_F32(VEC, MODE)                                                                                          \
   do {                                                                                                                 \
-    auto kernel = gemm_f32_kernel<BM, BN, TM, TN, KB, STAGES, VEC, MODE>;                                              \
+    auto kernel = gemm_f32_kernel<TM, TN, KB, STAGES, VEC, MODE>;                                                      \
     if (T::SMEM > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::SMEM);  \
-    gb_launch(kernel, grid, T::THREADS, T::SMEM, stream, c.x, c.w, c.bias, c.y, c.M, c.N, c.K, c.ldx, c.ldy, c.act,    \
-              c.col_scale);                                                                                            \
+    gb_launch(kernel, dim3((unsigned)tiles), 32 * PARTS, T::SMEM, stream, c.x, c.w, c.bias, c.y, c.M, c.N, c.K, c.ldx, \
+              c.ldy, c.act, c.col_scale, tiles_m);                                                                     \
   } while (0)
   if (mode == OUT_ACCUMULATE_F32) {
     if (vec) LAUNCH_F32(true, OUT_ACCUMULATE_F32);
@@ -221,43 +250,42 @@ static int launch_f32_tile(const F32Call& c, int mode, cudaStream_t stream) {
 // The tiles, small to large, and what four k of a tile cost on an SM in cycles, as measured on a B200 over M of
 // 1 to 2,048 rows and products of 1,024 x 2,048 to 151,936 x 1,024: `alone` when the SM has one CTA (a chain of
 // shared-memory reads and multiply-adds: it bounds products with few tiles), `shared` for every CTA more than the
-// chain hides (the shared-memory reads: a 16-byte read of a warp takes four cycles whether its lanes read one
-// address or 32).  The launcher takes the tile with the least of max(alone, shared x CTAs an SM).
-// One tile of 64 x 64 by 256 threads of 4 x 4, loaded without a pipeline, took (us, that kernel / these):
-// 301 x 6,144 x 1,024: 188 / 131; 301 x 1,024 x 3,072: 403 / 129; 3 x 151,936 x 1,024: 743 / 117;
-// 2,048 x 4,096 x 4,096: 2,435 / 1,757.  The same bits whatever the tile.
+// chain hides (the shared-memory reads; W's stream for the smallest two).  The launcher takes the tile with the least of
+// max(alone, shared x rounds), a round being a CTA on each of 148 SMs.  Tiles of 4 or 8 rows of x with one thread
+// for every result's whole sum took, up to 64 x 64 for prompts (us, those kernels / these): 1 x 4,096 x 4,096: 47.1 / 19.5;
+// 16 x 1,024 x 2,048: 24.0 / 10.6; 301 x 6,144 x 1,024: 160 / 101; 301 x 1,024 x 3,072: 149 / 61;
+// 2,048 x 4,096 x 4,096: 1,810 / 1,496; 3 x 151,936 x 1,024 (W's stream): 110 / 111.  The same bits whatever the tile.
 struct F32Cost {
   int bm, bn;
   float alone, shared;
 };
-static const F32Cost F32_TILES[] = {{4, 32, 100.f, 30.f},    {8, 32, 118.f, 33.f},   {16, 64, 174.f, 100.f},
-                                    {32, 64, 225.f, 140.f},  {64, 64, 405.f, 244.f}, {128, 128, 874.f, 868.f}};
+static const F32Cost F32_TILES[] = {{4, 32, 36.6f, 24.5f}, {8, 32, 38.f, 26.5f},  {16, 32, 52.f, 28.3f},
+                                    {32, 32, 65.f, 53.f},  {40, 32, 85.f, 66.6f}, {32, 64, 120.f, 100.f}};
 
 static int pick_f32_tile(int M, int N) {
-  int best = -1;
+  int best = 0;
   float least = 0.f;
   for (int i = 0; i < (int)(sizeof(F32_TILES) / sizeof(F32_TILES[0])); ++i) {
     const F32Cost& t = F32_TILES[i];
-    const int rows = (M + t.bm - 1) / t.bm;
-    if (rows > 65535) continue;             // what a grid has room for; the largest tile takes the most rows
-    const float cost = fmaxf(t.alone, t.shared * (float)rows * (float)((N + t.bn - 1) / t.bn) / 148.f);
-    if (best < 0 || cost < least) least = cost, best = i;
+    const long long tiles = (long long)((M + t.bm - 1) / t.bm) * ((N + t.bn - 1) / t.bn);
+    const float cost = fmaxf(t.alone, t.shared * (float)((tiles + 147) / 148));
+    if (i == 0 || cost < least) least = cost, best = i;
   }
   return best;
 }
 
 static int launch_f32(int tile, const F32Call& c, int mode, cudaStream_t stream) {
   switch (tile) {
-    case 0: return launch_f32_tile<4, 32, 4, 1, 64, 4>(c, mode, stream);
-    case 1: return launch_f32_tile<8, 32, 4, 1, 64, 4>(c, mode, stream);
-    case 2: return launch_f32_tile<16, 64, 4, 2, 32, 4>(c, mode, stream);
-    case 3: return launch_f32_tile<32, 64, 4, 4, 32, 3>(c, mode, stream);
-    case 4: return launch_f32_tile<64, 64, 4, 8, 16, 4>(c, mode, stream);
-    default: return launch_f32_tile<128, 128, 8, 8, 16, 3>(c, mode, stream);
+    case 0: return launch_f32_tile<1, 4, 32, 3>(c, mode, stream);
+    case 1: return launch_f32_tile<2, 4, 32, 3>(c, mode, stream);
+    case 2: return launch_f32_tile<4, 4, 32, 2>(c, mode, stream);
+    case 3: return launch_f32_tile<8, 4, 32, 2>(c, mode, stream);
+    case 4: return launch_f32_tile<10, 4, 32, 2>(c, mode, stream);
+    default: return launch_f32_tile<8, 8, 32, 2>(c, mode, stream);
   }
 }
 
-// Which of F32_TILES a float32 product of these sizes takes (-1: none).
+// Which of F32_TILES a float32 product of these sizes takes.
 GB_EXPORT int gb_gemm_ref_tile(int M, int N) { return pick_f32_tile(M, N); }
 
 // x: [M, K] rows ldx apart; w: [N, K]; y: [M, N] rows ldy apart.
@@ -277,8 +305,7 @@ GB_EXPORT int gb_gemm_ref(const void* x, const void* w, int in_dtype, const floa
   if (in_dtype == GB_F32) {
     if (out_dtype != GB_F32) return GB_ERR_DTYPE;
     const F32Call call{(const float*)x, (const float*)w, bias, (float*)y, M, N, K, ldx, ldy, act, col_scale};
-    const int tile = pick_f32_tile(M, N);
-    return tile < 0 ? GB_ERR_SIZE : launch_f32(tile, call, mode, stream);
+    return launch_f32(pick_f32_tile(M, N), call, mode, stream);
   } else if (in_dtype == GB_BF16) {
     if (mode == OUT_ACCUMULATE_F32) LAUNCH(bf16, float, OUT_ACCUMULATE_F32);
     else if (out_dtype == GB_F32) LAUNCH(bf16, float, OUT_STORE);
