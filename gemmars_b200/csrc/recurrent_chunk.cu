@@ -640,11 +640,14 @@ static int run(Prepare p, Scan s, int ntok, int heads_at_once, cudaStream_t stre
     // launches of 1,024 groups: 609, 632, 684; sixteen of 3,200 tokens in all, 2,048 groups a launch: 473, 491, 451; twelve of
     // 1,500, 3,072 groups: 232, 242, 203.
     // Few groups leave the chain to itself and want it short (more warps a group); many fill the SMs either way and
-    // want the least that a group costs.
+    // want the least that a group costs.  Without W (the scan alone, us, 1,600 tokens, (4, 1) / (2, 2)): 64 groups of a state
+    // space 86 / 117, 128 groups 100 / 117, four sequences' 512 groups 71 / 74, but sixteen's 2,048 groups 81 / 77.  Heads of
+    // up to 64 (linear attention, (2, 1) / (2, 2) / (4, 1)): 64 groups 73 / 71 / 71, 256 groups 99 / 72 / 102 (256 CTAs of
+    // two warps put two chains on most SMs and one on the rest), four sequences' 1,024 82 / 67 / 85.
     const long long groups = (long long)p.nseq * heads * ((s.V + 15) / 16);
     if constexpr (DP == 64)
-      launch_scan<DP, 2, 1, HAS_W, 4>(s, p.nseq, heads, stream);
-    else if (groups <= 148)
+      launch_scan<DP, 2, HAS_W ? 1 : 2, HAS_W, 4>(s, p.nseq, heads, stream);
+    else if (groups <= (HAS_W ? 1 : 4) * 148)
       launch_scan<DP, 4, 1, HAS_W, 3>(s, p.nseq, heads, stream);
     else if (!HAS_W || groups <= 8 * 148)
       launch_scan<DP, 2, 2, HAS_W, 4>(s, p.nseq, heads, stream);
