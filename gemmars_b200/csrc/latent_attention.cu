@@ -34,13 +34,15 @@ __device__ __forceinline__ void rotate_pair(float u, float v, float2 cs, float& 
 
 // A second copy of the cache rows (latents null: not wanted): latents and rotated key parts, rows ldl and ldr apart, token
 // by token.  With `cu` it is for keys and values that a prompt expands per head: sequence b's rows then start at
-// (cu[b] / 8 + b) * 8 (a multiple of 8, with room for every sequence's last, partly filled eight), and the queries lie
-// head by head as [dim | rd].
+// (cu[b] / 8 + b) * 8 (a multiple of 8, with room for every sequence's last, partly filled eight), the queries lie
+// head by head as [dim | rd], and the `rows` rows that no token fills are written as zeros.
 template <typename T>
 struct Copy {
   T *latents, *rotated;
   long long ldl, ldr;
   const int* cu;
+  long long rows;
+  __device__ __forceinline__ long long row(int b, int t) const { return (long long)(cu[b] / 8 + b) * 8 + (t - cu[b]); }
 };
 
 template <typename T> __device__ __forceinline__ void store4(T* to, float a, float b, float c, float d);
@@ -50,32 +52,91 @@ template <> __device__ __forceinline__ void store4<bf16>(bf16* to, float a, floa
   *(uint2*)to = make_uint2(*(const uint32_t*)&p, *(const uint32_t*)&q);
 }
 
-// One block per token.  Inputs are the float32 results of the layer's projections.  A token's angles are taken once
-// into shared memory, for the key part and all heads.  `wide` (interleaved pairs, everything in fours): a head a warp, four
-// dims a lane (16 heads of 64 rotated dims: 2,048 tokens 22 -> 20.9 us, 16 tokens 8.5 -> 7.3 us).
-template <typename T>
-__global__ void __launch_bounds__(256) latent_prepare_kernel(
+// A warp per token for its cache row, and a thread for every QUADS quads of its queries (or, where those are no quads, dims or
+// pairs): one where few tokens leave the chip idle, two loads in flight a thread for prompts.  Inputs are the float32 results of the layer's projections.  What bounds it is a chain of loads (position,
+// slot, page, the row), so nothing waits for a block: a warp holds a token's row and sums it alone, and a query's angles are
+// taken where they are used.  `wide`: interleaved pairs, everything in fours.  16 heads of 128 + 64 over rows of 512 + 64, with
+// the wait for the kernel before (us; a block a token, its row twice through memory, its angles through shared memory / so):
+// 2,048 tokens 20.9 / 16.6, 16 tokens 10.6 / 8.5; the layer, with the rows' zeros written here and not by two fills,
+// 145.5 / 132.0 and 65.7 / 65.4.
+constexpr int PREPARE_THREADS = 128, PREPARE_QUADS = 2, ROW_HELD = 16;
+template <typename T, int QUADS>
+__global__ void __launch_bounds__(PREPARE_THREADS) latent_prepare_kernel(
     const float* __restrict__ q_in, long long ldq, const float* __restrict__ kv_in, long long ldkv,
     const float* __restrict__ g_in, long long ldg, const float* __restrict__ norm_w, float eps,
     const float* __restrict__ inv_freq, int rot, float q_scale, T* __restrict__ q_nope, long long ldqn,
     T* __restrict__ q_lat, long long ldql, float* __restrict__ gate, T* __restrict__ cache,
     const int* __restrict__ page_table, int table_width, int page_size, const int* __restrict__ tok_pos,
-    const int* __restrict__ tok_seq, const int* __restrict__ seq_slot, int H, int dim, int rd, int rank,
-    Copy<T> ex, int half_layout, float rot_mag, int wide) {
-  extern __shared__ float2 turn[];          // [rot / 2] cosine and sine
-  __shared__ float scratch[34];
+    const int* __restrict__ tok_seq, const int* __restrict__ seq_slot, int ntok, int H, int dim, int rd, int rank,
+    Copy<T> ex, int half_layout, float rot_mag, int wide, int row_blocks, int token_blocks) {
   pdl_release_next();
   pdl_wait_prior();
-  const int t = blockIdx.x, tid = threadIdx.x;
+  const int halves = rd / 2 + (rd & 1);
+  if ((int)blockIdx.x >= row_blocks) {
+    // queries: the unrotated dims go to the absorbing product and the rotated ones straight into qa, or both into the
+    // head's own row
+    const int qd = dim + rd, rot_at = ex.cu ? dim : rank, nope_head = ex.cu ? qd : dim, lat_head = rot_at + rd;
+    const int block = (int)blockIdx.x - row_blocks, t = block / token_blocks;
+    const float* q = q_in + (size_t)t * ldq;
+    const float fpos = (float)tok_pos[t];
+    const int first = (block - t * token_blocks) * (QUADS * PREPARE_THREADS) + threadIdx.x;
+    if (wide) {       // four neighbouring dims at a time
+      const int quads = qd / 4, total = H * quads;
+      float4 v[QUADS];
+      int h[QUADS], d[QUADS];
+#pragma unroll
+      for (int u = 0; u < QUADS; ++u) {
+        const int e = first + u * PREPARE_THREADS;
+        h[u] = e < total ? e / quads : -1;
+        d[u] = (e - h[u] * quads) * 4;
+        if (h[u] >= 0) v[u] = *(const float4*)(q + h[u] * qd + d[u]);
+      }
+#pragma unroll
+      for (int u = 0; u < QUADS; ++u) {
+        if (h[u] < 0) continue;
+        float o[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
+        const bool turned = d[u] >= dim;
+        if (turned) {
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const int i = (d[u] - dim) / 2 + e;
+            if (2 * i < rot) rotate_pair(o[2 * e], o[2 * e + 1], cos_sin(fpos * inv_freq[i], rot_mag), o[2 * e], o[2 * e + 1]);
+          }
+        }
+        T* dst = turned ? q_lat + (size_t)t * ldql + (size_t)h[u] * lat_head + rot_at + d[u] - dim
+                        : q_nope + (size_t)t * ldqn + (size_t)h[u] * nope_head + d[u];
+        store4(dst, o[0] * q_scale, o[1] * q_scale, o[2] * q_scale, o[3] * q_scale);
+      }
+      return;
+    }
+    const int units = dim + halves;
+    for (int u = 0; u < QUADS; ++u) {
+      const int e = first + u * PREPARE_THREADS;
+      if (e >= H * units) return;
+      const int h = e / units, unit = e - h * units;
+      const float* src = q + h * qd;
+      if (unit < dim) {
+        q_nope[(size_t)t * ldqn + (size_t)h * nope_head + unit] = from_f32<T>(src[unit] * q_scale);
+        continue;
+      }
+      const int i = unit - dim;
+      const bool turns = 2 * i < rot;
+      const int a = turns && half_layout ? i : 2 * i, b = turns && half_layout ? i + rot / 2 : 2 * i + 1;
+      T* dst = q_lat + (size_t)t * ldql + (size_t)h * lat_head + rot_at;
+      float x = src[dim + a], y = b < rd ? src[dim + b] : 0.f;
+      if (turns) rotate_pair(x, y, cos_sin(fpos * inv_freq[i], rot_mag), x, y);
+      dst[a] = from_f32<T>(x * q_scale);
+      if (b < rd) dst[b] = from_f32<T>(y * q_scale);
+    }
+    return;
+  }
+  const int t = (int)blockIdx.x * (PREPARE_THREADS / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (t >= ntok) return;
   const int pos = tok_pos[t];
-  const float fpos = (float)pos;
   const float* kv = kv_in + (size_t)t * ldkv;
-  for (int i = tid; i < rot / 2; i += blockDim.x) turn[i] = cos_sin(fpos * inv_freq[i], rot_mag);
-  // the latent: x / sqrt(mean(x^2) + eps) * w
-  float ss = 0.f;
-  for (int i = tid; i < rank; i += blockDim.x) ss = fmaf(kv[i], kv[i], ss);
-  ss = block_sum(ss, scratch);              // also: the angles are there
-  const float rstd = 1.0f / sqrtf(ss / (float)rank + eps);
+  float x[ROW_HELD];                        // the row's first 512 numbers stay in registers
+#pragma unroll
+  for (int u = 0; u < ROW_HELD; ++u) x[u] = lane + 32 * u < rank ? kv[lane + 32 * u] : 0.f;
   // the row goes into the paged cache and, when asked for, into the rows to be expanded as well
   T *lat0 = nullptr, *lat1 = nullptr, *key0 = nullptr, *key1 = nullptr;
   if (cache != nullptr) {
@@ -85,26 +146,24 @@ __global__ void __launch_bounds__(256) latent_prepare_kernel(
     key0 = lat0 + rank;
   }
   if (ex.latents != nullptr) {
-    size_t row = t;
-    if (ex.cu) {
-      const int b = tok_seq[t];
-      row = (size_t)(ex.cu[b] / 8 + b) * 8 + (t - ex.cu[b]);
-    }
+    const long long row = ex.cu ? ex.row(tok_seq[t], t) : t;
     lat1 = ex.latents + row * ex.ldl;
     key1 = ex.rotated + row * ex.ldr;
-  }
-  for (int i = tid; i < rank; i += blockDim.x) {
-    const T v = from_f32<T>(kv[i] * rstd * norm_w[i]);
-    if (lat0) lat0[i] = v;
-    if (lat1) lat1[i] = v;
+    if (ex.cu) {                            // rows from this token's to the next one's, and before the first
+      const long long next = t + 1 < ntok ? ex.row(tok_seq[t + 1], t + 1) : ex.rows;
+      for (long long r = t > 0 ? row + 1 : 0; r < next; ++r) {
+        if (r == row) continue;
+        for (int i = lane; i < rank; i += 32) ex.latents[r * ex.ldl + i] = from_f32<T>(0.f);
+        for (int i = lane; i < rd; i += 32) ex.rotated[r * ex.ldr + i] = from_f32<T>(0.f);
+      }
+    }
   }
   // the shared rotated key part: pairs below `rot` turn, the rest passes
-  const int halves = rd / 2 + (rd & 1);
-  for (int i = tid; i < halves; i += blockDim.x) {
+  for (int i = lane; i < halves; i += 32) {
     const bool turns = 2 * i < rot;
     const int a = turns && half_layout ? i : 2 * i, b = turns && half_layout ? i + rot / 2 : 2 * i + 1;
     float u = kv[rank + a], v = b < rd ? kv[rank + b] : 0.f;
-    if (turns) rotate_pair(u, v, turn[i], u, v);
+    if (turns) rotate_pair(u, v, cos_sin((float)pos * inv_freq[i], rot_mag), u, v);
     for (int copy = 0; copy < 2; ++copy) {
       T* key = copy ? key1 : key0;
       if (!key) continue;
@@ -112,75 +171,64 @@ __global__ void __launch_bounds__(256) latent_prepare_kernel(
       if (b < rd) key[b] = from_f32<T>(v);
     }
   }
-  // queries: the unrotated dims go to the absorbing product and the rotated ones straight into qa, or both into the
-  // head's own row
-  const float* q = q_in + (size_t)t * ldq;
-  const int qd = dim + rd, rot_at = ex.cu ? dim : rank, nope_head = ex.cu ? qd : dim, lat_head = rot_at + rd;
-  if (wide) {       // four neighbouring dims a lane, a head a warp
-    for (int h = tid >> 5; h < H; h += 8)
-      for (int d = (tid & 31) * 4; d < qd; d += 128) {
-        const float4 v = *(const float4*)(q + h * qd + d);
-        float o[4] = {v.x, v.y, v.z, v.w};
-        const bool turned = d >= dim;
-        if (turned) {
+  // the latent: x / sqrt(mean(x^2) + eps) * w
+  float ss = 0.f;
 #pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            const int i = (d - dim) / 2 + e;
-            if (2 * i < rot) rotate_pair(o[2 * e], o[2 * e + 1], turn[i], o[2 * e], o[2 * e + 1]);
-          }
-        }
-        T* dst = turned ? q_lat + (size_t)t * ldql + (size_t)h * lat_head + rot_at + d - dim : q_nope + (size_t)t * ldqn + (size_t)h * nope_head + d;
-        store4(dst, o[0] * q_scale, o[1] * q_scale, o[2] * q_scale, o[3] * q_scale);
-      }
-    if (g_in != nullptr)
-      for (int h = tid; h < H; h += blockDim.x) gate[(size_t)t * H + h] = 1.0f / (1.0f + expf(-g_in[(size_t)t * ldg + h]));
-    return;
-  }
-  for (int e = tid; e < H * dim; e += blockDim.x) {
-    const int h = e / dim, d = e % dim;
-    q_nope[(size_t)t * ldqn + (size_t)h * nope_head + d] = from_f32<T>(q[h * qd + d] * q_scale);
-  }
-  for (int e = tid; e < H * halves; e += blockDim.x) {
-    const int h = e / halves, i = e % halves;
-    const bool turns = 2 * i < rot;
-    const int a = turns && half_layout ? i : 2 * i, b = turns && half_layout ? i + rot / 2 : 2 * i + 1;
-    const float* src = q + h * qd + dim;
-    T* dst = q_lat + (size_t)t * ldql + (size_t)h * lat_head + rot_at;
-    float u = src[a], v = b < rd ? src[b] : 0.f;
-    if (turns) rotate_pair(u, v, turn[i], u, v);
-    dst[a] = from_f32<T>(u * q_scale);
-    if (b < rd) dst[b] = from_f32<T>(v * q_scale);
-  }
+  for (int u = 0; u < ROW_HELD; ++u) ss = fmaf(x[u], x[u], ss);
+  for (int i = lane + 32 * ROW_HELD; i < rank; i += 32) ss = fmaf(kv[i], kv[i], ss);
+  ss = warp_sum(ss);
+  const float rstd = 1.0f / sqrtf(ss / (float)rank + eps);
+  auto put = [&](int i, float v) {
+    const T o = from_f32<T>(v * rstd * norm_w[i]);
+    if (lat0) lat0[i] = o;
+    if (lat1) lat1[i] = o;
+  };
+#pragma unroll
+  for (int u = 0; u < ROW_HELD; ++u)
+    if (lane + 32 * u < rank) put(lane + 32 * u, x[u]);
+  for (int i = lane + 32 * ROW_HELD; i < rank; i += 32) put(i, kv[i]);
   if (g_in != nullptr)
-    for (int h = tid; h < H; h += blockDim.x) gate[(size_t)t * H + h] = 1.0f / (1.0f + expf(-g_in[(size_t)t * ldg + h]));
+    for (int h = lane; h < H; h += 32) gate[(size_t)t * H + h] = 1.0f / (1.0f + expf(-g_in[(size_t)t * ldg + h]));
 }
 
-// latents, rotated, cu: see Copy; with cu, q_nope and q_lat are one buffer of rows [H, dim + rd].
+// latents, rotated, cu, rows: see Copy; with cu, q_nope and q_lat are one buffer of rows [H, dim + rd].
 GB_EXPORT int gb_latent_prepare(const float* q_in, long long ldq, const float* kv_in, long long ldkv, const float* g_in,
                                 long long ldg, const float* norm_w, float eps, const float* inv_freq, int rot,
                                 float q_scale, void* q_nope, long long ldqn, void* q_lat, long long ldql, float* gate,
                                 void* cache, int dtype, const int* page_table, int table_width, int page_size,
                                 const int* tok_pos, const int* tok_seq, const int* seq_slot, int ntok, int H, int dim,
-                                int rd, int rank, void* latents, long long ldl, void* rotated, long long ldr, const int* cu,
+                                int rd, int rank, void* latents, long long ldl, void* rotated, long long ldr, const int* cu, long long rows,
                                 int half_layout, float rot_mag, cudaStream_t stream) {
   if (ntok <= 0) return 0;
   if (H <= 0 || dim < 0 || rd < 0 || rank <= 0 || rot < 0 || rot > rd || (rot & 1) || rot > 8192) return GB_ERR_SIZE;
   if (rot > 0 && inv_freq == nullptr) return GB_ERR_ARG;
-  if (cu != nullptr && latents == nullptr) return GB_ERR_ARG;
+  if (cu != nullptr && (latents == nullptr || rows < ntok)) return GB_ERR_ARG;
   const int qd = dim + rd, head_end = (cu ? dim : rank) + rd;
   const int elem = dtype == GB_F32 ? 16 : 8;          // bytes of four results
   const int wide = (rot == 0 || !half_layout) && dim % 4 == 0 && rd % 4 == 0 && rank % 4 == 0 && ldq % 4 == 0 && ldqn % 4 == 0 &&
                    ldql % 4 == 0 && head_end % 4 == 0 && ((uintptr_t)q_in & 15) == 0 &&
                    ((uintptr_t)q_nope % elem) == 0 && ((uintptr_t)q_lat % elem) == 0 && qd > 0;
-#define LAUNCH(T)                                                                                                     \
-  gb_launch(latent_prepare_kernel<T>, dim3(ntok), dim3(256), (size_t)(rot / 2) * sizeof(float2), stream, q_in, ldq, kv_in, ldkv, \
+  const int units = H * (wide ? qd / 4 : dim + rd / 2 + (rd & 1));          // of a token
+  const int row_blocks = (ntok + PREPARE_THREADS / 32 - 1) / (PREPARE_THREADS / 32);
+  const int quads = (long long)ntok * units > 2048LL * 148 ? PREPARE_QUADS : 1;      // more than a chip of threads
+  const int token_blocks = (units + PREPARE_THREADS * quads - 1) / (PREPARE_THREADS * quads);
+  const long long blocks = row_blocks + (long long)ntok * token_blocks;
+  if (blocks > 0x7fffffffLL) return GB_ERR_SIZE;
+#define LAUNCH_QUADS(T, QUADS)                                                                                        \
+  gb_launch(latent_prepare_kernel<T, QUADS>, dim3((unsigned)blocks), dim3(PREPARE_THREADS), 0, stream, q_in, ldq, kv_in, ldkv, \
             g_in, ldg, norm_w, eps, inv_freq, rot, q_scale, (T*)q_nope, ldqn, (T*)q_lat, ldql, gate, (T*)cache, page_table, \
-            table_width, page_size, tok_pos, tok_seq, seq_slot, H, dim, rd, rank, Copy<T>{(T*)latents, (T*)rotated, ldl, ldr, cu}, \
-            half_layout, rot_mag, wide)
+            table_width, page_size, tok_pos, tok_seq, seq_slot, ntok, H, dim, rd, rank, Copy<T>{(T*)latents, (T*)rotated, ldl, ldr, cu, rows}, \
+            half_layout, rot_mag, wide, row_blocks, token_blocks)
+#define LAUNCH(T)                        \
+  do {                                              \
+    if (quads > 1) LAUNCH_QUADS(T, PREPARE_QUADS);  \
+    else LAUNCH_QUADS(T, 1);                        \
+  } while (0)
   if (dtype == GB_F32) LAUNCH(float);
   else if (dtype == GB_BF16) LAUNCH(bf16);
   else return GB_ERR_DTYPE;
 #undef LAUNCH
+#undef LAUNCH_QUADS
   return gb_launch_status();
 }
 

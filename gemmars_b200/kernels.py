@@ -900,8 +900,8 @@ def latent_prepare(q_in, kv_in, g_in, norm_w, eps, inv_freq, rot, q_scale, q_nop
     [T, heads * (rank + rd)]; ``gate`` [T, heads] = sigmoid(g_in) (float32; None: no gate).  ``dense``
     [T, rank + rd] (None: not wanted) receives the same rows as the cache, token by token.  ``expand``
     (latents [R, rank], key parts [R, rd], cu_seqlens), R = latent_expand_rows(T, sequences), instead of
-    ``dense``: the rows of sequence b from (cu_seqlens[b] // 8 + b) * 8 on, and the queries head by head as
-    [dim | rd]: ``q_nope`` and ``q_lat`` are then one [T, heads * (dim + rd)]."""
+    ``dense``: the rows of sequence b from (cu_seqlens[b] // 8 + b) * 8 on, zeros in those that no token fills, and the
+    queries head by head as [dim | rd]: ``q_nope`` and ``q_lat`` are then one [T, heads * (dim + rd)]."""
     _cuda(q_in, kv_in, g_in, norm_w, inv_freq, q_nope, q_lat, gate, cache, page_table, tok_pos, tok_seq, seq_slot)
     t = q_in.shape[0]
     assert q_in.dtype == torch.float32 and kv_in.dtype == torch.float32 and q_in.stride(1) == 1 and kv_in.stride(1) == 1
@@ -912,13 +912,13 @@ def latent_prepare(q_in, kv_in, g_in, norm_w, eps, inv_freq, rot, q_scale, q_nop
         rows = latent_expand_rows(t, cu.numel() - 1)
         assert lat.shape == (rows, rank) and keys.shape == (rows, rd) and lat.is_contiguous() and keys.is_contiguous()
         assert lat.dtype == keys.dtype == q_lat.dtype
-        copy = (lat.data_ptr(), rank, keys.data_ptr(), rd, cu.data_ptr())
+        copy = (lat.data_ptr(), rank, keys.data_ptr(), rd, cu.data_ptr(), rows)
     else:
         assert q_nope.shape == (t, heads * dim) and q_lat.shape == (t, heads * (rank + rd))
-        copy = (None, 0, None, 0, None)
+        copy = (None, 0, None, 0, None, 0)
         if dense is not None:
             assert dense.dtype == q_lat.dtype and dense.shape == (t, rank + rd) and dense.stride(1) == 1
-            copy = (dense.data_ptr(), dense.stride(0), dense[:, rank:].data_ptr(), dense.stride(0), None)
+            copy = (dense.data_ptr(), dense.stride(0), dense[:, rank:].data_ptr(), dense.stride(0), None, 0)
     assert q_nope.dtype == q_lat.dtype
     assert q_nope.stride(1) == 1 and q_lat.stride(1) == 1 and norm_w.dtype == torch.float32
     if g_in is not None:
@@ -931,8 +931,8 @@ def latent_prepare(q_in, kv_in, g_in, norm_w, eps, inv_freq, rot, q_scale, q_nop
     f = _fn("latent_attention", "gb_latent_prepare",
             [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_float, c_void_p, c_int, c_float,
              c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p,
-             c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_int,
-             c_float, c_void_p])
+             c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong,
+             c_int, c_float, c_void_p])
     _check(f(q_in.data_ptr(), q_in.stride(0), kv_in.data_ptr(), kv_in.stride(0), _ptr(g_in),
              g_in.stride(0) if g_in is not None else 0, norm_w.data_ptr(), eps, _ptr(inv_freq), rot, q_scale,
              q_nope.data_ptr(), q_nope.stride(0), q_lat.data_ptr(), q_lat.stride(0), _ptr(gate), _ptr(cache),

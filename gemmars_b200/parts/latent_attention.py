@@ -164,10 +164,9 @@ class LatentAttention(Part):
         dense = torch.empty((t, r + rd), dtype=self.act_dtype, device=h.device) if expand else None
         rows = None
         if on_tc:
-            # rows between two sequences, which no token fills, have to be finite
             n = kernels.latent_expand_rows(t, ctx.n_seqs)
-            rows = (torch.zeros((n, r), dtype=self.act_dtype, device=h.device),
-                    torch.zeros((n, rd), dtype=self.act_dtype, device=h.device), ctx.cu_seqlens)
+            rows = (torch.empty((n, r), dtype=self.act_dtype, device=h.device),
+                    torch.empty((n, rd), dtype=self.act_dtype, device=h.device), ctx.cu_seqlens)
             q_nope = qa = torch.empty((t, nh * (dim + rd)), dtype=self.act_dtype, device=h.device)
         else:
             q_nope = torch.empty((t, nh * dim), dtype=self.act_dtype, device=h.device)
