@@ -306,27 +306,47 @@ attention_capped_single_kernel(const bf16* __restrict__ q, long long q_stride, b
   const int win_blk = lo_first / KEYS, kept_blks = min((keep_first + KEYS - 1) / KEYS, win_blk);
   const int n_blks = kept_blks + last / KEYS - win_blk + 1;
   const int rank = (int)spread_rank(), spread = (int)spread_size();
-  for (int it = warp + rank * SPLIT; it < n_blks; it += SPLIT * spread) {
-    const int key0 = (it < kept_blks ? it : win_blk + it - kept_blks) * KEYS;
-    const int page = kv.page_table[(size_t)slot * kv.table_width + (key0 / kv.page_size) % kv.table_width];
+  // A warp's block is a chain of loads: its page, then its keys, then its values.  The page of the next block is asked for
+  // while this one is worked on, and the values together with the keys where the registers hold both: 8 sequences,
+  // 32 heads of 128 over 8, a window of 2,048 keys 21.7 -> 19.3 us.
+  constexpr bool AHEAD = HD <= 128 && VD <= 128;
+  auto key_of = [&](int it) { return (it < kept_blks ? it : win_blk + it - kept_blks) * KEYS; };
+  auto page_of = [&](int it) { return kv.page_table[(size_t)slot * kv.table_width + (key_of(it) / kv.page_size) % kv.table_width]; };
+  int it = warp + rank * SPLIT;
+  int page = it < n_blks ? page_of(it) : 0;
+  for (; it < n_blks; it += SPLIT * spread) {
+    const int key0 = key_of(it);
     const size_t page_base = ((size_t)page * kv.num_kv_heads + kvh) * kv.page_size * HD;
     const size_t value_base = ((size_t)page * kv.num_kv_heads + kvh) * kv.page_size * VD;
     const int in_page = key0 % kv.page_size;
+    const bf16* vbase = vcache + value_base + in_page + 8 * c;
+    uint4 kr[4][KB > 0 ? KB : 1], vr[AHEAD ? VD / 8 : 1];
+    uint2 kt[4];
+    auto bring_keys = [&](int j) {
+      const bf16* krow = kcache + page_base + (size_t)(in_page + 8 * (g >> 1) + 2 * j + (g & 1)) * HD;
+#pragma unroll
+      for (int kb = 0; kb < KB; ++kb) kr[j][kb] = *(const uint4*)(krow + kb * 32 + c * 8);
+      if (TAIL) kt[j] = *(const uint2*)(krow + KB * 32 + c * 4);
+    };
+    if (AHEAD) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) bring_keys(j);
+#pragma unroll
+      for (int d = 0; d < VD / 8; ++d) vr[AHEAD ? d : 0] = *(const uint4*)(vbase + (size_t)(d * 8 + g) * kv.page_size);
+    }
+    if (it + SPLIT * spread < n_blks) page = page_of(it + SPLIT * spread);
     float s[4][4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
+      if (!AHEAD) bring_keys(j);
       s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.f;
-      const bf16* krow = kcache + page_base + (size_t)(in_page + 8 * (g >> 1) + 2 * j + (g & 1)) * HD;
 #pragma unroll
       for (int kb = 0; kb < KB; ++kb) {
-        const uint4 k4 = *(const uint4*)(krow + kb * 32 + c * 8);
+        const uint4 k4 = kr[j][kb];
         mma16816(s[j], qa[kb][0], qb[kb][0], qa[kb][1], qb[kb][1], k4.x, k4.y);
         mma16816(s[j], qa[kb][2], qb[kb][2], qa[kb][3], qb[kb][3], k4.z, k4.w);
       }
-      if (TAIL) {
-        const uint2 k2 = *(const uint2*)(krow + KB * 32 + c * 4);
-        mma16816(s[j], qa[KB][0], qb[KB][0], qa[KB][1], qb[KB][1], k2.x, k2.y);
-      }
+      if (TAIL) mma16816(s[j], qa[KB][0], qb[KB][0], qa[KB][1], qb[KB][1], kt[j].x, kt[j].y);
     }
     float mx0 = -INFINITY, mx1 = -INFINITY;
 #pragma unroll
@@ -360,10 +380,9 @@ attention_capped_single_kernel(const bf16* __restrict__ q, long long q_stride, b
     }
     l0 = l0 * alpha0 + sum0;
     l1 = l1 * alpha1 + sum1;
-    const bf16* vbase = vcache + value_base + in_page + 8 * c;
 #pragma unroll
     for (int d = 0; d < VD / 8; ++d) {
-      const uint4 v4 = *(const uint4*)(vbase + (size_t)(d * 8 + g) * kv.page_size);
+      const uint4 v4 = AHEAD ? vr[AHEAD ? d : 0] : *(const uint4*)(vbase + (size_t)(d * 8 + g) * kv.page_size);
       o[d][0] *= alpha0; o[d][1] *= alpha0; o[d][2] *= alpha1; o[d][3] *= alpha1;
       mma16816(o[d], p[0][0], p[0][1], p[1][0], p[1][1], v4.x, v4.y);
       mma16816(o[d], p[2][0], p[2][1], p[3][0], p[3][1], v4.z, v4.w);
