@@ -1566,3 +1566,174 @@ GB_EXPORT int gb_matrix_memory(const float* q, const float* k, const float* v, c
 #undef GB_MEMORY
   return gb_launch_status();
 }
+
+// ------------------------------------------------------------------ a delta-rule layer's single tokens
+// A step in which every sequence brings one token: the filter, the delta rule and the gated norm that follows in one kernel
+// (short_filter_single_kernel, delta_rule_kernel and gated_group_norm_wide_kernel, in their orders of summing: the same bits).
+// A block is 32 columns of one (sequence, head), as there; the blocks of the heads that share a q/k head are a cluster, which
+// reads the filter's memory of q and k, meets, and one block writes it; a head's blocks send each other their parts of the
+// sum of squares.  What bounds a step is its kernels' boundaries: one
+// sequence, 16 heads of 128 x 128 over 8, a layer's step 24.4 us with the three kernels, 21.9 so.
+__device__ __forceinline__ void cluster_arrive_all() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait_all() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
+template <int P, typename O>
+__global__ void __launch_bounds__(32 * P) delta_step_kernel(const float* __restrict__ proj, long long ldp, const float* __restrict__ taps,
+                                                           float* __restrict__ filter_state, const float* __restrict__ A_log,
+                                                           const float* __restrict__ dt_bias, float* __restrict__ state,
+                                                           const int* __restrict__ seq_slot, const float* __restrict__ norm_w, int wn,
+                                                           O* __restrict__ out, int H, int G, int D, int V, int K, float qscale,
+                                                           float eps, float out_scale) {
+  constexpr int DP = P * SLICE;
+  __shared__ __align__(16) float kq[2][padded_size(P)];
+  __shared__ __align__(16) float vs[32], ys[32], squares[32], pre[5];
+  cluster_arrive_all();
+  pdl_release_next();
+  const int b = blockIdx.x, head = blockIdx.y, rep = H / G, g = head / rep, tid = threadIdx.x, lane = tid & 31;
+  const int part = tid % P, z = blockIdx.z, col = z * 32 + tid / P, Z = gridDim.z;
+  const int C = 2 * G * D + H * V, cq = g * D + tid, ck = G * D + g * D + tid, cv = 2 * G * D + head * V + z * 32 + tid;
+  // the weights do not depend on the kernel before this one
+  float wq[MAX_TAPS], wk[MAX_TAPS], wv[MAX_TAPS];
+#pragma unroll
+  for (int j = 0; j < MAX_TAPS; ++j) {
+    wq[j] = tid < D && j < K ? taps[(size_t)cq * K + j] : 0.f;
+    wk[j] = tid < D && j < K ? taps[(size_t)ck * K + j] : 0.f;
+    wv[j] = tid < 32 && j < K ? taps[(size_t)cv * K + j] : 0.f;
+  }
+  const float rate = expf(A_log[head]), dtb = dt_bias[head];
+  pdl_wait_prior();
+  const int slot = seq_slot[b];
+  float4* Sg = (float4*)(state + ((size_t)slot * H + head) * 8 * V * P * 4);
+  float S[SLICE];
+#pragma unroll
+  for (int r = 0; r < SLICE / 4; ++r) {
+    const float4 s4 = Sg[((size_t)r * V + col) * P + part];
+    S[4 * r] = s4.x; S[4 * r + 1] = s4.y; S[4 * r + 2] = s4.z; S[4 * r + 3] = s4.w;
+  }
+  const float* row = proj + (size_t)b * ldp;
+  float* hist = filter_state + (size_t)slot * (K - 1) * C;
+  const float beta_logit = row[C + H * V + head], a_logit = row[C + H * V + H + head];
+  const float gate = tid < 32 ? row[C + head * V + z * 32 + tid] : 0.f;
+  float held_q[MAX_TAPS], held_k[MAX_TAPS], held_v[MAX_TAPS];       // the memory, then the token: [K]
+  auto window = [&](int c, bool on, float (&held)[MAX_TAPS]) {
+#pragma unroll
+    for (int j = 0; j < MAX_TAPS; ++j) held[j] = on && j < K - 1 ? hist[(size_t)j * C + c] : on && j == K - 1 ? row[c] : 0.f;
+  };
+  window(cq, tid < D, held_q);
+  window(ck, tid < D, held_k);
+  window(cv, tid < 32, held_v);
+  auto filtered = [&](const float (&w)[MAX_TAPS], const float (&held)[MAX_TAPS]) {
+    float acc = 0.f;
+#pragma unroll
+    for (int j = 0; j < MAX_TAPS; ++j)
+      if (j < K) acc = fmaf(w[j], held[j], acc);
+    return silu_f(acc);
+  };
+  kq[0][padded(tid)] = tid < D ? filtered(wk, held_k) : 0.f;
+  kq[1][padded(tid)] = tid < D ? filtered(wq, held_q) : 0.f;
+  if (tid < 32) vs[tid] = filtered(wv, held_v);
+  __syncthreads();
+  if (tid < 32) {
+    float kk = 0.f, qq = 0.f, kdq = 0.f;
+    for (int i = lane; i < DP; i += 32) {
+      const float kv = kq[0][padded(i)], qv = kq[1][padded(i)];
+      kk = fmaf(kv, kv, kk); qq = fmaf(qv, qv, qq); kdq = fmaf(kv, qv, kdq);
+    }
+    kk = warp_sum(kk); qq = warp_sum(qq); kdq = warp_sum(kdq);
+    if (lane == 0) {
+      const float inv_k = 1.0f / sqrtf(kk + 1e-6f), inv_q = qscale / sqrtf(qq + 1e-6f);
+      const float decay = expf(-rate * softplus_f(a_logit + dtb));
+      pre[0] = decay; pre[1] = inv_k; pre[2] = sigmoid_f(beta_logit); pre[3] = kdq * inv_k * inv_q; pre[4] = decay * inv_q;
+    }
+  }
+  __syncthreads();
+  const float4 *ks = (const float4*)(kq[0] + part * (SLICE + 4)), *qs = (const float4*)(kq[1] + part * (SLICE + 4));
+  float4 kheld[SLICE / 4];
+  float sk = 0.f, sk2 = 0.f, sq = 0.f, sq2 = 0.f;
+#pragma unroll
+  for (int r = 0; r < SLICE / 4; ++r) {
+    const float4 kv = kheld[r] = ks[r], qv = qs[r];
+    sk = fmaf(S[4 * r], kv.x, sk); sk2 = fmaf(S[4 * r + 1], kv.y, sk2); sk = fmaf(S[4 * r + 2], kv.z, sk); sk2 = fmaf(S[4 * r + 3], kv.w, sk2);
+    sq = fmaf(S[4 * r], qv.x, sq); sq2 = fmaf(S[4 * r + 1], qv.y, sq2); sq = fmaf(S[4 * r + 2], qv.z, sq); sq2 = fmaf(S[4 * r + 3], qv.w, sq2);
+  }
+  sk = lanes_sum<P>(sk + sk2);
+  sq = lanes_sum<P>(sq + sq2);
+  const float decay = pre[0], inv_k = pre[1], u = pre[2] * (vs[tid / P] - decay * inv_k * sk), ku = inv_k * u;
+  if (part == 0) ys[tid / P] = fmaf(pre[3], u, pre[4] * sq);
+#pragma unroll
+  for (int r = 0; r < SLICE / 4; ++r) {
+    const float4 kv = kheld[r];
+    Sg[((size_t)r * V + col) * P + part] = make_float4(fmaf(kv.x, ku, decay * S[4 * r]), fmaf(kv.y, ku, decay * S[4 * r + 1]),
+                                                       fmaf(kv.z, ku, decay * S[4 * r + 2]), fmaf(kv.w, ku, decay * S[4 * r + 3]));
+  }
+  __syncthreads();
+  cluster_wait_all();                        // every block of the cluster has started
+  if (tid < 8) {                             // four columns' squares to every block of the head
+    const float4 v = *(const float4*)(ys + 4 * tid);
+    const float ss = fmaf(v.w, v.w, fmaf(v.z, v.z, fmaf(v.y, v.y, v.x * v.x)));
+    for (int to = 0; to < Z; ++to) {
+      uint32_t addr;
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
+                   : "=r"(addr) : "r"((uint32_t)__cvta_generic_to_shared(squares + z * 8 + tid)), "r"(head % rep + rep * to));
+      asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(ss) : "memory");
+    }
+  }
+  __syncwarp();
+  cluster_arrive_all();
+  cluster_wait_all();                        // the squares are there, and every block has read the filter's memory
+  auto keep = [&](int c, const float (&held)[MAX_TAPS]) {
+#pragma unroll
+    for (int j = 0; j < MAX_TAPS - 1; ++j)
+      if (j < K - 1) hist[(size_t)j * C + c] = held[j + 1];
+  };
+  if (head % rep == 0 && z == 0 && tid < D) {
+    keep(cq, held_q);
+    keep(ck, held_k);
+  }
+  if (tid < 32) {
+    keep(cv, held_v);
+    const int lanes = V / 4;                 // 16 or 32
+    float ss = lane < lanes ? squares[lane] : 0.f;
+    for (int o = lanes / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    ss = __shfl_sync(0xffffffffu, ss, 0);
+    const float inv = 1.0f / sqrtf(ss / (float)V + eps);
+    const int c = head * V + z * 32 + tid;
+    out[(size_t)b * H * V + c] = from_f32<O>(ys[tid] * inv * norm_w[c % wn] * silu_f(gate) * out_scale);
+  }
+}
+
+// proj: rows of [q (G D) | k (G D) | v (H V) | gate (H V) | b (H) | a (H)] float32; filter_state [slots, K - 1, 2 G D + H V];
+// state as gb_delta_rule; out [nseq, H V] in out_dtype.  D up to 128, V 64 or 128, H / G blocks of V / 32 at most 8.
+GB_EXPORT int gb_delta_step(const float* proj, long long ldp, const float* taps, float* filter_state, const float* A_log,
+                            const float* dt_bias, float* state, const int* seq_slot, const float* norm_w, int wn, void* out,
+                            int out_dtype, int nseq, int H, int G, int D, int V, int K, float qscale, float eps, float out_scale,
+                            cudaStream_t stream) {
+  if (nseq <= 0) return 0;
+  if (G <= 0 || H <= 0 || H % G || D <= 0 || D > 4 * SLICE || (V != 64 && V != 128) || H / G * (V / 32) > 8 || K < 2 || K > MAX_TAPS ||
+      wn <= 0 || ((uintptr_t)state & 15))
+    return GB_ERR_SIZE;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(nseq, H, V / 32);
+  cfg.blockDim = dim3(32 * lanes_for(D));
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 1;
+  attr[0].val.clusterDim.y = H / G;
+  attr[0].val.clusterDim.z = V / 32;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = GB_PDL_EARLY_START ? 2 : 1;
+#define GB_STEP(P, O)                                                                                                          \
+  (int)cudaLaunchKernelEx(&cfg, delta_step_kernel<P, O>, proj, ldp, taps, filter_state, A_log, dt_bias, state, seq_slot, norm_w, wn, \
+                          (O*)out, H, G, D, V, K, qscale, eps, out_scale)
+  if (out_dtype != GB_F32 && out_dtype != GB_BF16) return GB_ERR_DTYPE;
+  const bool f32 = out_dtype == GB_F32;
+  switch (lanes_for(D)) {
+    case 1: return f32 ? GB_STEP(1, float) : GB_STEP(1, bf16);
+    case 2: return f32 ? GB_STEP(2, float) : GB_STEP(2, bf16);
+    default: return f32 ? GB_STEP(4, float) : GB_STEP(4, bf16);
+  }
+#undef GB_STEP
+}

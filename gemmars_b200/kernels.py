@@ -1921,6 +1921,33 @@ def delta_rule(q, k, v, beta_logit, a_logit, a_log, dt_bias, state, cu_seqlens, 
            "delta_rule", "attention", _nbytes(y) * 2 + 2 * seq_slot.numel() * heads * dim * vdim * 4)
 
 
+def delta_step_usable(ntok: int, nseq: int, heads: int, groups: int, dim: int, vdim: int, taps: int) -> bool:
+    """Whether a gated delta layer's step runs as ``delta_step``: one token a sequence, and a q/k head's value heads in
+    blocks of 32 columns that fill at most a cluster of eight."""
+    return ntok == nseq and dim <= 128 and vdim in (64, 128) and heads // groups * (vdim // 32) <= 8 and 2 <= taps <= 8
+
+
+def delta_step(proj, taps, filter_state, a_log, dt_bias, state, seq_slot, norm_w, out, heads, groups, dim, vdim, q_scale, eps, out_scale):
+    """short_filter, delta_rule and gated_group_norm of a step in which every sequence brings one token, in one kernel with
+    the same bits: ``proj`` [T, q | k | v | gate | b | a] float32, the rest as there (see delta_step_usable)."""
+    _cuda(proj, taps, filter_state, a_log, dt_bias, state, seq_slot, norm_w, out)
+    c, k = taps.shape
+    t, hv = proj.shape[0], heads * vdim
+    assert delta_step_usable(t, seq_slot.numel(), heads, groups, dim, vdim, k) and c == 2 * groups * dim + hv
+    assert proj.dtype == torch.float32 and proj.stride(1) == 1 and proj.shape[1] >= c + hv + 2 * heads
+    assert taps.dtype == torch.float32 and taps.is_contiguous() and norm_w.dtype == torch.float32 and norm_w.numel() == vdim
+    assert filter_state.dtype == torch.float32 and filter_state.is_contiguous() and tuple(filter_state.shape[1:]) == (k - 1, c)
+    assert state.dtype == torch.float32 and state.is_contiguous() and tuple(state.shape[1:]) == (heads, recurrent_state_floats(dim, vdim))
+    assert out.is_contiguous() and out.shape == (t, hv)
+    f = _fn("recurrent", "gb_delta_step",
+            [c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int,
+             c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_float, c_void_p])
+    _check(f(proj.data_ptr(), proj.stride(0), taps.data_ptr(), filter_state.data_ptr(), a_log.data_ptr(), dt_bias.data_ptr(),
+             state.data_ptr(), seq_slot.data_ptr(), norm_w.data_ptr(), norm_w.numel(), out.data_ptr(), dtype_code(out.dtype), t, heads,
+             groups, dim, vdim, k, q_scale, eps, out_scale, _stream()),
+           "delta_step", "attention", _nbytes(proj, out) + 2 * t * heads * dim * vdim * 4)
+
+
 def ssd_scan(x, b, c, dt_raw, a_log, dt_bias, skip, state, cu_seqlens, seq_slot, y, heads, groups, n_state, vdim,
              chunked: bool = False):
     """The state-space recurrence with one decay per head over each sequence of the packed step

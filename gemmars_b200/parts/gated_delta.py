@@ -78,6 +78,12 @@ class GatedDeltaRule(Part):
         qk, hv, nh, c = self.qk, self.hv, self.heads, self.channels
         p = self.proj(h, out_dtype=torch.float32)
         t = p.shape[0]
+        out = torch.empty((t, hv), dtype=self.act_dtype, device=p.device)
+        if kernels.delta_step_usable(t, ctx.seq_slot.numel(), nh, self.kv_heads, self.dim, self.vdim, self.taps):
+            kernels.delta_step(p, self.filter, filter_state, self.a_log, self.dt_bias, state, ctx.seq_slot, self.norm, out, nh,
+                               self.kv_heads, self.dim, self.vdim, float(self.dim) ** -0.5, self.eps, self.out_scale)
+            self.o.add_into(out, residual)
+            return
         f = torch.empty((t, c), dtype=torch.float32, device=p.device)
         kernels.short_filter(p[:, :c], self.filter, None, filter_state, ctx.cu_seqlens, ctx.tok_seq, ctx.seq_slot, f, act=True)
         y = torch.empty((t, hv), dtype=torch.float32, device=p.device)
@@ -85,7 +91,6 @@ class GatedDeltaRule(Part):
                            self.a_log, self.dt_bias, state, ctx.cu_seqlens, ctx.seq_slot, y, nh, self.kv_heads, self.dim,
                            self.vdim, float(self.dim) ** -0.5,
                            chunked=kernels.chunk_scan("delta", self.compute, self.dim, self.heads, ctx))
-        out = torch.empty((t, hv), dtype=self.act_dtype, device=p.device)
         kernels.gated_group_norm(y, p[:, c:c + hv], self.norm, out, self.vdim, self.eps, False, self.out_scale)
         self.o.add_into(out, residual)
 

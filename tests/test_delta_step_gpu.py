@@ -1,0 +1,49 @@
+"""A gated delta layer's single tokens in one kernel: the bits of the filter, the recurrence and the norm one after the other."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("heads,groups,dim,vdim,taps", [(4, 2, 128, 128, 4), (8, 2, 64, 64, 2), (3, 3, 128, 64, 8), (2, 1, 36, 128, 3),
+                                                        (4, 1, 20, 64, 4), (2, 2, 100, 128, 5)])
+@pytest.mark.parametrize("seqs", [1, 5])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_the_bits_of_the_kernels_one_by_one(heads, groups, dim, vdim, taps, seqs, dtype):
+    from gemmars_b200 import kernels as k
+    assert k.delta_step_usable(seqs, seqs, heads, groups, dim, vdim, taps)
+    g = torch.Generator(device="cuda").manual_seed(heads * dim + seqs)
+    r = lambda *s: torch.randn(s, generator=g, device="cuda")       # noqa: E731
+    qk, hv = groups * dim, heads * vdim
+    c, width = 2 * qk + hv, 2 * qk + 2 * hv + 2 * heads
+    wide, filt = r(seqs, width + 8 - width % 4), r(c, taps)      # rows at 16-byte boundaries: the norm's wide form
+    a_log, dt_bias, norm = r(heads).abs().log(), r(heads), r(vdim)
+    slots = torch.tensor([(3 * i + 1) % 7 for i in range(seqs)], dtype=torch.int32, device="cuda")
+    states = [(r(8, taps - 1, c), r(8, heads, k.recurrent_state_floats(dim, vdim)))]
+    states.append(tuple(s.clone() for s in states[0]))
+    cu = torch.arange(seqs + 1, dtype=torch.int32, device="cuda")
+    seq = torch.arange(seqs, dtype=torch.int32, device="cuda")
+    outs = [torch.empty(seqs, hv, device="cuda", dtype=dtype) for _ in range(2)]
+    for step in range(3):                # on what the step before has left
+        proj = (wide.roll(step, 0) * (1 + 0.1 * step))[:, :width]
+        fs, st = states[0]
+        f, y = torch.empty(seqs, c, device="cuda"), torch.empty(seqs, hv, device="cuda")
+        k.short_filter(proj[:, :c], filt, None, fs, cu, seq, slots, f, act=True)
+        k.delta_rule(f[:, :qk], f[:, qk:2 * qk], f[:, 2 * qk:], proj[:, c + hv:c + hv + heads], proj[:, c + hv + heads:], a_log, dt_bias, st,
+                     cu, slots, y, heads, groups, dim, vdim, dim ** -0.5)
+        k.gated_group_norm(y, proj[:, c:c + hv], norm, outs[0], vdim, 1e-6, False, 0.7)
+        k.delta_step(proj, filt, states[1][0], a_log, dt_bias, states[1][1], slots, norm, outs[1], heads, groups, dim, vdim, dim ** -0.5,
+                     1e-6, 0.7)
+        assert torch.equal(outs[0], outs[1])
+        assert torch.equal(states[0][0], states[1][0])
+        # the decay's zero rows beyond the head's dims stay what they were times the decay in both
+        assert torch.equal(states[0][1], states[1][1])
+
+
+def test_what_is_refused_runs_as_before():
+    from gemmars_b200 import kernels as k
+    assert not k.delta_step_usable(5, 4, 4, 2, 128, 128, 4)          # a prompt among them
+    assert not k.delta_step_usable(4, 4, 4, 1, 128, 128, 4)          # sixteen blocks a q/k head
+    assert not k.delta_step_usable(4, 4, 4, 2, 256, 128, 4)
+    assert not k.delta_step_usable(4, 4, 4, 2, 128, 96, 4)
+    assert not k.delta_step_usable(4, 4, 4, 2, 128, 128, 1)
