@@ -531,28 +531,29 @@ __global__ void __launch_bounds__(32 * DS * NV + 32) chunk_scan_kernel(const Sca
       }
     }
     if (DS > 1) {
-      float* mine = exch + ((c & 1) * DS * NV + warp) * 512 + lane;
+      float4* mine = (float4*)(exch + ((c & 1) * DS * NV + warp) * 512) + lane;
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        if (HAS_W) mine[32 * e] = u[0][e], mine[32 * (4 + e)] = u[1][e];
-        mine[32 * (8 + e)] = y[0][e];
-        mine[32 * (12 + e)] = y[1][e];
+      for (int nt = 0; nt < 2; ++nt) {
+        if (HAS_W) mine[32 * nt] = make_float4(u[nt][0], u[nt][1], u[nt][2], u[nt][3]);
+        mine[32 * (2 + nt)] = make_float4(y[nt][0], y[nt][1], y[nt][2], y[nt][3]);
       }
     }
     asm volatile("bar.sync 0;" ::: "memory");     // the warps' parts are there, and block c + 1; block c - 1 may go
     const bool finishes = DS == 1 || part < 2;     // warp 0 the first half of the tokens, warp 1 the second
-    if (DS > 1) {                                  // the warps' parts, in their order
-      const float* group = exch + ((c & 1) * DS * NV + warp - part) * 512 + lane;
+    // the warps' parts, in their order: four numbers of part q (u of either half of the tokens, then y)
+    auto gather = [&](int q, float (&to)[4]) {
+      const float4* group = (const float4*)(exch + ((c & 1) * DS * NV + warp - part) * 512) + 32 * q + lane;
+      float4 sum = group[0];
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        if (HAS_W) u[0][e] = group[32 * e], u[1][e] = group[32 * (4 + e)];
-        if (finishes) y[0][e] = group[32 * (8 + 4 * part + e)];
-#pragma unroll
-        for (int o = 1; o < DS; ++o) {
-          if (HAS_W) u[0][e] += group[512 * o + 32 * e], u[1][e] += group[512 * o + 32 * (4 + e)];
-          if (finishes) y[0][e] += group[512 * o + 32 * (8 + 4 * part + e)];
-        }
+      for (int o = 1; o < DS; ++o) {
+        const float4 v = group[128 * o];
+        sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
       }
+      to[0] = sum.x; to[1] = sum.y; to[2] = sum.z; to[3] = sum.w;
+    };
+    if (DS > 1 && HAS_W) {
+      gather(0, u[0]);
+      gather(1, u[1]);
     }
     uint32_t uhi[2][4], ulo[2][4];
 #pragma unroll
@@ -582,6 +583,7 @@ __global__ void __launch_bounds__(32 * DS * NV + 32) chunk_scan_kernel(const Sca
       S[j][3] = fmaf(gf.y, S[j][3], whole(d[3], x[3], 2.f));
     }
     // Y = Q~ S + P U, of the tokens that this warp finishes
+    if (DS > 1 && finishes) gather(2 + part, y[0]);
     const bool u_clean = !finishes || all_finite(ulo);
 #pragma unroll
     for (int i = 0; i < (DS == 1 ? 2 : 1); ++i) {
