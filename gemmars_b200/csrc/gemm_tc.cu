@@ -1631,7 +1631,8 @@ GB_EXPORT int gb_gemm_tc_persistent(const void* x, const void* w, const float* b
 // w stacks `experts` matrices of N rows (2 N gated: gate rows, then up rows); tile_expert [M / bn].
 // mode 1: y float32 [M, N] = x W_g^T; mode 3: y bfloat16 [M, N] = row_scale * act(gate, up), act the
 // clamped form when limit > 0, or with scale_in act(row_scale * gate, row_scale * up); mode 0: y bfloat16 [M, N] = row_scale * act(x W_g^T) (no gate rows in w;
-// act 1: the exact GELU, 2: the square of relu).  bn: 128 or 256.  tile_rows [M / bn]: how many of a tile's rows exist
+// act 1: the exact GELU, 2: the square of relu).  bn: 128 or 256.  tile_expert null, with one expert: a product of all M rows,
+// any number of them, by one matrix (bn a multiple of 16 up to 256).  tile_rows [M / bn]: how many of a tile's rows exist
 // (null: all); the others' results are not written, or not to be read.
 GB_EXPORT int gb_gemm_tc_grouped(const void* x, const void* w, void* y, int mode, int M, int N, int K, long long ldx,
                                  long long ldy, int bn, int ctas, int experts, const int* tile_expert, const int* tile_rows,
@@ -1639,7 +1640,7 @@ GB_EXPORT int gb_gemm_tc_grouped(const void* x, const void* w, void* y, int mode
   if (M <= 0 || N <= 0 || experts <= 0) return 0;
   if (act < OUT_ACT_NONE || act > OUT_ACT_RELU2) return GB_ERR_ARG;
   if (K <= 0 || (K % 8) || (ldx % 8) || ((uintptr_t)x & 15) || ((uintptr_t)w & 15) || ctas <= 0) return GB_ERR_SIZE;
-  if ((bn != 128 && bn != 256) || M % bn || !tile_expert) return GB_ERR_SIZE;
+  if (tile_expert ? (bn != 128 && bn != 256) || M % bn : experts != 1 || tile_rows || bn < 16 || bn > 256 || bn % 16) return GB_ERR_SIZE;
   const bool gated = mode == EPI_SWIGLU_BF16;
   if (!gated && mode != EPI_STORE_F32 && mode != EPI_STORE_BF16) return GB_ERR_ARG;
   Grouped grp;
@@ -1651,6 +1652,7 @@ GB_EXPORT int gb_gemm_tc_grouped(const void* x, const void* w, void* y, int mode
   grp.act = mode == EPI_STORE_BF16 ? act : OUT_ACT_NONE;
   grp.scale_in = gated && row_scale ? scale_in : 0;
   const bool pair = pairs_pay(M, N, K, bn, ctas, gated ? BM / 2 : BM);
+  if (pair) bn = (bn + 31) / 32 * 32;
   CUtensorMap mw, mx;
   if (!persistent_w_map(&mw, w, (uint64_t)experts * grp.rows_per_expert, N, K, gated, grp)) return GB_ERR_ARG;
   if (!tensor_map(&mx, x, (uint64_t)M, (uint64_t)K, (uint64_t)ldx * 2, (uint32_t)(pair ? bn / 2 : bn))) return GB_ERR_ARG;

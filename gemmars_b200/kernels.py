@@ -450,6 +450,25 @@ _part_flags = {}
 PERSISTENT_SPLIT_LAST_ROUND = True
 
 
+def prompt_tile(m: int, tiles_n: int, sms: int, accumulate: bool = False) -> int:
+    """Tokens a tile of the persistent product of m rows by ``tiles_n`` tiles of features."""
+    # 256 tokens a tile.  Narrower tiles that fill the last round of tiles better were slower while a block
+    # of 64 inner elements took some 310 ns whatever its tokens: 240 tokens for 2,048 x 4,096 (1.5 % faster
+    # alone, 4 % slower inside a prompt step), and 128 tokens where 256 leave the last round nearly empty
+    # (2,048 x 2,560 is 160 tiles on 148 SMs; a 2,048-token prompt of a 4B-shaped model took 20.5 ms against
+    # 18.4, of a 32B-shaped one 35.3 ms against 30.9 over 16 layers).  With an elected issuing thread a block
+    # of 128 tokens takes 190 ns; the comparison has not been made again since.
+    bn = 128 if m <= 128 else 256
+    # Where those leave two SMs in five without a tile (a router, a low-rank factor, few tokens), the narrowest tiles that
+    # still are one round; a block of the inner dimension takes less time the narrower they are (us, 256 tokens a
+    # tile / so; 2,048 inner): 65 features of 2,048 tokens (8 tiles) 23.8 / 11.5, 576 of 2,048 (40) 17.7 / 13.1, 1,024
+    # of 2,048 (64) 17.7 / 13.6, 576 of 4,096 (80) 17.7 / 15.6, but 1,024 of 4,096 (128 tiles) 19.2 / 19.7.
+    # A product that adds cuts its tiles along the inner dimension instead.
+    if not accumulate and 5 * tiles_n * -(-m // bn) <= 3 * sms:
+        bn = min(bn, (-(-m // (sms // tiles_n)) + 15) // 16 * 16)
+    return bn
+
+
 def gemm_tc_persistent(x, w, out, bias=None, accumulate=False, swiglu=False, bn=None, ctas=None, split_last=None,
                        act="silu", plain_act=None, col_scale=None):
     """The tensor-core product for prompts (more than 64 rows of x): one CTA per SM walks the output
@@ -477,21 +496,7 @@ def gemm_tc_persistent(x, w, out, bias=None, accumulate=False, swiglu=False, bn=
     if bias is not None:
         assert bias.dtype == torch.float32 and bias.numel() == n
     if bn is None:
-        # 256 tokens a tile.  Narrower tiles that fill the last round of tiles better were slower while a block
-        # of 64 inner elements took some 310 ns whatever its tokens: 240 tokens for 2,048 x 4,096 (1.5 % faster
-        # alone, 4 % slower inside a prompt step), and 128 tokens where 256 leave the last round nearly empty
-        # (2,048 x 2,560 is 160 tiles on 148 SMs; a 2,048-token prompt of a 4B-shaped model took 20.5 ms against
-        # 18.4, of a 32B-shaped one 35.3 ms against 30.9 over 16 layers).  With an elected issuing thread a block
-        # of 128 tokens takes 190 ns; the comparison has not been made again since.
-        bn = 128 if m <= 128 else 256
-        # Where those leave two SMs in five without a tile (a router, a low-rank factor, few tokens), the narrowest tiles that
-        # still are one round; a block of the inner dimension takes less time the narrower they are (us, 256 tokens a
-        # tile / so; 2,048 inner): 65 features of 2,048 tokens (8 tiles) 23.8 / 11.5, 576 of 2,048 (40) 17.7 / 13.1, 1,024
-        # of 2,048 (64) 17.7 / 13.6, 576 of 4,096 (80) 17.7 / 15.6, but 1,024 of 4,096 (128 tiles) 19.2 / 19.7.
-        # A product that adds cuts its tiles along the inner dimension instead.
-        tiles_n, sms = -(-n // (64 if swiglu else 128)), ctas or sm_count(x.device)
-        if not accumulate and 5 * tiles_n * -(-m // bn) <= 3 * sms:
-            bn = min(bn, (-(-m // (sms // tiles_n)) + 15) // 16 * 16)
+        bn = prompt_tile(m, -(-n // (64 if swiglu else 128)), ctas or sm_count(x.device), accumulate)
     ctas = ctas or sm_count(x.device)
     flags = None
     if accumulate and split_last:
@@ -1469,12 +1474,13 @@ def gemm_tc_grouped(x, w, y, n, experts, tile_expert, row_scale=None, gated=Fals
     assert x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and x.stride(1) == 1 and w.is_contiguous()
     assert not (gated and act)
     assert y.shape == (rows, n) and y.is_contiguous() and y.dtype == (torch.bfloat16 if gated or act else torch.float32)
-    assert tile_expert.dtype == torch.int32 and tile_expert.numel() == rows // bn and rows % bn == 0
+    assert experts == 1 if tile_expert is None else (tile_expert.dtype == torch.int32 and tile_expert.numel() == rows // bn
+                                                     and rows % bn == 0)
     f = _fn("gemm_tc", "gb_gemm_tc_grouped",
             [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_longlong, c_longlong, c_int, c_int, c_int, c_void_p,
              c_void_p, c_void_p, c_float, c_float, c_float, c_int, c_int, c_void_p])
     _check(f(x.data_ptr(), w.data_ptr(), y.data_ptr(), 3 if gated else (0 if act else 1), rows, n, k, x.stride(0), y.stride(0), bn,
-             sm_count(x.device), experts, tile_expert.data_ptr(), _ptr(tile_rows), _ptr(row_scale), limit, alpha, shift, PLAIN_ACTS[act],
+             sm_count(x.device), experts, _ptr(tile_expert), _ptr(tile_rows), _ptr(row_scale), limit, alpha, shift, PLAIN_ACTS[act],
              1 if scale_in else 0, _stream()),
            "gemm_tc_grouped", "matmul", _nbytes(x, w, y))
 
@@ -1505,10 +1511,18 @@ def moe_experts_tc(h, idx, wts, sg, w_gate_up, w_down, shared_gate_up, shared_do
 
 
 def _shared_expert(h, sg, shared_gate_up, shared_down, residual, shared_limit, alpha, shift, col_scale=None):
-    """residual += sg * shared(h): two dense products of the framework's around the activation."""
+    """residual += sg * shared(h): two dense products of the framework's, the activation in the epilogue of the first for
+    prompts (us, apart / so: a layer of 2,048 tokens, 2,816 shared features 386 / 381; of 1,500, 1,024 features 146 / 138), a
+    kernel of its own for a few tokens."""
     if shared_down is None:
         return
     t, ffs = h.shape[0], shared_down.shape[1]
+    if t > GATED_TILE_128_MAX_TOKENS and shared_limit > 0 and gemm_tc_usable(h, shared_gate_up):
+        ys = torch.empty((t, ffs), dtype=torch.bfloat16, device=h.device)
+        gemm_tc_grouped(h, shared_gate_up, ys, ffs, 1, None, sg, gated=True, limit=shared_limit, alpha=alpha, shift=shift,
+                        bn=prompt_tile(t, -(-ffs // 64), sm_count(h.device)))
+        gemm(ys, shared_down, residual, accumulate=True, col_scale=col_scale)
+        return
     gu = torch.empty((t, 2 * ffs), dtype=torch.bfloat16, device=h.device)
     gemm(h, shared_gate_up, gu)
     ys = torch.empty((t, ffs), dtype=torch.bfloat16, device=h.device)

@@ -132,3 +132,19 @@ def test_groups_narrower_than_a_tile(k, monkeypatch, counts):
         tol = 2.0 ** -8 * want.abs() + 1.8 * (u.abs() * bound[:, :n] + (a.abs() + 1) * bound[:, n:]) + 2.0 ** -19 * (a.abs() + 1) * (u.abs() + 1)
         assert ((yg[at].double() - want).abs() <= tol).all()
     assert k.gemm_tc_status() == 0
+
+
+@pytest.mark.parametrize("t,width,ffs", [(129, 64, 72), (300, 200, 1024), (2048, 264, 320), (511, 128, 2816)])
+def test_shared_expert_with_its_activation_in_the_product(k, t, width, ffs):
+    x, w = operands(t, 2 * ffs, width, t)
+    down = (torch.randn(width, ffs, device="cuda") * ffs ** -0.5).bfloat16()
+    sg, residual = torch.rand(t, device="cuda"), torch.randn(t, width, device="cuda")
+    got = residual.clone()
+    k._shared_expert(x, sg, w, down, got, 1.5, 1.702, 1.0)
+    g, u = (x.double() @ w[:ffs].double().T).clamp(max=1.5), (x.double() @ w[ffs:].double().T).clamp(-1.5, 1.5)
+    act = g * torch.sigmoid(1.702 * g) * (u + 1) * sg[:, None].double()
+    want = residual.double() + act @ down.double().T
+    # an activation is rounded to bfloat16 once; what float32 sums and the clamps' edges add is far below its half step
+    tol = (2.0 ** -8 * act.abs() + 1e-4) @ down.double().abs().T + 2.0 ** -21 * (want.abs() + 4)
+    assert ((got.double() - want).abs() <= tol).all()
+    assert k.gemm_tc_status() == 0
