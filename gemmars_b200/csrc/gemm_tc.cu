@@ -871,6 +871,9 @@ struct Grouped {
   int rows_per_expert = 0;
   float limit = 0.f, alpha = 0.f, shift = 0.f;
   int act = 0, scale_in = 0;
+  // a batch of products of one size: group_rows rows of x and of the result each, one group after the other at any row, in
+  // group_tiles tiles of tokens (0: not a batch; then tile_expert, tile_rows are null)
+  int group_tiles = 0, group_rows = 0;
   int gate_rows_whole = 0;     // gated: map_w brings a tile's gate and up rows in one box (gated_map)
 };
 __device__ __forceinline__ void act_rows(uint32_t (&v)[16], float bias, int act, const float* row_scale, int row, int M) {
@@ -927,7 +930,24 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = PAIR ? (int)cluster_rank() : 0, walker = (int)blockIdx.x / CTAS, walkers = (int)gridDim.x / CTAS;
   constexpr int WALK_F = CTAS * TILE_F;             // features of the result per tile of the walk; rank r has the r-th TILE_F
-  const int tiles_m = (M + bn - 1) / bn, tiles_n = (N + WALK_F - 1) / WALK_F, tiles = tiles_m * tiles_n;
+  const int tiles_m = grp.group_tiles ? M / grp.group_rows * grp.group_tiles : (M + bn - 1) / bn;
+  const int tiles_n = (N + WALK_F - 1) / WALK_F, tiles = tiles_m * tiles_n;
+  // tile t: its first token and feature, its matrix (-1: a tile no group uses), and how many of its tokens exist
+  auto tile_at = [&](int t, int& m0, int& n0, int& e, int& rows) {
+    tile_origin(t, tiles_m, tiles_n, bn, WALK_F, m0, n0);
+    e = 0;
+    rows = bn;
+    if (grp.group_tiles) {
+      const int tm = m0 / bn;
+      e = tm / grp.group_tiles;
+      const int r = (tm - e * grp.group_tiles) * bn;
+      rows = min(bn, grp.group_rows - r);
+      m0 = e * grp.group_rows + r;
+    } else if (grp.tile_expert) {
+      e = grp.tile_expert[m0 / bn];
+      if (grp.tile_rows && e >= 0) rows = grp.tile_rows[m0 / bn];
+    }
+  };
   const int kb_total = (K + BK - 1) / BK;
 
   if (threadIdx.x == 0) {
@@ -969,16 +989,12 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
       uint32_t it = 0;
       bool ok = true;
       for (TileWalk w(tiles, kb_total, split, walker, walkers); w.more() && ok; w.next()) {
-        int m0, n0;
-        tile_origin(w.t, tiles_m, tiles_n, bn, WALK_F, m0, n0);
-        int w0 = n0 + rank * TILE_F;                   // the tile's first row of W
-        int x0 = m0 + rank * bn / 2;                   // a pair: rank 1 brings the second half of the MMA's tokens
-        if (grp.tile_expert) {
-          const int e = grp.tile_expert[m0 / bn];
-          if (e < 0) continue;
-          w0 += e * grp.rows_per_expert;
-          if (PAIR && grp.tile_rows) x0 = m0 + rank * (((grp.tile_rows[m0 / bn] + 31) & ~31) / 2);
-        }
+        int m0, n0, e, rows;
+        tile_at(w.t, m0, n0, e, rows);
+        if (e < 0) continue;
+        const int w0 = n0 + rank * TILE_F + e * grp.rows_per_expert;     // the tile's first row of W
+        // a pair: rank 1 brings the second half of the MMA's tokens
+        const int x0 = m0 + rank * ((rows < bn ? (rows + 31) & ~31 : bn) / 2);
         for (int kb = w.kb0; kb < w.kb1; ++kb, ++it) {
           const uint32_t s = it % STAGES;
           if (it >= STAGES && !mbar_wait(&empty_bar[s], ((it / STAGES) - 1) & 1)) {
@@ -1020,17 +1036,14 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
       // that is never filled
       if (grp.tile_expert) pdl_wait_prior();
       for (TileWalk w(tiles, kb_total, split, walker, walkers); w.more() && ok; w.next(), ++i) {
-        uint32_t width = (uint32_t)bn;
-        if (grp.tile_expert) {                         // a tile no group uses: not counted, as in the other roles
-          int m0, n0;
-          tile_origin(w.t, tiles_m, tiles_n, bn, WALK_F, m0, n0);
-          if (grp.tile_expert[m0 / bn] < 0) {
-            --i;
-            continue;
-          }
-          constexpr uint32_t UNIT = 16 * CTAS;
-          if (grp.tile_rows) width = ((uint32_t)grp.tile_rows[m0 / bn] + UNIT - 1) & ~(UNIT - 1);
+        constexpr int UNIT = 16 * CTAS;
+        int m0, n0, e, rows;
+        tile_at(w.t, m0, n0, e, rows);
+        if (e < 0) {                                   // not counted, as in the other roles
+          --i;
+          continue;
         }
+        const uint32_t width = rows < bn ? (uint32_t)((rows + UNIT - 1) & ~(UNIT - 1)) : (uint32_t)bn;
         const uint32_t idesc = idesc_rest | (width >> 3 << 17);
         const uint32_t b = i & 1;
         if (i >= 2 && !(PAIR ? mbar_wait_cluster(&acc_empty[b], ((i >> 1) - 1) & 1) : mbar_wait(&acc_empty[b], ((i >> 1) - 1) & 1))) {   // the epilogue has read this buffer out
@@ -1076,16 +1089,16 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
     const bool both = bn % 32 == 0;   // 32 tokens per round; the result's map is cut to match
     uint32_t i = 0;
     for (TileWalk w(tiles, kb_total, split, walker, walkers); w.more(); w.next(), ++i) {
-      int m0, n0;
-      tile_origin(w.t, tiles_m, tiles_n, bn, WALK_F, m0, n0);
+      int m0, n0, e, rows;
+      tile_at(w.t, m0, n0, e, rows);
       n0 += rank * TILE_F;
-      if (grp.tile_expert && grp.tile_expert[m0 / bn] < 0) {
+      if (e < 0) {
         --i;
         continue;
       }
       const uint32_t b = i & 1;
       const int n = n0 + f;
-      const int m_end = grp.tile_rows ? min(M, m0 + grp.tile_rows[m0 / bn]) : M;     // the tile's rows that exist
+      const int m_end = grp.tile_rows || grp.group_tiles ? min(M, m0 + rows) : M;     // the tile's rows that exist
       bool have = __all_sync(0xffffffffu, PAIR ? mbar_wait_cluster(&acc_full[b], (i >> 1) & 1) : mbar_wait(&acc_full[b], (i >> 1) & 1));
       if (!have && lane == 0) atomicCAS(&g_status, ST_OK, ST_TIMEOUT_TMEM);
       if (QKV) {   // the warps meet at barriers below: they leave together or not at all
@@ -1188,7 +1201,8 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
             scale_values(v, col_v);
             if (both) scale_values(v2, col_v);
           }
-          if (y_tma) {
+          // rows beyond a batch's group are the next one's
+          if (y_tma && !(grp.group_tiles && m_end < M && m0 + c + (both ? 32 : 16) > m_end)) {
             tile_out.send(v, v2, both, b_out, lane, n0 + warp * 32, m0 + c, N);
           } else {
             store_direct<MODE>(y, ldy, v, b_out, m0 + c, m_end, n, N);
@@ -1410,7 +1424,7 @@ int launch_persistent(const CUtensorMap& mw, const CUtensorMap& mx, const OutMap
     configured = true;
   }
   const int walkers = ctas / CTAS > 0 ? ctas / CTAS : 1;
-  const int tiles = ((M + bn - 1) / bn) * ((N + WALK_F - 1) / WALK_F);
+  const int tiles = (grp.group_tiles ? M / grp.group_rows * grp.group_tiles : (M + bn - 1) / bn) * ((N + WALK_F - 1) / WALK_F);
   // Where the last round of tiles would leave SMs idle and TMA adds the sums into the result: that
   // round's tiles in `split` parts along the inner dimension.  What a split costs, in blocks of the
   // inner dimension: the rounds of parts it makes, and, since the parts of a tile add one after the
@@ -1570,7 +1584,7 @@ GB_EXPORT int gb_gemm_tc_qkv(const void* x, const void* w, const float* bias, vo
   return GB_ERR_SIZE;
 }
 
-// The same product for prompts (M > 64): one CTA per SM walks the tiles and the epilogue of a tile
+// The same product for prompts (M > 64): one CTA per SM, or a pair of CTAs per two (pairs_pay), walks the tiles and the epilogue of a tile
 // runs under the MMAs of the next.  mode as gb_gemm_tc; bn: tokens per tile, a multiple of 16 up to
 // 256; ctas: CTAs to launch.  part_flags: null, or 4 * ctas int32 zeros: a product that adds into y
 // may then cut the tiles of a last round that is not full into parts along the inner dimension;
@@ -1670,6 +1684,33 @@ GB_EXPORT int gb_gemm_tc_grouped(const void* x, const void* w, void* y, int mode
   if (pair) return launch_persistent<256, 6, EPI_STORE_F32, true>(mw, mx, my, nullptr, y, M, N, K, ldy, bn, ctas, stream, QkvTail{}, nullptr, grp);
   if (bn > 128) return launch_persistent<256, 4, EPI_STORE_F32>(mw, mx, my, nullptr, y, M, N, K, ldy, bn, ctas, stream, QkvTail{}, nullptr, grp);
   return launch_persistent<128, 6, EPI_STORE_F32>(mw, mx, my, nullptr, y, M, N, K, ldy, bn, ctas, stream, QkvTail{}, nullptr, grp);
+}
+
+// `groups` products of one size in one walk of tiles: x [groups, T, K] bfloat16 (contiguous), w [groups, N, K] bfloat16, y
+// [groups, T, N] float32.  One launch whose last round of tiles is one, not `groups` of them: four of 2,048 x 4,096 x 4,096
+// 196 -> 164 us, a wkv layer of 700 tokens at 2,048 wide 189 -> 151.  bn: tokens a tile, a multiple of 16 up to 256.
+GB_EXPORT int gb_gemm_tc_batch(const void* x, const void* w, void* y, int groups, int T, int N, int K, int bn, int ctas,
+                               cudaStream_t stream) {
+  if (groups <= 0 || T <= 0 || N <= 0) return 0;
+  if (K <= 0 || (K % 8) || ((uintptr_t)x & 15) || ((uintptr_t)w & 15) || ctas <= 0 || bn < 16 || bn > 256 || bn % 16) return GB_ERR_SIZE;
+  if ((long long)groups * (T + bn) > 0x7fffffffLL || (long long)groups * N > 0x7fffffffLL) return GB_ERR_SIZE;
+  Grouped grp;
+  grp.rows_per_expert = N;
+  grp.group_tiles = (T + bn - 1) / bn;
+  grp.group_rows = T;
+  const bool pair = pairs_pay(groups * grp.group_tiles * bn, N, K, bn, ctas, BM);
+  if (pair) {
+    bn = (bn + 31) / 32 * 32;
+    grp.group_tiles = (T + bn - 1) / bn;
+  }
+  const int M = groups * T;
+  CUtensorMap mw, mx;
+  if (!tensor_map(&mw, w, (uint64_t)groups * N, (uint64_t)K, (uint64_t)K * 2, BM)) return GB_ERR_ARG;
+  if (!tensor_map(&mx, x, (uint64_t)M, (uint64_t)K, (uint64_t)K * 2, (uint32_t)(pair ? bn / 2 : bn))) return GB_ERR_ARG;
+  const OutMap my = out_map(y, EPI_STORE_F32, M, N, N, bn);
+  if (pair) return launch_persistent<256, 6, EPI_STORE_F32, true>(mw, mx, my, nullptr, y, M, N, K, N, bn, ctas, stream, QkvTail{}, nullptr, grp);
+  if (bn > 128) return launch_persistent<256, 4, EPI_STORE_F32>(mw, mx, my, nullptr, y, M, N, K, N, bn, ctas, stream, QkvTail{}, nullptr, grp);
+  return launch_persistent<128, 6, EPI_STORE_F32>(mw, mx, my, nullptr, y, M, N, K, N, bn, ctas, stream, QkvTail{}, nullptr, grp);
 }
 
 // Whether the products above take pairs of CTAs at these sizes: N features of the result; gated: mode 3.

@@ -1485,6 +1485,24 @@ def gemm_tc_grouped(x, w, y, n, experts, tile_expert, row_scale=None, gated=Fals
            "gemm_tc_grouped", "matmul", _nbytes(x, w, y))
 
 
+def gemm_batch(x, w, out):
+    """out[g] = x[g] @ w[g].T for x [G, T, K], w [G, N, K], out float32 [G, T, N], all contiguous: prompts in bfloat16 in one
+    launch, other steps a product at a time."""
+    groups, t, k = x.shape
+    n = w.shape[1]
+    assert w.shape == (groups, n, k) and out.shape == (groups, t, n) and x.is_contiguous() and w.is_contiguous() and out.is_contiguous()
+    if t <= 64 or not gemm_tc_usable(x[0], w[0]):
+        for g in range(groups):
+            gemm(x[g], w[g], out[g])
+        return
+    _cuda(x, w, out)
+    assert out.dtype == torch.float32
+    sms = sm_count(x.device)
+    f = _fn("gemm_tc", "gb_gemm_tc_batch", [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p])
+    _check(f(x.data_ptr(), w.data_ptr(), out.data_ptr(), groups, t, n, k, prompt_tile(t, groups * -(-n // 128), sms), sms, _stream()),
+           "gemm_tc_batch", "matmul", _nbytes(x, w, out))
+
+
 def moe_experts_tc(h, idx, wts, sg, w_gate_up, w_down, shared_gate_up, shared_down, residual, limit, shared_limit, alpha,
                    shift, col_scale=None, weigh_input=False, store=False):
     """As moe_experts_grouped for a prompt step, the experts' two products on the tcgen05 kernel: the

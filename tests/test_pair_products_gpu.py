@@ -148,3 +148,18 @@ def test_shared_expert_with_its_activation_in_the_product(k, t, width, ffs):
     tol = (2.0 ** -8 * act.abs() + 1e-4) @ down.double().abs().T + 2.0 ** -21 * (want.abs() + 4)
     assert ((got.double() - want).abs() <= tol).all()
     assert k.gemm_tc_status() == 0
+
+
+@pytest.mark.parametrize("sms", [4, 3, None])
+@pytest.mark.parametrize("groups,t,n,kk", [(4, 65, 200, 136), (3, 300, 384, 72), (2, 513, 128, 264), (4, 256, 1000, 64), (5, 270, 130, 4104)])
+def test_a_batch_of_products(k, monkeypatch, sms, groups, t, n, kk):
+    """Groups that start at any row: a tile's last piece of tokens ends at its group's last row."""
+    if sms:
+        monkeypatch.setattr(k, "sm_count", lambda device=None: sms)
+    x, w = operands(groups * t, groups * n, kk, t)
+    out = torch.full((groups, t, n), 7.0, device="cuda")
+    k.gemm_batch(x.view(groups, t, kk), w.view(groups, n, kk), out)
+    for g in range(groups):
+        want, bound = exact_and_bound(x[g * t:(g + 1) * t], w[g * n:(g + 1) * n])
+        assert ((out[g].double() - want).abs() <= bound + 2.0 ** -22 * want.abs()).all()
+    assert k.gemm_tc_status() == 0
