@@ -27,7 +27,7 @@
 // outputs and state, 1e-7): delta rule 2.2 / 2.5 and 3.6 / 3.5, with a decay per channel 1.9 / 1.8 and 2.2 / 1.9, state space
 // 1.0 / 1.4 and 1.8 / 1.8, read before 2.4 / 2.2 and 2.5 / 2.0, read after 1.9 / 1.9 and 1.7 / 1.6; of a layer's states,
 // whose inputs come from bfloat16 products, 54 / 54, 67 / 66 and 80 / 79 (delta rule, state space, read before).
-// A number that is not finite reaches what it reaches token by token: see mma_lower().
+// A number that is not finite reaches what it reaches token by token: see mend_lower().
 #include <type_traits>
 #include "common.cuh"
 
@@ -80,17 +80,18 @@ __device__ __forceinline__ void mma3_apart(float (&d)[4], float (&x)[4], const u
 __device__ __forceinline__ float whole(float d, float x, float links) { return d + fmaf(d, 4.3e-8f * (0.5f * (links + 1.f)), x); }
 
 // Over a chunk's tokens, by weights below a diagonal (T, P): d = (columns of V or U) x (weights of the eight tokens 8 nt ..), token i
-// from tokens up to i.  Above the diagonal the weights are zeros, and what they multiply must not reach the result where it is
-// not finite: without `clean`, a column's tokens before the first such one take the product without it.
-__device__ __forceinline__ void mma_lower(float (&d)[4], const uint32_t (&hi)[2][4], const uint32_t (&lo)[2][4], float4 w, int nt, bool clean,
-                                          int lane) {
+// from tokens up to i.
+__device__ __forceinline__ void mma_lower(float (&d)[4], const uint32_t (&hi)[2][4], const uint32_t (&lo)[2][4], float4 w, int nt) {
   float x[4] = {};
   d[0] = d[1] = d[2] = d[3] = 0.f;
   mma3(d, x, hi[0], lo[0], w.x, w.y);
   if (nt) mma3(d, x, hi[1], lo[1], w.z, w.w);
 #pragma unroll
   for (int e = 0; e < 4; ++e) d[e] = whole(d[e], x[e], nt ? 2.f : 1.f);
-  if (clean) return;
+}
+// Above the diagonal the weights are zeros, and what they multiply must not reach the result where it is not finite: a column's
+// tokens before the first such one take the product without it.  For operands that are not all finite.
+__device__ __forceinline__ void mend_lower(float (&d)[4], const uint32_t (&hi)[2][4], const uint32_t (&lo)[2][4], float4 w, int nt, int lane) {
   uint32_t h[2][4], l[2][4];
   int first[2] = {CT, CT};                      // of columns gr and gr + 8
 #pragma unroll
@@ -106,12 +107,11 @@ __device__ __forceinline__ void mma_lower(float (&d)[4], const uint32_t (&hi)[2]
   for (int o = 1; o <= 2; o <<= 1)
 #pragma unroll
     for (int c = 0; c < 2; ++c) first[c] = min(first[c], __shfl_xor_sync(0xffffffffu, first[c], o));
-  float f[4] = {}, fx[4] = {};
-  mma3(f, fx, h[0], l[0], w.x, w.y);
-  if (nt) mma3(f, fx, h[1], l[1], w.z, w.w);
+  float f[4];
+  mma_lower(f, h, l, w, nt);
 #pragma unroll
   for (int e = 0; e < 4; ++e)                   // result e: column e >> 1, token 2 t + (e & 1)
-    if (8 * nt + 2 * (lane & 3) + (e & 1) < first[e >> 1]) d[e] = whole(f[e], fx[e], nt ? 2.f : 1.f);
+    if (8 * nt + 2 * (lane & 3) + (e & 1) < first[e >> 1]) d[e] = f[e];
 }
 // Whether all of a warp's numbers in such an operand are finite (a low half is not finite where its number, or the high half, is not).
 __device__ __forceinline__ bool all_finite(const uint32_t (&lo)[2][4]) {
@@ -473,10 +473,57 @@ __global__ void __launch_bounds__(32 * DS * NV + 32) chunk_scan_kernel(const Sca
     const float2 z = in && in1 ? *(const float2*)(st + place(j, col0 + gr + 8)) : make_float2(0.f, 0.f);
     S[j][0] = x.x; S[j][1] = x.y; S[j][2] = z.x; S[j][3] = z.y;
   }
+  // Y = Q~ S + P U of a chunk, of the tokens that this warp finishes (the first warp the first half, the second the second).
+  // LATE: made under the next chunk's products with S, off the chain from chunk to chunk.  A delta rule's (2, 2) 200 -> 187 us
+  // (2,048 tokens, 32 heads of 128 x 128), linear attention at heads of 64 90.6 -> 89.1; four warps a group, whose chains
+  // are shorter, gain nothing.
+  constexpr bool LATE = DS == 2;
+  const bool finishes = DS == 1 || part < 2;
+  constexpr int HALF = DS == 1 ? 2 : 1;           // halves of the tokens that a warp finishes
   float* yrow = a.y + ((size_t)t0 * a.H + head) * V + col0 + gr;
+  uint32_t uhi[2][4] = {}, ulo[2][4] = {};        // the chunk before: what was written, Q~ S, its weights, whether all is finite
+  float ykept[HALF][4] = {}, pu[HALF][4];
+  const float4* pblk = (const float4*)smem + B::P / 4 + lane;
+  bool u_clean = true;
+  int left = 0;                                   // its rows that exist; none before the first
+  auto reads = [&]() {
+#pragma unroll
+    for (int i = 0; i < HALF; ++i) {
+      const int nt = DS == 1 ? i : part & 1;
+      if constexpr (LATE) {                       // without a branch: the first half takes zeros for the second's numbers
+        const uint32_t second = nt ? ~0u : 0u;
+        uint32_t h[4], l[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) h[e] = uhi[1][e] & second, l[e] = ulo[1][e] & second;
+        const float4 w = pblk[32 * nt];
+        float x[4] = {};
+        pu[i][0] = pu[i][1] = pu[i][2] = pu[i][3] = 0.f;
+        mma3(pu[i], x, uhi[0], ulo[0], w.x, w.y);
+        mma3(pu[i], x, h, l, w.z, w.w);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) pu[i][e] = whole(pu[i][e], x[e], nt ? 2.f : 1.f);
+      } else if (finishes) {
+        mma_lower(pu[i], uhi, ulo, pblk[32 * nt], nt);
+      }
+    }
+  };
+  auto leaves = [&]() {
+    if (!finishes) return;
+#pragma unroll
+    for (int i = 0; i < HALF; ++i) {
+      const int nt = DS == 1 ? i : part, row = 8 * nt + 2 * t;
+      if (!u_clean) mend_lower(pu[i], uhi, ulo, pblk[32 * nt], nt, lane);
+      float* to = yrow + (size_t)row * a.H * V;
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (row + (e & 1) < left && (e < 2 ? in0 : in1))
+          to[(size_t)(e & 1) * a.H * V + 8 * (e >> 1)] = (ykept[i][e] + pu[i][e]) * a.yscale;
+    }
+    if (left) yrow += (size_t)CT * a.H * V;
+  };
   asm volatile("bar.sync 0;" ::: "memory");
 #pragma unroll 1
-  for (int c = 0; c < chunks; ++c, yrow += (size_t)CT * a.H * V) {
+  for (int c = 0; c < chunks; ++c) {
     const float4* blk = (const float4*)(smem + (c % STAGES) * STAGE);
     const float* vs = (const float*)blk + B::FLOATS + 2 * t * LV + warp / DS * 16 + gr;
     uint32_t vhi[2][4], vlo[2][4];
@@ -485,6 +532,7 @@ __global__ void __launch_bounds__(32 * DS * NV + 32) chunk_scan_kernel(const Sca
 #pragma unroll
       for (int e = 0; e < 4; ++e)        // a left operand: columns gr, gr + 8 of tokens 2 t, 2 t + 1 of each half
         split(vs[(8 * h + (e >> 1)) * LV + 8 * (e & 1)], vhi[h][e], vlo[h][e]);
+    if (LATE) reads();
     // W S and Q~ S over this warp's channels, transposed: 16 columns by 16 tokens
     float y[2][4] = {}, yx[2][4] = {}, u[2][4] = {}, ux[2][4] = {};
 #pragma unroll
@@ -518,6 +566,7 @@ __global__ void __launch_bounds__(32 * DS * NV + 32) chunk_scan_kernel(const Sca
         y[nt][e] = whole(y[nt][e], yx[nt][e], NJ);
         if (HAS_W) u[nt][e] = -whole(u[nt][e], ux[nt][e], NJ);
       }
+    if (LATE) leaves();
     // + T V: the last warp's work, or the last two's, a half of the tokens each
     if (HAS_W && part >= DS - (DS == 4 ? 2 : 1)) {
       const bool v_clean = all_finite(vlo);
@@ -525,7 +574,9 @@ __global__ void __launch_bounds__(32 * DS * NV + 32) chunk_scan_kernel(const Sca
       for (int nt = 0; nt < 2; ++nt) {
         if (DS == 4 && nt != (part & 1)) continue;
         float d[4];
-        mma_lower(d, vhi, vlo, blk[B::T / 4 + 32 * nt + lane], nt, v_clean, lane);
+        const float4 w = blk[B::T / 4 + 32 * nt + lane];
+        mma_lower(d, vhi, vlo, w, nt);
+        if (!v_clean) mend_lower(d, vhi, vlo, w, nt, lane);
 #pragma unroll
         for (int e = 0; e < 4; ++e) u[nt][e] += d[e];
       }
@@ -539,7 +590,6 @@ __global__ void __launch_bounds__(32 * DS * NV + 32) chunk_scan_kernel(const Sca
       }
     }
     asm volatile("bar.sync 0;" ::: "memory");     // the warps' parts are there, and block c + 1; block c - 1 may go
-    const bool finishes = DS == 1 || part < 2;     // warp 0 the first half of the tokens, warp 1 the second
     // the warps' parts, in their order: four numbers of part q (u of either half of the tokens, then y)
     auto gather = [&](int q, float (&to)[4]) {
       const float4* group = (const float4*)(exch + ((c & 1) * DS * NV + warp - part) * 512) + 32 * q + lane;
@@ -555,7 +605,6 @@ __global__ void __launch_bounds__(32 * DS * NV + 32) chunk_scan_kernel(const Sca
       gather(0, u[0]);
       gather(1, u[1]);
     }
-    uint32_t uhi[2][4], ulo[2][4];
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       if (HAS_W) {
@@ -582,22 +631,23 @@ __global__ void __launch_bounds__(32 * DS * NV + 32) chunk_scan_kernel(const Sca
       S[j][2] = fmaf(gf.x, S[j][2], whole(d[2], x[2], 2.f));
       S[j][3] = fmaf(gf.y, S[j][3], whole(d[3], x[3], 2.f));
     }
-    // Y = Q~ S + P U, of the tokens that this warp finishes
-    if (DS > 1 && finishes) gather(2 + part, y[0]);
-    const bool u_clean = !finishes || all_finite(ulo);
+    if (DS > 1) {
+      if (finishes) gather(2 + part, ykept[0]);
+    } else {
 #pragma unroll
-    for (int i = 0; i < (DS == 1 ? 2 : 1); ++i) {
-      if (!finishes) break;
-      const int nt = DS == 1 ? i : part;
-      float d[4];
-      mma_lower(d, uhi, ulo, blk[B::P / 4 + 32 * nt + lane], nt, u_clean, lane);
-      const int row = 8 * nt + 2 * t, rows = t1 - t0 - c * CT;
-      float* to = yrow + (size_t)row * a.H * V;
-#pragma unroll
-      for (int e = 0; e < 4; ++e)
-        if (row + (e & 1) < rows && (e < 2 ? in0 : in1))
-          to[(size_t)(e & 1) * a.H * V + 8 * (e >> 1)] = (y[i][e] + d[e]) * a.yscale;
+      for (int e = 0; e < 4; ++e) ykept[0][e] = y[0][e], ykept[HALF - 1][e] = y[1][e];
     }
+    u_clean = !finishes || all_finite(ulo);
+    pblk = blk + B::P / 4 + lane;
+    left = t1 - t0 - c * CT;
+    if (!LATE) {
+      reads();
+      leaves();
+    }
+  }
+  if (LATE) {
+    reads();
+    leaves();
   }
   pdl_release_next();
 #pragma unroll
