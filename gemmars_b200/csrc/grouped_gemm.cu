@@ -354,8 +354,8 @@ __global__ void __launch_bounds__(256) moe_combine_wide_kernel(const float* __re
 
 // y[t, f] = act(gu[t, f], gu[t, F + f]) * scale[t]: the activation of a dense (shared) expert.  Bound by memory; eight features a
 // thread where rows of both lie at 16-byte boundaries: 2,048 tokens of 2,816 features (35 MB) 13 us a feature a thread, 9.7
-// so.  Prompts have it in the epilogue of the product before (the gated mode of gemm_tc.cu); this is for up to 128 tokens and
-// experts without a limit.
+// so.  Prompts have it in the epilogue of the product before (the gated mode of gemm_tc.cu); this is for up to 128 tokens
+// and for what that product does not take (a limit of 0, an inner dimension that TMA cannot address).
 __device__ __forceinline__ float gated_value(float g, float u, float sc, float limit, float alpha, float shift) {
   g = fminf(g, limit);
   u = fminf(fmaxf(u, -limit), limit);
