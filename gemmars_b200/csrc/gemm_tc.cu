@@ -27,6 +27,7 @@
 // Every wait on an mbarrier is bounded: after WAIT_LIMIT polls the thread records a code in
 // the status word and goes on to the common exit, where tensor memory is freed.
 #include "tc_common.cuh"
+#include "store_ring.h"
 
 namespace {
 
@@ -138,14 +139,19 @@ constexpr int PIECE_BYTES = PIECE_TOKENS * PIECE_FEATURES * 4;          // float
 constexpr int PIECES = 2;                                               // pieces of a warp in flight
 constexpr int OUT_STAGING_BYTES = 4 * PIECES * PIECE_BYTES;             // four warps
 
+struct StoreQueue {                   // the TMA stores of one thread
+  __device__ __forceinline__ void commit() const { tma_store_commit(); }
+  template <int N> __device__ __forceinline__ void wait_read() const { tma_store_wait_read<N>(); }
+};
+
 template <int MODE, int SLOT_BYTES = PIECE_BYTES>
 struct TileOut {
   static constexpr int FEATURES = PIECE_FEATURES;
   const CUtensorMap* map;
   uint8_t* pieces;   // this warp's pieces, 128-byte aligned
-  uint32_t sent;
+  StoreRing<PIECES> ring;
   __device__ __forceinline__ TileOut(const CUtensorMap* m, uint8_t* staging, int warp)
-      : map(m), pieces(staging + warp * PIECES * SLOT_BYTES), sent(0) {}
+      : map(m), pieces(staging + warp * PIECES * SLOT_BYTES) {}
   __device__ __forceinline__ static void put(uint8_t* p, int token, int lane, float r) {
     if (MODE == EPI_STORE_BF16 || MODE == EPI_SWIGLU_BF16 || MODE == EPI_QKV_BF16)
       ((bf16*)p)[token * FEATURES + lane] = __float2bfloat16_rn(r);
@@ -154,22 +160,22 @@ struct TileOut {
   }
   // the piece to fill next; waits until the request that last used its memory has read it
   __device__ __forceinline__ uint8_t* next(int lane) {
-    if (sent >= PIECES) {
-      if (lane == 0) tma_store_wait_read<PIECES - 1>();
-      __syncwarp();
-    }
-    return pieces + (sent % PIECES) * SLOT_BYTES;
+    ring.reuse(lane == 0, StoreQueue());
+    __syncwarp();
+    return pieces + ring.place() * SLOT_BYTES;
   }
-  // after every lane has put its values: one request for the whole piece
-  __device__ __forceinline__ void post(uint8_t* p, int lane, int x, int row, int N) {
+  // after every lane has put its values: one group of requests for the whole piece, `send` (by lane 0) if there is something of it
+  template <typename Send>
+  __device__ __forceinline__ void post(int lane, bool there, Send send) {
     fence_smem_to_tma();
     __syncwarp();
-    if (lane == 0 && x < N) {
+    ring.post(lane == 0, there, StoreQueue(), send);
+  }
+  __device__ __forceinline__ void post(uint8_t* p, int lane, int x, int row, int N) {
+    post(lane, x < N, [&] {
       if (MODE == EPI_ACCUMULATE_F32) tma_add_2d(map, p, x, row);
       else tma_store_2d(map, p, x, row);
-      tma_store_commit();
-    }
-    ++sent;
+    });
   }
   // lo, hi: tokens 0-15 and (with `both`) 16-31 of this lane's feature; x: the warp's first
   // feature; row: the first token.  The map's pieces are 32 tokens long with `both`, else 16.
@@ -1167,14 +1173,10 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
             if (both) {
               tile_out.post(p, lane, x, m0 + c, N);
             } else {                              // the map's pieces are 16 tokens; the tile may end after the first
-              fence_smem_to_tma();
-              __syncwarp();
-              if (lane == 0 && x < N) {
+              tile_out.post(lane, x < N, [&] {
                 tma_store_2d(&map_y, p, x, m0 + c);
                 if (c + 16 < bn) tma_store_2d(&map_y, p + 16 * GATED_FEATURES * 2, x, m0 + c + 16);
-                tma_store_commit();
-              }
-              ++tile_out.sent;
+              });
             }
           } else if (n < N) {
             const int end = min(m_end, m0 + bn);
