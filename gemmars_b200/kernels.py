@@ -1953,11 +1953,16 @@ def delta_rule(q, k, v, beta_logit, a_logit, a_log, dt_bias, state, cu_seqlens, 
            "delta_rule", "attention", _nbytes(y) * 2 + 2 * seq_slot.numel() * heads * dim * vdim * 4)
 
 
-def delta_step_usable(ntok: int, nseq: int, heads: int, groups: int, dim: int, vdim: int, taps: int) -> bool:
+def delta_step_usable(ntok: int, nseq: int, heads: int, groups: int, dim: int, vdim: int, taps: int, row: int = 0) -> bool:
     """Whether a gated delta layer's step runs as ``delta_step``: one token a sequence, and a q/k head's value heads in
     blocks of 32 columns that fill at most a cluster of eight.  At most a block an SM: one sequence of 16 heads of 128 took
-    24.4 us in kernels of their own and 21.9 so, but a drawn step of about 41 us, 56 where this kernel ran without the line."""
-    return ntok == nseq and nseq * heads * (vdim // 32) <= 148 and dim <= 128 and vdim in (64, 128) and heads // groups * (vdim // 32) <= 8 and 2 <= taps <= 8
+    24.4 us in kernels of their own and 21.9 so, but a drawn step of about 41 us, 56 where this kernel ran without the line.
+    ``row``: floats from one row of the projection to the next (0: rows at 16-byte boundaries).  The kernel sums a head's
+    squares as the norm does for rows and gates at 16-byte boundaries; the norm of other rows has another order, and a
+    token's bits must not depend on how many sequences its step has."""
+    gate = 2 * groups * dim + heads * vdim
+    return (ntok == nseq and nseq * heads * (vdim // 32) <= 148 and dim <= 128 and vdim in (64, 128) and heads // groups * (vdim // 32) <= 8
+            and 2 <= taps <= 8 and row % 4 == 0 and gate % 4 == 0)
 
 
 def delta_step(proj, taps, filter_state, a_log, dt_bias, state, seq_slot, norm_w, out, heads, groups, dim, vdim, q_scale, eps, out_scale):
@@ -1966,7 +1971,8 @@ def delta_step(proj, taps, filter_state, a_log, dt_bias, state, seq_slot, norm_w
     _cuda(proj, taps, filter_state, a_log, dt_bias, state, seq_slot, norm_w, out)
     c, k = taps.shape
     t, hv = proj.shape[0], heads * vdim
-    assert delta_step_usable(t, seq_slot.numel(), heads, groups, dim, vdim, k) and c == 2 * groups * dim + hv
+    assert delta_step_usable(t, seq_slot.numel(), heads, groups, dim, vdim, k, proj.stride(0)) and c == 2 * groups * dim + hv
+    assert proj.data_ptr() % 16 == 0 and out.data_ptr() % 16 == 0
     assert proj.dtype == torch.float32 and proj.stride(1) == 1 and proj.shape[1] >= c + hv + 2 * heads
     assert taps.dtype == torch.float32 and taps.is_contiguous() and norm_w.dtype == torch.float32 and norm_w.numel() == vdim
     assert filter_state.dtype == torch.float32 and filter_state.is_contiguous() and tuple(filter_state.shape[1:]) == (k - 1, c)

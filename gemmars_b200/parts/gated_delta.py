@@ -79,7 +79,7 @@ class GatedDeltaRule(Part):
         p = self.proj(h, out_dtype=torch.float32)
         t = p.shape[0]
         out = torch.empty((t, hv), dtype=self.act_dtype, device=p.device)
-        if kernels.delta_step_usable(t, ctx.seq_slot.numel(), nh, self.kv_heads, self.dim, self.vdim, self.taps):
+        if kernels.delta_step_usable(t, ctx.seq_slot.numel(), nh, self.kv_heads, self.dim, self.vdim, self.taps, p.stride(0)):
             kernels.delta_step(p, self.filter, filter_state, self.a_log, self.dt_bias, state, ctx.seq_slot, self.norm, out, nh,
                                self.kv_heads, self.dim, self.vdim, float(self.dim) ** -0.5, self.eps, self.out_scale)
             self.o.add_into(out, residual)

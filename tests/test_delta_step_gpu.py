@@ -47,3 +47,54 @@ def test_what_is_refused_runs_as_before():
     assert not k.delta_step_usable(4, 4, 4, 2, 256, 128, 4)
     assert not k.delta_step_usable(4, 4, 4, 2, 128, 96, 4)
     assert not k.delta_step_usable(4, 4, 4, 2, 128, 128, 1)
+
+
+def _layer(heads, groups, dim, vdim, hidden=64, conv=4):
+    from gemmars_b200.csrc import build
+    from gemmars_b200.parts.base import build_part
+    from gemmars_b200.parts.plan import PartSpec
+    part = build_part("mixer", PartSpec("gated_delta", {"hidden_size": hidden, "heads": heads, "kv_heads": groups, "dim": dim, "vdim": vdim,
+                                                        "conv": conv, "norm_eps": 1e-6}), "float32")
+    build.ensure(part.kernel_units())
+    g = torch.Generator(device="cuda").manual_seed(heads * dim)
+    part.load({n: torch.randn(w.shape, generator=g, device="cuda") * (w.shape[-1] ** -0.5 if len(w.shape) == 2 else 0.5)
+               for n, w in part.wants().items()})
+    return part
+
+
+@pytest.mark.parametrize("heads,groups,dim,vdim", [(3, 3, 128, 64), (1, 1, 33, 64), (5, 5, 64, 128), (4, 2, 128, 128)])
+def test_a_token_alone_has_the_bits_of_the_same_token_among_many(heads, groups, dim, vdim):
+    """Rows of a layer's own width, which are at 16-byte boundaries or not: one sequence may take the one kernel, many do not."""
+    from gemmars_b200.cache.pool import SequenceCache
+    from gemmars_b200.parts.base import StepContext
+    part = _layer(heads, groups, dim, vdim)
+    many = 150
+    g = torch.Generator(device="cuda").manual_seed(7)
+    h = torch.randn(many, 64, generator=g, device="cuda")
+    past = [torch.randn(s.shape, generator=g, device="cuda") for s in part.cache_needs()]
+    ints = lambda v: torch.tensor(list(v), dtype=torch.int32, device="cuda")       # noqa: E731
+    rows, states = [], []
+    for n in (1, many):
+        cache = SequenceCache([(0, part.cache_needs())], 64 * many, n, 0, 64, torch.float32, torch.device("cuda"))
+        for _ in range(n):
+            cache.extend(cache.open(), 1)
+        cache.sync()
+        caches = cache.views(0)
+        for c, p in zip(caches, past):
+            c[:n] = p
+        ctx = StepContext(compute="float32", act_dtype=torch.float32, device=torch.device("cuda"), n_tokens=n, n_seqs=n, tok_pos=ints([0] * n),
+                          tok_seq=ints(range(n)), seq_slot=ints(range(n)), seq_start=ints([0] * n), seq_len=ints([1] * n),
+                          cu_seqlens=ints(range(n + 1)), is_decode=True, max_new=1, max_total=1, cache=cache, page_size=64, host=None)
+        out = torch.zeros(n, 64, device="cuda")
+        part.forward(ctx, h[:n], out, caches)
+        rows.append(out[0])
+        states.append([c[0].clone() for c in caches])
+    assert torch.equal(*rows)
+    assert all(torch.equal(a, b) for a, b in zip(*states))
+
+
+def test_rows_that_the_norm_sums_in_another_order_are_refused():
+    from gemmars_b200 import kernels as k
+    assert k.delta_step_usable(1, 1, 4, 2, 128, 128, 4, 2 * 256 + 2 * 512 + 8)
+    assert not k.delta_step_usable(1, 1, 3, 3, 128, 64, 4, 2 * 384 + 2 * 192 + 6)        # rows
+    assert not k.delta_step_usable(1, 1, 1, 1, 33, 64, 4, 2 * 33 + 2 * 64 + 2)           # the gate's place in them
