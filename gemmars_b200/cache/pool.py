@@ -24,6 +24,8 @@ from typing import Dict, List, Optional, Sequence, Tuple
 import numpy as np
 import torch
 
+from .. import kernels
+
 PAGE_SIZE = 64
 
 
@@ -185,11 +187,14 @@ class KVGroup:
     def table_rows(self, rows: np.ndarray) -> np.ndarray:
         return self._table[rows]
 
-    def put_rows(self, rows: np.ndarray, values: torch.Tensor) -> None:
+    def put_rows(self, rows: np.ndarray, values: torch.Tensor, at: Optional[torch.Tensor] = None) -> None:
         """Puts ``rows`` of the page table in their places from ``values`` [rows, width] (``table_rows``), which a step's
-        index block has brought to the device."""
-        for i, r in enumerate(rows.tolist()):
-            self.page_table[r].copy_(values[i])
+        index block has brought to the device, and with them their numbers ``at`` (int32; None: a copy a row)."""
+        if at is None:
+            for i, r in enumerate(rows.tolist()):
+                self.page_table[r].copy_(values[i])
+        elif len(rows):
+            kernels.put_rows(values, at, self.page_table)
         self._dirty.difference_update(rows.tolist())
 
     def sync(self) -> None:

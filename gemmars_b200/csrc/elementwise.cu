@@ -62,6 +62,23 @@ GB_EXPORT int gb_embed_gather(const void* table, int table_dtype, const int* tok
   return gb_launch_status();
 }
 
+// ------------------------------------------------------------------ page table rows
+// table[rows[r], :] = values[r, :], a block a row: all rows of a group that changed in one launch (a copy a row takes the
+// host some 12 us each).
+__global__ void put_rows_kernel(const int* __restrict__ values, const int* __restrict__ rows, int* __restrict__ table, int width) {
+  pdl_release_next();
+  pdl_wait_prior();
+  int* to = table + (size_t)rows[blockIdx.x] * width;
+  const int* from = values + (size_t)blockIdx.x * width;
+  for (int i = threadIdx.x; i < width; i += blockDim.x) to[i] = from[i];
+}
+
+GB_EXPORT int gb_put_rows(const int* values, const int* rows, int* table, int n, int width, cudaStream_t stream) {
+  if (n <= 0 || width <= 0) return 0;
+  gb_launch(put_rows_kernel, dim3(n), dim3(128), 0, stream, values, rows, table, width);
+  return gb_launch_status();
+}
+
 // ------------------------------------------------------------------ RMSNorm
 // out[r, :] = x[src(r), :] * (mean(x^2) + eps)^-1/2 * w, statistics in float32.
 // rows_index (optional) gathers: src(r) = rows_index[r].

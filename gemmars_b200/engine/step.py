@@ -202,18 +202,20 @@ class Runner:
         tok_seq = np.repeat(np.arange(b), lens)
         tok_pos = np.arange(t) - cu[tok_seq] + starts[tok_seq]
         tokens = np.concatenate([toks[i][off:off + n] for i, off, n in part])
-        # Page table rows that changed go out with the step's index block and are put in their places on the device: a copy
-        # of their own out of pageable memory returns only when all steps before have run, so that the device stood idle
-        # while the host prepared a prompt's launches (110 us of 1,880 for 2,048 tokens through two layers of 8B sizes, of
-        # 1,550 for 301 float32 tokens).  Each row is a copy on the device, so many rows take that one copy all the same.
+        # Page table rows that changed go out with the step's index block and are put in their places on the device, a launch a
+        # group: a copy of their own out of pageable memory returns only when all steps before have run, so that the device
+        # stood idle while the host prepared a prompt's launches (110 us of 1,880 for 2,048 tokens through two layers of 8B
+        # sizes, of 1,550 for 301 float32 tokens).  A step of two layers, own copy / so, us: of 8B sizes, 2,048 tokens, 4 rows of 40
+        # 1,700 / 1,550, 64 of 160 1,840 / 1,700; of 1,024 wide, 256 tokens, where the host's time is the step's, 4 rows of 12
+        # 545 / 516, 16 of 36 590 / 604, 64 of 132 908 / 936.
         changed = []
         n_rows, n_numbers = cache.changed()
-        if n_rows <= 16 and n_numbers <= self.max_step_tokens:
+        if n_rows + n_numbers <= self.max_step_tokens:
             changed = [(g, g.changed_rows()) for g in cache.kv_groups]
         else:
             cache.sync()
         block = np.concatenate([tokens, tok_pos, tok_seq, slots, starts, lens, cu, np.asarray(rows, dtype=np.int64)]
-                               + [g.table_rows(r).reshape(-1) for g, r in changed]).astype(np.int32)
+                               + [v for g, r in changed for v in (r, g.table_rows(r).reshape(-1))], dtype=np.int32, casting="same_kind")
         dev = self._ring.stage(block, self.device)
         o = 0
 
@@ -226,7 +228,8 @@ class Runner:
         d_tokens, d_pos, d_seq = take(t), take(t), take(t)
         d_slot, d_start, d_len, d_cu, d_rows = take(b), take(b), take(b), take(b + 1), take(len(rows))
         for g, r in changed:
-            g.put_rows(r, take(len(r) * g.table_width).view(len(r), g.table_width))
+            at = take(len(r))
+            g.put_rows(r, take(len(r) * g.table_width).view(len(r), g.table_width), at)
         ctx = StepContext(
             compute=self.model.compute, act_dtype=self.model.act_dtype, device=self.device, n_tokens=t, n_seqs=b,
             tok_pos=d_pos, tok_seq=d_seq, seq_slot=d_slot, seq_start=d_start, seq_len=d_len, cu_seqlens=d_cu,

@@ -234,6 +234,16 @@ def head_norm_rope_cache(qkv, nh, nkv, hd, rot, q_weight, k_weight, eps, inv_fre
         count_launches(1)   # prompts: the values go through a second, transposing kernel
 
 
+def put_rows(values: torch.Tensor, rows: torch.Tensor, table: torch.Tensor):
+    """table[rows[r]] = values[r]: int32, ``values`` [R, width], ``rows`` [R] (each named once and a row of ``table``)."""
+    _cuda(values, rows, table)
+    assert values.dtype == rows.dtype == table.dtype == torch.int32 and values.shape == (rows.numel(), table.shape[1])
+    assert values.is_contiguous() and rows.is_contiguous() and table.is_contiguous()
+    f = _fn("elementwise", "gb_put_rows", [c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p])
+    _check(f(values.data_ptr(), rows.data_ptr(), table.data_ptr(), rows.numel(), table.shape[1], _stream()), "put_rows",
+           "elementwise", 2 * _nbytes(values))
+
+
 def silu_mul(gu: torch.Tensor, out: torch.Tensor):
     """out[t, i] = silu(gu[t, i]) * gu[t, I + i]."""
     _cuda(gu, out)
