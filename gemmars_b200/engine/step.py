@@ -37,6 +37,12 @@ class StepItem:
     want: Sequence[int] = ()      # places among ``tokens`` whose logits are asked for
 
 
+def index_block_numbers(max_step_tokens: int, n_slots: int) -> int:
+    """The most numbers that a step's index block holds: a token's id, position and sequence, its row if it is wanted, five
+    of every sequence, and page table rows (``Runner._run`` sends at most as many numbers as a step has tokens)."""
+    return 5 * max_step_tokens + 5 * n_slots + 1
+
+
 class _PinnedRing:
     """A few pinned host buffers used in turn for the step's index block; a buffer is written
     again only after the copy that last read it has finished.  They are allocated once, for the
@@ -81,7 +87,7 @@ class Runner:
         self._pool = None
         self._length_matters = model.capture_depends_on_length
         self._broken = set()      # slots a failed step left in a state that cannot be restored
-        self._ring = _PinnedRing(4 * self.max_step_tokens + 8 * self.cache.n_slots + 64) if self.device.type == "cuda" else None
+        self._ring = _PinnedRing(index_block_numbers(self.max_step_tokens, self.cache.n_slots)) if self.device.type == "cuda" else None
         self.steps_run = 0
         self.tokens_run = 0
 

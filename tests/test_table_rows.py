@@ -76,3 +76,23 @@ def test_a_prompt_step_sends_its_rows_with_its_index_block(model_folders, monkey
     for i in (0, 23):
         want = np.asarray(plain.forward(pcfg, w, prompts[i]))[-1]
         assert np.abs(out[i].double().cpu().numpy() - want).max() <= 1e-4 * np.abs(want).max()
+
+
+@pytest.mark.gpu
+def test_the_largest_step_pins_no_new_memory(model_folders):
+    """As many tokens as a step takes, every one's logits wanted, and page table rows beside them."""
+    from tiny_configs import TINY_C
+
+    from gemmars_b200 import Engine
+    from gemmars_b200.engine.step import Runner, StepItem
+    model = Engine.load(model_folders(TINY_C), "dtype=float32;max_batch=8;max_tokens=512").runner.model
+    runner = Runner(model, 8192, max_batch=8, prefill_chunk=256, max_step_tokens=256)
+    pinned = [b.data_ptr() for b in runner._ring.bufs]
+    rng = np.random.default_rng(1)
+    for lens in ((200, 56), (32,) * 8, (256,)):
+        slots = [runner.open() for _ in lens]
+        assert sum(runner.cache.changed()) <= runner.max_step_tokens
+        runner.step([StepItem(s, rng.integers(0, 301, n).tolist(), list(range(n))) for s, n in zip(slots, lens)])
+        for s in slots:
+            runner.close(s)
+    assert [b.data_ptr() for b in runner._ring.bufs] == pinned
