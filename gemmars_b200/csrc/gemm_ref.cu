@@ -213,6 +213,116 @@ __global__ void __launch_bounds__(32 * PARTS)
   }
 }
 
+// The same sums for short inner dimensions and many results, where the four warps' parts are a block or two and their meeting
+// most of the time: a CTA of 128 threads works 64 rows by 64 with whole sums, 4 x 8 results a thread, and adds up a part's even
+// and odd sums when the part ends: the same bits.  What bounds it: the results' way to memory and, from 64 inner elements on, the
+// 16-byte reads.  See short_pays.
+struct F32Short {
+  static constexpr int BM = 64, BN = 64, TM = 4, TN = 8, KB = 16, STAGES = 4, LD = KB + 4, MAX_K = 192;
+  static constexpr int STAGE_FLOATS = (BM + BN) * LD;
+};
+static_assert(F32Short::STAGES * F32Short::STAGE_FLOATS * sizeof(float) <= 48 * 1024, "static shared memory");
+
+template <bool VEC, int MODE>
+__global__ void __launch_bounds__(128)
+    gemm_f32_short_kernel(const float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ bias, float* __restrict__ y,
+                          int M, int N, int K, long long ldx, long long ldy, int act, const float* __restrict__ col_scale, int tiles_m) {
+  using T = F32Short;
+  constexpr int BM = T::BM, BN = T::BN, TM = T::TM, TN = T::TN, KB = T::KB, STAGES = T::STAGES, LD = T::LD, CH = KB / 4;
+  __shared__ __align__(16) float smem[STAGES * T::STAGE_FLOATS];
+  pdl_release_next();
+  const int tid = threadIdx.x, ty = tid >> 3, tx = tid & 7;
+  const int m0 = blockIdx.x % tiles_m * BM, n0 = blockIdx.x / tiles_m * BN;
+  const int blocks = (K + KB - 1) / KB, length = part_length(K);
+  auto bring = [&](int block, const float* base, long long ld, int row0, int rows_have, float* dst) {
+    static_assert(BM == BN, "as many rows of both");
+#pragma unroll
+    for (int i = 0; i < BM * CH / 128; ++i) {
+      const int r = (tid + 128 * i) / CH, c = tid % CH * 4, k = block * KB + c;
+      float* d = dst + r * LD + c;
+      const bool row_in = row0 + r < rows_have;
+      const float* src = base + (size_t)(row_in ? row0 + r : 0) * ld;
+      if (VEC) {
+        const bool in = row_in && k < K;
+        copy16(d, in ? src + k : base, in ? 16 : 0);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const bool in = row_in && k + j < K;
+          copy4(d + j, in ? src + k + j : base, in ? 4 : 0);
+        }
+      }
+    }
+  };
+#pragma unroll
+  for (int s = 0; s < STAGES - 1; ++s)
+    if (s < blocks) bring(s, w, K, n0, N, smem + s * T::STAGE_FLOATS + BM * LD);
+  pdl_wait_prior();
+#pragma unroll
+  for (int s = 0; s < STAGES - 1; ++s) {
+    if (s < blocks) bring(s, x, ldx, m0, M, smem + s * T::STAGE_FLOATS);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  uint64_t acc[TM][TN] = {};
+  float sum[TM][TN];
+#pragma unroll 1
+  for (int b = 0; b < blocks; ++b) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
+    __syncthreads();                       // block b is there for all, and block b - 1 has been read by all
+    if (b + STAGES - 1 < blocks) {
+      float* to = smem + (b + STAGES - 1) % STAGES * T::STAGE_FLOATS;
+      bring(b + STAGES - 1, x, ldx, m0, M, to);
+      bring(b + STAGES - 1, w, K, n0, N, to + BM * LD);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    const float *xs = smem + b % STAGES * T::STAGE_FLOATS + ty * LD, *ws = smem + b % STAGES * T::STAGE_FLOATS + (BM + tx) * LD;
+#pragma unroll
+    for (int kk = 0; kk < KB; kk += 4) {
+      ulonglong2 a[TM];
+#pragma unroll
+      for (int i = 0; i < TM; ++i) a[i] = *(const ulonglong2*)(xs + i * 16 * LD + kk);
+#pragma unroll
+      for (int j = 0; j < TN; ++j) {
+        const ulonglong2 v = *(const ulonglong2*)(ws + j * 8 * LD + kk);
+#pragma unroll
+        for (int i = 0; i < TM; ++i) fma2(acc[i][j], a[i].x, v.x);
+#pragma unroll
+        for (int i = 0; i < TM; ++i) fma2(acc[i][j], a[i].y, v.y);
+      }
+    }
+    const int end = (b + 1) * KB;
+    if (end % length == 0 || b + 1 == blocks) {          // a part ends
+#pragma unroll
+      for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int j = 0; j < TN; ++j) {
+          const float part = even_and_odd(acc[i][j]);
+          sum[i][j] = end <= length ? part : sum[i][j] + part;
+          acc[i][j] = 0;
+        }
+    }
+  }
+  const bool fewer = (PARTS - 1) * length >= K;           // parts without an element, which are added as zeros
+#pragma unroll
+  for (int i = 0; i < TM; ++i) {
+    const int gm = m0 + i * 16 + ty;
+    if (gm >= M) continue;
+#pragma unroll
+    for (int j = 0; j < TN; ++j) {
+      const int gn = n0 + j * 8 + tx;
+      if (gn >= N) continue;
+      float v = sum[i][j];
+      if (fewer) v += 0.f;
+      if (bias) v += bias[gn];
+      if (act == ACT_GELU) v = 0.5f * v * (1.0f + erff(v * 0.70710678118654752f));
+      else if (act == ACT_RELU2) v = fmaxf(v, 0.f) * fmaxf(v, 0.f);
+      if (col_scale) v *= col_scale[gn];
+      float* dst = y + (size_t)gm * ldy + gn;
+      *dst = MODE == OUT_ACCUMULATE_F32 ? *dst + v : v;
+    }
+  }
+}
+
 struct F32Call {
   const float *x, *w, *bias;
   float* y;
@@ -222,10 +332,14 @@ struct F32Call {
   const float* col_scale;
 };
 
+static bool f32_vec(const F32Call& c) {
+  return c.K % 4 == 0 && c.ldx % 4 == 0 && (((uintptr_t)c.x | (uintptr_t)c.w) & 15) == 0;
+}
+
 template <int TM, int TN, int KB, int STAGES>
 static int launch_f32_tile(const F32Call& c, int mode, cudaStream_t stream) {
   using T = F32Tile<TM, TN, KB, STAGES>;
-  const bool vec = c.K % 4 == 0 && c.ldx % 4 == 0 && (((uintptr_t)c.x | (uintptr_t)c.w) & 15) == 0;
+  const bool vec = f32_vec(c);
   const int tiles_m = (c.M + T::BM - 1) / T::BM;
   const long long tiles = (long long)tiles_m * ((c.N + T::BN - 1) / T::BN);
   if (tiles > 0x7fffffffLL) return GB_ERR_SIZE;
@@ -244,6 +358,24 @@ static int launch_f32_tile(const F32Call& c, int mode, cudaStream_t stream) {
     else LAUNCH_F32(false, OUT_STORE);
   }
 #undef LAUNCH_F32
+  return gb_launch_status();
+}
+
+static int launch_f32_short(const F32Call& c, int mode, cudaStream_t stream) {
+  const int tiles_m = (c.M + F32Short::BM - 1) / F32Short::BM;
+  const long long tiles = (long long)tiles_m * ((c.N + F32Short::BN - 1) / F32Short::BN);
+  if (tiles > 0x7fffffffLL) return GB_ERR_SIZE;
+#define LAUNCH_SHORT(VEC, MODE)                                                                                                \
+  gb_launch(gemm_f32_short_kernel<VEC, MODE>, dim3((unsigned)tiles), 128, 0, stream, c.x, c.w, c.bias, c.y, c.M, c.N, c.K, c.ldx, \
+            c.ldy, c.act, c.col_scale, tiles_m)
+  if (mode == OUT_ACCUMULATE_F32) {
+    if (f32_vec(c)) LAUNCH_SHORT(true, OUT_ACCUMULATE_F32);
+    else LAUNCH_SHORT(false, OUT_ACCUMULATE_F32);
+  } else {
+    if (f32_vec(c)) LAUNCH_SHORT(true, OUT_STORE);
+    else LAUNCH_SHORT(false, OUT_STORE);
+  }
+#undef LAUNCH_SHORT
   return gb_launch_status();
 }
 
@@ -285,7 +417,17 @@ static int launch_f32(int tile, const F32Call& c, int mode, cudaStream_t stream)
   }
 }
 
-// Which of F32_TILES a float32 product of these sizes takes.
+// Whether gemm_f32_short_kernel is the faster of the two.  us, four parts / whole sums: 2,048 x 4,096 by K of 16 60.3 / 21.6, 64 71.7 /
+// 41.2, 96 73.8 / 55.6, 128 78.5 / 69.3, 160 106 / 84, 192 110 / 98, 224 111 / 113; 2,048 x 1,024 by 16 18.0 / 9.4, 96 21.9 / 18.9, 128
+// 22.5 / 23.4, 160 30.9 / 27.3, 192 32.0 / 31.8; 301 x 4,096 by 64 14.0 / 11.5, 96 14.4 / 14.8, 160 20.1 / 21.3; 1,024 x 1,024 by 64 9.8 / 9.0,
+// 96 10.8 / 11.7; 301 x 2,048 by 16 6.4 / 5.5, 32 6.5 / 6.3, 64 7.4 / 9.0; 64 x 4,096 by 16 4.3 / 5.0.
+static bool short_pays(int M, int N, int K) {
+  const long long results = (long long)M * N;
+  return K <= F32Short::MAX_K && results >= (K <= 32 ? 1 << 19 : K <= 64 ? 1 << 20 : K <= 96 || K > 128 ? 1 << 21 : 1 << 22);
+}
+GB_EXPORT int gb_gemm_ref_short(int M, int N, int K) { return short_pays(M, N, K) ? 1 : 0; }
+
+// Which of F32_TILES a float32 product of these sizes takes where four warps share a tile.
 GB_EXPORT int gb_gemm_ref_tile(int M, int N) { return pick_f32_tile(M, N); }
 
 // x: [M, K] rows ldx apart; w: [N, K]; y: [M, N] rows ldy apart.
@@ -305,7 +447,7 @@ GB_EXPORT int gb_gemm_ref(const void* x, const void* w, int in_dtype, const floa
   if (in_dtype == GB_F32) {
     if (out_dtype != GB_F32) return GB_ERR_DTYPE;
     const F32Call call{(const float*)x, (const float*)w, bias, (float*)y, M, N, K, ldx, ldy, act, col_scale};
-    return launch_f32(pick_f32_tile(M, N), call, mode, stream);
+    return short_pays(M, N, K) ? launch_f32_short(call, mode, stream) : launch_f32(pick_f32_tile(M, N), call, mode, stream);
   } else if (in_dtype == GB_BF16) {
     if (mode == OUT_ACCUMULATE_F32) LAUNCH(bf16, float, OUT_ACCUMULATE_F32);
     else if (out_dtype == GB_F32) LAUNCH(bf16, float, OUT_STORE);
