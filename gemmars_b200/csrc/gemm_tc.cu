@@ -1396,14 +1396,17 @@ int launch_mode(int mode, const CUtensorMap& mw, const CUtensorMap& mx, const Ou
 // tokens and has six stages where one CTA has four: a block of 64 inner elements by 256 tokens in 275 to 285 ns where one
 // CTA takes 304 to 320.  It starts and ends with a barrier of the cluster, some 0.8 us a launch, and its tiles are twice as
 // large.  So: not where that makes more rounds of tiles than the faster block gives back, and where there is one round only
-// from 4,096 inner elements on.  Measured (us, one CTA / pairs; 148 SMs): 12,352 x 4,096 by 2,048 tokens 177.8 / 145.4,
-// 4,096 x 4,096 by 2,048 53.8 / 49.7, 3,136 x 1,024 by 1,300 (two rounds) 17.1 / 16.3, 4,096 x 4,096 by 1,000 (one) 27.7 /
-// 26.9; 2,048 x 2,048 by 2,048 (one) 16.2 / 17.2, 4,672 x 2,048 by 2,048 (two rounds against three) 30.6 / 35.9.
+// above 4,096 inner elements.  Measured (us, one CTA / pairs; 148 SMs): 12,352 x 4,096 by 2,048 tokens 177.8 / 145.4,
+// 4,096 x 4,096 by 2,048 53.8 / 49.7, 3,136 x 1,024 by 1,300 (two rounds) 17.1 / 16.3; 4,672 x 2,048 by 2,048 (two rounds
+// against three) 30.6 / 35.9.  One round, by 2,048 / 3,072 / 4,096 / 6,144 inner elements: 2,048 features by 2,048 tokens 16.7,
+// 21.8, 26.9, 38.5 / 17.5, 22.3, 27.5, 38.4, 4,096 by 1,000 17.9, 22.0, 27.8, 39.6 / 19.3, 22.9, 28.0, 39.6, 4,096 by 700 16.4,
+// 21.7, 26.9, 37.1 / 17.4, 22.5, 27.0, 36.0; adding into the result, 4,096 and 6,144: 27.3, 41.4 / 28.3, 42.4, 28.3, 41.6 / 28.9, 40.8
+// and 29.8, 37.6 / 30.1, 36.7.
 bool pairs_pay(int M, int N, int K, int bn, int ctas, int tile_features) {
   if (bn <= 128 || ctas < 2) return false;
   const long long tiles_m = (M + bn - 1) / bn, tiles_n = (N + tile_features - 1) / tile_features;
   const long long rounds = (tiles_m * tiles_n + ctas - 1) / ctas, pair_rounds = (tiles_m * ((tiles_n + 1) / 2) + ctas / 2 - 1) / (ctas / 2);
-  return 0.92 * pair_rounds < rounds && (rounds > 1 || K >= 4096);
+  return 0.92 * pair_rounds < rounds && (rounds > 1 || K > 4096);
 }
 
 template <int BN, int STAGES, int MODE, bool PAIR = false>

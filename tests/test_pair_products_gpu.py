@@ -163,3 +163,10 @@ def test_a_batch_of_products(k, monkeypatch, sms, groups, t, n, kk):
         want, bound = exact_and_bound(x[g * t:(g + 1) * t], w[g * n:(g + 1) * n])
         assert ((out[g].double() - want).abs() <= bound + 2.0 ** -22 * want.abs()).all()
     assert k.gemm_tc_status() == 0
+
+
+def test_one_round_of_tiles_takes_pairs_where_they_are_the_faster(k):
+    """Both sides measured: up to 4,096 inner elements a single round is the faster with one CTA a tile."""
+    for m, n, kk, paired in ((2048, 2048, 4096, 0), (1000, 4096, 4096, 0), (700, 4096, 6144, 1), (2048, 2048, 6144, 1), (2048, 4096, 4096, 1),
+                             (2048, 4672, 2048, 0)):
+        assert pairs(k, m, n, kk, 256, 148) == paired
