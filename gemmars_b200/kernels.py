@@ -1963,16 +1963,21 @@ def delta_rule(q, k, v, beta_logit, a_logit, a_log, dt_bias, state, cu_seqlens, 
            "delta_rule", "attention", _nbytes(y) * 2 + 2 * seq_slot.numel() * heads * dim * vdim * 4)
 
 
-def delta_step_usable(ntok: int, nseq: int, heads: int, groups: int, dim: int, vdim: int, taps: int, row: int = 0) -> bool:
+def delta_step_usable(ntok: int, nseq: int, heads: int, groups: int, dim: int, vdim: int, taps: int, row: int = 0,
+                      sms: Optional[int] = None) -> bool:
     """Whether a gated delta layer's step runs as ``delta_step``: one token a sequence, and a q/k head's value heads in
-    blocks of 32 columns that fill at most a cluster of eight.  At most a block an SM: one sequence of 16 heads of 128 took
-    24.4 us in kernels of their own and 21.9 so, but a drawn step of about 41 us, 56 where this kernel ran without the line.
+    blocks of 32 columns that fill at most a cluster of eight.  At most as many blocks as there is room for at once (a thread has
+    168 registers, so three blocks of the 128 threads that heads of 65 to 128 dims take lie on an SM, six of 64): the blocks of a
+    cluster wait for one another, and a second round of them costs more than two kernels' boundaries.  us, filter, recurrence and
+    norm apart / in one: heads of 128 x 128, 64 blocks 7.0 / 5.7, 256 8.1 / 6.9, 384 9.3 / 7.0, 512 9.4 / 12.1, 2,048 17.8 / 31.5; of
+    64 x 64, 768 blocks 8.7 / 6.8, 1,024 8.9 / 11.6; of 32 x 64, 768 8.2 / 5.7, 1,536 8.6 / 10.4.  A layer's step, 16 heads, one
+    sequence 20.6 / 18.5, five 22.6 / 21.9, eight 23.2 / 26.7; 32 heads, three 43.3 / 40.9, four 44.7 / 46.0.
     ``row``: floats from one row of the projection to the next (0: rows at 16-byte boundaries).  The kernel sums a head's
     squares as the norm does for rows and gates at 16-byte boundaries; the norm of other rows has another order, and a
     token's bits must not depend on how many sequences its step has."""
     gate = 2 * groups * dim + heads * vdim
-    return (ntok == nseq and nseq * heads * (vdim // 32) <= 148 and dim <= 128 and vdim in (64, 128) and heads // groups * (vdim // 32) <= 8
-            and 2 <= taps <= 8 and row % 4 == 0 and gate % 4 == 0)
+    return (ntok == nseq and dim <= 128 and vdim in (64, 128) and nseq * heads * (vdim // 32) <= (3 if dim > 64 else 6) * (sms or sm_count())
+            and heads // groups * (vdim // 32) <= 8 and 2 <= taps <= 8 and row % 4 == 0 and gate % 4 == 0)
 
 
 def delta_step(proj, taps, filter_state, a_log, dt_bias, state, seq_slot, norm_w, out, heads, groups, dim, vdim, q_scale, eps, out_scale):
@@ -1985,6 +1990,7 @@ def delta_step(proj, taps, filter_state, a_log, dt_bias, state, seq_slot, norm_w
     assert proj.data_ptr() % 16 == 0 and out.data_ptr() % 16 == 0
     assert proj.dtype == torch.float32 and proj.stride(1) == 1 and proj.shape[1] >= c + hv + 2 * heads
     assert taps.dtype == torch.float32 and taps.is_contiguous() and norm_w.dtype == torch.float32 and norm_w.numel() == vdim
+    assert a_log.dtype == dt_bias.dtype == torch.float32 and a_log.numel() == dt_bias.numel() == heads
     assert filter_state.dtype == torch.float32 and filter_state.is_contiguous() and tuple(filter_state.shape[1:]) == (k - 1, c)
     assert state.dtype == torch.float32 and state.is_contiguous() and tuple(state.shape[1:]) == (heads, recurrent_state_floats(dim, vdim))
     assert out.is_contiguous() and out.shape == (t, hv)

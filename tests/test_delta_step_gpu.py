@@ -98,3 +98,47 @@ def test_rows_that_the_norm_sums_in_another_order_are_refused():
     assert k.delta_step_usable(1, 1, 4, 2, 128, 128, 4, 2 * 256 + 2 * 512 + 8)
     assert not k.delta_step_usable(1, 1, 3, 3, 128, 64, 4, 2 * 384 + 2 * 192 + 6)        # rows
     assert not k.delta_step_usable(1, 1, 1, 1, 33, 64, 4, 2 * 33 + 2 * 64 + 2)           # the gate's place in them
+
+
+def _both(seqs, slots, heads, groups, dim, vdim, taps=4):
+    """Outputs and states of the three kernels and of the one, from the same past."""
+    from gemmars_b200 import kernels as k
+    g = torch.Generator(device="cuda").manual_seed(seqs)
+    r = lambda *s: torch.randn(s, generator=g, device="cuda")       # noqa: E731
+    qk, hv, n_slots = groups * dim, heads * vdim, max(slots) + 1
+    c, width = 2 * qk + hv, 2 * qk + 2 * hv + 2 * heads
+    proj, filt = r(seqs, width + -width % 4)[:, :width], r(c, taps)
+    a_log, dt_bias, norm = r(heads).abs().log(), r(heads), r(vdim)
+    fs, st = r(n_slots, taps - 1, c), r(n_slots, heads, k.recurrent_state_floats(dim, vdim))
+    slots = torch.tensor(slots, dtype=torch.int32, device="cuda")
+    cu = torch.arange(seqs + 1, dtype=torch.int32, device="cuda")
+    made = []
+    for one in (False, True):
+        f1, s1, out = fs.clone(), st.clone(), torch.empty(seqs, hv, device="cuda")
+        if one:
+            k.delta_step(proj, filt, f1, a_log, dt_bias, s1, slots, norm, out, heads, groups, dim, vdim, dim ** -0.5, 1e-6, 1.0)
+        else:
+            f, y = torch.empty(seqs, c, device="cuda"), torch.empty(seqs, hv, device="cuda")
+            k.short_filter(proj[:, :c], filt, None, f1, cu, cu[:-1], slots, f, act=True)
+            k.delta_rule(f[:, :qk], f[:, qk:2 * qk], f[:, 2 * qk:], proj[:, c + hv:c + hv + heads], proj[:, c + hv + heads:], a_log, dt_bias, s1,
+                         cu, slots, y, heads, groups, dim, vdim, dim ** -0.5)
+            k.gated_group_norm(y, proj[:, c:c + hv], norm, out, vdim, 1e-6, False)
+        made.append((out, f1, s1))
+    return made
+
+
+@pytest.mark.parametrize("heads,groups,dim,vdim,per_sm", [(8, 4, 128, 128, 3), (4, 4, 64, 64, 6), (16, 8, 32, 64, 6)])
+def test_as_many_blocks_as_there_is_room_for(heads, groups, dim, vdim, per_sm):
+    from gemmars_b200 import kernels as k
+    most = per_sm * k.sm_count() // (heads * vdim // 32)
+    assert k.delta_step_usable(most, most, heads, groups, dim, vdim, 4) and not k.delta_step_usable(most + 1, most + 1, heads, groups, dim, vdim, 4)
+    apart, one = _both(most, list(range(most)), heads, groups, dim, vdim)
+    assert all(torch.equal(a, b) for a, b in zip(apart, one))
+
+
+def test_rows_that_pad_a_captured_step_share_a_slot():
+    """Three rows on the spare slot: the others' outputs and states are what they are without them."""
+    apart, one = _both(7, [2, 0, 5, 1, 6, 6, 6], 4, 2, 128, 128)
+    for a, b in zip(apart, one):
+        rows = [0, 1, 2, 3] if a.shape[0] == 7 and a.dim() == 2 else [0, 1, 2, 5]
+        assert torch.equal(a[rows], b[rows])
