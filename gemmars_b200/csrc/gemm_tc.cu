@@ -870,6 +870,7 @@ constexpr int EIGHT_WARPS_THREADS = 320, QKV_STAGING_BYTES = 65 * 1024;   // pie
 // rows exist: the MMAs are as wide as those (a multiple of 16) and only those leave; what the others hold, which the
 // loads still bring, counts nothing.  `act` (bfloat16 results of a
 // product without a gate, grouped or not): an activation of every result (out_act), then the row's scale.
+constexpr int BATCH_GROUPS = 4;
 struct Grouped {
   const int* tile_expert = nullptr;
   const int* tile_rows = nullptr;
@@ -878,8 +879,10 @@ struct Grouped {
   float limit = 0.f, alpha = 0.f, shift = 0.f;
   int act = 0, scale_in = 0;
   // a batch of products of one size: group_rows rows of x and of the result each, one group after the other at any row, in
-  // group_tiles tiles of tokens (0: not a batch; then tile_expert, tile_rows are null)
+  // group_tiles tiles of tokens (0: not a batch; then tile_expert, tile_rows are null); a group's matrix has a map of its own,
+  // the first one's being map_w
   int group_tiles = 0, group_rows = 0;
+  CUtensorMap group_w[BATCH_GROUPS - 1] = {};
   int gate_rows_whole = 0;     // gated: map_w brings a tile's gate and up rows in one box (gated_map)
 };
 __device__ __forceinline__ void act_rows(uint32_t (&v)[16], float bias, int act, const float* row_scale, int row, int M) {
@@ -999,6 +1002,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
         tile_at(w.t, m0, n0, e, rows);
         if (e < 0) continue;
         const int w0 = n0 + rank * TILE_F + e * grp.rows_per_expert;     // the tile's first row of W
+        const CUtensorMap* w_map = MODE == EPI_STORE_F32 && grp.group_tiles && e > 0 ? &grp.group_w[e - 1] : &map_w;
         // a pair: rank 1 brings the second half of the MMA's tokens
         const int x0 = m0 + rank * ((rows < bn ? (rows + 31) & ~31 : bn) / 2);
         for (int kb = w.kb0; kb < w.kb1; ++kb, ++it) {
@@ -1016,7 +1020,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
           };
           if (rank == 0) mbar_expect_tx(&full_bar[s], stage_tx);
           if (!GATED) {
-            load(a, &map_w, w0);
+            load(a, w_map, w0);
           } else if (grp.gate_rows_whole) {      // one box: 8 gate rows, the same features' 8 up rows, and so on
             if (PAIR) tma_load_4d_pair(a, &map_w, kb * BK, w0 / 8, bar);
             else tma_load_4d(a, &map_w, kb * BK, w0 / 8, &full_bar[s]);
@@ -1691,16 +1695,16 @@ GB_EXPORT int gb_gemm_tc_grouped(const void* x, const void* w, void* y, int mode
   return launch_persistent<128, 6, EPI_STORE_F32>(mw, mx, my, nullptr, y, M, N, K, ldy, bn, ctas, stream, QkvTail{}, nullptr, grp);
 }
 
-// `groups` products of one size in one walk of tiles: x [groups, T, K] bfloat16 (contiguous), w [groups, N, K] bfloat16, y
-// [groups, T, N] float32.  One launch whose last round of tiles is one, not `groups` of them: four of 2,048 x 4,096 x 4,096
-// 196 -> 164 us, a wkv layer of 700 tokens at 2,048 wide 189 -> 151.  bn: tokens a tile, a multiple of 16 up to 256.
-GB_EXPORT int gb_gemm_tc_batch(const void* x, const void* w, void* y, int groups, int T, int N, int K, int bn, int ctas,
+// `groups` (up to 4) products of one size in one walk of tiles: x [groups, T, K] bfloat16 (contiguous), w[g] [N, K] bfloat16
+// (addresses on the host), y [groups, T, N] float32.  One launch whose last round of tiles is one, not `groups` of them: four of
+// 2,048 x 4,096 x 4,096 196 -> 164 us, a wkv layer of 700 tokens at 2,048 wide 189 -> 151.  bn: tokens a tile, a multiple of 16 up
+// to 256.
+GB_EXPORT int gb_gemm_tc_batch(const void* x, const void* const* w, void* y, int groups, int T, int N, int K, int bn, int ctas,
                                cudaStream_t stream) {
   if (groups <= 0 || T <= 0 || N <= 0) return 0;
-  if (K <= 0 || (K % 8) || ((uintptr_t)x & 15) || ((uintptr_t)w & 15) || ctas <= 0 || bn < 16 || bn > 256 || bn % 16) return GB_ERR_SIZE;
-  if ((long long)groups * (T + bn) > 0x7fffffffLL || (long long)groups * N > 0x7fffffffLL) return GB_ERR_SIZE;
+  if (groups > BATCH_GROUPS || K <= 0 || (K % 8) || ((uintptr_t)x & 15) || ctas <= 0 || bn < 16 || bn > 256 || bn % 16) return GB_ERR_SIZE;
+  if ((long long)groups * (T + bn) > 0x7fffffffLL) return GB_ERR_SIZE;
   Grouped grp;
-  grp.rows_per_expert = N;
   grp.group_tiles = (T + bn - 1) / bn;
   grp.group_rows = T;
   const bool pair = pairs_pay(groups * grp.group_tiles * bn, N, K, bn, ctas, BM);
@@ -1710,7 +1714,10 @@ GB_EXPORT int gb_gemm_tc_batch(const void* x, const void* w, void* y, int groups
   }
   const int M = groups * T;
   CUtensorMap mw, mx;
-  if (!tensor_map(&mw, w, (uint64_t)groups * N, (uint64_t)K, (uint64_t)K * 2, BM)) return GB_ERR_ARG;
+  for (int g = 0; g < groups; ++g) {
+    if ((uintptr_t)w[g] & 15) return GB_ERR_SIZE;
+    if (!tensor_map(g ? &grp.group_w[g - 1] : &mw, w[g], (uint64_t)N, (uint64_t)K, (uint64_t)K * 2, BM)) return GB_ERR_ARG;
+  }
   if (!tensor_map(&mx, x, (uint64_t)M, (uint64_t)K, (uint64_t)K * 2, (uint32_t)(pair ? bn / 2 : bn))) return GB_ERR_ARG;
   const OutMap my = out_map(y, EPI_STORE_F32, M, N, N, bn);
   if (pair) return launch_persistent<256, 6, EPI_STORE_F32, true>(mw, mx, my, nullptr, y, M, N, K, N, bn, ctas, stream, QkvTail{}, nullptr, grp);

@@ -1495,22 +1495,29 @@ def gemm_tc_grouped(x, w, y, n, experts, tile_expert, row_scale=None, gated=Fals
            "gemm_tc_grouped", "matmul", _nbytes(x, w, y))
 
 
+BATCH_GROUPS = 4
+
+
 def gemm_batch(x, w, out):
-    """out[g] = x[g] @ w[g].T for x [G, T, K], w [G, N, K], out float32 [G, T, N], all contiguous: prompts in bfloat16 in one
-    launch, other steps a product at a time."""
+    """out[g] = x[g] @ w[g].T for x [G, T, K], G matrices w[g] [N, K], out float32 [G, T, N], all contiguous: prompts in bfloat16 in a
+    launch for four products, other steps a product at a time."""
     groups, t, k = x.shape
-    n = w.shape[1]
-    assert w.shape == (groups, n, k) and out.shape == (groups, t, n) and x.is_contiguous() and w.is_contiguous() and out.is_contiguous()
-    if t <= 64 or not gemm_tc_usable(x[0], w[0]):
+    n = w[0].shape[0]
+    assert len(w) == groups and all(m.shape == (n, k) and m.is_contiguous() for m in w)
+    assert out.shape == (groups, t, n) and x.is_contiguous() and out.is_contiguous()
+    if t <= 64 or not all(gemm_tc_usable(x[0], m) for m in w):
         for g in range(groups):
             gemm(x[g], w[g], out[g])
         return
-    _cuda(x, w, out)
+    _cuda(x, *w, out)
     assert out.dtype == torch.float32
     sms = sm_count(x.device)
     f = _fn("gemm_tc", "gb_gemm_tc_batch", [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p])
-    _check(f(x.data_ptr(), w.data_ptr(), out.data_ptr(), groups, t, n, k, prompt_tile(t, groups * -(-n // 128), sms), sms, _stream()),
-           "gemm_tc_batch", "matmul", _nbytes(x, w, out))
+    for g in range(0, groups, BATCH_GROUPS):
+        some = w[g:g + BATCH_GROUPS]
+        places = (c_void_p * len(some))(*(m.data_ptr() for m in some))
+        _check(f(x[g].data_ptr(), places, out[g].data_ptr(), len(some), t, n, k, prompt_tile(t, len(some) * -(-n // 128), sms), sms,
+                 _stream()), "gemm_tc_batch", "matmul", _nbytes(x[g:g + len(some)], *some, out[g:g + len(some)]))
 
 
 def moe_experts_tc(h, idx, wts, sg, w_gate_up, w_down, shared_gate_up, shared_down, residual, limit, shared_limit, alpha,

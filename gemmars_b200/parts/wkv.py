@@ -43,7 +43,7 @@ class DecayedLinearAttention(Part):
         if not 1 <= self.dim <= 256:
             raise ValueError(f"wkv: heads of {self.dim} are not supported by the kernel (1 to 256)")
         self.inner = self.heads * self.dim
-        self.mu = self.rkvg = self.w1 = self.w2 = self.w0 = self.u = self.norm = self.o = None
+        self.mu = self.r = self.k = self.v = self.g = self.w1 = self.w2 = self.w0 = self.u = self.norm = self.o = None
 
     def wants(self):
         h, n = self.hidden_size, self.inner
@@ -56,7 +56,7 @@ class DecayedLinearAttention(Part):
 
     def load(self, t):
         self.mu = torch.stack([t[f"mu_{s}"] for s in MIXES]).to(torch.float32).contiguous()
-        self.rkvg = torch.stack([t[s] for s in ("r", "k", "v", "g")]).contiguous()
+        self.r, self.k, self.v, self.g = (Linear(t[s]) for s in ("r", "k", "v", "g"))
         self.w1, self.w2 = Linear(t["w1"]), t["w2"].contiguous()
         self.w0, self.u, self.norm = t["w0"].contiguous(), t["u"].contiguous(), t["norm"].contiguous()
         self.o = Linear(t["o"])
@@ -70,7 +70,8 @@ class DecayedLinearAttention(Part):
 
     def weight_bytes(self):
         small = sum(4 * t.numel() for t in (self.mu, self.w0, self.u, self.norm) if t is not None)
-        return self.w1.bytes() + self.o.bytes() + sum(m.numel() * m.element_size() for m in (self.rkvg, self.w2)) + small
+        mats = sum(m.bytes() for m in (self.r, self.k, self.v, self.g, self.w1, self.o))
+        return mats + self.w2.numel() * self.w2.element_size() + small
 
     def forward(self, ctx, h, residual, caches, writes_cache=True):
         if not writes_cache:
@@ -78,7 +79,7 @@ class DecayedLinearAttention(Part):
         before, state = caches
         mixes = kernels.shift_mix(h, self.mu, before, ctx.cu_seqlens, ctx.tok_seq, ctx.seq_slot)
         r, k, v, gate = made = torch.empty((4, h.shape[0], self.inner), dtype=torch.float32, device=h.device)
-        kernels.gemm_batch(mixes[:4], self.rkvg, made)
+        kernels.gemm_batch(mixes[:4], [m.weight for m in (self.r, self.k, self.v, self.g)], made)
         decay = kernels.lowrank_decay(self.w1(mixes[4], out_dtype=torch.float32), self.w2, self.w0)
         y = torch.empty((h.shape[0], self.inner), dtype=torch.float32, device=h.device)
         kernels.wkv_scan(r, k, decay, v, self.u, state, ctx.cu_seqlens, ctx.seq_slot, y, self.heads, self.dim, self.dim,

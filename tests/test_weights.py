@@ -125,3 +125,16 @@ def test_random_weights_are_seeded_and_load(tmp_path):
     assert all(t.dtype == torch.bfloat16 for t in got.values())      # kept as stored
     f32 = write_random_model(str(tmp_path / "m32"), TINY_A, seed=5, dtype=torch.float32)
     assert ModelFiles(f32).info("model.norm.weight")[0] == torch.float32
+
+
+def test_a_wkv_part_uses_its_matrices_as_they_were_loaded():
+    """Its four projections run in one launch, but no second copy of them is made for it."""
+    import torch
+    from gemmars_b200.parts.base import build_part
+    from gemmars_b200.parts.plan import PartSpec
+    part = build_part("mixer", PartSpec("wkv", {"hidden_size": 64, "heads": 2, "dim": 32, "rank": 8, "norm_eps": 1e-6}), "bfloat16")
+    t = {n: torch.randn(w.shape).to(torch.bfloat16 if w.role == "matrix" else torch.float32) for n, w in part.wants().items()}
+    part.load(t)
+    held = {v.weight.data_ptr() for v in vars(part).values() if hasattr(v, "weight")}
+    assert {t[s].data_ptr() for s in ("r", "k", "v", "g", "o")} <= held
+    assert part.weight_bytes() == sum(v.numel() * v.element_size() for v in t.values())
