@@ -1473,13 +1473,15 @@ def gemm_tc_grouped(x, w, y, n, experts, tile_expert, row_scale=None, gated=Fals
                     bn=MOE_TC_TILE, act=None, scale_in=False, tile_rows=None):
     """The tcgen05 product over groups of rows: x [rows, K] holds the groups one after the other, each
     starting at a multiple of ``bn`` rows; w stacks the groups' matrices ([experts * n, K], or
-    [experts * 2 n, K] gated); tile_expert names the group of every tile of ``bn`` rows (-1: none).
+    [experts * 2 n, K] gated); tile_expert names the group of every tile of ``bn`` rows (-1: none; None: one matrix for
+    all rows, any number of them).
     y float32 [rows, n], or with ``gated`` bfloat16 [rows, n] = row_scale * act(gate, up), or with
     ``act`` (one of PLAIN_ACTS) bfloat16 [rows, n] = row_scale * act(x w^T) (no gate rows).  ``scale_in``
-    (gated): act(row_scale * gate, row_scale * up).  ``tile_rows`` [rows / bn] (None: all): how many of a tile's rows
-    exist; what y holds in the others is not to be read."""
+    (gated): act(row_scale * gate, row_scale * up).  ``tile_rows`` [rows / bn] (with tile_expert; None: all): how many of a
+    tile's rows exist; what y holds in the others is not to be read."""
     _cuda(x, w, y, tile_expert, row_scale, tile_rows)
-    assert tile_rows is None or (tile_rows.dtype == torch.int32 and tile_rows.numel() == tile_expert.numel())
+    assert tile_rows is None or (tile_expert is not None and tile_rows.dtype == torch.int32 and tile_rows.numel() == tile_expert.numel())
+    assert row_scale is None or (row_scale.dtype == torch.float32 and row_scale.is_contiguous() and row_scale.numel() >= x.shape[0])
     rows, k = x.shape
     assert x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and x.stride(1) == 1 and w.is_contiguous()
     assert not (gated and act)

@@ -170,3 +170,13 @@ def test_one_round_of_tiles_takes_pairs_where_they_are_the_faster(k):
     for m, n, kk, paired in ((2048, 2048, 4096, 0), (1000, 4096, 4096, 0), (700, 4096, 6144, 1), (2048, 2048, 6144, 1), (2048, 4096, 4096, 1),
                              (2048, 4672, 2048, 0)):
         assert pairs(k, m, n, kk, 256, 148) == paired
+
+
+def test_a_product_without_groups_refuses_what_belongs_to_groups(k):
+    x, w = operands(256, 128, 64, 1)
+    y = torch.empty(256, 128, device="cuda")
+    tile_rows = torch.full((1,), 256, dtype=torch.int32, device="cuda")
+    with pytest.raises(AssertionError):
+        k.gemm_tc_grouped(x, w, y, 128, 1, None, tile_rows=tile_rows, bn=256)
+    with pytest.raises(AssertionError):
+        k.gemm_tc_grouped(x, w, y, 128, 1, None, torch.ones(255, device="cuda"), bn=256)
