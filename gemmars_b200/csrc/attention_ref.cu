@@ -394,23 +394,39 @@ static int launch_ref(int ntok, int rep, const PagedKV& kv, cudaStream_t stream,
   return gb_launch_status();
 }
 
-// q: [ntok, nh, hd] rows q_stride apart (already normed, rotated, scaled); out likewise.  apart: tokens seldom share their
-// sequence and first key (single tokens, or most of a prompt past its window), so that a block would work its four one after
-// the other: one token a block then.  The same bits either way.
+// Query heads of a kv head that a block works.
+static int block_heads(int rep) { return rep >= 3 ? 4 : rep; }
+
+// The form for a step whose neighbouring tokens share their sequence and first key, by its size: 16 (sixteen queries a block), 4
+// (four tokens) or 1 (one).  The larger forms read a chunk's keys for more queries but leave fewer blocks.  us, one / four tokens /
+// sixteen queries, heads of 128: 16 heads over 8: 100 tokens 25 / 18 / 18, 150 43 / 39 / 29, 301 110 / 79 / 49, 1,024 868 / 553 / 285; 32 over
+// 8: 64 tokens 22 / 17 / 16, 100 29 / 21 / 21, 301 128 / 91 / 78; 8 over 8: 200 tokens 51 / 27 / 32, 301 92 / 50 / 46; 16 over 16: 100 tokens
+// 35 / 16 / 21, 150 60 / 34 / 33, 200 89 / 45 / 36.  Sixteen queries want a block an SM (147 blocks: 145 tokens, 73, 289, 145 of those),
+// and heads of up to 128; four tokens two.  With two or four heads a block the second line lies at or beyond the first: four tokens
+// are then for wider heads, and for steps whose tokens share less (see the caller's rule).
+static int form_by_size(int ntok, int nh, int nkv, int hd) {
+  const int heads = block_heads(nh / nkv), columns = nkv * ((nh / nkv + heads - 1) / heads), tile_tokens = 16 / heads;
+  if (hd <= CHUNK && (long long)((ntok + tile_tokens - 1) / tile_tokens) * columns >= 148) return 16;
+  return (long long)ntok * columns >= 4 * 2 * 148 ? 4 : 1;
+}
+GB_EXPORT int gb_attention_ref_form(int ntok, int nh, int nkv, int hd) {
+  return ntok > 0 && nkv > 0 && nh >= nkv && nh % nkv == 0 ? form_by_size(ntok, nh, nkv, hd) : 1;
+}
+
+// q: [ntok, nh, hd] rows q_stride apart (already normed, rotated, scaled); out likewise.  form: 1, 4 or 16 as above, or 0: by size.
+// Tokens of a block that do not share their sequence and first key are worked one after the other.  The same bits whatever it is.
 GB_EXPORT int gb_attention_ref(const void* q, long long q_stride, void* out, long long out_stride, int dtype,
                                const void* kcache, const void* vcache, const int* page_table, int table_width,
                                int page_size, int nkv, int hd, const int* tok_pos, const int* tok_seq,
-                               const int* seq_slot, int ntok, int nh, int window, int apart, cudaStream_t stream) {
+                               const int* seq_slot, int ntok, int nh, int window, int form, cudaStream_t stream) {
   if (ntok <= 0) return 0;
   if (hd <= 0 || hd > 2 * CHUNK || nkv <= 0 || nh % nkv) return GB_ERR_SIZE;
+  if (form != 0 && form != 1 && form != 4 && form != 16) return GB_ERR_ARG;
+  if (form == 16 && hd > CHUNK) return GB_ERR_SIZE;
   PagedKV kv{page_table, table_width, page_size, nkv, hd};
-  const int rep = nh / nkv, heads = rep >= 3 ? 4 : rep;
-  // Positions of a prompt share their keys: four tokens a block, once that leaves two blocks an SM (us, one / four; 16 heads of
-  // 128 over 8: 1,024 tokens 869 / 554, but in a window of 128 278 / 569, and 2,048 in one of 512 1,818 / 3,465)
-  const bool four = !apart && (long long)ntok * nkv * ((rep + heads - 1) / heads) >= 4 * 2 * 148;
-  // ... and sixteen queries once those leave a block an SM
-  const int tile_tokens = 16 / heads;
-  const bool tiles = !apart && hd <= CHUNK && (long long)((ntok + tile_tokens - 1) / tile_tokens) * nkv * ((rep + heads - 1) / heads) >= 148;
+  const int rep = nh / nkv, heads = block_heads(rep);
+  if (form == 0) form = form_by_size(ntok, nh, nkv, hd);
+  const bool four = form == 4, tiles = form == 16;
   const int wide = hd % 4 == 0 && (((uintptr_t)kcache | (uintptr_t)vcache) & 15) == 0;
 #define REF(T, TOKENS, HEADS)                                                                                              \
   launch_ref<T, TOKENS, HEADS>(ntok, rep, kv, stream, (const T*)q, q_stride, (T*)out, out_stride, (const T*)kcache, (const T*)vcache, \

@@ -737,17 +737,69 @@ def check_status() -> None:
 # --------------------------------------------------------------------------- attention
 
 def attention_tokens_apart(window: Optional[int], max_new: int, max_total: int) -> bool:
-    """Whether a step's tokens seldom share their sequence and first key: sequences bring a few tokens each, or the longest one's
-    tokens are past the window (from there on every token has a first key of its own) by more than an eighth.  A block of
-    four tokens works such tokens one after the other (us, one / four tokens a block, 16 heads of 128 over 8; of 1,212 tokens of
-    two prompts in a window of 512 the longer one's last 188 are past it: 678 / 834; none past it 664 / 421)."""
+    """Whether a step's tokens seldom share their sequence and first key, from what is known without the sequences' lengths:
+    sequences bring a few tokens each, or the longest one's tokens are past the window (from there on every token has a first
+    key of its own) by more than an eighth.  With the lengths, attention_ref_form tells more."""
     return max_new < 4 or (window is not None and 8 * (max_total - window) > max_new)
 
 
+def attention_ref_passes(window: Optional[int], lens, starts, tokens: int):
+    """Keys that blocks of ``tokens`` neighbouring tokens of a step walk, a pass for each run of them that shares its sequence
+    and first key: (of the block that walks most, of all).  Sequences bring ``lens`` tokens after ``starts``."""
+    longest = total = at = here = 0              # the open block: tokens in it, keys that they walk
+    for n, s in zip(lens, starts):
+        shared = n if window is None else min(n, max(0, window - s))         # tokens up to the window's end start at key 0
+        for left, past in ((shared, False), (n - shared, True)):
+            while left:
+                if at == 0 and left >= tokens:   # whole blocks
+                    blocks = left // tokens
+                    last = s + blocks * tokens
+                    most = tokens * window if past else last
+                    total += blocks * most if past else blocks * (s + tokens + last) // 2
+                    longest, s, left = max(longest, most), last, left - blocks * tokens
+                    continue
+                some = min(left, tokens - at)
+                s, at, left = s + some, at + some, left - some
+                keys = some * window if past else s
+                here, total = here + keys, total + keys
+                longest = max(longest, here)
+                if at == tokens:
+                    at = here = 0
+    return longest, total
+
+
+# A block's time goes with the keys of its passes, and a step takes about the time of its longest block and of all blocks' keys
+# shared out over so many places: by form, and by the heads a block works (fitted to the figures of attention_ref_form and to prompts)
+ATTENTION_REF_PLACES = {1: {1: 593, 2: 483, 4: 421}, 4: {1: 367, 2: 190, 4: 170}, 16: {1: 165, 2: 185, 4: 220}}
+
+
+def attention_ref_form(window: Optional[int], lens, starts, nh: int, nkv: int, hd: int) -> int:
+    """How many tokens a block of the plain attention works (1, 4; 16: sixteen queries), by the step's size and by how many of its
+    tokens share their sequence and first key: the others of a block are worked one after the other.  us, one / four tokens /
+    sixteen queries a block, heads of 128: a prompt of 301 beside 8 single tokens of 2,000, 16 heads over 8: 249 / 976 / 934, 16 of
+    8,000 751 / 3,883 / 5,744; of 1,024 beside 16 of 2,000 1,001 / 1,419 / 1,767, 40 of 500 908 / 745 / 671; 16 heads over 16, 8 of 2,000
+    1,533 / 1,228 / 1,817; 32 over 8, 16 of 2,000 1,128 / 1,468 / 1,249, 40 of 500 1,034 / 825 / 675.  Past a window of 512, 16 heads over 8: 528
+    tokens 286 / 409 / 544, 700 455 / 696 / 689; over 16: 528 445 / 373 / 1,086, 700 746 / 720 / 1,314; past one of 2,048: 2,098 tokens 3,462 /
+    3,180 / 3,089 and 5,708 / 3,211 / 5,508; prompts of 512 and 586 over 8, 32 heads 655 / 714 / 616."""
+    by_size = _fn("attention_ref", "gb_attention_ref_form", [c_int] * 4)(sum(lens), nh, nkv, hd)
+    heads = 4 if nh // nkv >= 3 else nh // nkv
+    columns = nkv * -(-(nh // nkv) // heads)
+    best, least = 1, None
+    for form, tokens in ((1, 1), (4, 4), (16, 16 // heads)):
+        if form > by_size:
+            break
+        longest, total = attention_ref_passes(window, lens, starts, tokens)
+        cost = longest + total * columns / ATTENTION_REF_PLACES[form][heads]
+        if least is None or cost < least:
+            best, least = form, cost
+    return best
+
+
 def attention_ref(q, out, nh, kcache, vcache, page_table, page_size, tok_pos, tok_seq, seq_slot, window=None, cache_bytes: int = 0,
-                  apart: Optional[bool] = None):
-    """Causal grouped-query attention of q [T, nh*hd] (row stride free) over the paged cache.  ``apart`` (None: with a window):
-    see attention_tokens_apart; the bits are the same either way."""
+                  apart: Optional[bool] = None, form: int = 0):
+    """Causal grouped-query attention of q [T, nh*hd] (row stride free) over the paged cache.  ``form``: see attention_ref_form
+    (0: one token a block if ``apart``, else by the step's size); ``apart`` (None: with a window, or as many sequences as tokens):
+    see attention_tokens_apart.  The bits are the same whatever they are."""
     _cuda(q, out, kcache, vcache, page_table, tok_pos, tok_seq, seq_slot)
     nkv, hd = kcache.shape[1], kcache.shape[3]
     assert q.stride(-1) == 1 and out.stride(-1) == 1 and q.dtype == out.dtype == kcache.dtype
@@ -755,10 +807,10 @@ def attention_ref(q, out, nh, kcache, vcache, page_table, page_size, tok_pos, to
             [c_void_p, c_longlong, c_void_p, c_longlong, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
              c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p])
     if apart is None:
-        apart = window is not None
+        apart = window is not None or q.shape[0] == seq_slot.numel()
     _check(f(q.data_ptr(), q.stride(0), out.data_ptr(), out.stride(0), dtype_code(q.dtype), kcache.data_ptr(),
              vcache.data_ptr(), page_table.data_ptr(), page_table.shape[1], page_size, nkv, hd, tok_pos.data_ptr(),
-             tok_seq.data_ptr(), seq_slot.data_ptr(), q.shape[0], nh, window or 0, int(apart), _stream()), "attention_ref",
+             tok_seq.data_ptr(), seq_slot.data_ptr(), q.shape[0], nh, window or 0, form or int(apart), _stream()), "attention_ref",
            "attention", _nbytes(q, out) + cache_bytes)
 
 
@@ -1696,8 +1748,14 @@ def attention(ctx, q, out, nh, kcache, vcache, page_table, page_size, window=Non
         prefill(q, out, nh, kcache, vcache, page_table, page_size, ctx.cu_seqlens, ctx.seq_start, ctx.seq_slot, window,
                 cache_bytes=cached)
         return
+    form = 0
+    if ctx.host is not None and ctx.max_new > 1:
+        key = ("attention_ref", window, nh, kcache.shape[1], kcache.shape[3])
+        form = ctx.extras.get(key)
+        if form is None:
+            form = ctx.extras[key] = attention_ref_form(window, ctx.host["seq_len"], ctx.host["seq_start"], nh, kcache.shape[1], kcache.shape[3])
     attention_ref(q, out, nh, kcache, vcache, page_table, page_size, ctx.tok_pos, ctx.tok_seq, ctx.seq_slot, window,
-                  cache_bytes=cached, apart=attention_tokens_apart(window, ctx.max_new, ctx.max_total))
+                  cache_bytes=cached, apart=attention_tokens_apart(window, ctx.max_new, ctx.max_total), form=form)
 
 
 # a step whose sequences bring at most this many tokens each runs the per-position decode kernel
