@@ -308,7 +308,8 @@ attention_capped_single_kernel(const bf16* __restrict__ q, long long q_stride, b
   const int rank = (int)spread_rank(), spread = (int)spread_size();
   // A warp's block is a chain of loads: its page, then its keys, then its values.  The page of the next block is asked for
   // while this one is worked on, and the values together with the keys where the registers hold both: 8 sequences,
-  // 32 heads of 128 over 8, a window of 2,048 keys 21.7 -> 19.3 us.
+  // 32 heads of 128 over 8, a window of 2,048 keys 21.7 -> 19.3 us, although keys and values of 128 take all 255 registers and
+  // 28 bytes are spilled.
   constexpr bool AHEAD = HD <= 128 && VD <= 128;
   auto key_of = [&](int it) { return (it < kept_blks ? it : win_blk + it - kept_blks) * KEYS; };
   auto page_of = [&](int it) { return kv.page_table[(size_t)slot * kv.table_width + (key_of(it) / kv.page_size) % kv.table_width]; };

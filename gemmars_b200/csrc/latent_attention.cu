@@ -57,8 +57,8 @@ template <> __device__ __forceinline__ void store4<bf16>(bf16* to, float a, floa
 // slot, page, the row), so nothing waits for a block: a warp holds a token's row and sums it alone, and a query's angles are
 // taken where they are used.  `wide`: interleaved pairs, everything in fours.  16 heads of 128 + 64 over rows of 512 + 64, with
 // the wait for the kernel before (us; a block a token, its row twice through memory, its angles through shared memory / so):
-// 2,048 tokens 20.9 / 16.6, 16 tokens 10.6 / 8.5; the layer, with the rows' zeros written here and not by two fills,
-// 145.5 / 132.0 and 65.7 / 65.4.
+// 2,048 tokens 20.9 / 16.6, 16 tokens 10.6 / 8.5; the layer of 2,048 tokens, with the rows' zeros written here and not by two fills,
+// 145.5 / 132.0 where one side's runs differ by up to a fifth; of 16 single tokens 65.7 / 65.4.
 constexpr int PREPARE_THREADS = 128, PREPARE_QUADS = 2, ROW_HELD = 16;
 template <typename T, int QUADS>
 __global__ void __launch_bounds__(PREPARE_THREADS) latent_prepare_kernel(
@@ -210,7 +210,10 @@ GB_EXPORT int gb_latent_prepare(const float* q_in, long long ldq, const float* k
                    ((uintptr_t)q_nope % elem) == 0 && ((uintptr_t)q_lat % elem) == 0 && qd > 0;
   const int units = H * (wide ? qd / 4 : dim + rd / 2 + (rd & 1));          // of a token
   const int row_blocks = (ntok + PREPARE_THREADS / 32 - 1) / (PREPARE_THREADS / 32);
-  const int quads = (long long)ntok * units > 2048LL * 148 ? PREPARE_QUADS : 1;      // more than a chip of threads
+  // Two quads a thread where there are more than a chip of threads.  us, one / two, by units of 148 threads: 996 (8 heads, 768 tokens)
+  // 5.9 / 5.6, 1,328 (16 heads, 256) 6.0 / 6.1, 1,328 (32 heads, 128) 5.9 / 5.9, 1,992 6.1 / 6.1 and 6.8 / 6.3, 2,656 6.6 / 6.6 and 6.3 / 6.4,
+  // 3,985 7.9 / 6.9, 10,627 (16 heads, 2,048) 17.6 / 14.7.
+  const int quads = (long long)ntok * units > 2048LL * 148 ? PREPARE_QUADS : 1;
   const int token_blocks = (units + PREPARE_THREADS * quads - 1) / (PREPARE_THREADS * quads);
   const long long blocks = row_blocks + (long long)ntok * token_blocks;
   if (blocks > 0x7fffffffLL) return GB_ERR_SIZE;
