@@ -782,6 +782,8 @@ def attention_ref_form(window: Optional[int], lens, starts, nh: int, nkv: int, h
     tokens 286 / 409 / 544, 700 455 / 696 / 689; over 16: 528 445 / 373 / 1,086, 700 746 / 720 / 1,314; past one of 2,048: 2,098 tokens 3,462 /
     3,180 / 3,089 and 5,708 / 3,211 / 5,508; prompts of 512 and 586 over 8, 32 heads 655 / 714 / 616."""
     by_size = _fn("attention_ref", "gb_attention_ref_form", [c_int] * 4)(sum(lens), nh, nkv, hd)
+    if by_size == 1:                             # also heads that the kernel refuses
+        return 1
     heads = 4 if nh // nkv >= 3 else nh // nkv
     columns = nkv * -(-(nh // nkv) // heads)
     best, least = 1, None

@@ -86,3 +86,8 @@ def test_the_plain_attention_takes_the_form_that_was_the_fastest(nh, nkv, lens, 
 def test_heads_too_wide_for_sixteen_queries_take_four_tokens():
     from gemmars_b200 import kernels
     assert kernels.attention_ref_form(None, [300], [0], 16, 8, 200) == 4 and kernels.attention_ref_form(None, [100], [0], 16, 8, 200) == 1
+
+
+def test_heads_that_the_plain_attention_refuses_are_left_to_it():
+    from gemmars_b200 import kernels
+    assert [kernels.attention_ref_form(None, [500], [0], nh, nkv, 64) for nh, nkv in ((2, 4), (6, 4))] == [1, 1]
